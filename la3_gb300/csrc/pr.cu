@@ -17,13 +17,9 @@
 // so nothing is contracted into an FMA and the result is bit-identical to
 // the reference built without contraction.
 //
-// Kernel layout (pr_pull): one warp owns 32 consecutive rows; it streams the
-// rows' in-edges in chunks of 32 x 8 entries through shared memory (coalesced
-// index loads, gathered x values) and each lane adds its own row's values in
-// order.  Rows longer than kLongRow are skipped there and summed by a single
-// lane that walks the row sequentially with its warp prefetching the values;
-// those warps are the first blocks of the same launch, so the long chains
-// start first.
+// Kernel layout (k_pr_pull): rows of at most kMedRow in-edges in tiles of 32,
+// a lane each; longer rows a warp each, the longest a block each, summed in
+// parallel with the result of the sequential sum (see "exact sums" below).
 #include <algorithm>
 #include <cstring>
 #include <vector>
@@ -38,6 +34,7 @@ namespace la3g {
 static constexpr double kAlpha = 0.15;
 static constexpr double kTol = 1e-5;
 static constexpr uint32_t kLongRow = 1024;
+static constexpr uint32_t kMedRow = 64;  // FP64: longer rows leave the tiles
 static constexpr int kChunk = 256;  // edges staged per warp per step
 static constexpr int kWarpsPerBlock = 8;
 
@@ -46,8 +43,9 @@ struct PrScratch
   uint32_t* deg = nullptr;      // [nslots] out-degree
   double* rank = nullptr;       // [nslots]
   double* x[2] = {nullptr, nullptr};  // [nslots] messages (scatter values)
-  uint32_t* long_rows = nullptr;      // rows with degree > kLongRow, descending
-  uint32_t nlong = 0;
+  uint32_t* long_rows = nullptr;      // rows with degree > kMedRow, descending
+  uint32_t nlong = 0;                 // of which > kLongRow (they come first)
+  uint32_t nheavy = 0;                // all of them
   int* flag = nullptr;          // any-activated flag
   float* xf[2] = {nullptr, nullptr};  // FP32 study
   float* rankf = nullptr;
@@ -94,7 +92,8 @@ __global__ void k_mark_long(const uint32_t* __restrict__ ptr, uint32_t nrows, ui
   for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < nrows; r += gridDim.x * blockDim.x)
   {
     uint32_t d = ptr[r + 1] - ptr[r];
-    if (d > kLongRow)
+    if (d > kLongRow) atomicAdd(count + 1, 1u);
+    if (d > kMedRow)
     {
       uint32_t i = atomicAdd(count, 1u);
       keys[i] = ~d;  // ascending sort of ~d = descending degree
@@ -120,75 +119,273 @@ __device__ __forceinline__ void pr_finish_row(uint32_t r, double acc, const uint
   if (flag && fabs(__dsub_rn(nr, old)) > kTol) *flag = 1;
 }
 
-// Rows [row_lo, row_hi).  Blocks [0, long_blocks) take the long rows (one
-// warp per row, descending length); the rest take 32-row tiles.
+// ---- exact sums --------------------------------------------------------------
+//
+// acc = RN(acc + v) one value after another, v >= 0, is a serial chain of
+// FP64 additions (about 55 cycles each here: a 10k-edge row took 320 us).
+// While acc stays inside one binade its ulp 2^e is fixed, and acc = m 2^e with
+// an integer m: adding v adds v / 2^e rounded to an integer, which does not
+// depend on m except that a tie goes to the even result.  One value is thus a
+// function of m's parity, (increment if m is even, increment if m is odd), and
+// such functions compose associatively: any stretch of a row that stays in one
+// binade can be summed in parallel, in integers, with the sequential result
+// bit for bit.  Where m would reach 2^53 (acc enters the next binade, at most
+// once per doubling of the sum), the thread that holds that value adds its few
+// values with real FP64 additions, and the rest is taken up with the new
+// exponent.  On R-MAT 2^16 (1M edges): 328 -> 45 us per iteration.
+struct ExactSum
+{
+  uint64_t m;  // value m 2^(e - 1075); m < 2^53
+  int e;       // exponent field of the ulp's binade (1 for denormals); -1 while the sum is 0
+};
+
+struct ParityFn  // increments for m even / odd
+{
+  uint64_t a, b;
+};
+
+static constexpr uint64_t kExactTop = 1ull << 53;
+static constexpr int kExactPer = 8;  // consecutive values per thread and step
+
+__device__ __forceinline__ ExactSum exact_of(double v)
+{
+  const uint64_t bits = (uint64_t) __double_as_longlong(v), f = bits & ((1ull << 52) - 1);
+  const int e = (int) (bits >> 52);  // v >= 0
+  if (!bits) return {0, -1};
+  return e ? ExactSum{f | (1ull << 52), e} : ExactSum{f, 1};
+}
+
+__device__ __forceinline__ double exact_double(uint64_t m, int e)
+{
+  return m ? __longlong_as_double((long long) (((uint64_t) (e - 1) << 52) + m)) : 0.0;
+}
+
+// v as a function of m's parity, with ulp exponent e; an increment of
+// kExactTop or more leaves the binade whatever m is.
+__device__ __forceinline__ ParityFn exact_fn(double v, int e)
+{
+  const uint64_t bits = (uint64_t) __double_as_longlong(v);
+  int ev = (int) (bits >> 52);
+  uint64_t mant = bits & ((1ull << 52) - 1);
+  if (ev) mant |= 1ull << 52;
+  else ev = 1;
+  const int s = e - ev;
+  if (s < 0) return mant ? ParityFn{kExactTop, kExactTop} : ParityFn{0, 0};
+  if (s > 53) return {0, 0};  // below half an ulp
+  const uint64_t f = mant >> s;
+  const uint64_t rem = s ? mant << (64 - s) : 0;  // the dropped bits, left-aligned
+  const uint64_t up = rem > (1ull << 63), tie = rem == (1ull << 63);
+  const uint64_t odd = f & 1;
+  return {f + (tie ? odd : up), f + (tie ? odd ^ 1 : up)};
+}
+
+__device__ __forceinline__ ParityFn exact_then(ParityFn f, ParityFn g)
+{
+  return {f.a + ((f.a & 1) ? g.b : g.a), f.b + ((f.b & 1) ? g.a : g.b)};
+}
+
+__device__ __forceinline__ ParityFn exact_shfl_up(ParityFn f, int d)
+{
+  return {__shfl_up_sync(0xffffffffu, f.a, d), __shfl_up_sync(0xffffffffu, f.b, d)};
+}
+
+// The thread's kExactPer values of the chunk that starts at entry `base`
+// (a multiple of 4, so that the column indices load as 16-byte vectors);
+// entries outside [b, e) count as 0, which adds nothing.  in_col is
+// allocated past its last entry for the vectors that straddle the end.
+__device__ __forceinline__ void exact_load(const uint32_t* __restrict__ col, const double* __restrict__ x, uint32_t base,
+                                           uint32_t b, uint32_t e, double v[kExactPer])
+{
+#pragma unroll
+  for (int q = 0; q < kExactPer; q += 4)
+  {
+    const uint32_t i = base + q;
+    uint4 c = make_uint4(0, 0, 0, 0);
+    if (i < e) c = *reinterpret_cast<const uint4*>(col + i);
+    v[q] = i >= b && i < e ? x[c.x] : 0.0;
+    v[q + 1] = i + 1 >= b && i + 1 < e ? x[c.y] : 0.0;
+    v[q + 2] = i + 2 >= b && i + 2 < e ? x[c.z] : 0.0;
+    v[q + 3] = i + 3 >= b && i + 3 < e ? x[c.w] : 0.0;
+  }
+}
+
+__device__ __forceinline__ ParityFn exact_mine(const double v[kExactPer], int e)
+{
+  ParityFn f{0, 0};
+#pragma unroll
+  for (int q = 0; q < kExactPer; q++) f = exact_then(f, exact_fn(v[q], e));
+  return f;
+}
+
+// Inclusive scan over the warp's lanes, in lane order.
+__device__ __forceinline__ ParityFn exact_scan(ParityFn f, int lane)
+{
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1)
+  {
+    const ParityFn g = exact_shfl_up(f, o);
+    if (lane >= o) f = exact_then(g, f);
+  }
+  return f;
+}
+
+// One row by one warp.
+__device__ __forceinline__ double exact_row_warp(const uint32_t* __restrict__ col, const double* __restrict__ x,
+                                                 uint32_t b, uint32_t e, int lane)
+{
+  ExactSum s{0, -1};
+  double v[kExactPer];
+  exact_load(col, x, (b & ~3u) + lane * kExactPer, b, e, v);
+  for (uint64_t base = b & ~3u; base < e; base += 32 * kExactPer)
+  {
+    int from = 0;  // lanes below are in the sum already
+    for (;;)
+    {
+      const ParityFn f = exact_scan(lane >= from ? exact_mine(v, s.e) : ParityFn{0, 0}, lane);
+      const uint64_t incl = s.m + ((s.m & 1) ? f.b : f.a);
+      const unsigned over = __ballot_sync(0xffffffffu, incl >= kExactTop);
+      if (!over)
+      {
+        s.m = __shfl_sync(0xffffffffu, incl, 31);
+        break;
+      }
+      const int L = __ffs(over) - 1;
+      uint64_t before = __shfl_up_sync(0xffffffffu, incl, 1);
+      if (lane == 0) before = s.m;
+      double acc = 0.0;
+      if (lane == L)
+      {
+        acc = exact_double(before, s.e);
+#pragma unroll
+        for (int q = 0; q < kExactPer; q++) acc = __dadd_rn(acc, v[q]);
+      }
+      s = exact_of(__shfl_sync(0xffffffffu, acc, L));
+      from = L + 1;
+      if (from == 32) break;
+    }
+    if (base + 32 * kExactPer < e) exact_load(col, x, (uint32_t) base + (32 + lane) * kExactPer, b, e, v);
+  }
+  return exact_double(s.m, s.e);
+}
+
+// One row by one block (WARPS warps): the warps' functions meet in shared
+// memory, every thread composes them and keeps its own copy of the sum.
+template <int WARPS>
+__device__ __forceinline__ double exact_row_block(const uint32_t* __restrict__ col, const double* __restrict__ x,
+                                                  uint32_t b, uint32_t e)
+{
+  __shared__ ParityFn s_fn[2][WARPS];
+  __shared__ double s_acc;
+  __shared__ int s_from;
+  constexpr uint32_t kStep = WARPS * 32 * kExactPer;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  ExactSum s{0, -1};
+  double v[kExactPer], nv[kExactPer];
+  int buf = 0;
+  exact_load(col, x, (b & ~3u) + threadIdx.x * kExactPer, b, e, v);
+  for (uint64_t base = b & ~3u; base < e; base += kStep)
+  {
+    const bool more = base + kStep < e;
+    if (more) exact_load(col, x, (uint32_t) (base + kStep) + threadIdx.x * kExactPer, b, e, nv);
+    int from = 0;
+    for (;;)
+    {
+      const ParityFn f = exact_scan((int) threadIdx.x >= from ? exact_mine(v, s.e) : ParityFn{0, 0}, lane);
+      if (lane == 31) s_fn[buf][w] = f;
+      __syncthreads();
+      uint64_t m = s.m, mine = 0;  // the sum before warp k; before this warp
+      int cross = -1;
+#pragma unroll
+      for (int k = 0; k < WARPS; k++)
+      {
+        if (k == w) mine = m;
+        const ParityFn g = s_fn[buf][k];
+        if (cross < 0)
+        {
+          m += (m & 1) ? g.b : g.a;
+          if (m >= kExactTop) cross = k;
+        }
+      }
+      buf ^= 1;
+      if (cross < 0)
+      {
+        s.m = m;
+        break;
+      }
+      if (w == cross)
+      {
+        const uint64_t incl = mine + ((mine & 1) ? f.b : f.a);
+        const int L = __ffs(__ballot_sync(0xffffffffu, incl >= kExactTop)) - 1;
+        uint64_t before = __shfl_up_sync(0xffffffffu, incl, 1);
+        if (lane == 0) before = mine;
+        if (lane == L)
+        {
+          double acc = exact_double(before, s.e);
+#pragma unroll
+          for (int q = 0; q < kExactPer; q++) acc = __dadd_rn(acc, v[q]);
+          s_acc = acc;
+          s_from = w * 32 + L + 1;
+        }
+      }
+      __syncthreads();
+      s = exact_of(s_acc);
+      from = s_from;
+      if (from == WARPS * 32) break;
+    }
+#pragma unroll
+    for (int q = 0; q < kExactPer; q++) v[q] = nv[q];
+  }
+  __syncthreads();  // s_fn, s_acc and s_from are free for the next row
+  return exact_double(s.m, s.e);
+}
+
+// Rows [row_lo, row_hi).  Blocks [0, long_blocks) take the rows above
+// kLongRow (a block per row, descending length), the next med_blocks the rest
+// of the rows above kMedRow (a warp per row), the others 32-row tiles.
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 k_pr_pull(const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col, const double* __restrict__ x,
           double* __restrict__ xnext, double* __restrict__ rank, const uint32_t* __restrict__ deg,
-          const uint32_t* __restrict__ long_rows, uint32_t nlong, uint32_t long_blocks, uint32_t row_lo,
-          uint32_t row_hi, int* flag, int write_x)
+          const uint32_t* __restrict__ long_rows, uint32_t nlong, uint32_t nheavy, uint32_t long_blocks,
+          uint32_t med_blocks, uint32_t row_lo, uint32_t row_hi, int* flag, int write_x)
 {
   __shared__ double sx[kWarpsPerBlock][kChunk];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   if (blockIdx.x < long_blocks)
   {
-    for (uint32_t li = blockIdx.x * kWarpsPerBlock + wib; li < nlong; li += long_blocks * kWarpsPerBlock)
+    for (uint32_t li = blockIdx.x; li < nlong; li += long_blocks)
     {
-      uint32_t r = long_rows[li];
-      if (r < row_lo || r >= row_hi) continue;
-      uint32_t b = ptr[r], e = ptr[r + 1];
-      double acc = 0.0;
-      // prefetch one chunk ahead; lane 0 adds sequentially
-      double v[kChunk / 32];
-#pragma unroll
-      for (int k = 0; k < kChunk / 32; k++)
-      {
-        uint32_t i = b + k * 32 + lane;
-        v[k] = i < e ? x[col[i]] : 0.0;
-      }
-      for (uint32_t base = b; base < e; base += kChunk)
-      {
-#pragma unroll
-        for (int k = 0; k < kChunk / 32; k++) sx[wib][k * 32 + lane] = v[k];
-        __syncwarp();
-        uint32_t nb = base + kChunk;
-#pragma unroll
-        for (int k = 0; k < kChunk / 32; k++)
-        {
-          uint32_t i = nb + k * 32 + lane;
-          v[k] = i < e ? x[col[i]] : 0.0;
-        }
-        if (lane == 0)
-        {
-          uint32_t n = min((uint32_t) kChunk, e - base);
-          if (n == kChunk)
-          {
-#pragma unroll 32
-            for (uint32_t j = 0; j < kChunk; j++) acc = __dadd_rn(acc, sx[wib][j]);
-          }
-          else
-          {
-            for (uint32_t j = 0; j < n; j++) acc = __dadd_rn(acc, sx[wib][j]);
-          }
-        }
-        __syncwarp();
-      }
+      const uint32_t r = long_rows[li];
+      if (r < row_lo || r >= row_hi) continue;  // the same for the whole block
+      const double acc = exact_row_block<kWarpsPerBlock>(col, x, ptr[r], ptr[r + 1]);
+      if (threadIdx.x == 0) pr_finish_row(r, acc, deg, rank, xnext, flag, write_x);
+    }
+    return;
+  }
+  if (blockIdx.x < long_blocks + med_blocks)
+  {
+    for (uint32_t li = nlong + (blockIdx.x - long_blocks) * kWarpsPerBlock + wib; li < nheavy;
+         li += med_blocks * kWarpsPerBlock)
+    {
+      const uint32_t r = long_rows[li];
+      if (r < row_lo || r >= row_hi) continue;  // the same for the whole warp
+      const double acc = exact_row_warp(col, x, ptr[r], ptr[r + 1], lane);
       if (lane == 0) pr_finish_row(r, acc, deg, rank, xnext, flag, write_x);
     }
     return;
   }
   const uint32_t ntiles = (row_hi - row_lo + 31) / 32;
-  const uint32_t nwarps = (gridDim.x - long_blocks) * kWarpsPerBlock;
-  for (uint32_t t = (blockIdx.x - long_blocks) * kWarpsPerBlock + wib; t < ntiles; t += nwarps)
+  const uint32_t first = long_blocks + med_blocks;
+  const uint32_t nwarps = (gridDim.x - first) * kWarpsPerBlock;
+  for (uint32_t t = (blockIdx.x - first) * kWarpsPerBlock + wib; t < ntiles; t += nwarps)
   {
     const uint32_t r0 = row_lo + t * 32;
     const uint32_t r = r0 + lane;
     const bool valid = r < row_hi;
     uint32_t rb = valid ? ptr[r] : 0, re = valid ? ptr[r + 1] : 0;
-    const bool mine = valid && (re - rb) <= kLongRow;
+    const bool mine = valid && (re - rb) <= kMedRow;
     if (!mine) { rb = 0; re = 0; }
     // Walk the short rows' edges in chunks; each chunk starts at the lowest
-    // edge any lane still needs, which skips over the long rows' edges.
+    // edge any lane still needs, which skips over the longer rows' edges.
     const uint32_t te = ptr[min(r0 + 32, row_hi)];
     double acc = 0.0;
     uint32_t cur = rb;  // next edge of my row to add
@@ -250,33 +447,34 @@ static int pr_prepare(la3g_graph* G, PrScratch** out)
     k_outdeg<<<grid_for(g.nent, 256), 256, 0, s>>>(g.in_col, g.nent, ps->deg);
     LA3G_LAUNCHED();
   }
-  // long rows, sorted by descending degree
+  // long and medium rows, sorted by descending degree
   DevBuf keys, vals, keys2, vals2, cnt;
   LA3G_TRY(keys.alloc((size_t) g.nrows() * 4 + 4));
   LA3G_TRY(vals.alloc((size_t) g.nrows() * 4 + 4));
-  LA3G_TRY(cnt.alloc(4));
-  LA3G_CUDA(cudaMemsetAsync(cnt.p, 0, 4, s));
+  LA3G_TRY(cnt.alloc(8));
+  LA3G_CUDA(cudaMemsetAsync(cnt.p, 0, 8, s));
   if (g.nrows())
   {
     k_mark_long<<<grid_for(g.nrows(), 256), 256, 0, s>>>(g.in_ptr, g.nrows(), keys.as<uint32_t>(), vals.as<uint32_t>(),
                                                          cnt.as<uint32_t>());
     LA3G_LAUNCHED();
   }
-  uint32_t nlong = 0;
-  LA3G_CUDA(cudaMemcpyAsync(&nlong, cnt.p, 4, cudaMemcpyDeviceToHost, s));
+  uint32_t n[2] = {0, 0};
+  LA3G_CUDA(cudaMemcpyAsync(n, cnt.p, 8, cudaMemcpyDeviceToHost, s));
   LA3G_CUDA(cudaStreamSynchronize(s));
-  ps->nlong = nlong;
-  LA3G_TRY(galloc(G, &ps->long_rows, nlong + 1));
-  if (nlong)
+  ps->nheavy = n[0];
+  ps->nlong = n[1];
+  LA3G_TRY(galloc(G, &ps->long_rows, (size_t) n[0] + 1));
+  if (n[0])
   {
-    LA3G_TRY(keys2.alloc((size_t) nlong * 4 + 4));
+    LA3G_TRY(keys2.alloc((size_t) n[0] * 4 + 4));
     size_t tb = 0;
     LA3G_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, keys.as<uint32_t>(), keys2.as<uint32_t>(), vals.as<uint32_t>(),
-                                              ps->long_rows, nlong, 0, 32, s));
+                                              ps->long_rows, n[0], 0, 32, s));
     DevBuf tmp;
     LA3G_TRY(tmp.alloc(tb));
     LA3G_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, tb, keys.as<uint32_t>(), keys2.as<uint32_t>(), vals.as<uint32_t>(),
-                                              ps->long_rows, nlong, 0, 32, s));
+                                              ps->long_rows, n[0], 0, 32, s));
   }
   LA3G_CUDA(cudaStreamSynchronize(s));
   ps->ready = true;
@@ -289,17 +487,18 @@ static int pr_launch(la3g_graph* G, PrScratch* ps, const double* x, double* xnex
 {
   DevGraph& g = G->g;
   if (row_hi <= row_lo) return LA3G_OK;
-  const uint32_t long_blocks = ps->nlong ? std::min<uint32_t>((ps->nlong + kWarpsPerBlock - 1) / kWarpsPerBlock, num_sms()) : 0;
+  const uint32_t long_blocks = std::min<uint32_t>(ps->nlong, num_sms() * 4);
+  const uint32_t med_blocks =
+      std::min<uint32_t>((ps->nheavy - ps->nlong + kWarpsPerBlock - 1) / kWarpsPerBlock, num_sms() * 8);
   const uint32_t ntiles = (row_hi - row_lo + 31) / 32;
   const uint32_t tile_blocks = std::min<uint32_t>((ntiles + kWarpsPerBlock - 1) / kWarpsPerBlock, num_sms() * 8);
-  uint64_t edges = 0;  // algorithmic bytes: 4 B index per edge + per-row ptr, x, rank, xnext
-  (void) edges;
+  // algorithmic bytes: 4 B index per edge + per-row ptr, x, rank, xnext
   double bytes = 4.0 * (double) g.nent + 4.0 * (row_hi - row_lo + 1) + 8.0 * (double) g.nslots +
                  (write_x ? 16.0 : 8.0) * (row_hi - row_lo) + 4.0 * (row_hi - row_lo);
   ProfileScope p("pr_pull_f64", G->stream, bytes);
-  k_pr_pull<<<long_blocks + std::max<uint32_t>(tile_blocks, 1), kWarpsPerBlock * 32, 0, G->stream>>>(
-      g.in_ptr, g.in_col, x, xnext, ps->rank, ps->deg, ps->long_rows, ps->nlong, long_blocks, row_lo, row_hi, flag,
-      write_x ? 1 : 0);
+  k_pr_pull<<<long_blocks + med_blocks + std::max<uint32_t>(tile_blocks, 1), kWarpsPerBlock * 32, 0, G->stream>>>(
+      g.in_ptr, g.in_col, x, xnext, ps->rank, ps->deg, ps->long_rows, ps->nlong, ps->nheavy, long_blocks, med_blocks,
+      row_lo, row_hi, flag, write_x ? 1 : 0);
   LA3G_LAUNCHED();
   return LA3G_OK;
 }
