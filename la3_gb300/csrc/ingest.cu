@@ -277,7 +277,7 @@ static int build_graph(la3g_graph* G, const uint32_t* a, const uint32_t* b, cons
 
   // Pull CSR.
   LA3G_TRY(galloc(G, &g.in_ptr, N + 1));
-  LA3G_TRY(galloc(G, &g.in_col, mu + 4));  // read as 16-byte vectors up to the last entry
+  LA3G_TRY(galloc(G, &g.in_col, mu + 1));
   if (g.weighted()) LA3G_TRY(galloc(G, &g.in_w, mu + 1));
   if (mu)
   {

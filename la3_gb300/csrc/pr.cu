@@ -17,9 +17,11 @@
 // so nothing is contracted into an FMA and the result is bit-identical to
 // the reference built without contraction.
 //
-// Kernel layout (k_pr_pull): rows of at most kMedRow in-edges in tiles of 32,
-// a lane each; longer rows a warp each, the longest a block each, summed in
-// parallel with the result of the sequential sum (see "exact sums" below).
+// Kernel layout: the calls run over a copy of the matrix made for them once
+// per graph (see "the pull layout"): rows in descending length, columns
+// renumbered in descending out-degree.  Rows of at most kShortRow in-edges go
+// a lane each, longer ones a warp each, the longest a block each; FP64 rows are
+// summed in parallel with the result of the sequential sum (see "exact sums").
 #include <algorithm>
 #include <cstring>
 #include <vector>
@@ -33,22 +35,54 @@ namespace la3g {
 
 static constexpr double kAlpha = 0.15;
 static constexpr double kTol = 1e-5;
-static constexpr uint32_t kLongRow = 1024;
-static constexpr uint32_t kMedRow = 64;  // FP64: longer rows leave the tiles
-static constexpr int kChunk = 256;  // edges staged per warp per step
+static constexpr uint32_t kLongRow = 1024;  // longer rows: a block each
+// Rows up to this: a lane each.  Of 64, 128, 256 and 512, 256 was fastest for
+// FP32 on R-MAT 2^22 (50 iterations: 14.8, 14.5, 13.5, 14.3 ms) and as good as
+// any for FP64 on R-MAT 2^16.
+static constexpr uint32_t kShortRow = 256;
 static constexpr int kWarpsPerBlock = 8;
+
+// ---- the pull layout --------------------------------------------------------
+//
+// A pull is bound by its gathers x[col]: one random 4- or 8-byte read per
+// edge, and at R-MAT 2^22 one column in a hundred is behind half of the
+// edges.  By position those hot columns are spread over the whole of x, a
+// 32-byte sector each, and L1 keeps few of them; numbered by descending
+// out-degree ("slots") they share sectors and lines.
+// Rows are numbered by descending in-degree ("q"; the regular rows, then the
+// sinks), so that 32 neighbouring rows have almost the same length and can go
+// a lane each: such a slice is stored column-major (step t of its lanes is
+// contiguous), its rows padded to the first one's length with slot N, where x
+// is 0.  The longer rows come first, each padded to a multiple of 4 entries
+// (16-byte index loads).  Every row keeps the order of its entries, so sums
+// come out as over the pull CSR.  FP32, R-MAT 2^22, 50 iterations: 34.0 ms over
+// the pull CSR by position, 13.7 ms here (240 G edges/s); what is left is the
+// L1 misses of the gathers (36 % hits; neither 32 to 200 KB of the hottest
+// messages in shared memory nor L1 eviction hints were faster).
+struct PrRange  // q's of one class (regular rows or sinks)
+{
+  uint32_t q0, q1, q2, q3;  // [q0, q1) above kLongRow, [q1, q2) above kShortRow, [q2, q3) slices
+};
+
+struct PrLayout
+{
+  uint32_t* qpos = nullptr;  // [nslots] position of row q (identity beyond the rows)
+  uint32_t* xi = nullptr;    // [nslots] slot of q's own message
+  uint32_t* degq = nullptr;  // [nslots] out-degree of q
+  uint64_t* off = nullptr;   // [nrows + 1] first entry of row q; of a slice: of its first row
+  uint32_t* col = nullptr;   // the entries' slots
+  PrRange reg{}, sink{};
+};
 
 struct PrScratch
 {
-  uint32_t* deg = nullptr;      // [nslots] out-degree
-  double* rank = nullptr;       // [nslots]
-  double* x[2] = {nullptr, nullptr};  // [nslots] messages (scatter values)
-  uint32_t* long_rows = nullptr;      // rows with degree > kMedRow, descending
-  uint32_t nlong = 0;                 // of which > kLongRow (they come first)
-  uint32_t nheavy = 0;                // all of them
+  uint32_t* deg = nullptr;      // [nslots] out-degree by position
+  PrLayout L;
+  double* rank = nullptr;       // [nslots] by q
+  double* x[2] = {nullptr, nullptr};  // [nslots + 1] messages (scatter values) by slot
   int* flag = nullptr;          // any-activated flag
-  float* xf[2] = {nullptr, nullptr};  // FP32 study
-  float* rankf = nullptr;
+  float* xf[2] = {nullptr, nullptr};  // FP32 study: messages by slot (tiled: by position)
+  float* rankf = nullptr;       // by q (tiled: by position until the loop has ended)
   double* resid = nullptr;
   bool ready = false;
   // tiled layout of the regular rows (la3g_pr_f32_tiled), built on first use
@@ -59,6 +93,8 @@ struct PrScratch
   uint32_t* tptr = nullptr;      // [ncols + 1] first entry of each non-empty column
   uint16_t* trow = nullptr;      // [nent] row of each entry, local to its tile
   uint32_t* tecol = nullptr;     // [nent] column of each entry (the hypersparse tiles' form)
+  float* trankf = nullptr;       // [nslots] by position
+  float* txf[2] = {nullptr, nullptr};  // [nslots] by position
   int tile_blocks = 0;           // resident blocks per SM of the tiled kernel
 };
 
@@ -70,35 +106,144 @@ __global__ void k_outdeg(const uint32_t* __restrict__ col, uint64_t m, uint32_t*
     atomicAdd(&deg[col[e]], 1u);
 }
 
-__global__ void k_pr_init(uint32_t N, uint32_t nreg, uint32_t src_base, uint32_t iso_base,
-                          const uint32_t* __restrict__ deg, double* rank, double* x0, double* x1)
+// Sort keys of the columns (descending out-degree) and of the rows (regular
+// before sinks, descending in-degree); `mask` is at least any degree.
+__global__ void k_pr_keys(uint32_t N, uint32_t nrows, uint32_t nreg, uint32_t mask, const uint32_t* __restrict__ ptr,
+                          const uint32_t* __restrict__ deg, uint32_t* ckey, uint32_t* rkey, uint32_t* iota)
 {
   for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < N; p += gridDim.x * blockDim.x)
   {
-    rank[p] = kAlpha;
-    // init(vid, other, s) returns true for everyone, so regular and source
-    // vertices scatter rank / degree (pr.h:34-37); sinks and isolated
-    // vertices have no out-edges and are never read as columns.
-    double xv = 0.0;
-    if (p < nreg || (p >= src_base && p < iso_base)) xv = __ddiv_rn(kAlpha, (double) deg[p]);
-    x0[p] = xv;
-    x1[p] = xv;
+    ckey[p] = mask - deg[p];
+    if (p < nrows) rkey[p] = (p < nreg ? 0u : mask + 1) + (mask - (ptr[p + 1] - ptr[p]));
+    iota[p] = p;
   }
 }
 
-__global__ void k_mark_long(const uint32_t* __restrict__ ptr, uint32_t nrows, uint32_t* keys, uint32_t* vals,
-                            uint32_t* count)
+// Row classes from the sorted keys: bounds[0..3] = q1, q2 of the regular rows,
+// q1, q2 of the sinks (one thread each).
+__global__ void k_pr_bounds(uint32_t nrows, uint32_t nreg, uint32_t mask, const uint32_t* __restrict__ rkey,
+                            uint32_t* bounds)
 {
-  for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < nrows; r += gridDim.x * blockDim.x)
+  const uint32_t t = threadIdx.x, lim = (t & 1) ? kShortRow : kLongRow;
+  uint32_t lo = t < 2 ? 0 : nreg, hi = t < 2 ? nreg : nrows;
+  const uint32_t key = (t < 2 ? 0u : mask + 1) + (mask > lim ? mask - lim : 0u);  // the first row with lim or fewer
+  while (lo < hi)
   {
-    uint32_t d = ptr[r + 1] - ptr[r];
-    if (d > kLongRow) atomicAdd(count + 1, 1u);
-    if (d > kMedRow)
+    const uint32_t mid = (lo + hi) >> 1;
+    if (rkey[mid] < key) lo = mid + 1;
+    else hi = mid;
+  }
+  bounds[t] = lo;
+}
+
+// Slot of each position; the rows' own arrays by q; the entries each row takes
+// (a slice: its rows together, 32 or fewer, the first one's length each).
+__global__ void k_pr_slots(uint32_t N, const uint32_t* __restrict__ order, uint32_t* slot)
+{
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) slot[order[i]] = i;
+}
+
+__global__ void k_pr_rows(uint32_t N, uint32_t nrows, uint32_t nreg, uint32_t mask, const uint32_t* __restrict__ rkey,
+                          const uint32_t* __restrict__ bounds, const uint32_t* __restrict__ deg,
+                          const uint32_t* __restrict__ slot, uint32_t* qpos, uint32_t* xi, uint32_t* degq, uint64_t* take)
+{
+  for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < N; q += gridDim.x * blockDim.x)
+  {
+    if (q >= nrows) qpos[q] = q;
+    const uint32_t p = q < nrows ? qpos[q] : q;
+    xi[q] = slot[p];
+    degq[q] = deg[p];
+    if (q > nrows) continue;
+    uint64_t n = 0;
+    if (q < nrows)
     {
-      uint32_t i = atomicAdd(count, 1u);
-      keys[i] = ~d;  // ascending sort of ~d = descending degree
-      vals[i] = r;
+      const uint32_t q2 = bounds[q < nreg ? 1 : 3];
+      if (q < q2) n = (mask - (rkey[q] & mask) + 3) & ~3u;
+      else
+      {
+        n = mask - (rkey[q2 + ((q - q2) & ~31u)] & mask);
+        // the last slice ends on a multiple of 4, where the sinks' long rows start
+        if (q + 1 == (q < nreg ? nreg : nrows)) n += (0 - (((q - q2) & 31u) + 1) * n) & 3;
+      }
     }
+    take[q] = n;
+  }
+  if (nrows == N && blockIdx.x == 0 && threadIdx.x == 0) take[N] = 0;
+}
+
+// Blocks of a kernel over a PrRange: [0, nlong) a block per row, then nmed a
+// warp per row, the rest a warp per slice.
+struct PrBlocks
+{
+  uint32_t nlong, nmed, total;
+};
+
+static PrBlocks pr_blocks(const PrRange& r)
+{
+  PrBlocks b;
+  b.nlong = std::min<uint32_t>(r.q1 - r.q0, num_sms() * 4);
+  b.nmed = std::min<uint32_t>((r.q2 - r.q1 + kWarpsPerBlock - 1) / kWarpsPerBlock, num_sms() * 8);
+  const uint32_t slices = (r.q3 - r.q2 + 31) / 32;
+  b.total = b.nlong + b.nmed + std::min<uint32_t>((slices + kWarpsPerBlock - 1) / kWarpsPerBlock, num_sms() * 8);
+  return b;
+}
+
+__global__ void __launch_bounds__(kWarpsPerBlock * 32)
+k_pr_fill(PrRange R, PrBlocks B, const uint32_t* __restrict__ qpos, const uint64_t* __restrict__ off,
+          const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col, const uint32_t* __restrict__ slot,
+          uint32_t zero, uint32_t* __restrict__ out)
+{
+  const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  if (blockIdx.x < B.nlong + B.nmed)
+  {
+    const bool block = blockIdx.x < B.nlong;  // a block or a warp per row
+    const uint32_t step = block ? blockDim.x : 32, at = block ? threadIdx.x : lane;
+    const uint32_t hi = block ? R.q1 : R.q2;
+    uint32_t q = block ? R.q0 + blockIdx.x : R.q1 + (blockIdx.x - B.nlong) * kWarpsPerBlock + wib;
+    for (; q < hi; q += block ? B.nlong : B.nmed * kWarpsPerBlock)
+    {
+      const uint32_t p = qpos[q], b = ptr[p], n = ptr[p + 1] - b;
+      uint32_t* o = out + off[q];
+      for (uint32_t i = at; i < ((n + 3) & ~3u); i += step) o[i] = i < n ? slot[col[b + i]] : zero;
+    }
+    return;
+  }
+  const uint32_t nw = (gridDim.x - B.nlong - B.nmed) * kWarpsPerBlock;
+  for (uint32_t q0 = R.q2 + ((blockIdx.x - B.nlong - B.nmed) * kWarpsPerBlock + wib) * 32; q0 < R.q3; q0 += nw * 32)
+  {
+    const uint32_t cnt = min(32u, R.q3 - q0);
+    uint32_t b = 0, n = 0;
+    if (lane < cnt)
+    {
+      const uint32_t p = qpos[q0 + lane];
+      b = ptr[p];
+      n = ptr[p + 1] - b;
+    }
+    const uint32_t width = (uint32_t) (off[q0 + 1] - off[q0]);
+    uint32_t* o = out + off[q0];
+    if (lane < cnt)
+      for (uint32_t t = 0; t < width; t++) o[t * cnt + lane] = t < n ? slot[col[b + t]] : zero;
+  }
+}
+
+// x: regular and source vertices scatter rank / degree (init(vid, other, s)
+// returns true for everyone, pr.h:34-37); sinks and isolated vertices have no
+// out-edges and are never read as columns.  Slot N is the padding's.
+template <class T>
+__global__ void k_pr_init(uint32_t N, uint32_t nreg, uint32_t src_base, uint32_t iso_base,
+                          const uint32_t* __restrict__ degq, const uint32_t* __restrict__ xi, T* rank, T* x0, T* x1)
+{
+  for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q <= N; q += gridDim.x * blockDim.x)
+  {
+    T xv = 0;
+    if (q < N)
+    {
+      rank[q] = (T) kAlpha;
+      if (q < nreg || (q >= src_base && q < iso_base)) xv = (T) kAlpha / (T) degq[q];
+    }
+    const uint32_t k = q < N ? xi[q] : N;
+    x0[k] = xv;
+    x1[k] = xv;
   }
 }
 
@@ -109,13 +254,13 @@ __device__ __forceinline__ double pr_apply(double partial)
   return __dadd_rn(kAlpha, __dmul_rn(1.0 - kAlpha, y));
 }
 
-__device__ __forceinline__ void pr_finish_row(uint32_t r, double acc, const uint32_t* __restrict__ deg, double* rank,
-                                              double* xnext, int* flag, bool write_x)
+__device__ __forceinline__ void pr_finish_row(uint32_t q, double acc, const PrLayout& L, double* rank, double* xnext,
+                                              int* flag, bool write_x)
 {
-  double old = rank[r];
+  double old = rank[q];
   double nr = pr_apply(acc);
-  rank[r] = nr;
-  if (write_x) xnext[r] = __ddiv_rn(nr, (double) deg[r]);
+  rank[q] = nr;
+  if (write_x) xnext[L.xi[q]] = __ddiv_rn(nr, (double) L.degq[q]);
   if (flag && fabs(__dsub_rn(nr, old)) > kTol) *flag = 1;
 }
 
@@ -132,7 +277,7 @@ __device__ __forceinline__ void pr_finish_row(uint32_t r, double acc, const uint
 // bit for bit.  Where m would reach 2^53 (acc enters the next binade, at most
 // once per doubling of the sum), the thread that holds that value adds its few
 // values with real FP64 additions, and the rest is taken up with the new
-// exponent.  On R-MAT 2^16 (1M edges): 328 -> 45 us per iteration.
+// exponent.  On R-MAT 2^16 (1M edges): 328 -> 26 us per iteration.
 struct ExactSum
 {
   uint64_t m;  // value m 2^(e - 1075); m < 2^53
@@ -145,7 +290,11 @@ struct ParityFn  // increments for m even / odd
 };
 
 static constexpr uint64_t kExactTop = 1ull << 53;
-static constexpr int kExactPer = 8;  // consecutive values per thread and step
+// Consecutive values per thread and step: a step costs the functions of a
+// thread's values and, at a new binade, as many FP64 additions (R-MAT 2^16, 20
+// iterations, the whole call: 8 values 700 us, 4 values 630).
+static constexpr int kExactPer = 4;
+static constexpr int kAhead = 8;  // entries of a slice's lane per step
 
 __device__ __forceinline__ ExactSum exact_of(double v)
 {
@@ -189,31 +338,29 @@ __device__ __forceinline__ ParityFn exact_shfl_up(ParityFn f, int d)
   return {__shfl_up_sync(0xffffffffu, f.a, d), __shfl_up_sync(0xffffffffu, f.b, d)};
 }
 
-// The thread's kExactPer values of the chunk that starts at entry `base`
-// (a multiple of 4, so that the column indices load as 16-byte vectors);
-// entries outside [b, e) count as 0, which adds nothing.  in_col is
-// allocated past its last entry for the vectors that straddle the end.
-__device__ __forceinline__ void exact_load(const uint32_t* __restrict__ col, const double* __restrict__ x, uint32_t base,
-                                           uint32_t b, uint32_t e, double v[kExactPer])
+// A thread's kExactPer consecutive values from entry i of a row of n entries
+// (both multiples of 4; entries beyond n count as 0, which adds nothing).
+__device__ __forceinline__ void exact_load(const uint32_t* __restrict__ col, const double* __restrict__ x, uint32_t i,
+                                           uint32_t n, double v[kExactPer])
 {
 #pragma unroll
-  for (int q = 0; q < kExactPer; q += 4)
+  for (int k = 0; k < kExactPer; k += 4)
   {
-    const uint32_t i = base + q;
+    const bool in = i + k < n;
     uint4 c = make_uint4(0, 0, 0, 0);
-    if (i < e) c = *reinterpret_cast<const uint4*>(col + i);
-    v[q] = i >= b && i < e ? x[c.x] : 0.0;
-    v[q + 1] = i + 1 >= b && i + 1 < e ? x[c.y] : 0.0;
-    v[q + 2] = i + 2 >= b && i + 2 < e ? x[c.z] : 0.0;
-    v[q + 3] = i + 3 >= b && i + 3 < e ? x[c.w] : 0.0;
+    if (in) c = __ldcs(reinterpret_cast<const uint4*>(col + i + k));
+    v[k] = in ? x[c.x] : 0.0;
+    v[k + 1] = in ? x[c.y] : 0.0;
+    v[k + 2] = in ? x[c.z] : 0.0;
+    v[k + 3] = in ? x[c.w] : 0.0;
   }
 }
 
-__device__ __forceinline__ ParityFn exact_mine(const double v[kExactPer], int e)
+__device__ __forceinline__ ParityFn exact_mine(const double (&v)[kExactPer], int e)
 {
   ParityFn f{0, 0};
 #pragma unroll
-  for (int q = 0; q < kExactPer; q++) f = exact_then(f, exact_fn(v[q], e));
+  for (int k = 0; k < kExactPer; k++) f = exact_then(f, exact_fn(v[k], e));
   return f;
 }
 
@@ -229,14 +376,14 @@ __device__ __forceinline__ ParityFn exact_scan(ParityFn f, int lane)
   return f;
 }
 
-// One row by one warp.
+// One row of n entries (a multiple of 4) by one warp.
 __device__ __forceinline__ double exact_row_warp(const uint32_t* __restrict__ col, const double* __restrict__ x,
-                                                 uint32_t b, uint32_t e, int lane)
+                                                 uint32_t n, int lane)
 {
   ExactSum s{0, -1};
   double v[kExactPer];
-  exact_load(col, x, (b & ~3u) + lane * kExactPer, b, e, v);
-  for (uint64_t base = b & ~3u; base < e; base += 32 * kExactPer)
+  exact_load(col, x, lane * kExactPer, n, v);
+  for (uint32_t base = 0; base < n; base += 32 * kExactPer)  // a warp's rows end at kLongRow
   {
     int from = 0;  // lanes below are in the sum already
     for (;;)
@@ -257,22 +404,22 @@ __device__ __forceinline__ double exact_row_warp(const uint32_t* __restrict__ co
       {
         acc = exact_double(before, s.e);
 #pragma unroll
-        for (int q = 0; q < kExactPer; q++) acc = __dadd_rn(acc, v[q]);
+        for (int k = 0; k < kExactPer; k++) acc = __dadd_rn(acc, v[k]);
       }
       s = exact_of(__shfl_sync(0xffffffffu, acc, L));
       from = L + 1;
       if (from == 32) break;
     }
-    if (base + 32 * kExactPer < e) exact_load(col, x, (uint32_t) base + (32 + lane) * kExactPer, b, e, v);
+    if (base + 32 * kExactPer < n) exact_load(col, x, base + (32 + lane) * kExactPer, n, v);
   }
   return exact_double(s.m, s.e);
 }
 
-// One row by one block (WARPS warps): the warps' functions meet in shared
+// One row of n entries (a multiple of 4) by one block (WARPS warps): the warps' functions meet in shared
 // memory, every thread composes them and keeps its own copy of the sum.
 template <int WARPS>
 __device__ __forceinline__ double exact_row_block(const uint32_t* __restrict__ col, const double* __restrict__ x,
-                                                  uint32_t b, uint32_t e)
+                                                  uint64_t n)
 {
   __shared__ ParityFn s_fn[2][WARPS];
   __shared__ double s_acc;
@@ -282,11 +429,12 @@ __device__ __forceinline__ double exact_row_block(const uint32_t* __restrict__ c
   ExactSum s{0, -1};
   double v[kExactPer], nv[kExactPer];
   int buf = 0;
-  exact_load(col, x, (b & ~3u) + threadIdx.x * kExactPer, b, e, v);
-  for (uint64_t base = b & ~3u; base < e; base += kStep)
+  const uint32_t at = threadIdx.x * kExactPer;
+  exact_load(col, x, at, (uint32_t) min(n, (uint64_t) kStep), v);
+  for (uint64_t base = 0; base < n; base += kStep)
   {
-    const bool more = base + kStep < e;
-    if (more) exact_load(col, x, (uint32_t) (base + kStep) + threadIdx.x * kExactPer, b, e, nv);
+    const uint64_t next = base + kStep;
+    if (next < n) exact_load(col + next, x, at, (uint32_t) min(n - next, (uint64_t) kStep), nv);
     int from = 0;
     for (;;)
     {
@@ -322,7 +470,7 @@ __device__ __forceinline__ double exact_row_block(const uint32_t* __restrict__ c
         {
           double acc = exact_double(before, s.e);
 #pragma unroll
-          for (int q = 0; q < kExactPer; q++) acc = __dadd_rn(acc, v[q]);
+          for (int k = 0; k < kExactPer; k++) acc = __dadd_rn(acc, v[k]);
           s_acc = acc;
           s_from = w * 32 + L + 1;
         }
@@ -333,86 +481,77 @@ __device__ __forceinline__ double exact_row_block(const uint32_t* __restrict__ c
       if (from == WARPS * 32) break;
     }
 #pragma unroll
-    for (int q = 0; q < kExactPer; q++) v[q] = nv[q];
+    for (int k = 0; k < kExactPer; k++) v[k] = nv[k];
   }
   __syncthreads();  // s_fn, s_acc and s_from are free for the next row
   return exact_double(s.m, s.e);
 }
 
-// Rows [row_lo, row_hi).  Blocks [0, long_blocks) take the rows above
-// kLongRow (a block per row, descending length), the next med_blocks the rest
-// of the rows above kMedRow (a warp per row), the others 32-row tiles.
+// One pull over the rows of R.
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
-k_pr_pull(const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col, const double* __restrict__ x,
-          double* __restrict__ xnext, double* __restrict__ rank, const uint32_t* __restrict__ deg,
-          const uint32_t* __restrict__ long_rows, uint32_t nlong, uint32_t nheavy, uint32_t long_blocks,
-          uint32_t med_blocks, uint32_t row_lo, uint32_t row_hi, int* flag, int write_x)
+k_pr_pull(PrRange R, PrBlocks B, PrLayout L, uint32_t zero, const double* __restrict__ x, double* __restrict__ xnext,
+          double* __restrict__ rank, int* flag, int write_x)
 {
-  __shared__ double sx[kWarpsPerBlock][kChunk];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  if (blockIdx.x < long_blocks)
+  if (blockIdx.x < B.nlong)
   {
-    for (uint32_t li = blockIdx.x; li < nlong; li += long_blocks)
+    for (uint32_t q = R.q0 + blockIdx.x; q < R.q1; q += B.nlong)
     {
-      const uint32_t r = long_rows[li];
-      if (r < row_lo || r >= row_hi) continue;  // the same for the whole block
-      const double acc = exact_row_block<kWarpsPerBlock>(col, x, ptr[r], ptr[r + 1]);
-      if (threadIdx.x == 0) pr_finish_row(r, acc, deg, rank, xnext, flag, write_x);
+      const uint64_t o = L.off[q];
+      const double acc = exact_row_block<kWarpsPerBlock>(L.col + o, x, L.off[q + 1] - o);
+      if (threadIdx.x == 0) pr_finish_row(q, acc, L, rank, xnext, flag, write_x);
     }
     return;
   }
-  if (blockIdx.x < long_blocks + med_blocks)
+  if (blockIdx.x < B.nlong + B.nmed)
   {
-    for (uint32_t li = nlong + (blockIdx.x - long_blocks) * kWarpsPerBlock + wib; li < nheavy;
-         li += med_blocks * kWarpsPerBlock)
+    for (uint32_t q = R.q1 + (blockIdx.x - B.nlong) * kWarpsPerBlock + wib; q < R.q2; q += B.nmed * kWarpsPerBlock)
     {
-      const uint32_t r = long_rows[li];
-      if (r < row_lo || r >= row_hi) continue;  // the same for the whole warp
-      const double acc = exact_row_warp(col, x, ptr[r], ptr[r + 1], lane);
-      if (lane == 0) pr_finish_row(r, acc, deg, rank, xnext, flag, write_x);
+      const uint64_t o = L.off[q];
+      const double acc = exact_row_warp(L.col + o, x, (uint32_t) (L.off[q + 1] - o), lane);
+      if (lane == 0) pr_finish_row(q, acc, L, rank, xnext, flag, write_x);
     }
     return;
   }
-  const uint32_t ntiles = (row_hi - row_lo + 31) / 32;
-  const uint32_t first = long_blocks + med_blocks;
-  const uint32_t nwarps = (gridDim.x - first) * kWarpsPerBlock;
-  for (uint32_t t = (blockIdx.x - first) * kWarpsPerBlock + wib; t < ntiles; t += nwarps)
+  const uint32_t first = B.nlong + B.nmed, nw = (gridDim.x - first) * kWarpsPerBlock;
+  for (uint32_t q0 = R.q2 + ((blockIdx.x - first) * kWarpsPerBlock + wib) * 32; q0 < R.q3; q0 += nw * 32)
   {
-    const uint32_t r0 = row_lo + t * 32;
-    const uint32_t r = r0 + lane;
-    const bool valid = r < row_hi;
-    uint32_t rb = valid ? ptr[r] : 0, re = valid ? ptr[r + 1] : 0;
-    const bool mine = valid && (re - rb) <= kMedRow;
-    if (!mine) { rb = 0; re = 0; }
-    // Walk the short rows' edges in chunks; each chunk starts at the lowest
-    // edge any lane still needs, which skips over the longer rows' edges.
-    const uint32_t te = ptr[min(r0 + 32, row_hi)];
-    double acc = 0.0;
-    uint32_t cur = rb;  // next edge of my row to add
-    for (;;)
-    {
-      const uint32_t base = __reduce_min_sync(0xffffffffu, cur < re ? cur : 0xffffffffu);
-      if (base == 0xffffffffu) break;
-      const uint32_t lim = min(base + kChunk, te);
+    const uint32_t cnt = min(32u, R.q3 - q0), width = (uint32_t) (L.off[q0 + 1] - L.off[q0]);
+    const uint32_t* col = L.col + L.off[q0] + lane;
+    if ((uint32_t) lane >= cnt) continue;
+    // one step of kAhead additions (a serial chain) while the next step's
+    // messages and the slots of the one after are on their way
+    double acc = 0.0, v[kAhead];
+    uint32_t c[kAhead];
 #pragma unroll
-      for (int k = 0; k < kChunk / 32; k++)
-      {
-        uint32_t i = base + k * 32 + lane;
-        if (i < lim) sx[wib][k * 32 + lane] = x[col[i]];
-      }
-      __syncwarp();
-      const uint32_t stop = min(re, lim);
-      for (; cur < stop; cur++) acc = __dadd_rn(acc, sx[wib][cur - base]);
-      __syncwarp();
+    for (int u = 0; u < kAhead; u++) c[u] = (uint32_t) u < width ? __ldcs(col + u * cnt) : zero;
+#pragma unroll
+    for (int u = 0; u < kAhead; u++) v[u] = x[c[u]];
+#pragma unroll
+    for (int u = 0; u < kAhead; u++) c[u] = kAhead + u < width ? __ldcs(col + (kAhead + u) * cnt) : zero;
+    for (uint32_t t = 0; t < width; t += kAhead)
+    {
+      double nv[kAhead];
+#pragma unroll
+      for (int u = 0; u < kAhead; u++) nv[u] = x[c[u]];
+#pragma unroll
+      for (int u = 0; u < kAhead; u++) c[u] = t + 2 * kAhead + u < width ? __ldcs(col + (t + 2 * kAhead + u) * cnt) : zero;
+#pragma unroll
+      for (int u = 0; u < kAhead; u++) acc = __dadd_rn(acc, v[u]);
+#pragma unroll
+      for (int u = 0; u < kAhead; u++) v[u] = nv[u];
     }
-    if (mine) pr_finish_row(r, acc, deg, rank, xnext, flag, write_x);
+    pr_finish_row(q0 + lane, acc, L, rank, xnext, flag, write_x);
   }
 }
 
-__global__ void k_scatter_pos(uint32_t N, const uint32_t* __restrict__ id_of_pos, const double* __restrict__ val,
-                              double* __restrict__ out)
+// Ranks by id; vertices that are not rows keep alpha (in FP64 in either form).
+template <class T>
+__global__ void k_rank_by_id(uint32_t N, uint32_t nrows, const uint32_t* __restrict__ qpos, const uint32_t* __restrict__ id_of_pos,
+                             const T* __restrict__ rank, double* __restrict__ out)
 {
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < N; p += gridDim.x * blockDim.x) out[id_of_pos[p]] = val[p];
+  for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < N; q += gridDim.x * blockDim.x)
+    out[id_of_pos[qpos[q]]] = q < nrows ? (double) rank[q] : kAlpha;
 }
 
 __global__ void k_scatter_pos_u32(uint32_t N, const uint32_t* __restrict__ id_of_pos, const uint32_t* __restrict__ val,
@@ -434,12 +573,14 @@ static int pr_prepare(la3g_graph* G, PrScratch** out)
     G->slot[kSlotPr] = ps;
     G->slot_free[kSlotPr] = pr_scratch_free;
   }
-  const uint32_t N = g.nslots;
+  const uint32_t N = g.nslots, nrows = g.nrows();
+  PrLayout& L = ps->L;
   LA3G_TRY(galloc(G, &ps->deg, N));
-  LA3G_TRY(galloc(G, &ps->rank, N));
-  LA3G_TRY(galloc(G, &ps->x[0], N));
-  LA3G_TRY(galloc(G, &ps->x[1], N));
   LA3G_TRY(galloc(G, &ps->flag, 4));
+  LA3G_TRY(galloc(G, &L.qpos, N));
+  LA3G_TRY(galloc(G, &L.xi, N));
+  LA3G_TRY(galloc(G, &L.degq, N));
+  LA3G_TRY(galloc(G, &L.off, (size_t) nrows + 1));
   LA3G_CUDA(cudaMemsetAsync(ps->deg, 0, (size_t) N * 4, s));
   if (g.nent)
   {
@@ -447,34 +588,57 @@ static int pr_prepare(la3g_graph* G, PrScratch** out)
     k_outdeg<<<grid_for(g.nent, 256), 256, 0, s>>>(g.in_col, g.nent, ps->deg);
     LA3G_LAUNCHED();
   }
-  // long and medium rows, sorted by descending degree
-  DevBuf keys, vals, keys2, vals2, cnt;
-  LA3G_TRY(keys.alloc((size_t) g.nrows() * 4 + 4));
-  LA3G_TRY(vals.alloc((size_t) g.nrows() * 4 + 4));
-  LA3G_TRY(cnt.alloc(8));
-  LA3G_CUDA(cudaMemsetAsync(cnt.p, 0, 8, s));
-  if (g.nrows())
+  // no self-loops and no duplicates: degrees are below N, which is at most 2^31
+  int bits = 1;
+  while (((uint64_t) (N - 1) >> bits) != 0) bits++;
+  const uint32_t mask = (1u << bits) - 1;
+  // one allocation for the temporaries: four key / value arrays, the rows'
+  // entry counts, the library calls' storage, the class bounds
+  size_t tb0 = 0, tb1 = 0;
+  uint32_t* null32 = nullptr;
+  uint64_t* null64 = nullptr;
+  LA3G_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb0, null32, null32, null32, null32, (int64_t) N, 0, bits + 1, s));
+  LA3G_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb1, null64, null64, (int64_t) nrows + 1, s));
+  const size_t n4 = ((size_t) N * 4 + 255) & ~(size_t) 255, n8 = ((size_t) N * 8 + 8 + 255) & ~(size_t) 255;
+  DevBuf tmp;
+  LA3G_TRY(tmp.alloc(5 * n4 + n8 + 256 + std::max(tb0, tb1)));
+  char* t = tmp.as<char>();
+  uint32_t *key = (uint32_t*) t, *rkey = (uint32_t*) (t + n4), *key2 = (uint32_t*) (t + 2 * n4);
+  uint32_t *iota = (uint32_t*) (t + 3 * n4), *slot = (uint32_t*) (t + 4 * n4);
+  uint64_t* take = (uint64_t*) (t + 5 * n4);
+  uint32_t* bounds = (uint32_t*) (t + 5 * n4 + n8);
+  void* lib = t + 5 * n4 + n8 + 256;
+  k_pr_keys<<<grid_for(N, 256), 256, 0, s>>>(N, nrows, g.nreg, mask, g.in_ptr, ps->deg, key, rkey, iota);
+  LA3G_LAUNCHED();
+  uint32_t* order = L.xi;  // the columns' order, until xi is written
+  LA3G_CUDA(cub::DeviceRadixSort::SortPairs(lib, tb0, key, key2, iota, order, (int64_t) N, 0, bits, s));
+  k_pr_slots<<<grid_for(N, 256), 256, 0, s>>>(N, order, slot);
+  LA3G_LAUNCHED();
+  if (nrows)
   {
-    k_mark_long<<<grid_for(g.nrows(), 256), 256, 0, s>>>(g.in_ptr, g.nrows(), keys.as<uint32_t>(), vals.as<uint32_t>(),
-                                                         cnt.as<uint32_t>());
+    LA3G_CUDA(cub::DeviceRadixSort::SortPairs(lib, tb0, rkey, key, iota, L.qpos, (int64_t) nrows, 0, bits + 1, s));
+    k_pr_bounds<<<1, 4, 0, s>>>(nrows, g.nreg, mask, key, bounds);
     LA3G_LAUNCHED();
   }
-  uint32_t n[2] = {0, 0};
-  LA3G_CUDA(cudaMemcpyAsync(n, cnt.p, 8, cudaMemcpyDeviceToHost, s));
+  k_pr_rows<<<grid_for(N, 256), 256, 0, s>>>(N, nrows, g.nreg, mask, key, bounds, ps->deg, slot, L.qpos, L.xi, L.degq,
+                                             take);
+  LA3G_LAUNCHED();
+  LA3G_CUDA(cub::DeviceScan::ExclusiveSum(lib, tb1, take, L.off, (int64_t) nrows + 1, s));
+  uint32_t hb[4] = {0, 0, 0, 0};
+  uint64_t total = 0;
+  if (nrows) LA3G_CUDA(cudaMemcpyAsync(hb, bounds, 16, cudaMemcpyDeviceToHost, s));
+  LA3G_CUDA(cudaMemcpyAsync(&total, L.off + nrows, 8, cudaMemcpyDeviceToHost, s));
   LA3G_CUDA(cudaStreamSynchronize(s));
-  ps->nheavy = n[0];
-  ps->nlong = n[1];
-  LA3G_TRY(galloc(G, &ps->long_rows, (size_t) n[0] + 1));
-  if (n[0])
+  L.reg = PrRange{0, hb[0], hb[1], g.nreg};
+  L.sink = PrRange{g.nreg, hb[2], hb[3], nrows};
+  if (!nrows) L.sink = PrRange{0, 0, 0, 0};
+  LA3G_TRY(galloc(G, &L.col, (size_t) total + 4));
+  for (const PrRange& r : {L.reg, L.sink})
   {
-    LA3G_TRY(keys2.alloc((size_t) n[0] * 4 + 4));
-    size_t tb = 0;
-    LA3G_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, keys.as<uint32_t>(), keys2.as<uint32_t>(), vals.as<uint32_t>(),
-                                              ps->long_rows, n[0], 0, 32, s));
-    DevBuf tmp;
-    LA3G_TRY(tmp.alloc(tb));
-    LA3G_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, tb, keys.as<uint32_t>(), keys2.as<uint32_t>(), vals.as<uint32_t>(),
-                                              ps->long_rows, n[0], 0, 32, s));
+    if (r.q3 == r.q0) continue;
+    const PrBlocks b = pr_blocks(r);
+    k_pr_fill<<<b.total, kWarpsPerBlock * 32, 0, s>>>(r, b, L.qpos, L.off, g.in_ptr, g.in_col, slot, N, L.col);
+    LA3G_LAUNCHED();
   }
   LA3G_CUDA(cudaStreamSynchronize(s));
   ps->ready = true;
@@ -482,138 +646,139 @@ static int pr_prepare(la3g_graph* G, PrScratch** out)
   return LA3G_OK;
 }
 
-static int pr_launch(la3g_graph* G, PrScratch* ps, const double* x, double* xnext, uint32_t row_lo, uint32_t row_hi,
-                     int* flag, bool write_x)
+static int pr_launch(la3g_graph* G, PrScratch* ps, const PrRange& r, const double* x, double* xnext, int* flag,
+                     bool write_x)
 {
   DevGraph& g = G->g;
-  if (row_hi <= row_lo) return LA3G_OK;
-  const uint32_t long_blocks = std::min<uint32_t>(ps->nlong, num_sms() * 4);
-  const uint32_t med_blocks =
-      std::min<uint32_t>((ps->nheavy - ps->nlong + kWarpsPerBlock - 1) / kWarpsPerBlock, num_sms() * 8);
-  const uint32_t ntiles = (row_hi - row_lo + 31) / 32;
-  const uint32_t tile_blocks = std::min<uint32_t>((ntiles + kWarpsPerBlock - 1) / kWarpsPerBlock, num_sms() * 8);
+  const uint32_t rows = r.q3 - r.q0;
+  if (!rows) return LA3G_OK;
+  const PrBlocks b = pr_blocks(r);
   // algorithmic bytes: 4 B index per edge + per-row ptr, x, rank, xnext
-  double bytes = 4.0 * (double) g.nent + 4.0 * (row_hi - row_lo + 1) + 8.0 * (double) g.nslots +
-                 (write_x ? 16.0 : 8.0) * (row_hi - row_lo) + 4.0 * (row_hi - row_lo);
+  double bytes = 4.0 * (double) g.nent + 4.0 * (rows + 1) + 8.0 * (double) g.nslots + (write_x ? 16.0 : 8.0) * rows +
+                 4.0 * rows;
   ProfileScope p("pr_pull_f64", G->stream, bytes);
-  k_pr_pull<<<long_blocks + med_blocks + std::max<uint32_t>(tile_blocks, 1), kWarpsPerBlock * 32, 0, G->stream>>>(
-      g.in_ptr, g.in_col, x, xnext, ps->rank, ps->deg, ps->long_rows, ps->nlong, ps->nheavy, long_blocks, med_blocks,
-      row_lo, row_hi, flag, write_x ? 1 : 0);
+  k_pr_pull<<<b.total, kWarpsPerBlock * 32, 0, G->stream>>>(r, b, ps->L, g.nslots, x, xnext, ps->rank, flag,
+                                                            write_x ? 1 : 0);
   LA3G_LAUNCHED();
   return LA3G_OK;
 }
 
 // ------------------------------------------------------------------ FP32 study
 
-__global__ void k_prf_init(uint32_t N, uint32_t nrows_reg, uint32_t src_base, uint32_t iso_base,
-                           const uint32_t* __restrict__ deg, float* rankf, double* rank, float* x0, float* x1)
-{
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < N; p += gridDim.x * blockDim.x)
-  {
-    rankf[p] = (float) kAlpha;
-    rank[p] = kAlpha;
-    float xv = 0.0f;
-    bool scat = (p < nrows_reg) || (p >= src_base && p < iso_base);
-    if (scat && deg[p]) xv = (float) kAlpha / (float) deg[p];
-    x0[p] = xv;
-    x1[p] = xv;
-  }
-}
+__device__ __forceinline__ float prf_next(float acc) { return (float) kAlpha + (float) (1.0 - kAlpha) * acc; }
 
-__device__ __forceinline__ double prf_finish(uint32_t r, float acc, float* __restrict__ xnext, float* __restrict__ rankf,
-                                             double* __restrict__ rank, const uint32_t* __restrict__ deg, int write_x)
+__device__ __forceinline__ double prf_finish(uint32_t q, float acc, const PrLayout& L, float* __restrict__ xnext,
+                                             float* __restrict__ rankf, int write_x)
 {
-  const float nr = (float) kAlpha + (float) (1.0 - kAlpha) * acc;
-  const double d = fabs((double) nr - (double) rankf[r]);
-  rankf[r] = nr;
-  rank[r] = (double) nr;
-  if (write_x) xnext[r] = nr / (float) deg[r];
+  const float nr = prf_next(acc);
+  const double d = fabs((double) nr - (double) rankf[q]);
+  rankf[q] = nr;
+  if (write_x) xnext[L.xi[q]] = nr / (float) L.degq[q];
   return d;
 }
 
-// FP32 SpMV with FP32 accumulation (any order inside a row is allowed
-// here).  The first `long_blocks` blocks take the rows longer than
-// kLongRow, one block per row with a shared-memory reduction; the others
-// give each row of at most kLongRow edges a group of 4 lanes (eight rows
-// per warp), so average-degree rows keep the lanes busy.  The L1 residual
-// is reduced in FP64.
-__global__ void __launch_bounds__(256)
-k_prf_pull(const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col, const float* __restrict__ x,
-           float* __restrict__ xnext, float* __restrict__ rankf, double* __restrict__ rank,
-           const uint32_t* __restrict__ deg, const uint32_t* __restrict__ long_rows, uint32_t nlong,
-           uint32_t long_blocks, uint32_t row_lo, uint32_t row_hi, double* resid, int write_x)
+// One FP32 pull over the rows of R, FP32 accumulation.  A row of at most
+// kLongRow entries has four partial sums, entry i in sum i % 4, combined
+// (0 + 2) + (1 + 3): a lane holds all four in a slice, a group of four lanes
+// one each above kShortRow.  A longer row has one per thread of its block.
+// The L1 residual is reduced in FP64.
+__global__ void __launch_bounds__(kWarpsPerBlock * 32)
+k_prf_pull(PrRange R, PrBlocks B, PrLayout L, uint32_t zero, const float* __restrict__ x, float* __restrict__ xnext,
+           float* __restrict__ rankf, double* resid, int write_x)
 {
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   double local = 0.0;
-  if (blockIdx.x < long_blocks)
+  if (blockIdx.x < B.nlong)
   {
-    __shared__ float part[8];
-    for (uint32_t k = blockIdx.x; k < nlong; k += long_blocks)
+    __shared__ float part[kWarpsPerBlock];
+    for (uint32_t q = R.q0 + blockIdx.x; q < R.q1; q += B.nlong)
     {
-      const uint32_t r = long_rows[k];
-      if (r < row_lo || r >= row_hi) continue;  // uniform per block
+      const uint64_t o = L.off[q], n = L.off[q + 1] - o;
+      const uint32_t* col = L.col + o;
       float acc = 0.0f;
-      for (uint32_t i = ptr[r] + threadIdx.x; i < ptr[r + 1]; i += blockDim.x) acc += x[col[i]];
+      for (uint64_t i = threadIdx.x; i < n; i += 4 * kWarpsPerBlock * 32)
+      {
+        float v[4];
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-      if (lane == 0) part[threadIdx.x >> 5] = acc;
+        for (int u = 0; u < 4; u++)
+        {
+          const uint64_t k = i + u * kWarpsPerBlock * 32;
+          v[u] = x[k < n ? __ldcs(col + k) : zero];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) acc += v[u];
+      }
+#pragma unroll
+      for (int o2 = 16; o2 > 0; o2 >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o2);
+      if (lane == 0) part[wib] = acc;
       __syncthreads();
       if (threadIdx.x == 0)
       {
         float t = 0.0f;
-        for (int w = 0; w < (int) (blockDim.x >> 5); w++) t += part[w];
-        local += prf_finish(r, t, xnext, rankf, rank, deg, write_x);
+        for (int w = 0; w < kWarpsPerBlock; w++) t += part[w];
+        local += prf_finish(q, t, L, xnext, rankf, write_x);
       }
       __syncthreads();
     }
-    if (threadIdx.x == 0 && local != 0.0) atomicAdd(resid, local);
-    return;
   }
-  // short rows: 4 lanes per row, each keeping four independent loads in
-  // flight per step (the step is bound by memory latency)
-  constexpr uint32_t G = 4;
-  const uint32_t sub = lane & (G - 1);
-  const uint32_t group = ((blockIdx.x - long_blocks) * blockDim.x + threadIdx.x) / G;
-  const uint32_t ngroups = ((gridDim.x - long_blocks) * blockDim.x) / G;
-  const uint32_t nrows = row_hi - row_lo;
-  // all groups of a warp run the same number of rounds
-  const uint32_t rounds = (nrows + ngroups - 1) / ngroups;
-  for (uint32_t k = 0; k < rounds; k++)
+  else if (blockIdx.x < B.nlong + B.nmed)
   {
-    const uint32_t r = row_lo + group + k * ngroups;
-    float acc = 0.0f;
-    bool mine = false;
-    if (r < row_hi)
+    // eight rows per warp, four lanes each; a warp's lanes go round together
+    const uint32_t sub = lane & 3;
+    const uint32_t nw = B.nmed * kWarpsPerBlock;
+    for (uint32_t q0 = R.q1 + ((blockIdx.x - B.nlong) * kWarpsPerBlock + wib) * 8; q0 < R.q2; q0 += nw * 8)
     {
-      const uint32_t b = ptr[r], e = ptr[r + 1];
-      mine = (e - b) <= kLongRow;
-      if (mine)
-        for (uint32_t i = b + sub; i < e; i += 4 * G)
+      const uint32_t q = q0 + (lane >> 2);
+      float acc = 0.0f;
+      if (q < R.q2)
+      {
+        const uint64_t o = L.off[q];
+        const uint32_t n = (uint32_t) (L.off[q + 1] - o);
+        const uint32_t* col = L.col + o;
+        for (uint32_t i = sub; i < n; i += 32)
         {
-          uint32_t c[4];
+          float v[8];
 #pragma unroll
-          for (int u = 0; u < 4; u++) c[u] = i + u * G < e ? col[i + u * G] : 0xFFFFFFFFu;
-          float v[4];
+          for (int u = 0; u < 8; u++) v[u] = x[i + 4 * u < n ? __ldcs(col + i + 4 * u) : zero];
 #pragma unroll
-          for (int u = 0; u < 4; u++) v[u] = c[u] != 0xFFFFFFFFu ? x[c[u]] : 0.0f;
-#pragma unroll
-          for (int u = 0; u < 4; u++) acc += v[u];
+          for (int u = 0; u < 8; u++) acc += v[u];
         }
+      }
+      acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+      acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+      if (q < R.q2 && sub == 0) local += prf_finish(q, acc, L, xnext, rankf, write_x);
     }
-#pragma unroll
-    for (int o = G / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (mine && sub == 0) local += prf_finish(r, acc, xnext, rankf, rank, deg, write_x);
   }
+  else
+  {
+    const uint32_t first = B.nlong + B.nmed, nw = (gridDim.x - first) * kWarpsPerBlock;
+    for (uint32_t q0 = R.q2 + ((blockIdx.x - first) * kWarpsPerBlock + wib) * 32; q0 < R.q3; q0 += nw * 32)
+    {
+      const uint32_t cnt = min(32u, R.q3 - q0), width = (uint32_t) (L.off[q0 + 1] - L.off[q0]);
+      const uint32_t* col = L.col + L.off[q0] + lane;
+      if ((uint32_t) lane >= cnt) continue;
+      float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+      for (uint32_t t = 0; t < width; t += 8)
+      {
+        float v[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) v[u] = x[t + u < width ? __ldcs(col + (t + u) * cnt) : zero];
+#pragma unroll
+        for (int u = 0; u < 8; u++) acc[u & 3] += v[u];
+      }
+      local += prf_finish(q0 + lane, (acc[0] + acc[2]) + (acc[1] + acc[3]), L, xnext, rankf, write_x);
+    }
+  }
+  // one FP64 atomic per block (per-warp atomics on one word serialise)
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(0xffffffffu, local, o);
-  // one FP64 atomic per block (per-warp atomics on one word serialise)
-  __shared__ double wsum[8];
-  if (lane == 0) wsum[threadIdx.x >> 5] = local;
+  __shared__ double wsum[kWarpsPerBlock];
+  if (lane == 0) wsum[wib] = local;
   __syncthreads();
   if (threadIdx.x == 0)
   {
     double t = 0.0;
-    for (int w = 0; w < (int) (blockDim.x >> 5); w++) t += wsum[w];
+    for (int w = 0; w < kWarpsPerBlock; w++) t += wsum[w];
     if (t != 0.0) atomicAdd(resid, t);
   }
 }
@@ -787,6 +952,44 @@ static int pr_build_tiles(la3g_graph* G, PrScratch* ps)
   return LA3G_OK;
 }
 
+__global__ void k_prf_tile_init(uint32_t N, uint32_t nreg, uint32_t src_base, uint32_t iso_base,
+                                const uint32_t* __restrict__ deg, float* rankf, float* x0, float* x1)
+{
+  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < N; p += gridDim.x * blockDim.x)
+  {
+    rankf[p] = (float) kAlpha;
+    const bool scat = p < nreg || (p >= src_base && p < iso_base);
+    x0[p] = x1[p] = scat ? (float) kAlpha / (float) deg[p] : 0.0f;
+  }
+}
+
+__device__ __forceinline__ double prf_tile_finish(uint32_t p, float acc, float* __restrict__ xnext,
+                                                  float* __restrict__ rankf, const uint32_t* __restrict__ deg)
+{
+  const float nr = prf_next(acc);
+  const double d = fabs((double) nr - (double) rankf[p]);
+  rankf[p] = nr;
+  xnext[p] = nr / (float) deg[p];
+  return d;
+}
+
+// The tiled loop's results in the pull layout, for the sink pass and the output.
+__global__ void k_prf_from_tiles(uint32_t N, const uint32_t* __restrict__ qpos, const uint32_t* __restrict__ xi,
+                                 const float* __restrict__ trankf, const float* __restrict__ tx, float* rankf, float* x)
+{
+  for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q <= N; q += gridDim.x * blockDim.x)
+  {
+    if (q == N)
+    {
+      x[N] = 0.0f;
+      continue;
+    }
+    const uint32_t p = qpos[q];
+    rankf[q] = trankf[p];
+    x[xi[q]] = tx[p];
+  }
+}
+
 __global__ void __launch_bounds__(kTileThreads)
 k_prf_tiles(const uint32_t* __restrict__ tile_col, const uint32_t* __restrict__ tcol,
             const uint32_t* __restrict__ tptr, const uint16_t* __restrict__ trow,
@@ -794,7 +997,7 @@ k_prf_tiles(const uint32_t* __restrict__ tile_col, const uint32_t* __restrict__ 
             const uint32_t* __restrict__ in_ptr, const uint32_t* __restrict__ in_col,
             const uint32_t* __restrict__ long_rows, uint32_t nlong, uint32_t long_blocks,
             const float* __restrict__ x, float* __restrict__ xnext, float* __restrict__ rankf,
-            double* __restrict__ rank, const uint32_t* __restrict__ deg, double* resid)
+            const uint32_t* __restrict__ deg, double* resid)
 {
   extern __shared__ float ys[];  // kTileRows accumulators
   __shared__ uint32_t s_big[kTileBigCap];
@@ -807,7 +1010,6 @@ k_prf_tiles(const uint32_t* __restrict__ tile_col, const uint32_t* __restrict__ 
   for (uint32_t k = blockIdx.x; blockIdx.x < long_blocks && k < nlong; k += long_blocks)
   {
     const uint32_t r = long_rows[k];
-    if (r >= nreg) continue;  // a sink row (uniform per block)
     float acc = 0.0f;
     for (uint32_t i = in_ptr[r] + tid; i < in_ptr[r + 1]; i += kTileThreads) acc += x[in_col[i]];
 #pragma unroll
@@ -818,7 +1020,7 @@ k_prf_tiles(const uint32_t* __restrict__ tile_col, const uint32_t* __restrict__ 
     {
       float t = 0.0f;
       for (uint32_t w = 0; w < kTileThreads / 32; w++) t += s_lpart[w];
-      local += prf_finish(r, t, xnext, rankf, rank, deg, 1);
+      local += prf_tile_finish(r, t, xnext, rankf, deg);
     }
     __syncthreads();
   }
@@ -901,7 +1103,7 @@ k_prf_tiles(const uint32_t* __restrict__ tile_col, const uint32_t* __restrict__ 
     __syncthreads();
     for (uint32_t i = tid; i < nr; i += kTileThreads)
       if (in_ptr[r0 + i + 1] - in_ptr[r0 + i] <= kLongRow)  // long rows are finished by the flat kernel
-        local += prf_finish(r0 + i, ys[i], xnext, rankf, rank, deg, 1);
+        local += prf_tile_finish(r0 + i, ys[i], xnext, rankf, deg);
     __syncthreads();
   }
 #pragma unroll
@@ -931,12 +1133,17 @@ extern "C" int la3g_pr(la3g_graph* G, uint32_t iters, double* rank_out, uint32_t
   LA3G_TRY(pr_prepare(G, &ps));
   cudaStream_t s = G->stream;
   const uint32_t N = g.nslots;
+  if (!ps->rank)
+  {
+    LA3G_TRY(galloc(G, &ps->rank, N));
+    LA3G_TRY(galloc(G, &ps->x[0], (size_t) N + 1));
+    LA3G_TRY(galloc(G, &ps->x[1], (size_t) N + 1));
+  }
   T.device_begin();
-  k_pr_init<<<grid_for(N, 256), 256, 0, s>>>(N, g.nreg, g.src_base(), g.iso_base(), ps->deg, ps->rank, ps->x[0], ps->x[1]);
+  k_pr_init<double><<<grid_for((uint64_t) N + 1, 256), 256, 0, s>>>(N, g.nreg, g.src_base(), g.iso_base(), ps->L.degq,
+                                                                    ps->L.xi, ps->rank, ps->x[0], ps->x[1]);
   LA3G_LAUNCHED();
   tls_launches++;
-  // k_pr_init gives regular and source vertices a message; sinks and
-  // isolated vertices never scatter (their x stays 0 and is never read).
   uint32_t it = 0;
   int cur = 0;
   const bool until = iters == 0;
@@ -944,7 +1151,7 @@ extern "C" int la3g_pr(la3g_graph* G, uint32_t iters, double* rank_out, uint32_t
   {
     if (!until && it >= iters) break;
     if (until) LA3G_CUDA(cudaMemsetAsync(ps->flag, 0, 4, s));
-    LA3G_TRY(pr_launch(G, ps, ps->x[cur], ps->x[cur ^ 1], 0, g.nreg, until ? ps->flag : nullptr, true));
+    LA3G_TRY(pr_launch(G, ps, ps->L.reg, ps->x[cur], ps->x[cur ^ 1], until ? ps->flag : nullptr, true));
     cur ^= 1;
     it++;
     if (until)
@@ -956,7 +1163,7 @@ extern "C" int la3g_pr(la3g_graph* G, uint32_t iters, double* rank_out, uint32_t
     }
   }
   // sink pass from the final messages (vertex_program_execute.hpp:131-148)
-  LA3G_TRY(pr_launch(G, ps, ps->x[cur], ps->x[cur ^ 1], g.nreg, g.nreg + g.nsink, nullptr, false));
+  LA3G_TRY(pr_launch(G, ps, ps->L.sink, ps->x[cur], ps->x[cur ^ 1], nullptr, false));
   T.device_end();
   if (st)
   {
@@ -971,7 +1178,8 @@ extern "C" int la3g_pr(la3g_graph* G, uint32_t iters, double* rank_out, uint32_t
     LA3G_TRY(tmp.alloc((size_t) N * 8));
     if (rank_out)
     {
-      k_scatter_pos<<<grid_for(N, 256), 256, 0, s>>>(N, g.id_of_pos, ps->rank, tmp.as<double>());
+      k_rank_by_id<double><<<grid_for(N, 256), 256, 0, s>>>(N, g.nrows(), ps->L.qpos, g.id_of_pos, ps->rank,
+                                                              tmp.as<double>());
       LA3G_LAUNCHED();
       LA3G_CUDA(cudaMemcpyAsync(rank_out, tmp.p, (size_t) N * 8, cudaMemcpyDeviceToHost, s));
       LA3G_CUDA(cudaStreamSynchronize(s));
@@ -1003,8 +1211,8 @@ static int pr_f32_run(la3g_graph* G, uint32_t iters, double tol, double* rank_ou
   if (!ps->rankf)
   {
     LA3G_TRY(galloc(G, &ps->rankf, N));
-    LA3G_TRY(galloc(G, &ps->xf[0], N));
-    LA3G_TRY(galloc(G, &ps->xf[1], N));
+    LA3G_TRY(galloc(G, &ps->xf[0], (size_t) N + 1));
+    LA3G_TRY(galloc(G, &ps->xf[1], (size_t) N + 1));
     LA3G_TRY(galloc(G, &ps->resid, 1));
   }
   if (tiled && !ps->tile_col)
@@ -1013,17 +1221,25 @@ static int pr_f32_run(la3g_graph* G, uint32_t iters, double tol, double* rank_ou
     LA3G_CUDA(cudaFuncSetAttribute(k_prf_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) (kTileRows * 4)));
     LA3G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ps->tile_blocks, k_prf_tiles, kTileThreads,
                                                             kTileRows * 4));
+    LA3G_TRY(galloc(G, &ps->trankf, N));
+    LA3G_TRY(galloc(G, &ps->txf[0], N));
+    LA3G_TRY(galloc(G, &ps->txf[1], N));
   }
+  const PrLayout& L = ps->L;
+  const uint32_t nlong = L.reg.q1;  // regular rows above kLongRow: qpos[0 .. nlong)
   T.device_begin();
-  k_prf_init<<<grid_for(N, 256), 256, 0, s>>>(N, g.nreg, g.src_base(), g.iso_base(), ps->deg, ps->rankf, ps->rank,
-                                              ps->xf[0], ps->xf[1]);
+  if (tiled)
+    k_prf_tile_init<<<grid_for(N, 256), 256, 0, s>>>(N, g.nreg, g.src_base(), g.iso_base(), ps->deg, ps->trankf,
+                                                     ps->txf[0], ps->txf[1]);
+  else
+    k_pr_init<float><<<grid_for((uint64_t) N + 1, 256), 256, 0, s>>>(N, g.nreg, g.src_base(), g.iso_base(), L.degq, L.xi,
+                                                                     ps->rankf, ps->xf[0], ps->xf[1]);
   LA3G_LAUNCHED();
   tls_launches++;
   int cur = 0;
   uint32_t it = 0;
   double res = 0.0;
-  const uint32_t long_blocks = ps->nlong ? std::min<uint32_t>(ps->nlong, num_sms() * 2) : 0;
-  const unsigned blocks = long_blocks + std::max<uint32_t>(grid_for((uint64_t) g.nreg * 4, 256, num_sms() * 8), 1);
+  const PrBlocks rb = pr_blocks(L.reg), sb = pr_blocks(L.sink);
   // algorithmic bytes per iteration (FP32 form of the FP64 count): column
   // index per edge, row offsets, x read, rank read + write, next x write
   const double it_bytes = 4.0 * g.nent + 4.0 * (g.nreg + 1) + 4.0 * N + 8.0 * g.nreg + 8.0 * g.nreg + 4.0 * g.nreg;
@@ -1037,19 +1253,18 @@ static int pr_f32_run(la3g_graph* G, uint32_t iters, double tol, double* rank_ou
       ProfileScope p("pr_tiles_f32", s, 12.0 * ps->tile_ncols + 2.0 * ps->tile_nent + 4.0 * (g.nreg + 1) + 8.0 * g.nreg +
                                             8.0 * g.nreg + 4.0 * g.nreg);
       // long rows first (a block each), then the tiles
-      const uint32_t lblocks = ps->nlong ? std::min<uint32_t>(ps->nlong, num_sms()) : 0;
+      const uint32_t lblocks = std::min<uint32_t>(nlong, num_sms());
       const unsigned tgrid = std::min<unsigned>(std::max<uint32_t>(ps->ntiles, 1), num_sms() * std::max(ps->tile_blocks, 1));
       k_prf_tiles<<<lblocks + tgrid, kTileThreads, kTileRows * 4, s>>>(
-          ps->tile_col, ps->tcol, ps->tptr, ps->trow, ps->tecol, ps->ntiles, g.nreg, g.in_ptr, g.in_col, ps->long_rows,
-          ps->nlong,
-          lblocks, ps->xf[cur], ps->xf[cur ^ 1], ps->rankf, ps->rank, ps->deg, ps->resid);
+          ps->tile_col, ps->tcol, ps->tptr, ps->trow, ps->tecol, ps->ntiles, g.nreg, g.in_ptr, g.in_col, L.qpos, nlong,
+          lblocks, ps->txf[cur], ps->txf[cur ^ 1], ps->trankf, ps->deg, ps->resid);
       LA3G_LAUNCHED();
     }
-    else
+    else if (g.nreg)
     {
       ProfileScope p("pr_pull_f32", s, it_bytes);
-      k_prf_pull<<<blocks, 256, 0, s>>>(g.in_ptr, g.in_col, ps->xf[cur], ps->xf[cur ^ 1], ps->rankf, ps->rank, ps->deg,
-                                        ps->long_rows, ps->nlong, long_blocks, 0, g.nreg, ps->resid, 1);
+      k_prf_pull<<<rb.total, kWarpsPerBlock * 32, 0, s>>>(L.reg, rb, L, N, ps->xf[cur], ps->xf[cur ^ 1], ps->rankf,
+                                                          ps->resid, 1);
       LA3G_LAUNCHED();
     }
     cur ^= 1;
@@ -1063,12 +1278,17 @@ static int pr_f32_run(la3g_graph* G, uint32_t iters, double tol, double* rank_ou
   }
   // the residual of the last iteration (the sink pass below reuses the counter)
   if (tol <= 0) LA3G_CUDA(cudaMemcpyAsync(&res, ps->resid, 8, cudaMemcpyDeviceToHost, s));
+  if (tiled)
+  {
+    k_prf_from_tiles<<<grid_for((uint64_t) N + 1, 256), 256, 0, s>>>(N, L.qpos, L.xi, ps->trankf, ps->txf[cur],
+                                                                     ps->rankf, ps->xf[cur]);
+    LA3G_LAUNCHED();
+  }
   if (g.nsink)
   {
-    const unsigned sb = long_blocks + std::max<uint32_t>(grid_for((uint64_t) g.nsink * 4, 256, num_sms() * 8), 1);
     LA3G_CUDA(cudaMemsetAsync(ps->resid, 0, 8, s));
-    k_prf_pull<<<sb, 256, 0, s>>>(g.in_ptr, g.in_col, ps->xf[cur], ps->xf[cur ^ 1], ps->rankf, ps->rank, ps->deg,
-                                  ps->long_rows, ps->nlong, long_blocks, g.nreg, g.nreg + g.nsink, ps->resid, 0);
+    k_prf_pull<<<sb.total, kWarpsPerBlock * 32, 0, s>>>(L.sink, sb, L, N, ps->xf[cur], ps->xf[cur ^ 1], ps->rankf,
+                                                        ps->resid, 0);
     LA3G_LAUNCHED();
   }
   T.device_end();
@@ -1083,7 +1303,7 @@ static int pr_f32_run(la3g_graph* G, uint32_t iters, double tol, double* rank_ou
   {
     DevBuf tmp;
     LA3G_TRY(tmp.alloc((size_t) N * 8));
-    k_scatter_pos<<<grid_for(N, 256), 256, 0, s>>>(N, g.id_of_pos, ps->rank, tmp.as<double>());
+    k_rank_by_id<float><<<grid_for(N, 256), 256, 0, s>>>(N, g.nrows(), L.qpos, g.id_of_pos, ps->rankf, tmp.as<double>());
     LA3G_LAUNCHED();
     LA3G_CUDA(cudaMemcpyAsync(rank_out, tmp.p, (size_t) N * 8, cudaMemcpyDeviceToHost, s));
   }
