@@ -37,24 +37,21 @@ static constexpr float kB = 0.75f;
 
 struct Bm25Scratch
 {
+  IrScratch ir;
   float* length = nullptr;      // [nslots] DtState.length by position
-  float* score = nullptr;       // [nslots]
-  uint32_t* stamp = nullptr;    // [nslots] query id that last touched the doc
-  uint32_t* touched = nullptr;  // [nslots] touched docs of the current query
-  unsigned long long* ctr = nullptr;  // [0] touched count, [1] tokens, [2] postings
-  uint32_t* qin = nullptr;      // query vertex ids (device copy)
-  uint32_t* qpos = nullptr;     // paired (position, idf bits) after the push emulation
-  unsigned long long* cand = nullptr;  // kTopBlocks * kTopKMax candidates
-  unsigned long long* best = nullptr;  // kTopKMax
-  uint32_t qcap = 0;
+  unsigned long long* tok = nullptr;  // token count
   uint32_t term_row0 = 0;       // first regular position of a term (docs come first)
-  uint32_t query_id = 0;
   uint64_t tokens = 0;
   float avg = 0.0f;
   bool prepared = false;
 };
 
-static void bm25_scratch_free(void* p) { delete (Bm25Scratch*) p; }
+static void bm25_scratch_free(void* p)
+{
+  Bm25Scratch* b = (Bm25Scratch*) p;
+  if (b->ir.out) cudaFreeHost(b->ir.out);
+  delete b;
+}
 
 // IDF on term rows [row_lo, row_hi).
 __global__ void k_bm25_idf(const uint32_t* __restrict__ ptr, uint32_t row_lo, uint32_t row_hi, uint32_t ndocs,
@@ -130,90 +127,22 @@ __global__ void k_bm25_pair(const uint32_t* __restrict__ q, uint32_t nq, uint32_
   out[0] = cnt;
 }
 
-// One term: every doc of the term adds its contribution; a doc appears once
-// per term, so there are no races inside a launch.
-// gather reads the row's mirror state, taken when the TFIDF program was
-// first initialised: docs hold K(d); terms (not active then) hold zero.  A
-// term row is reached only by a query that names a document vertex.
-__global__ void k_bm25_term(const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col,
-                            const uint32_t* __restrict__ w, const uint32_t* __restrict__ qpos, uint32_t nq,
-                            uint32_t j, const float* __restrict__ length, uint32_t term_row0, float* score,
-                            uint32_t* stamp, uint32_t qid, uint32_t* touched, unsigned long long* ctr)
+// One posting adds (tf * 2.2) / (tf + K(d)) * idf.  gather reads the row's
+// mirror state, taken when the TFIDF program was first initialised: docs hold
+// K(d); terms (not active then) hold zero.  A term row is reached only by a
+// query that names a document vertex.
+struct Bm25Scorer
 {
-  const uint32_t cnt = qpos[0];
-  if (j >= cnt) return;
-  const uint32_t t = qpos[1 + j];                          // j-th smallest pushed index
-  const float idf = __uint_as_float(qpos[1 + nq + j]);     // value of slot j
-  const uint32_t b = ptr[t], e = ptr[t + 1];
-  if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&ctr[2], (unsigned long long) (e - b));  // postings walked
-  const float k1p1 = __fadd_rn(kK1, 1.0f);
-  for (uint32_t i = b + blockIdx.x * blockDim.x + threadIdx.x; i < e; i += gridDim.x * blockDim.x)
+  const float* __restrict__ length;
+  uint32_t term_row0;
+  __device__ __forceinline__ float value(float idf) const { return idf; }
+  __device__ __forceinline__ float own(uint32_t d) const { return d < term_row0 ? length[d] : 0.0f; }
+  __device__ __forceinline__ float term(float kd, float wf, float idf) const
   {
-    const uint32_t d = col[i];
-    const float wf = (float) w[i];
-    const float kd = d < term_row0 ? length[d] : 0.0f;
-    const float c = __fmul_rn(__fdiv_rn(__fmul_rn(wf, k1p1), __fadd_rn(wf, kd)), idf);
-    if (stamp[d] != qid)
-    {
-      stamp[d] = qid;
-      score[d] = __fadd_rn(0.0f, c);
-      unsigned long long slot = atomicAdd(&ctr[0], 1ull);
-      touched[slot] = d;
-    }
-    else
-    {
-      score[d] = __fadd_rn(score[d], c);
-    }
+    return __fmul_rn(__fdiv_rn(__fmul_rn(wf, __fadd_rn(kK1, 1.0f)), __fadd_rn(wf, kd)), idf);
   }
-}
-
-__device__ __forceinline__ unsigned long long bm25_key(float s, uint32_t id)
-{
-  // order-preserving map of the score (with -0 == +0), then smaller id first
-  uint32_t u = __float_as_uint(s);
-  if ((u & 0x7FFFFFFFu) == 0) u = 0;
-  u = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-  return ((unsigned long long) u << 32) | (0xFFFFFFFFu - id);
-}
-
-__global__ void __launch_bounds__(kTopThreads)
-k_bm25_top_partial(const uint32_t* __restrict__ touched, const unsigned long long* __restrict__ ctr,
-                   const float* __restrict__ score, const uint32_t* __restrict__ id_of_pos, int k,
-                   unsigned long long* cand)
-{
-  unsigned long long mine[kTopKMax];
-  for (int i = 0; i < k; i++) mine[i] = 0;
-  const uint64_t n = ctr[0];
-  for (uint64_t i = (uint64_t) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t) gridDim.x * blockDim.x)
-  {
-    uint32_t d = touched[i];
-    keep_best(mine, k, bm25_key(score[d], id_of_pos[d]));
-  }
-  block_topk(mine, k, cand + (size_t) blockIdx.x * k);
-}
-
-__global__ void __launch_bounds__(kTopThreads)
-k_bm25_top_final(const unsigned long long* __restrict__ cand, int ncand, int k, unsigned long long* best)
-{
-  unsigned long long mine[kTopKMax];
-  for (int i = 0; i < k; i++) mine[i] = 0;
-  for (int i = threadIdx.x; i < ncand; i += blockDim.x) keep_best(mine, k, cand[i]);
-  block_topk(mine, k, best);
-}
-
-__global__ void k_bm25_dump(const uint32_t* __restrict__ touched, const unsigned long long* __restrict__ ctr,
-                            const float* __restrict__ score, const uint32_t* __restrict__ id_of_pos, float* all,
-                            uint8_t* act)
-{
-  const uint64_t n = ctr[0];
-  for (uint64_t i = (uint64_t) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t) gridDim.x * blockDim.x)
-  {
-    uint32_t d = touched[i];
-    uint32_t id = id_of_pos[d];
-    if (all) all[id] = score[d];
-    if (act) act[id] = 1;
-  }
-}
+  __device__ __forceinline__ float done(uint32_t, float y) const { return y; }
+};
 
 __global__ void k_f32_by_id(uint32_t N, const uint32_t* __restrict__ id_of_pos, const float* __restrict__ v, float* out)
 {
@@ -230,13 +159,8 @@ static int bm25_scratch(la3g_graph* G, Bm25Scratch** out)
   G->slot_free[kSlotBm25] = bm25_scratch_free;
   const uint32_t N = G->g.nslots;
   LA3G_TRY(galloc(G, &b->length, N));
-  LA3G_TRY(galloc(G, &b->score, N));
-  LA3G_TRY(galloc(G, &b->stamp, N));
-  LA3G_TRY(galloc(G, &b->touched, N));
-  LA3G_TRY(galloc(G, &b->ctr, 4));
-  LA3G_TRY(galloc(G, &b->cand, (size_t) kTopBlocks * kTopKMax));
-  LA3G_TRY(galloc(G, &b->best, kTopKMax));
-  LA3G_CUDA(cudaMemsetAsync(b->stamp, 0, (size_t) N * 4, G->stream));
+  LA3G_TRY(galloc(G, &b->tok, 1));
+  LA3G_TRY(ir_scratch(G, &b->ir));
   *out = b;
   return LA3G_OK;
 }
@@ -277,7 +201,7 @@ extern "C" int la3g_bm25_prepare(la3g_graph* G, uint64_t* ntokens_out, float* av
   LA3G_TRY(bipartite_first_term_row(G, &tb));
   b->term_row0 = tb;
   LA3G_CUDA(cudaMemsetAsync(b->length, 0, (size_t) N * 4, s));
-  LA3G_CUDA(cudaMemsetAsync(b->ctr, 0, 4 * 8, s));
+  LA3G_CUDA(cudaMemsetAsync(b->tok, 0, 8, s));
   {
     ProfileScope p("bm25_idf", s, 4.0 * (g.nreg - tb + 1) + 4.0 * (g.nreg - tb));
     k_bm25_idf<<<grid_for(g.nreg - tb, 256), 256, 0, s>>>(g.in_ptr, tb, g.nreg, g.nleft, b->length);
@@ -288,10 +212,10 @@ extern "C" int la3g_bm25_prepare(la3g_graph* G, uint64_t* ntokens_out, float* av
     k_bm25_dl<<<grid_for(tb, 256), 256, 0, s>>>(g.in_ptr, g.in_w, 0, tb, 0.0f, b->length);
     LA3G_LAUNCHED();
   }
-  k_bm25_tokens<<<grid_for(N, 256), 256, 0, s>>>(b->length, N, b->ctr + 1);
+  k_bm25_tokens<<<grid_for(N, 256), 256, 0, s>>>(b->length, N, b->tok);
   LA3G_LAUNCHED();
   unsigned long long tok = 0;
-  LA3G_CUDA(cudaMemcpyAsync(&tok, b->ctr + 1, 8, cudaMemcpyDeviceToHost, s));
+  LA3G_CUDA(cudaMemcpyAsync(&tok, b->tok, 8, cudaMemcpyDeviceToHost, s));
   LA3G_CUDA(cudaStreamSynchronize(s));
   // avg = collection_ntokens / (float) ndocs (bm25.cpp:38): uint64 -> float, float divide
   const float avg = (float) tok / (float) g.nleft;
@@ -326,89 +250,6 @@ extern "C" int la3g_bm25_query(la3g_graph* G, const uint32_t* term_vids, uint32_
   if (k > kTopKMax) return set_error(LA3G_EINVAL, "k = %u exceeds the maximum of %d", k, kTopKMax);
   Bm25Scratch* b = (Bm25Scratch*) G->slot[kSlotBm25];
   if (!b || !b->prepared) return set_error(LA3G_EINVAL, "call la3g_bm25_prepare first");
-  DevGraph& g = G->g;
-  cudaStream_t s = G->stream;
-  const uint32_t N = g.nslots;
-  CallTimer T(G, st);
-  if (nterms > b->qcap || !b->qpos)
-  {
-    uint32_t cap = std::max<uint32_t>(64, nterms);
-    LA3G_TRY(galloc(G, &b->qin, cap));
-    LA3G_TRY(galloc(G, &b->qpos, 1 + 2 * (size_t) cap));
-    b->qcap = cap;
-  }
-  if (++b->query_id == 0)
-  {
-    LA3G_CUDA(cudaMemsetAsync(b->stamp, 0, (size_t) N * 4, s));
-    b->query_id = 1;
-  }
-  T.device_begin();
-  if (nterms) LA3G_CUDA(cudaMemcpyAsync(b->qin, term_vids, (size_t) nterms * 4, cudaMemcpyHostToDevice, s));
-  LA3G_CUDA(cudaMemsetAsync(b->ctr, 0, 8, s));
-  LA3G_CUDA(cudaMemsetAsync(b->ctr + 2, 0, 8, s));
-  LA3G_CUDA(cudaMemsetAsync(b->qpos, 0, 4, s));
-  if (nterms)
-  {
-    k_bm25_pair<<<1, 1, 0, s>>>(b->qin, nterms, N, g.nreg, g.pos_of_id, b->length, b->qpos);
-    LA3G_LAUNCHED();
-    tls_launches++;
-  }
-  // the distinct regular terms, ascending; at most nterms launches
-  for (uint32_t j = 0; j < nterms; j++)
-  {
-    ProfileScope p("bm25_term", s, 0.0);
-    k_bm25_term<<<num_sms() * 4, 256, 0, s>>>(g.in_ptr, g.in_col, g.in_w, b->qpos, nterms, j, b->length, b->term_row0,
-                                        b->score, b->stamp, b->query_id, b->touched, b->ctr);
-    LA3G_LAUNCHED();
-  }
-  const int kk = (int) k;
-  if (kk > 0)
-  {
-    k_bm25_top_partial<<<kTopBlocks, kTopThreads, 0, s>>>(b->touched, b->ctr, b->score, g.id_of_pos, kk, b->cand);
-    LA3G_LAUNCHED();
-    k_bm25_top_final<<<1, kTopThreads, 0, s>>>(b->cand, kTopBlocks * kk, kk, b->best);
-    LA3G_LAUNCHED();
-    tls_launches += 2;
-  }
-  T.device_end();
-  unsigned long long ntouched = 0, postings = 0;
-  LA3G_CUDA(cudaMemcpyAsync(&ntouched, b->ctr, 8, cudaMemcpyDeviceToHost, s));
-  LA3G_CUDA(cudaMemcpyAsync(&postings, b->ctr + 2, 8, cudaMemcpyDeviceToHost, s));
-  unsigned long long best[kTopKMax];
-  if (kk > 0) LA3G_CUDA(cudaMemcpyAsync(best, b->best, (size_t) kk * 8, cudaMemcpyDeviceToHost, s));
-  if (all_scores_out || active_out)
-  {
-    DevBuf a, c;
-    if (all_scores_out) { LA3G_TRY(a.alloc((size_t) N * 4)); LA3G_CUDA(cudaMemsetAsync(a.p, 0, (size_t) N * 4, s)); }
-    if (active_out) { LA3G_TRY(c.alloc(N)); LA3G_CUDA(cudaMemsetAsync(c.p, 0, N, s)); }
-    k_bm25_dump<<<num_sms() * 4, 256, 0, s>>>(b->touched, b->ctr, b->score, g.id_of_pos, a.as<float>(), c.as<uint8_t>());
-    LA3G_LAUNCHED();
-    if (all_scores_out) LA3G_CUDA(cudaMemcpyAsync(all_scores_out, a.p, (size_t) N * 4, cudaMemcpyDeviceToHost, s));
-    if (active_out) LA3G_CUDA(cudaMemcpyAsync(active_out, c.p, N, cudaMemcpyDeviceToHost, s));
-    LA3G_CUDA(cudaStreamSynchronize(s));
-  }
-  LA3G_TRY(T.finish());
-  uint32_t n = (uint32_t) std::min<unsigned long long>(ntouched, (unsigned long long) k);
-  for (uint32_t i = 0; i < n; i++)
-  {
-    uint32_t u = (uint32_t) (best[i] >> 32);
-    u = (u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u;
-    float sc;
-    std::memcpy(&sc, &u, 4);
-    if (ids_out) ids_out[i] = 0xFFFFFFFFu - (uint32_t) best[i];
-    if (scores_out) scores_out[i] = sc;
-  }
-  if (nout) *nout = n;
-  // algorithmic bytes: doc id + tf per posting walked, K(d) read and score
-  // written per touched doc, the top-k pass over the touched docs
-  const double bytes = 8.0 * (double) postings + 12.0 * (double) ntouched;
-  profile_add_bytes("bm25_term", bytes);
-  if (st)
-  {
-    st->iterations = 1;
-    st->teps_edges = ntouched;
-    st->edges_examined = postings;
-    st->algo_bytes = (uint64_t) bytes;
-  }
-  return LA3G_OK;
+  return ir_query(G, &b->ir, Bm25Scorer{b->length, b->term_row0}, b->length, 0xFFFFFFFFu, "bm25_term", term_vids, nterms, k,
+                  ids_out, scores_out, nout, all_scores_out, active_out, st);
 }

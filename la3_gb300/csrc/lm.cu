@@ -40,25 +40,22 @@ static constexpr float kMu = 2000.0f;
 
 struct LmScratch
 {
+  IrScratch ir;
   float* length = nullptr;      // [nslots] DtState.length by position
   float* factor = nullptr;      // [nslots] log10f(mu / (length + mu)) by position
-  float* score = nullptr;       // [nslots]
-  uint32_t* stamp = nullptr;    // [nslots] query id that last touched the vertex
-  uint32_t* touched = nullptr;  // [nslots] active vertices of the current query
-  unsigned long long* ctr = nullptr;  // [0] touched count, [1] tokens, [2] postings
-  uint32_t* qin = nullptr;
-  uint32_t* qpos = nullptr;
-  unsigned long long* cand = nullptr;
-  unsigned long long* best = nullptr;
-  uint32_t qcap = 0;
+  unsigned long long* tok = nullptr;  // token count
   uint32_t term_row0 = 0;
-  uint32_t query_id = 0;
   uint64_t tokens = 0;
   bool prepared = false;
   bool leftover = false;        // the TL pass's activity is still set (first query)
 };
 
-static void lm_scratch_free(void* p) { delete (LmScratch*) p; }
+static void lm_scratch_free(void* p)
+{
+  LmScratch* b = (LmScratch*) p;
+  if (b->ir.out) cudaFreeHost(b->ir.out);
+  delete b;
+}
 
 // TL on term rows [row_lo, row_hi): a warp per row, lanes load 32 entries at
 // a time and the sum runs through them in entry (ascending doc) order.
@@ -83,62 +80,23 @@ __global__ void k_lm_tl(const uint32_t* __restrict__ ptr, const uint32_t* __rest
   }
 }
 
-// One term: every doc of the term adds log10(1 + tf / (mu * msg)); a doc
-// appears once per term, so there are no races inside a launch.
-__global__ void k_lm_term(const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col,
-                          const uint32_t* __restrict__ w, const uint32_t* __restrict__ qpos, uint32_t nq, uint32_t j,
-                          float* score, uint32_t* stamp, uint32_t qid, uint32_t* touched, unsigned long long* ctr)
+// One posting adds log10(1 + tf / (mu * msg)); a touched vertex then takes
+// score = y + (float) nterms * factor.
+struct LmScorer
 {
-  const uint32_t cnt = qpos[0];
-  if (j >= cnt) return;
-  const uint32_t t = qpos[1 + j];
-  const float msg = __uint_as_float(qpos[1 + nq + j]);
-  const uint32_t b = ptr[t], e = ptr[t + 1];
-  if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&ctr[2], (unsigned long long) (e - b));
-  const float den = __fmul_rn(kMu, msg);
-  for (uint32_t i = b + blockIdx.x * blockDim.x + threadIdx.x; i < e; i += gridDim.x * blockDim.x)
+  const float* __restrict__ factor;
+  float nterms;
+  __device__ __forceinline__ float value(float msg) const { return __fmul_rn(kMu, msg); }
+  __device__ __forceinline__ float own(uint32_t) const { return 0.0f; }
+  __device__ __forceinline__ float term(float, float wf, float den) const
   {
-    const uint32_t d = col[i];
-    const float q = __fdiv_rn((float) w[i], den);
-    const float c = (float) log10(__dadd_rn(1.0, (double) q));
-    if (stamp[d] != qid)
-    {
-      stamp[d] = qid;
-      score[d] = __fadd_rn(0.0f, c);
-      touched[atomicAdd(&ctr[0], 1ull)] = d;
-    }
-    else
-    {
-      score[d] = __fadd_rn(score[d], c);
-    }
+    return (float) log10(__dadd_rn(1.0, (double) __fdiv_rn(wf, den)));
   }
-}
-
-// apply on the touched vertices: score = y + (float) nterms * factor.
-__global__ void k_lm_apply(const uint32_t* __restrict__ touched, const unsigned long long* __restrict__ ctr,
-                           const float* __restrict__ factor, float nterms, float* score)
-{
-  const uint64_t n = ctr[0];
-  for (uint64_t i = (uint64_t) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t) gridDim.x * blockDim.x)
+  __device__ __forceinline__ float done(uint32_t d, float y) const
   {
-    const uint32_t d = touched[i];
-    score[d] = __fadd_rn(score[d], __fmul_rn(nterms, factor[d]));
+    return __fadd_rn(y, __fmul_rn(nterms, factor[d]));
   }
-}
-
-// The first query after prepare: the term rows the TL pass left active and
-// this query did not reach join its pool with score 0.
-__global__ void k_lm_leftover(uint32_t row_lo, uint32_t row_hi, uint32_t* stamp, uint32_t qid, float* score,
-                              uint32_t* touched, unsigned long long* ctr)
-{
-  for (uint32_t r = row_lo + blockIdx.x * blockDim.x + threadIdx.x; r < row_hi; r += gridDim.x * blockDim.x)
-    if (stamp[r] != qid)
-    {
-      stamp[r] = qid;
-      score[r] = 0.0f;
-      touched[atomicAdd(&ctr[0], 1ull)] = r;
-    }
-}
+};
 
 static int lm_scratch(la3g_graph* G, LmScratch** out)
 {
@@ -151,13 +109,8 @@ static int lm_scratch(la3g_graph* G, LmScratch** out)
   const uint32_t N = G->g.nslots;
   LA3G_TRY(galloc(G, &b->length, N));
   LA3G_TRY(galloc(G, &b->factor, N));
-  LA3G_TRY(galloc(G, &b->score, N));
-  LA3G_TRY(galloc(G, &b->stamp, N));
-  LA3G_TRY(galloc(G, &b->touched, N));
-  LA3G_TRY(galloc(G, &b->ctr, 4));
-  LA3G_TRY(galloc(G, &b->cand, (size_t) kTopBlocks * kTopKMax));
-  LA3G_TRY(galloc(G, &b->best, kTopKMax));
-  LA3G_CUDA(cudaMemsetAsync(b->stamp, 0, (size_t) N * 4, G->stream));
+  LA3G_TRY(galloc(G, &b->tok, 1));
+  LA3G_TRY(ir_scratch(G, &b->ir));
   *out = b;
   return LA3G_OK;
 }
@@ -181,16 +134,16 @@ extern "C" int la3g_lm_prepare(la3g_graph* G, uint64_t* ntokens_out, float* leng
   LA3G_TRY(bipartite_first_term_row(G, &tb));
   b->term_row0 = tb;
   LA3G_CUDA(cudaMemsetAsync(b->length, 0, (size_t) N * 4, s));
-  LA3G_CUDA(cudaMemsetAsync(b->ctr, 0, 4 * 8, s));
+  LA3G_CUDA(cudaMemsetAsync(b->tok, 0, 8, s));
   {
     ProfileScope p("lm_dl", s, 8.0 * g.nent / 2);
     k_bm25_dl<<<grid_for(tb, 256), 256, 0, s>>>(g.in_ptr, g.in_w, 0, tb, 0.0f, b->length);
     LA3G_LAUNCHED();
   }
-  k_bm25_tokens<<<grid_for(N, 256), 256, 0, s>>>(b->length, N, b->ctr + 1);
+  k_bm25_tokens<<<grid_for(N, 256), 256, 0, s>>>(b->length, N, b->tok);
   LA3G_LAUNCHED();
   unsigned long long tok = 0;
-  LA3G_CUDA(cudaMemcpyAsync(&tok, b->ctr + 1, 8, cudaMemcpyDeviceToHost, s));
+  LA3G_CUDA(cudaMemcpyAsync(&tok, b->tok, 8, cudaMemcpyDeviceToHost, s));
   LA3G_CUDA(cudaStreamSynchronize(s));
   if (g.nreg > tb)
   {
@@ -234,103 +187,12 @@ extern "C" int la3g_lm_query(la3g_graph* G, const uint32_t* term_vids, uint32_t 
   if (k > kTopKMax) return set_error(LA3G_EINVAL, "k = %u exceeds the maximum of %d", k, kTopKMax);
   LmScratch* b = (LmScratch*) G->slot[kSlotLm];
   if (!b || !b->prepared) return set_error(LA3G_EINVAL, "call la3g_lm_prepare first");
-  DevGraph& g = G->g;
-  cudaStream_t s = G->stream;
-  const uint32_t N = g.nslots;
-  CallTimer T(G, st);
-  if (nterms > b->qcap || !b->qpos)
-  {
-    uint32_t cap = std::max<uint32_t>(64, nterms);
-    LA3G_TRY(galloc(G, &b->qin, cap));
-    LA3G_TRY(galloc(G, &b->qpos, 1 + 2 * (size_t) cap));
-    b->qcap = cap;
-  }
-  if (++b->query_id == 0)
-  {
-    LA3G_CUDA(cudaMemsetAsync(b->stamp, 0, (size_t) N * 4, s));
-    b->query_id = 1;
-  }
-  T.device_begin();
-  if (nterms) LA3G_CUDA(cudaMemcpyAsync(b->qin, term_vids, (size_t) nterms * 4, cudaMemcpyHostToDevice, s));
-  LA3G_CUDA(cudaMemsetAsync(b->ctr, 0, 8, s));
-  LA3G_CUDA(cudaMemsetAsync(b->ctr + 2, 0, 8, s));
-  LA3G_CUDA(cudaMemsetAsync(b->qpos, 0, 4, s));
-  if (nterms)
-  {
-    k_bm25_pair<<<1, 1, 0, s>>>(b->qin, nterms, N, g.nreg, g.pos_of_id, b->length, b->qpos);
-    LA3G_LAUNCHED();
-    tls_launches++;
-  }
-  for (uint32_t j = 0; j < nterms; j++)
-  {
-    ProfileScope p("lm_term", s, 0.0);
-    k_lm_term<<<num_sms() * 4, 256, 0, s>>>(g.in_ptr, g.in_col, g.in_w, b->qpos, nterms, j, b->score, b->stamp,
-                                      b->query_id, b->touched, b->ctr);
-    LA3G_LAUNCHED();
-  }
+  // the leftover activity of the TL pass lasts for one query
+  // (tfidf.reset_activity() after it, lm.cpp:86)
+  const uint32_t leftover_from = b->leftover ? b->term_row0 : 0xFFFFFFFFu;
   // query_nterms = queries[q].size() (lm.cpp:66), as float in the apply
-  k_lm_apply<<<num_sms() * 4, 256, 0, s>>>(b->touched, b->ctr, b->factor, (float) nterms, b->score);
-  LA3G_LAUNCHED();
-  tls_launches++;
-  if (b->leftover)
-  {
-    if (g.nreg > b->term_row0)
-    {
-      k_lm_leftover<<<grid_for(g.nreg - b->term_row0, 256), 256, 0, s>>>(b->term_row0, g.nreg, b->stamp, b->query_id,
-                                                                         b->score, b->touched, b->ctr);
-      LA3G_LAUNCHED();
-      tls_launches++;
-    }
-    b->leftover = false;  // tfidf.reset_activity() after the query (lm.cpp:86)
-  }
-  const int kk = (int) k;
-  if (kk > 0)
-  {
-    k_bm25_top_partial<<<kTopBlocks, kTopThreads, 0, s>>>(b->touched, b->ctr, b->score, g.id_of_pos, kk, b->cand);
-    LA3G_LAUNCHED();
-    k_bm25_top_final<<<1, kTopThreads, 0, s>>>(b->cand, kTopBlocks * kk, kk, b->best);
-    LA3G_LAUNCHED();
-    tls_launches += 2;
-  }
-  T.device_end();
-  unsigned long long ntouched = 0, postings = 0;
-  LA3G_CUDA(cudaMemcpyAsync(&ntouched, b->ctr, 8, cudaMemcpyDeviceToHost, s));
-  LA3G_CUDA(cudaMemcpyAsync(&postings, b->ctr + 2, 8, cudaMemcpyDeviceToHost, s));
-  unsigned long long best[kTopKMax];
-  if (kk > 0) LA3G_CUDA(cudaMemcpyAsync(best, b->best, (size_t) kk * 8, cudaMemcpyDeviceToHost, s));
-  if (all_scores_out || active_out)
-  {
-    DevBuf a, c;
-    if (all_scores_out) { LA3G_TRY(a.alloc((size_t) N * 4)); LA3G_CUDA(cudaMemsetAsync(a.p, 0, (size_t) N * 4, s)); }
-    if (active_out) { LA3G_TRY(c.alloc(N)); LA3G_CUDA(cudaMemsetAsync(c.p, 0, N, s)); }
-    k_bm25_dump<<<num_sms() * 4, 256, 0, s>>>(b->touched, b->ctr, b->score, g.id_of_pos, a.as<float>(), c.as<uint8_t>());
-    LA3G_LAUNCHED();
-    if (all_scores_out) LA3G_CUDA(cudaMemcpyAsync(all_scores_out, a.p, (size_t) N * 4, cudaMemcpyDeviceToHost, s));
-    if (active_out) LA3G_CUDA(cudaMemcpyAsync(active_out, c.p, N, cudaMemcpyDeviceToHost, s));
-    LA3G_CUDA(cudaStreamSynchronize(s));
-  }
-  LA3G_TRY(T.finish());
-  uint32_t n = (uint32_t) std::min<unsigned long long>(ntouched, (unsigned long long) k);
-  for (uint32_t i = 0; i < n; i++)
-  {
-    uint32_t u = (uint32_t) (best[i] >> 32);
-    u = (u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u;
-    float sc;
-    std::memcpy(&sc, &u, 4);
-    if (ids_out) ids_out[i] = 0xFFFFFFFFu - (uint32_t) best[i];
-    if (scores_out) scores_out[i] = sc;
-  }
-  if (nout) *nout = n;
-  // algorithmic bytes: doc id + tf per posting walked, factor read and score
-  // written per touched vertex, the top-k pass over them
-  const double bytes = 8.0 * (double) postings + 12.0 * (double) ntouched;
-  profile_add_bytes("lm_term", bytes);
-  if (st)
-  {
-    st->iterations = 1;
-    st->teps_edges = ntouched;
-    st->edges_examined = postings;
-    st->algo_bytes = (uint64_t) bytes;
-  }
+  LA3G_TRY(ir_query(G, &b->ir, LmScorer{b->factor, (float) nterms}, b->length, leftover_from, "lm_term", term_vids, nterms,
+                    k, ids_out, scores_out, nout, all_scores_out, active_out, st));
+  b->leftover = false;
   return LA3G_OK;
 }
