@@ -395,8 +395,7 @@ void la3g_server_free(la3g_server* s);
  * one fixed device array of about 12.8 MB, so nvertices is limited to
  * 1048576 (2^20); larger graphs are rejected with LA3G_EINVAL.  Each call
  * looks up the array's address on the current device (no allocation).  The
- * call waits for its stream at every BFS level, since it reads the frontier
- * size back to the host, and again before it returns, also after an error.
+ * call waits for its stream before it returns, also after an error.
  * Calls share the array, so calls that overlap on the GPU race; run them one
  * at a time.  row_ptr must be non-decreasing with row_ptr[nvertices] = the
  * entry count; that is not checked, while neighbour ids >= nvertices are

@@ -1,4 +1,5 @@
 // Errors, allocation, timing and kernel profiling shared by the library.
+#include <algorithm>
 #include <chrono>
 #include <cstdarg>
 #include <cstring>
@@ -44,6 +45,16 @@ int num_sms()
     cached[dev] = v;  // the same value from any thread: a benign race
   }
   return cached[dev];
+}
+
+int cooperative_blocks(const void* f, int threads, uint64_t want, int max_per_sm, unsigned* out)
+{
+  int per_sm = 0;
+  LA3G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, threads, 0));
+  if (per_sm < 1) return set_error(LA3G_ECUDA, "a cooperative kernel does not fit an SM");
+  const uint64_t most = (uint64_t) std::min(per_sm, max_per_sm) * num_sms();
+  *out = (unsigned) std::max<uint64_t>(1, std::min<uint64_t>(most, (want + threads - 1) / threads));
+  return LA3G_OK;
 }
 
 double now_ms()

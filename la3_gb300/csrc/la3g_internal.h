@@ -115,6 +115,53 @@ __device__ __forceinline__ uint32_t block_min_u32(uint32_t v)
   return v;
 }
 
+// Barrier over the blocks of a cooperative launch.  `count` starts at zero; a
+// block that waits more than `limit` polls sets *err and every block leaves its
+// kernel at its next barrier (sync() returns false in all its threads).  Every
+// thread of every block calls sync() the same number of times.  Like
+// cooperative groups' grid barrier it is a fence at device scope, after which
+// ordinary loads see what the other blocks wrote before it.
+struct GridBarrier
+{
+  unsigned int* count;
+  int* err;
+  long long limit;
+  unsigned int phase = 0;
+  __device__ bool sync()
+  {
+    __shared__ int s_ok;
+    phase++;
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+      const unsigned int target = phase * gridDim.x;
+      __threadfence();
+      atomicAdd(count, 1u);
+      volatile unsigned int* c = count;
+      long long polls = 0;
+      int ok = 1;
+      while ((int) (*c - target) < 0)
+        if (++polls > limit || ((polls & 63) == 0 && *(volatile int*) err))
+        {
+          atomicExch(err, 1);
+          ok = 0;
+          break;
+        }
+      __threadfence();
+      s_ok = ok;
+    }
+    __syncthreads();
+    return s_ok;
+  }
+};
+
+// Polls of a barrier before it gives up (a few seconds).
+static constexpr long long kBarrierPolls = 1ll << 23;
+
+// Blocks of a cooperative launch of `f`: enough for `want` threads, at most
+// as many as are resident at once (and max_per_sm per SM).
+int cooperative_blocks(const void* f, int threads, uint64_t want, int max_per_sm, unsigned* out);
+
 // Kernel-level profiling: when on, a launch is bracketed by events on its
 // stream and its time accumulated under `name` with `bytes` algorithmic
 // bytes.  Always counts the launch.
