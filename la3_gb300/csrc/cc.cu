@@ -6,12 +6,17 @@
 // vertex 0 has no edges no label is ever 0, combine is a plain min, and
 // the fixed point is: every vertex with edges carries the least id of its
 // component, every isolated vertex its own id.  That fixed point is computed
-// here with a lock-free union-find whose roots are always the least id of
-// their set (a root is only ever hooked under a root with a smaller id),
-// followed by full path compression.  Edges are processed Afforest-style
-// (Sutton et al.): each vertex first unites with two neighbours, the giant
-// component is found by sampling, and only vertices outside it then walk
-// their remaining edges.
+// here with a lock-free union-find over the rows' positions (a root is only
+// ever hooked under a smaller position), full path compression, and the least
+// id of each tree.  Edges are processed Afforest-style (Sutton et al.): each row
+// first hooks under its least neighbour, without atomics, then its tree is
+// linked with a few more neighbours' by one atomicMin each, which may be lost;
+// the giant component is found by sampling, and only rows outside it walk
+// their edges (all of them: the graph is symmetric, so an edge that leaves the
+// giant component is seen from its other end).  Positions, not ids, order the
+// trees: the neighbours' ids need not be looked up, and a graph whose
+// neighbours have consecutive ids (a path, a road network in order) does not
+// hook into one long chain, since the bucket hash spreads them.
 //
 // When vertex 0 does have edges, label 0 behaves as "no value yet" and the
 // outcome depends on the order messages arrive in, so that case runs the
@@ -26,9 +31,14 @@
 
 namespace la3g {
 
+static constexpr int kCcFlags = 8;  // chains left by the compressions, one flag each
+
 struct CcScratch
 {
-  uint32_t* label = nullptr;   // by original id (union-find parents)
+  uint32_t* label = nullptr;   // by original id
+  uint32_t* parent = nullptr;  // [rows] union-find by position
+  uint32_t* least = nullptr;   // [rows] least id of each root's tree
+  uint32_t* deep = nullptr;    // [kCcFlags]
   uint32_t* probe = nullptr;   // roots of sampled vertices
   uint32_t* lab_pos = nullptr; // BSP path: labels by position
   uint32_t* msg = nullptr;
@@ -36,7 +46,7 @@ struct CcScratch
   int* flag = nullptr;
   unsigned long long* walked = nullptr;  // [0] rows, [1] edges k_cc_rest walked
   unsigned long long* hwalked = nullptr; // pinned mirror
-  uint32_t* giant = nullptr;   // the sampled giant component's root
+  uint32_t* giant = nullptr;   // the sampled giant component's root, and the samples in it
   int zero_has_edges = -1;     // whether vertex 0 has edges (-1: not looked up yet)
 };
 
@@ -45,11 +55,6 @@ static void cc_scratch_free(void* p)
   CcScratch* s = (CcScratch*) p;
   if (s->hwalked) cudaFreeHost(s->hwalked);
   delete s;
-}
-
-__global__ void k_cc_init(uint32_t N, uint32_t* parent)
-{
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < N; v += gridDim.x * blockDim.x) parent[v] = v;
 }
 
 __device__ __forceinline__ uint32_t cc_find(uint32_t* parent, uint32_t v)
@@ -80,120 +85,196 @@ __device__ __forceinline__ void cc_union(uint32_t* parent, uint32_t a, uint32_t 
   }
 }
 
-// Afforest-style sampling round r: every row unites with its r-th
-// neighbour (rounds are separated by a full path compression, which keeps
-// the finds of the next round short).
-__global__ void k_cc_sample(const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col,
-                            const uint32_t* __restrict__ id_of_pos, uint32_t nrows, uint32_t r, uint32_t* parent)
+// First round: a row starts under the least of itself and its neighbours, the
+// first of its entries.  Parents only ever point to smaller positions, so plain
+// stores make a forest; what a row leaves out here the later passes see.
+// (Uniting with two neighbours in turn by compare-and-swap took 161 + 280 us on
+// R-MAT 2^22; this takes 23 us, the link rounds 41 + 30.)
+__global__ void k_cc_hook(const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col, uint32_t nrows,
+                          uint32_t* parent, uint32_t* least, uint32_t* deep)
 {
   for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < nrows; u += gridDim.x * blockDim.x)
   {
-    const uint32_t i = ptr[u] + r;
-    if (i < ptr[u + 1]) cc_union(parent, id_of_pos[u], id_of_pos[col[i]]);
+    parent[u] = min(u, col[ptr[u]]);
+    least[u] = 0xFFFFFFFFu;
+  }
+  if (blockIdx.x == 0 && threadIdx.x < kCcFlags) deep[threadIdx.x] = 0;
+}
+
+// Later rounds, each after a full compression: a row's tree and that of one
+// more neighbour (spread over the row) are linked by a single atomicMin on the
+// larger root, which may lose to a smaller parent set at the same time; no
+// retries and no finds, since k_cc_rest unites what is lost.  The rounds after
+// the second are for graphs whose giant component is not found by then: with
+// it half formed, k_cc_rest would unite most edges one by one (R-MAT 2^22 after
+// one round only: 4 ms).  They return at once when *giant_share says that
+// kCcEnough of the samples are in it.
+static constexpr uint32_t kCcLinks = 2, kCcMoreLinks = 2;
+static constexpr uint32_t kCcSamples = 1024, kCcEnough = 900;
+__global__ void k_cc_link(const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col, uint32_t nrows, uint32_t round,
+                          const uint32_t* __restrict__ giant_share, uint32_t* parent)
+{
+  if (giant_share && *giant_share >= kCcEnough) return;
+  for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < nrows; u += gridDim.x * blockDim.x)
+  {
+    const uint32_t b = ptr[u], e = ptr[u + 1];
+    // the last entry, the middle one, then the quarters
+    const uint32_t c = col[round == 0 ? e - 1 : b + (uint32_t) ((uint64_t) (e - b) * (round == 1 ? 2 : round == 2 ? 1 : 3) / 4)];
+    const uint32_t ru = parent[u], rv = parent[c];
+    const uint32_t lo = min(ru, rv), hi = max(ru, rv);
+    if (lo != hi && parent[hi] > lo) atomicMin(&parent[hi], lo);
   }
 }
 
-// Remaining edges (from the k-th neighbour on) of the rows whose root is not
-// the sampled giant root; the graph is symmetric, so every edge that leaves
-// the giant component is seen from its other endpoint.  One warp per row.
+// The edges of the rows whose root is not the sampled giant root: a lane
+// looks at a row each, the warp then walks the edges of those found together.
 __global__ void __launch_bounds__(256)
-k_cc_rest(const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col, const uint32_t* __restrict__ id_of_pos,
-          uint32_t nrows, uint32_t k, const uint32_t* __restrict__ giant_ptr, uint32_t* parent,
-          unsigned long long* walked)
+k_cc_rest(const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col, uint32_t nrows,
+          const uint32_t* __restrict__ giant_ptr, uint32_t* parent, unsigned long long* walked)
 {
   const uint32_t giant = *giant_ptr;
-  const int lane = threadIdx.x & 31;
-  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+  const uint32_t lane = threadIdx.x & 31;
   unsigned long long rows = 0, edges = 0;
-  for (uint32_t u = warp; u < nrows; u += nwarps)
+  for (uint32_t u0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); u0 < nrows; u0 += gridDim.x * blockDim.x)
   {
-    const uint32_t b = ptr[u] + k, e = ptr[u + 1];
-    if (b >= e) continue;
-    const uint32_t iu = id_of_pos[u];
-    if (cc_find(parent, iu) == giant) continue;
-    rows++;
-    edges += e - b;
-    for (uint32_t i = b + lane; i < e; i += 32) cc_union(parent, iu, id_of_pos[col[i]]);
+    const uint32_t u = u0 + lane;
+    uint32_t b = 0, e = 0;
+    const bool out = u < nrows && cc_find(parent, u) != giant;
+    if (out)
+    {
+      b = ptr[u];
+      e = ptr[u + 1];
+      rows++;
+      edges += e - b;
+    }
+    for (unsigned m = __ballot_sync(0xffffffffu, out); m; m &= m - 1)
+    {
+      const int src = __ffs(m) - 1;
+      const uint32_t b0 = __shfl_sync(0xffffffffu, b, src), e0 = __shfl_sync(0xffffffffu, e, src);
+      for (uint32_t i = b0 + lane; i < e0; i += 32) cc_union(parent, u0 + src, col[i]);
+    }
   }
-  if (lane == 0 && rows)
+  rows = block_sum_u64(rows);
+  edges = block_sum_u64(edges);
+  if (threadIdx.x == 0 && rows)
   {
     atomicAdd(&walked[0], rows);
     atomicAdd(&walked[1], edges);
   }
 }
 
-__global__ void k_cc_probe(const uint32_t* __restrict__ id_of_pos, uint32_t nrows, uint32_t nsamples, uint64_t seed,
+__global__ void k_cc_probe(uint32_t nrows, uint32_t nsamples, uint64_t seed, const uint32_t* __restrict__ giant_share,
                            uint32_t* parent, uint32_t* out)
 {
+  if (giant_share && *giant_share >= kCcEnough) return;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nsamples; i += gridDim.x * blockDim.x)
   {
     uint64_t x = seed + 0x9E3779B97F4A7C15ull * (i + 1);
     x = (x ^ (x >> 30)) * 0xBF58476D1CE4E5B9ull;
     x = (x ^ (x >> 27)) * 0x94D049BB133111EBull;
     x ^= x >> 31;
-    out[i] = cc_find(parent, id_of_pos[(uint32_t) (x % nrows)]);
+    out[i] = cc_find(parent, (uint32_t) (x % nrows));
   }
 }
 
-// The most frequent root among the samples (ties: the smallest), on the
-// device: one block sorts them in shared memory and counts runs.
-template <uint32_t NS>
-__global__ void __launch_bounds__(NS) k_cc_giant(const uint32_t* __restrict__ probe, uint32_t* giant)
+// giant[0]: the most frequent root among the samples (ties: the smallest),
+// giant[1]: how many they are.  One block counts them in a hash table in shared
+// memory, a warp's equal ones with one addition.  again: after rounds that were
+// skipped if the first sample had kCcEnough; nothing to do then.
+__global__ void __launch_bounds__(kCcSamples) k_cc_giant(const uint32_t* __restrict__ probe, uint32_t* giant, int again)
 {
-  __shared__ uint32_t v[NS];
-  __shared__ uint32_t best_len, best_val;
+  constexpr uint32_t kSlots = 2 * kCcSamples;
+  __shared__ uint32_t key[kSlots], cnt[kSlots];
+  __shared__ unsigned long long best;
+  if (again && giant[1] >= kCcEnough) return;
   const uint32_t t = threadIdx.x;
-  v[t] = probe[t];
+  for (uint32_t i = t; i < kSlots; i += kCcSamples)
+  {
+    key[i] = 0xFFFFFFFFu;
+    cnt[i] = 0;
+  }
+  if (t == 0) best = 0;
+  __syncthreads();
+  const uint32_t r = probe[t];
+  const unsigned same = __match_any_sync(0xffffffffu, r);
+  const bool leads = (int) (t & 31) == __ffs(same) - 1;
+  uint32_t slot = (r * 0x9E3779B1u) % kSlots;
+  if (leads)
+  {
+    for (;; slot = (slot + 1) % kSlots)
+    {
+      const uint32_t k = atomicCAS(&key[slot], 0xFFFFFFFFu, r);
+      if (k == 0xFFFFFFFFu || k == r) break;
+    }
+    atomicAdd(&cnt[slot], __popc(same));
+  }
+  __syncthreads();
+  if (leads) atomicMax(&best, (unsigned long long) cnt[slot] << 32 | (0xFFFFFFFFu - r));
+  __syncthreads();
   if (t == 0)
   {
-    best_len = 0;
-    best_val = 0xFFFFFFFFu;
+    giant[0] = 0xFFFFFFFFu - (uint32_t) best;
+    giant[1] = (uint32_t) (best >> 32);
   }
-  __syncthreads();
-  for (uint32_t size = 2; size <= NS; size <<= 1)
-    for (uint32_t stride = size >> 1; stride > 0; stride >>= 1)
-    {
-      const uint32_t j = t ^ stride;
-      if (j > t)
-      {
-        const bool up = (t & size) == 0;
-        const uint32_t a = v[t], b = v[j];
-        if ((a > b) == up)
-        {
-          v[t] = b;
-          v[j] = a;
-        }
-      }
-      __syncthreads();
-    }
-  // run starts: thread t owns the run beginning at t
-  if (t == 0 || v[t] != v[t - 1])
-  {
-    uint32_t e = t + 1;
-    while (e < NS && v[e] == v[t]) e++;
-    const uint32_t len = e - t;
-    // longest run, the smallest root among equal lengths: pack (len, ~val) into one word
-    atomicMax(&best_len, len);
-  }
-  __syncthreads();
-  if ((t == 0 || v[t] != v[t - 1]))
-  {
-    uint32_t e = t + 1;
-    while (e < NS && v[e] == v[t]) e++;
-    if (e - t == best_len) atomicMin(&best_val, v[t]);
-  }
-  __syncthreads();
-  if (t == 0) *giant = best_val;
 }
 
-__global__ void k_cc_flatten(uint32_t N, uint32_t* parent)
+// Full compression.  A chain longer than kCcWalk is cut short at that ancestor
+// and reported in *deep; the second pass (second: after the first one) then
+// walks what is left, and has nothing to do otherwise.  (Walking every chain to
+// its end at once, 2^20 vertices hooked one under the other took 19 ms; finds
+// with path halving cannot be used here, since a late halving store may
+// overwrite a root.)
+static constexpr uint32_t kCcWalk = 512;
+__global__ void k_cc_flatten(uint32_t nrows, const uint32_t* __restrict__ giant_share, uint32_t* parent, uint32_t* deep,
+                             int second)
 {
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < N; v += gridDim.x * blockDim.x)
+  if (giant_share && *giant_share >= kCcEnough) return;  // after a round that was skipped
+  if (second && !*deep) return;
+  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < nrows; v += gridDim.x * blockDim.x)
   {
-    uint32_t r = v;
-    while (parent[r] != r) r = parent[r];
+    uint32_t r = v, p = parent[v], n = 0;
+    while (p != r)
+    {
+      r = p;
+      if (!second && ++n == kCcWalk)
+      {
+        *deep = 1;
+        break;
+      }
+      p = parent[r];
+    }
     parent[v] = r;
+  }
+}
+
+// The least id of each tree (compressed): the lanes of a warp that share a
+// root, most of them under the giant one, first take theirs together.
+__global__ void k_cc_least(uint32_t nrows, const uint32_t* __restrict__ id_of_pos, const uint32_t* __restrict__ parent,
+                           uint32_t* least)
+{
+  for (uint32_t u0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); u0 < nrows; u0 += gridDim.x * blockDim.x)
+  {
+    const uint32_t u = u0 + (threadIdx.x & 31);
+    uint32_t r = 0xFFFFFFFFu, id = 0xFFFFFFFFu;
+    if (u < nrows)
+    {
+      r = parent[u];
+      id = id_of_pos[u];
+    }
+    const uint32_t first = __shfl_sync(0xffffffffu, r, 0);
+    const uint32_t m = __reduce_min_sync(0xffffffffu, r == first ? id : 0xFFFFFFFFu);
+    if (r == first) id = (threadIdx.x & 31) == 0 ? m : 0xFFFFFFFFu;
+    if (id != 0xFFFFFFFFu && least[r] > id) atomicMin(&least[r], id);
+  }
+}
+
+__global__ void k_cc_labels(uint32_t N, uint32_t nrows, const uint32_t* __restrict__ id_of_pos,
+                            const uint32_t* __restrict__ parent, const uint32_t* __restrict__ least, uint32_t* label)
+{
+  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < N; p += gridDim.x * blockDim.x)
+  {
+    const uint32_t id = id_of_pos[p];
+    label[id] = p < nrows ? least[parent[p]] : id;
   }
 }
 
@@ -288,57 +369,91 @@ extern "C" int la3g_cc(la3g_graph* G, uint32_t* label_out, la3g_stats* st)
   const bool zero_has_edges = cs->zero_has_edges == 1;
   uint32_t iters = 0;
   bool rest_counted = false;
+  uint32_t first = 0;  // link rounds before the first sample
   T.device_begin();
   if (!zero_has_edges && nrows)
   {
-    const uint32_t k = 2, nsamples = 1024;
-    k_cc_init<<<grid_for(N, 256), 256, 0, s>>>(N, cs->label);
-    LA3G_LAUNCHED();
-    tls_launches++;
-    for (uint32_t r = 0; r < k; r++)
+    if (!cs->parent)
     {
-      {
-        // row offsets, one index, two ids, and the two finds' parents
-        ProfileScope p("cc_sample", s, 8.0 * nrows + 4.0 * nrows + 8.0 * nrows + 8.0 * nrows);
-        k_cc_sample<<<grid_for(nrows, 256), 256, 0, s>>>(g.in_ptr, g.in_col, g.id_of_pos, nrows, r, cs->label);
-        LA3G_LAUNCHED();
-      }
-      {
-        ProfileScope p("cc_flatten", s, 8.0 * N);
-        k_cc_flatten<<<grid_for(N, 256), 256, 0, s>>>(N, cs->label);
-        LA3G_LAUNCHED();
-      }
+      LA3G_TRY(galloc(G, &cs->least, nrows));
+      LA3G_TRY(galloc(G, &cs->deep, kCcFlags));
+      LA3G_TRY(galloc(G, &cs->probe, kCcSamples));
+      LA3G_TRY(galloc(G, &cs->giant, 2));
+      LA3G_TRY(galloc(G, &cs->parent, nrows));
     }
-    if (!cs->probe) LA3G_TRY(galloc(G, &cs->probe, nsamples));
-    k_cc_probe<<<4, 256, 0, s>>>(g.id_of_pos, nrows, nsamples, 0x5A3Dull, cs->label, cs->probe);
-    LA3G_LAUNCHED();
-    tls_launches++;
-    if (!cs->giant) LA3G_TRY(galloc(G, &cs->giant, 1));
-    k_cc_giant<1024><<<1, 1024, 0, s>>>(cs->probe, cs->giant);
-    LA3G_LAUNCHED();
-    tls_launches++;
+    int nflat = 0;
+    auto flatten = [&](const uint32_t* share) -> int {
+      ProfileScope p("cc_flatten", s, 8.0 * nrows);
+      for (int second = 0; second < 2; second++)
+      {
+        k_cc_flatten<<<grid_for(nrows, 256), 256, 0, s>>>(nrows, share, cs->parent, cs->deep + nflat, second);
+        LA3G_LAUNCHED();
+      }
+      tls_launches++;
+      nflat++;
+      return LA3G_OK;
+    };
+    auto link = [&](uint32_t r, const uint32_t* share) -> int {
+      // row offsets, one index, the two roots
+      ProfileScope p("cc_link", s, (8.0 + 4.0 + 8.0) * nrows);
+      k_cc_link<<<grid_for(nrows, 256), 256, 0, s>>>(g.in_ptr, g.in_col, nrows, r, share, cs->parent);
+      LA3G_LAUNCHED();
+      return LA3G_OK;
+    };
+    auto sample = [&](bool again) -> int {
+      k_cc_probe<<<4, 256, 0, s>>>(nrows, kCcSamples, 0x5A3Dull, again ? cs->giant + 1 : nullptr, cs->parent, cs->probe);
+      LA3G_LAUNCHED();
+      k_cc_giant<<<1, kCcSamples, 0, s>>>(cs->probe, cs->giant, again ? 1 : 0);
+      LA3G_LAUNCHED();
+      tls_launches += 2;
+      return LA3G_OK;
+    };
+    {
+      // row offset, one index, the parent and the least id's start
+      ProfileScope p("cc_hook", s, 16.0 * nrows);
+      k_cc_hook<<<grid_for(nrows, 256), 256, 0, s>>>(g.in_ptr, g.in_col, nrows, cs->parent, cs->least, cs->deep);
+      LA3G_LAUNCHED();
+    }
+    LA3G_TRY(flatten(nullptr));
+    // rows of a few entries have hardly more neighbours to link with
+    const bool sparse = g.nent < 3ull * nrows;
+    const uint32_t rounds = sparse ? 1 : kCcLinks + kCcMoreLinks;
+    first = sparse ? 1 : kCcLinks;
+    for (uint32_t r = 0; r < rounds; r++)
+    {
+      const uint32_t* share = r < first ? nullptr : cs->giant + 1;
+      LA3G_TRY(link(r, share));
+      LA3G_TRY(flatten(share));
+      if (r + 1 == first) LA3G_TRY(sample(false));
+    }
+    if (rounds > first) LA3G_TRY(sample(true));
     LA3G_CUDA(cudaMemsetAsync(cs->walked, 0, 16, s));
     {
-      // every row: its offsets, id and root (16 B); the walked rows' edges:
-      // index, neighbour id and its root (12 B each), added once the walked
+      // every row: its root (4 B); the walked rows: offsets (8 B), and per edge
+      // its index and the neighbour's root (8 B each), added once the walked
       // counts are back on the host
-      ProfileScope p("cc_rest", s, 16.0 * nrows);
-      k_cc_rest<<<grid_for((uint64_t) nrows * 32, 256, num_sms() * 32), 256, 0, s>>>(g.in_ptr, g.in_col, g.id_of_pos, nrows,
-                                                                               k, cs->giant, cs->label, cs->walked);
+      ProfileScope p("cc_rest", s, 4.0 * nrows);
+      k_cc_rest<<<grid_for(nrows, 256, num_sms() * 32), 256, 0, s>>>(g.in_ptr, g.in_col, nrows, cs->giant, cs->parent,
+                                                                     cs->walked);
       LA3G_LAUNCHED();
     }
     LA3G_CUDA(cudaMemcpyAsync(cs->hwalked, cs->walked, 16, cudaMemcpyDeviceToHost, s));
     rest_counted = true;
+    LA3G_TRY(flatten(nullptr));
     {
-      ProfileScope p("cc_flatten", s, 8.0 * N);
-      k_cc_flatten<<<grid_for(N, 256), 256, 0, s>>>(N, cs->label);
+      // ids, roots and the labels by id
+      ProfileScope p("cc_labels", s, 8.0 * nrows + 12.0 * N);
+      k_cc_least<<<grid_for(nrows, 256), 256, 0, s>>>(nrows, g.id_of_pos, cs->parent, cs->least);
       LA3G_LAUNCHED();
+      k_cc_labels<<<grid_for(N, 256), 256, 0, s>>>(N, nrows, g.id_of_pos, cs->parent, cs->least, cs->label);
+      LA3G_LAUNCHED();
+      tls_launches++;
     }
     iters = 1;
   }
   else if (!zero_has_edges)
   {
-    k_cc_init<<<grid_for(N, 256), 256, 0, s>>>(N, cs->label);
+    k_cc_labels<<<grid_for(N, 256), 256, 0, s>>>(N, 0, g.id_of_pos, nullptr, nullptr, cs->label);
     LA3G_LAUNCHED();
     tls_launches++;
     iters = 1;
@@ -388,13 +503,15 @@ extern "C" int la3g_cc(la3g_graph* G, uint32_t* label_out, la3g_stats* st)
   LA3G_TRY(T.finish());
   if (rest_counted)
   {
-    profile_add_bytes("cc_rest", 12.0 * (double) cs->hwalked[1]);
+    const double rest = 8.0 * (double) cs->hwalked[0] + 8.0 * (double) cs->hwalked[1];
+    profile_add_bytes("cc_rest", rest);
     if (st)
     {
-      // two sampled neighbours per row (28 B), three compressions (8 B per
-      // vertex each), every row's root test (16 B), the walked edges (12 B)
-      st->edges_examined = 2ull * nrows + cs->hwalked[1];
-      st->algo_bytes = (uint64_t) (56.0 * nrows + 24.0 * N + 16.0 * nrows + 12.0 * (double) cs->hwalked[1]);
+      // the hook and link rounds (16 and 20 B per row), a compression after
+      // each and at the end (8 B), every row's root test (4 B), the walked
+      // edges, the labels
+      st->edges_examined = (uint64_t) (1 + first) * nrows + cs->hwalked[1];
+      st->algo_bytes = (uint64_t) ((16.0 + 20.0 * first + 8.0 * (first + 2) + 4.0 + 8.0) * nrows + 12.0 * N + rest);
     }
   }
   return LA3G_OK;
