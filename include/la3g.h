@@ -273,20 +273,20 @@ int la3g_bfs_batch(la3g_graph* g, const uint32_t* roots, uint32_t nroots, uint8_
 int la3g_sssp_batch(la3g_graph* g, const uint32_t* roots, uint32_t nroots, uint32_t* dist_out,
                     la3g_stats* st);
 
-/* Tunes the batched BFS for this graph (level mode: per-level CUDA graph or
- * persistent kernel; block size; push/pull threshold) by timing each
- * combination on the given roots (best of two runs); the best is kept on the
- * graph handle for batches of the same number of 64-root words (batches of
- * other sizes use the nearest tuned size).  report (nullable) receives a
- * JSON list of the timings. */
+/* Tunes the batched BFS for this graph (mode: levels that push or pull, or
+ * pull only; block size; push/pull threshold) by timing each combination on
+ * the given roots (best of two runs); the best is kept on the graph handle for
+ * batches of the same number of 64-root words (batches of other sizes use the
+ * nearest tuned size).  report (nullable) receives a JSON list of the
+ * timings. */
 int la3g_batch_autotune(la3g_graph* g, const uint32_t* roots, uint32_t nroots, char* report, size_t cap);
 
 /* Sets the batched-BFS configuration by hand (dropping tuned ones): mode 0 =
- * per-level CUDA graph, 1 = persistent kernel; block 128 / 256 / 512;
- * push_frac in [0, 1]. */
+ * levels push or pull by push_frac, 1 = every level pulls; block 128 / 256 /
+ * 512; push_frac in [0, 1]. */
 int la3g_batch_config(la3g_graph* g, int mode, int block, double push_frac);
 
-/* The persistent batched-BFS kernel's grid barriers wait at most `polls`
+/* In mode 1 the batched-BFS kernel's grid barriers wait at most `polls`
  * polls per block (default 2^26, restored by polls < 0); a block that runs
  * out sets an error word, every block leaves its kernel, and the call returns
  * LA3G_ETIMEOUT with the device left usable.  No counterpart in the

@@ -494,12 +494,12 @@ def batch_autotune(G: Graph, roots: Sequence[int]) -> list:
 
 
 def batch_config(G: Graph, mode: int, block: int = 256, push_frac: float = 0.05) -> None:
-    """mode 0: per-level CUDA graph; 1: persistent kernel."""
+    """mode 0: levels push or pull by push_frac; 1: every level pulls."""
     N.check(N.lib().la3g_batch_config(G._h, mode, block, push_frac))
 
 
 def batch_set_wait_limit(G: Graph, polls: int = -1) -> None:
-    """Grid-barrier poll limit of the persistent batched-BFS kernel (< 0: the default)."""
+    """Grid-barrier poll limit of the batched-BFS kernel in mode 1 (< 0: the default)."""
     N.check(N.lib().la3g_batch_set_wait_limit(G._h, polls))
 
 

@@ -10,11 +10,11 @@
 // run bottom-up (pull) when the frontier is dense and top-down (push, an
 // atomicOr per edge and word) when it is sparse.  Per-word "alive" masks
 // record which roots still discovered something; words whose roots are all
-// finished are skipped (done-masks).  Levels run either as a CUDA graph of
-// one level replayed from the host (the level number and buffer parity live
-// in device memory, so one captured graph serves every level), or inside one
-// persistent cooperative kernel with a grid barrier whose waits are bounded
-// (a barrier that waits too long records an error and every block returns).
+// finished are skipped (done-masks).  All levels run inside one cooperative
+// kernel with a grid barrier whose waits are bounded (a barrier that waits too
+// long records an error and every block returns): with a host round trip per
+// level a batch of 64 roots on R-MAT 2^18 spent a third of its time between
+// kernels.
 // BFS levels are order-free, so hops equal the single-root runs; a batch
 // whose BFS would exceed 254 levels (where the reference's uint8 hops wrap)
 // is rerun root by root with la3g_bfs.
@@ -41,37 +41,37 @@ namespace la3g {
 
 struct BatchConfig
 {
-  int mode = 0;          // 0 = per-level CUDA graph, 1 = persistent cooperative kernel
+  int mode = 0;          // 0 = pushing or pulling levels, 1 = pulling levels only
   int block = 256;       // threads per block of the level kernels
   double push_frac = 0.05;  // push when frontier edges * words < push_frac * m * words
   bool tuned = false;
 };
 
-// Polls a block of the persistent kernel makes at a grid barrier before it
-// gives up (sets the error word, every block leaves, the call returns
-// LA3G_ETIMEOUT); la3g_batch_set_wait_limit changes it per graph.
+// Polls a block makes at a grid barrier before it gives up (sets the error
+// word, every block leaves, the call returns LA3G_ETIMEOUT);
+// la3g_batch_set_wait_limit changes it per graph for mode 1.
 static constexpr long long kDefaultWaitPolls = 1ll << 26;
 
 struct BatchScratch
 {
-  long long wait_polls = kDefaultWaitPolls;  // grid-barrier poll limit of the persistent kernel
+  long long wait_polls = kDefaultWaitPolls;  // grid-barrier poll limit in mode 1
   uint32_t cap_r = 0;        // roots the buffers were sized for
   uint64_t* vis = nullptr;   // [N][W]
   uint64_t* buf[2] = {nullptr, nullptr};  // frontier / next, [N][W]
-  uint64_t* alive[2] = {nullptr, nullptr};  // [W] per-word "discovered something" masks
+  uint64_t* alive[3] = {nullptr, nullptr, nullptr};  // [W] per-word "discovered something" masks
   uint8_t* hops = nullptr;   // [N][W * 64] by position (vertex-major)
   uint32_t* rpos = nullptr;  // root positions
   uint32_t* active = nullptr;  // push: active (vertex, word) pairs of small vertices
   uint32_t* phub = nullptr;    // push: pairs of hub vertices, and their first task numbers
   uint32_t* phub_t0 = nullptr;
-  unsigned long long* ctr = nullptr;  // [0] new bits, [1] small pairs, [2] frontier edges*words, [3] level,
-                                      // [4] levels that found something, [5] hub slots / tasks (packed)
-  unsigned long long* hctr = nullptr;
-  unsigned int* bar = nullptr;        // grid barrier: count, generation
-  int* err = nullptr;
-  cudaGraphExec_t pull_exec = nullptr;
-  uint32_t pull_exec_w = 0, pull_exec_block = 0;
-  cudaStream_t pull_exec_stream = nullptr;
+  // BFS: [0..2] new bits of the levels in turn, [3] small pairs, [4] hub slots
+  // and tasks (packed).  SSSP: [c], [2 + c] list c's small pairs and packed
+  // hubs, [4 + c] smallest distance list c holds
+  unsigned long long* ctr = nullptr;
+  unsigned long long* hctr = nullptr;  // pinned, written by the kernels: [0] levels / iterations, [1] status
+  unsigned int* bar = nullptr;         // grid barrier: count, error word
+  uint8_t* tpos = nullptr;             // results by root and id, before they leave the device
+  size_t tpos_bytes = 0;
   BatchConfig cfg;                           // set by hand, or the default
   std::vector<std::pair<uint32_t, BatchConfig>> tuned;  // autotuned, by words per batch
   // SSSP
@@ -91,7 +91,6 @@ struct BatchScratch
 static void batch_scratch_free(void* p)
 {
   BatchScratch* b = (BatchScratch*) p;
-  if (b->pull_exec) cudaGraphExecDestroy(b->pull_exec);
   if (b->hctr) cudaFreeHost(b->hctr);
   delete b;
 }
@@ -130,236 +129,165 @@ __global__ void k_ms_roots(const uint32_t* __restrict__ rpos, uint32_t R, uint32
   }
 }
 
-// Bottom-up level over (vertex, word) pairs (pull_scan: a lane per pair,
-// the warp for long in-edge lists).  Reads the level from ctr[3]; front /
-// next alternate with its parity.  tid / nthreads count whole warps.
-__device__ __forceinline__ void ms_pull_body(const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col,
-                                             uint32_t nrows, uint32_t N, uint32_t W, uint64_t* vis, uint64_t* const* buf,
-                                             uint64_t* const* alive, uint8_t* hops, unsigned long long* ctr,
-                                             uint64_t tid, uint64_t nthreads)
+struct MsArgs
 {
-  const uint32_t level = (uint32_t) ctr[3];
-  const uint64_t* __restrict__ front = buf[level & 1];
-  uint64_t* next = buf[(level + 1) & 1];
-  const uint64_t* alive_now = alive[level & 1];
-  uint64_t* alive_next = alive[(level + 1) & 1];
-  const uint8_t hop = (uint8_t) (level + 1);
-  unsigned long long cnt = 0;
-  const uint64_t NW = (uint64_t) nrows * W;
-  // a warp takes 32 consecutive pairs at a time (pull_scan is warp-collective)
-  const int lane = threadIdx.x & 31;
-  for (uint64_t base = (tid >> 5) * 32; base < NW; base += (nthreads >> 5) * 32)
-  {
-    const uint64_t i = base + lane;
-    const bool ok = i < NW;
-    const uint32_t v = ok ? (uint32_t) (i / W) : 0, w = ok ? (uint32_t) (i % W) : 0;
-    const uint64_t seen = ok ? vis[i] : ~0ull;
-    const uint64_t want = ok ? ~seen & alive_now[w] : 0;
-    const uint64_t nb = pull_scan(v, w, W, want, ptr, col, front, lane);
-    if (!ok) continue;
-    next[i] = nb;
-    if (nb)
-    {
-      vis[i] = seen | nb;
-      cnt += __popcll(nb);
-      atomicOr((unsigned long long*) &alive_next[w], (unsigned long long) nb);
-      hops_record(hops + i * 64, nb, hop);
-    }
-  }
-  for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-  if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(&ctr[0], cnt);
-}
-
-struct BufPair
-{
-  uint64_t* p[2];
+  const uint32_t *ptr, *col;
+  uint32_t nrows, N, W, R;
+  uint64_t* vis;
+  uint64_t* buf[2];    // the frontier of level l in buf[l & 1]
+  uint64_t* alive[3];  // the roots still active at level l in alive[l % 3]
+  uint8_t* hops;
+  PairList list;       // pushing levels: the frontier's pairs
+  unsigned long long* ctr;
+  unsigned int* bar;
+  long long wait_polls;
+  // a level pushes when its new bits x mean degree stay below the limit
+  double mean_deg, push_limit;
+  unsigned long long* out;  // pinned: levels run, status
 };
 
-__global__ void k_ms_pull(const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col, uint32_t nrows, uint32_t N,
-                          uint32_t W, uint64_t* vis, BufPair buf, BufPair alive, uint8_t* hops, unsigned long long* ctr)
-{
-  ms_pull_body(ptr, col, nrows, N, W, vis, buf.p, alive.p, hops, ctr, (uint64_t) blockIdx.x * blockDim.x + threadIdx.x,
-               (uint64_t) gridDim.x * blockDim.x);
-}
+static constexpr uint32_t kMsAliveShared = 256;  // words of the alive mask gathered per block
 
-// End of a level: clear the alive mask two levels ahead, advance the level.
-__global__ void k_ms_advance(uint32_t W, BufPair alive, unsigned long long* ctr)
+// What a warp found for 32 consecutive pairs: visited bits, hop bytes, the
+// roots still alive (in shared memory first: thousands of pairs would meet at
+// a few global words).
+__device__ __forceinline__ uint32_t ms_found(const MsArgs& A, uint64_t base, bool ok, uint64_t nb, uint64_t seen, uint8_t hop,
+                                             int lane, unsigned long long* s_alive, unsigned long long* alive_next)
 {
-  const uint32_t level = (uint32_t) ctr[3];
-  uint64_t* stale = alive.p[level & 1];  // becomes the "next" mask of the next level
-  for (uint32_t w = threadIdx.x; w < W; w += blockDim.x) stale[w] = 0;
-  __syncthreads();
-  if (threadIdx.x == 0) ctr[3] = level + 1;
-}
-
-// Top-down level: list the nonzero frontier words, push them to neighbours
-// (masked by visited), then apply.
-__global__ void k_ms_list(uint32_t nrows, uint32_t W, BufPair buf, const uint32_t* __restrict__ ptr, PairList out,
-                          const unsigned long long* __restrict__ ctr)
-{
-  const uint32_t level = (uint32_t) ctr[3];
-  const uint64_t* front = buf.p[level & 1];
-  const uint64_t NW = (uint64_t) nrows * W;
-  for (uint64_t i = (uint64_t) blockIdx.x * blockDim.x + threadIdx.x; i < NW; i += (uint64_t) gridDim.x * blockDim.x)
-    if (front[i])
-    {
-      const uint32_t v = (uint32_t) (i / W);
-      bs_list_pair((uint32_t) i, ptr[v + 1] - ptr[v], out);
-    }
-}
-
-__global__ void k_ms_push(const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col, uint32_t W, BufPair buf,
-                          const uint64_t* __restrict__ vis, PairList list, const unsigned long long* __restrict__ ctr)
-{
-  const uint32_t level = (uint32_t) ctr[3];
-  ms_push_pairs(ptr, col, W, buf.p[level & 1], vis, buf.p[(level + 1) & 1], list);
-}
-
-__global__ void k_ms_apply(uint32_t nrows, uint32_t N, uint32_t W, uint64_t* vis, BufPair buf, BufPair alive,
-                           uint8_t* hops, unsigned long long* ctr)
-{
-  const uint32_t level = (uint32_t) ctr[3];
-  uint64_t* next = buf.p[(level + 1) & 1];
-  uint64_t* alive_next = alive.p[(level + 1) & 1];
-  const uint8_t hop = (uint8_t) (level + 1);
-  unsigned long long cnt = 0;
-  const uint64_t NW = (uint64_t) nrows * W;
-  for (uint64_t i = (uint64_t) blockIdx.x * blockDim.x + threadIdx.x; i < NW; i += (uint64_t) gridDim.x * blockDim.x)
+  const uint64_t i = base + lane;
+  if (ok) A.buf[hop & 1][i] = nb;
+  if (nb)
   {
-    const uint64_t nb = next[i] & ~vis[i];
-    next[i] = nb;
-    if (nb)
+    A.vis[i] = seen | nb;
+    const uint32_t w = (uint32_t) (i % A.W);
+    if (A.W <= kMsAliveShared)
     {
-      vis[i] |= nb;
-      cnt += __popcll(nb);
-      atomicOr((unsigned long long*) &alive_next[i % W], (unsigned long long) nb);
-      hops_record(hops + i * 64, nb, hop);
+      if ((*(volatile unsigned long long*) &s_alive[w] & nb) != nb) atomicOr(&s_alive[w], (unsigned long long) nb);
     }
+    else if ((__ldcg(&alive_next[w]) & nb) != nb) atomicOr(&alive_next[w], (unsigned long long) nb);
   }
-  for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-  if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(&ctr[0], cnt);
+  hops_record_warp(A.hops + base * 64, nb, hop, lane);
+  return __popcll(nb);
 }
 
-// The front buffer must be zero before it is reused as "next" two levels
-// later; the pull kernel overwrites every word, the push path clears it.
-__global__ void k_ms_clear(uint64_t n, BufPair buf, unsigned long long* ctr)
+// All levels of a batch.  A pulling level (pull_scan: a lane per (vertex,
+// word) pair, the warp for long in-edge lists) writes every word of the next
+// frontier; a pushing one lists the frontier's nonzero words and clears the
+// next, pushes them to the neighbours (masked by visited), then applies.
+__global__ void __launch_bounds__(512) k_ms_run(MsArgs A)
 {
-  const uint32_t level = (uint32_t) ctr[3];
-  uint64_t* next = buf.p[(level + 1) & 1];
-  for (uint64_t i = (uint64_t) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t) gridDim.x * blockDim.x)
-    next[i] = 0;
-}
-
-// Grid barrier for the persistent kernel: bounded spin (at most `limit`
-// polls); on timeout the error word is set and every block leaves.
-__device__ bool grid_barrier(unsigned int* bar, int* err, unsigned int nblocks, long long limit)
-{
-  __syncthreads();
-  bool ok = true;
-  if (threadIdx.x == 0)
+  __shared__ unsigned long long s_alive[kMsAliveShared], s_got[3];
+  GridBarrier bar{A.bar, (int*) (A.bar + 1), A.wait_polls};
+  const int lane = threadIdx.x & 31;
+  const uint64_t tid = (uint64_t) blockIdx.x * blockDim.x + threadIdx.x, nth = (uint64_t) gridDim.x * blockDim.x;
+  const uint64_t NW = (uint64_t) A.nrows * A.W;
+  unsigned long long found = A.R;  // level 0: every root
+  uint32_t level = 0;
+  for (; level < 255 && found; level++)
   {
-    volatile unsigned int* vgen = bar + 1;
-    const unsigned int gen = *vgen;
-    __threadfence();
-    if (atomicAdd(bar, 1u) == nblocks - 1)
+    const uint64_t* front = A.buf[level & 1];
+    uint64_t* next = A.buf[(level + 1) & 1];
+    const uint64_t* alive_now = A.alive[level % 3];
+    unsigned long long* alive_next = (unsigned long long*) A.alive[(level + 1) % 3];
+    const uint8_t hop = (uint8_t) (level + 1);
+    for (uint64_t w = tid; w < A.W; w += nth) A.alive[(level + 2) % 3][w] = 0;
+    if (tid == 0) A.ctr[(level + 2) % 3] = 0;
+    for (uint32_t w = threadIdx.x; w < kMsAliveShared; w += blockDim.x) s_alive[w] = 0;
+    const bool push = (double) found * A.mean_deg < A.push_limit;
+    if (push)
     {
-      atomicExch(bar, 0u);
-      __threadfence();
-      atomicAdd(bar + 1, 1u);
-    }
-    else
-    {
-      long long spins = 0;
-      while (*vgen == gen)
+      for (uint64_t i = tid; i < NW; i += nth)
       {
-        if (spins++ >= limit || *(volatile int*) err)
+        next[i] = 0;
+        if (front[i])
         {
-          atomicExch(err, 1);
-          ok = false;
-          break;
+          const uint32_t v = (uint32_t) (i / A.W);
+          bs_list_pair((uint32_t) i, A.ptr[v + 1] - A.ptr[v], A.list);
         }
-        __nanosleep(64);
       }
-    }
-    __threadfence();
-  }
-  __shared__ int s_ok;
-  if (threadIdx.x == 0) s_ok = ok && !*(volatile int*) err;
-  __syncthreads();
-  return s_ok;
-}
-
-// All pull levels in one cooperative launch.
-__global__ void k_ms_persistent(const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col, uint32_t nrows,
-                                uint32_t N, uint32_t W, uint64_t* vis, BufPair buf, BufPair alive, uint8_t* hops,
-                                unsigned long long* ctr, unsigned int* bar, int* err, uint32_t max_levels,
-                                long long wait_limit)
-{
-  const uint64_t tid = (uint64_t) blockIdx.x * blockDim.x + threadIdx.x;
-  const uint64_t nth = (uint64_t) gridDim.x * blockDim.x;
-  for (uint32_t it = 0; it < max_levels; it++)
-  {
-    ms_pull_body(ptr, col, nrows, N, W, vis, buf.p, alive.p, hops, ctr, tid, nth);
-    if (!grid_barrier(bar, err, gridDim.x, wait_limit)) return;
-    const unsigned long long found = ctr[0];
-    if (!grid_barrier(bar, err, gridDim.x, wait_limit)) return;
-    if (blockIdx.x == 0)
-    {
-      const uint32_t level = (uint32_t) ctr[3];
-      uint64_t* stale = alive.p[level & 1];
-      for (uint32_t w = threadIdx.x; w < W; w += blockDim.x) stale[w] = 0;
-      __syncthreads();
+      if (!bar.sync()) return;
       if (threadIdx.x == 0)
       {
-        ctr[3] = level + 1;
-        ctr[4] += found ? 1 : 0;
-        ctr[0] = 0;
+        s_got[0] = __ldcg(A.list.nsmall);
+        s_got[1] = __ldcg(A.list.packed);
       }
+      __syncthreads();
+      ms_push_pairs(A.ptr, A.col, A.W, front, A.vis, next, A.list, (uint32_t) s_got[0], s_got[1]);
+      if (!bar.sync()) return;
+      if (tid == 0) *A.list.nsmall = *A.list.packed = 0;
     }
-    if (!grid_barrier(bar, err, gridDim.x, wait_limit)) return;
-    if (!found) return;
+    else __syncthreads();
+    uint32_t cnt = 0;
+    for (uint64_t base = (tid >> 5) * 32; base < NW; base += (nth >> 5) * 32)
+    {
+      const uint64_t i = base + lane;
+      const bool ok = i < NW;
+      const uint64_t seen = ok ? A.vis[i] : ~0ull;
+      uint64_t nb;
+      if (push) nb = ok ? next[i] & ~seen : 0;
+      else
+      {
+        const uint32_t v = ok ? (uint32_t) (i / A.W) : 0, w = ok ? (uint32_t) (i % A.W) : 0;
+        nb = pull_scan(v, w, A.W, ok ? ~seen & alive_now[w] : 0, A.ptr, A.col, front, lane);
+      }
+      cnt += ms_found(A, base, ok, nb, seen, hop, lane, s_alive, alive_next);
+    }
+    const unsigned long long total = block_sum_u64(cnt);  // (its barriers order s_alive too)
+    if (threadIdx.x == 0 && total) atomicAdd(&A.ctr[(level + 1) % 3], total);
+    if (A.W <= kMsAliveShared)
+      for (uint32_t w = threadIdx.x; w < A.W; w += blockDim.x)
+        if (s_alive[w]) atomicOr(&alive_next[w], s_alive[w]);
+    if (!bar.sync()) return;
+    if (threadIdx.x == 0) s_got[2] = __ldcg(&A.ctr[(level + 1) % 3]);
+    __syncthreads();
+    found = s_got[2];
+  }
+  if (tid == 0)
+  {
+    A.out[0] = level;
+    A.out[1] = found ? 2 : 1;  // 2: more levels than a byte of hops holds
   }
 }
 
-// Hops to out[root][id] in two passes, so that no pass gathers across the
-// whole [N][W * 64] array: a tiled transpose by position (32 positions x 32
-// roots per tile through shared memory; reads and writes move 32-byte runs)
-// into tpos[root][position], then a gather by id inside one root's N-byte
-// row, which stays in L2.
-__global__ void __launch_bounds__(256) k_ms_out_pos(uint32_t N, uint32_t R, uint32_t W, const uint8_t* __restrict__ hops,
-                                                    uint8_t* tpos)
+// Hops to out[root][id]: a block takes 128 ids and the 64 roots of a word, reads
+// each id's 64 bytes (16 lanes, 4 bytes each), transposes them in shared memory
+// and writes runs of 128 bytes.  (A transpose by position and a gather by id
+// took 36 + 54 us for 64 roots on R-MAT 2^18; this takes 14 us.)
+__global__ void __launch_bounds__(256) k_ms_out(uint32_t N, uint32_t R, uint32_t W, const uint32_t* __restrict__ pos_of_id,
+                                                const uint8_t* __restrict__ hops, uint8_t* __restrict__ out)
 {
-  __shared__ uint8_t t[32][33];
-  const uint32_t tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const uint32_t np = (N + 31) / 32, nr = (R + 31) / 32;
-  const uint64_t RW = (uint64_t) W * 64;
-  for (uint64_t tile = blockIdx.x; tile < (uint64_t) np * nr; tile += gridDim.x)
+  __shared__ uint8_t t[64][132];
+  const uint32_t tid = threadIdx.x, nid = (N + 127) / 128;
+  for (uint64_t tile = blockIdx.x; tile < (uint64_t) nid * W; tile += gridDim.x)
   {
-    const uint32_t p0 = (uint32_t) (tile % np) * 32, r0 = (uint32_t) (tile / np) * 32;
-    for (uint32_t k = ty; k < 32; k += 8)
+    const uint32_t id0 = (uint32_t) (tile % nid) * 128, w = (uint32_t) (tile / nid);
+    uint32_t v[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++)
     {
-      const uint32_t p = p0 + k;
-      t[k][tx] = p < N && r0 + tx < R ? hops[(uint64_t) p * RW + r0 + tx] : 255;
+      const uint32_t id = id0 + k * 16 + (tid >> 4);
+      v[k] = id < N ? *reinterpret_cast<const uint32_t*>(hops + ((uint64_t) pos_of_id[id] * W + w) * 64 + 4 * (tid & 15)) : 0;
     }
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+#pragma unroll
+      for (int q = 0; q < 4; q++) t[4 * (tid & 15) + q][k * 16 + (tid >> 4)] = (uint8_t) (v[k] >> (8 * q));
     __syncthreads();
-    for (uint32_t k = ty; k < 32; k += 8)
-    {
-      const uint32_t r = r0 + k, p = p0 + tx;
-      if (r < R && p < N) tpos[(uint64_t) r * N + p] = t[tx][k];
-    }
+    const uint32_t nr = min(64u, R - w * 64), x = tid & 127;
+    if (id0 + x < N)
+      for (uint32_t r = tid >> 7; r < nr; r += 2) out[(uint64_t) (w * 64 + r) * N + id0 + x] = t[r][x];
     __syncthreads();
   }
 }
 
-__global__ void k_ms_out_id(uint32_t N, uint32_t R, const uint32_t* __restrict__ pos_of_id, const uint8_t* __restrict__ tpos,
-                            uint8_t* out)
+// The buffer results are put in order in before they leave the device.
+static int batch_out_buffer(la3g_graph* G, BatchScratch* b, size_t bytes)
 {
-  const uint64_t RN = (uint64_t) R * N;
-  for (uint64_t i = (uint64_t) blockIdx.x * blockDim.x + threadIdx.x; i < RN; i += (uint64_t) gridDim.x * blockDim.x)
-  {
-    const uint64_t r = i / N;
-    out[i] = tpos[r * N + pos_of_id[i - r * N]];
-  }
+  if (bytes <= b->tpos_bytes) return LA3G_OK;
+  b->tpos_bytes = 0;
+  LA3G_TRY(galloc(G, &b->tpos, bytes));
+  b->tpos_bytes = bytes;
+  return LA3G_OK;
 }
 
 static int batch_scratch(la3g_graph* G, BatchScratch** out)
@@ -373,8 +301,7 @@ static int batch_scratch(la3g_graph* G, BatchScratch** out)
     G->slot_free[kSlotBatch] = batch_scratch_free;
     LA3G_TRY(galloc(G, &b->ctr, 8));
     LA3G_TRY(galloc(G, &b->bar, 2));
-    LA3G_TRY(galloc(G, &b->err, 1));
-    LA3G_CUDA(cudaHostAlloc(&b->hctr, 8 * sizeof(unsigned long long), cudaHostAllocDefault));
+    LA3G_CUDA(cudaHostAlloc(&b->hctr, 2 * sizeof(unsigned long long), cudaHostAllocMapped));
   }
   *out = b;
   return LA3G_OK;
@@ -388,19 +315,13 @@ static int ms_bfs_alloc(la3g_graph* G, BatchScratch* b, uint32_t R)
   LA3G_TRY(galloc(G, &b->vis, (size_t) N * W));
   LA3G_TRY(galloc(G, &b->buf[0], (size_t) N * W));
   LA3G_TRY(galloc(G, &b->buf[1], (size_t) N * W));
-  LA3G_TRY(galloc(G, &b->alive[0], W));
-  LA3G_TRY(galloc(G, &b->alive[1], W));
+  for (int k = 0; k < 3; k++) LA3G_TRY(galloc(G, &b->alive[k], W));
   LA3G_TRY(galloc(G, &b->hops, (size_t) N * W * 64));
   LA3G_TRY(galloc(G, &b->rpos, R));
   LA3G_TRY(galloc(G, &b->active, (size_t) N * W));
   LA3G_TRY(galloc(G, &b->phub, (size_t) N * W));
   LA3G_TRY(galloc(G, &b->phub_t0, (size_t) N * W));
   b->cap_r = R;
-  if (b->pull_exec)
-  {
-    cudaGraphExecDestroy(b->pull_exec);
-    b->pull_exec = nullptr;
-  }
   return LA3G_OK;
 }
 
@@ -420,120 +341,50 @@ static int ms_bfs_run(la3g_graph* G, BatchScratch* b, const uint32_t* roots_host
   cudaStream_t s = G->stream;
   const uint32_t N = g.nslots, nrows = g.nrows(), W = (R + 63) / 64;
   LA3G_TRY(ms_bfs_alloc(G, b, R));
-  BufPair buf{{b->buf[0], b->buf[1]}}, alive{{b->alive[0], b->alive[1]}};
   LA3G_CUDA(cudaMemcpyAsync(b->active, roots_host, (size_t) R * 4, cudaMemcpyHostToDevice, s));
   k_root_pos<<<grid_for(R, 256), 256, 0, s>>>(b->active, R, N, g.pos_of_id, b->rpos);
   LA3G_LAUNCHED();
   k_ms_init<<<num_sms() * 8, 256, 0, s>>>(N, W, R, b->vis, b->buf[0], b->buf[1]);
   LA3G_LAUNCHED();
   LA3G_CUDA(cudaMemsetAsync(b->hops, 0xFF, (size_t) N * W * 64, s));
-  LA3G_CUDA(cudaMemsetAsync(b->alive[0], 0, (size_t) W * 8, s));
-  LA3G_CUDA(cudaMemsetAsync(b->alive[1], 0, (size_t) W * 8, s));
+  for (int k = 0; k < 3; k++) LA3G_CUDA(cudaMemsetAsync(b->alive[k], 0, (size_t) W * 8, s));
   LA3G_CUDA(cudaMemsetAsync(b->ctr, 0, 8 * 8, s));
+  LA3G_CUDA(cudaMemsetAsync(b->bar, 0, 8, s));
   k_ms_roots<<<grid_for(R, 256), 256, 0, s>>>(b->rpos, R, N, W, b->vis, b->buf[0], b->hops, b->alive[0]);
   LA3G_LAUNCHED();
-  tls_launches += 4;
-  *wrap = false;
-  *edges_words = 0;
-  const unsigned blocks = num_sms() * (2048 / cfg.block);
-  if (cfg.mode == 1)
+  tls_launches += 3;
+  MsArgs A;
+  A.ptr = g.in_ptr;
+  A.col = g.in_col;
+  A.nrows = nrows;
+  A.N = N;
+  A.W = W;
+  A.R = R;
+  A.vis = b->vis;
+  for (int k = 0; k < 2; k++) A.buf[k] = b->buf[k];
+  for (int k = 0; k < 3; k++) A.alive[k] = b->alive[k];
+  A.hops = b->hops;
+  A.list = PairList{b->active, b->phub, b->phub_t0, b->ctr + 3, b->ctr + 4};
+  A.ctr = b->ctr;
+  A.bar = b->bar;
+  A.wait_polls = cfg.mode == 1 ? b->wait_polls : kDefaultWaitPolls;
+  A.mean_deg = (double) g.nent / std::max<uint32_t>(1, nrows);
+  A.push_limit = cfg.mode == 1 ? 0.0 : cfg.push_frac * (double) g.nent * 64.0 * W;
+  A.out = b->hctr;
+  b->hctr[1] = 0;
+  unsigned grid = 0;
+  LA3G_TRY(cooperative_blocks((const void*) k_ms_run, cfg.block, std::max<uint64_t>((uint64_t) nrows * W, g.nent / 8),
+                              2048 / cfg.block, &grid));
   {
-    // persistent cooperative kernel (pull levels)
-    int per_sm = 0;
-    LA3G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ms_persistent, cfg.block, 0));
-    int dev = 0, sms = num_sms();
-    LA3G_CUDA(cudaGetDevice(&dev));
-    LA3G_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    unsigned grid = (unsigned) std::max(1, per_sm) * (unsigned) sms;
-    LA3G_CUDA(cudaMemsetAsync(b->bar, 0, 8, s));
-    LA3G_CUDA(cudaMemsetAsync(b->err, 0, 4, s));
-    const uint32_t* ptr = g.in_ptr;
-    const uint32_t* col = g.in_col;
-    uint64_t* vis = b->vis;
-    uint8_t* hops = b->hops;
-    unsigned long long* ctr = b->ctr;
-    unsigned int* bar = b->bar;
-    int* err = b->err;
-    uint32_t maxl = 255;
-    long long wait_limit = b->wait_polls;
-    void* args[] = {(void*) &ptr, (void*) &col, (void*) &nrows, (void*) &N, (void*) &W, (void*) &vis, (void*) &buf,
-                    (void*) &alive, (void*) &hops, (void*) &ctr, (void*) &bar, (void*) &err, (void*) &maxl,
-                    (void*) &wait_limit};
-    {
-      ProfileScope p("msbfs_persistent", s, 0.0);
-      LA3G_CUDA(cudaLaunchCooperativeKernel((void*) k_ms_persistent, grid, cfg.block, args, 0, s));
-    }
-    int herr = 0;
-    LA3G_CUDA(cudaMemcpyAsync(&herr, b->err, 4, cudaMemcpyDeviceToHost, s));
-    LA3G_CUDA(cudaMemcpyAsync(b->hctr, b->ctr, 8 * 8, cudaMemcpyDeviceToHost, s));
-    LA3G_CUDA(cudaStreamSynchronize(s));
-    if (herr) return set_error(LA3G_ETIMEOUT, "batched BFS: a grid barrier wait ran out");
-    *levels = (uint32_t) b->hctr[3];
-    *wrap = b->hctr[3] >= 255;
-    *edges_words = (uint64_t) *levels * g.nent * W;
-    return LA3G_OK;
+    void* args[] = {(void*) &A};
+    ProfileScope p("msbfs", s, 0.0);
+    LA3G_CUDA(cudaLaunchCooperativeKernel((const void*) k_ms_run, grid, cfg.block, args, 0, s));
   }
-  // per-level: the bottom-up level is one captured graph replayed each level
-  if (!b->pull_exec || b->pull_exec_w != W || b->pull_exec_block != (uint32_t) cfg.block || b->pull_exec_stream != s)
-  {
-    if (b->pull_exec) cudaGraphExecDestroy(b->pull_exec);
-    b->pull_exec = nullptr;
-    cudaStream_t cap;
-    LA3G_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
-    cudaGraph_t graph;
-    cudaError_t e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
-    if (e == cudaSuccess)
-    {
-      k_ms_pull<<<blocks, cfg.block, 0, cap>>>(g.in_ptr, g.in_col, nrows, N, W, b->vis, buf, alive, b->hops, b->ctr);
-      k_ms_advance<<<1, 256, 0, cap>>>(W, alive, b->ctr);
-      e = cudaStreamEndCapture(cap, &graph);
-    }
-    if (e == cudaSuccess)
-    {
-      e = cudaGraphInstantiate(&b->pull_exec, graph, 0);
-      cudaGraphDestroy(graph);
-    }
-    cudaStreamDestroy(cap);
-    if (e != cudaSuccess) return set_error(LA3G_ECUDA, "graph capture of the BFS level failed: %s", cudaGetErrorString(e));
-    b->pull_exec_w = W;
-    b->pull_exec_block = (uint32_t) cfg.block;
-    b->pull_exec_stream = s;
-  }
-  uint64_t front_bits = 0;
-  for (uint32_t level = 0; level < 255; level++)
-  {
-    // frontier popcount of level 0 = number of valid roots (approximate: R)
-    const uint64_t fb = level == 0 ? R : front_bits;
-    const bool push = (double) fb * ((double) g.nent / std::max<uint32_t>(1, nrows)) <
-                      cfg.push_frac * (double) g.nent * 64.0 * W;
-    LA3G_CUDA(cudaMemsetAsync(b->ctr, 0, 2 * 8, s));
-    if (push)
-    {
-      ProfileScope p("msbfs_push", s, 0.0);
-      const PairList pl{b->active, b->phub, b->phub_t0, b->ctr + 1, b->ctr + 5};
-      LA3G_CUDA(cudaMemsetAsync(b->ctr + 5, 0, 8, s));
-      k_ms_clear<<<blocks, cfg.block, 0, s>>>((uint64_t) N * W, buf, b->ctr);
-      k_ms_list<<<blocks, cfg.block, 0, s>>>(nrows, W, buf, g.in_ptr, pl, b->ctr);
-      k_ms_push<<<blocks, cfg.block, 0, s>>>(g.in_ptr, g.in_col, W, buf, b->vis, pl, b->ctr);
-      k_ms_apply<<<blocks, cfg.block, 0, s>>>(nrows, N, W, b->vis, buf, alive, b->hops, b->ctr);
-      k_ms_advance<<<1, 256, 0, s>>>(W, alive, b->ctr);
-      LA3G_LAUNCHED();
-      tls_launches += 4;
-    }
-    else
-    {
-      ProfileScope p("msbfs_pull", s, 0.0);
-      LA3G_CUDA(cudaGraphLaunch(b->pull_exec, s));
-      tls_launches += 1;
-    }
-    *edges_words += (uint64_t) g.nent * W;
-    LA3G_CUDA(cudaMemcpyAsync(b->hctr, b->ctr, 4 * 8, cudaMemcpyDeviceToHost, s));
-    LA3G_CUDA(cudaStreamSynchronize(s));
-    front_bits = b->hctr[0];
-    *levels = level + 1;
-    if (front_bits == 0) return LA3G_OK;
-  }
-  *wrap = true;
+  LA3G_CUDA(cudaStreamSynchronize(s));
+  if (!b->hctr[1]) return set_error(LA3G_ETIMEOUT, "batched BFS: a grid barrier wait ran out");
+  *levels = (uint32_t) b->hctr[0];
+  *wrap = b->hctr[1] == 2;
+  *edges_words = (uint64_t) *levels * g.nent * W;
   return LA3G_OK;
 }
 
@@ -589,14 +440,92 @@ __global__ void k_bs_sinks(const uint32_t* __restrict__ ptr, const uint32_t* __r
   }
 }
 
-__global__ void k_bs_out(uint32_t N, uint32_t R, const uint32_t* __restrict__ id_of_pos, const uint32_t* __restrict__ dist,
-                         uint32_t* out)
+// Distances to out[root][id]: a block takes 32 ids and 32 roots, reads each id's
+// 128 bytes and writes runs of 128 bytes by id.
+__global__ void __launch_bounds__(256) k_bs_out(uint32_t N, uint32_t R, const uint32_t* __restrict__ pos_of_id,
+                                                const uint32_t* __restrict__ dist, uint32_t* __restrict__ out)
 {
-  const uint64_t n = (uint64_t) N * R;
-  for (uint64_t i = (uint64_t) blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t) gridDim.x * blockDim.x)
+  __shared__ uint32_t t[32][33];
+  const uint32_t tx = threadIdx.x & 31, ty = threadIdx.x >> 5, nid = (N + 31) / 32, nr = (R + 31) / 32;
+  for (uint64_t tile = blockIdx.x; tile < (uint64_t) nid * nr; tile += gridDim.x)
   {
-    const uint32_t p = (uint32_t) (i / R), r = (uint32_t) (i % R);
-    out[(uint64_t) r * N + id_of_pos[p]] = dist[i];
+    const uint32_t id0 = (uint32_t) (tile % nid) * 32, r0 = (uint32_t) (tile / nid) * 32;
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+    {
+      const uint32_t id = id0 + ty + 8 * k;
+      t[ty + 8 * k][tx] = id < N && r0 + tx < R ? dist[(uint64_t) pos_of_id[id] * R + r0 + tx] : 0u;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+    {
+      const uint32_t r = r0 + ty + 8 * k;
+      if (r < R && id0 + tx < N) out[(uint64_t) r * N + id0 + tx] = t[tx][ty + 8 * k];
+    }
+    __syncthreads();
+  }
+}
+
+struct BsArgs
+{
+  const uint32_t *ptr, *reg_end, *row, *wgt;
+  uint32_t N, R, W;
+  uint64_t* front[2];
+  PairList L[2];            // their counters: ctr[c], ctr[2 + c]
+  uint32_t* dist;
+  unsigned long long* ctr;
+  unsigned int* bar;
+  uint32_t delta;           // kNoWindow: no window
+  unsigned long long* out;  // pinned: iterations, status
+};
+
+// All iterations of a batch's SSSP: relax the listed pairs, then form the next
+// list (see lanes.cuh), a grid barrier after each.  With a window, the smallest
+// distance a list holds collects in ctr[4 + c] during the relaxation that
+// forms it and sets the next limit.
+__global__ void __launch_bounds__(256, 4) k_bs_run(BsArgs A)
+{
+  __shared__ unsigned long long s_got[3];
+  GridBarrier bar{A.bar, (int*) (A.bar + 1), kDefaultWaitPolls};
+  const uint64_t tid = (uint64_t) blockIdx.x * blockDim.x + threadIdx.x;
+  uint32_t iters = 0, limit = A.delta;
+  int cur = 0;
+  auto counts = [&]() {
+    if (threadIdx.x < 3) s_got[threadIdx.x] = __ldcg(&A.ctr[2 * threadIdx.x + cur]);
+    __syncthreads();
+  };
+  counts();
+  for (;;)
+  {
+    const unsigned long long ns = s_got[0], pk = s_got[1];
+    __syncthreads();  // s_got is free
+    if (iters > 1000000) break;
+    iters++;
+    unsigned int* pend = (unsigned int*) &A.ctr[4 + (cur ^ 1)];
+    if (tid == 0) A.ctr[cur ^ 1] = A.ctr[2 + (cur ^ 1)] = 0;  // the list formed next
+    bs_relax_all(A.ptr, A.reg_end, A.row, A.wgt, A.R, A.W, A.front[cur], A.L[cur], (uint32_t) ns, pk, A.front[cur ^ 1],
+                 A.dist, A.delta == kNoWindow ? kNoWindow : limit, A.delta == kNoWindow ? nullptr : pend);
+    if (!bar.sync()) return;
+    // every block has read this list's smallest distance: it starts over for
+    // the list after the next
+    if (tid == 0) *(unsigned int*) &A.ctr[4 + cur] = 0xFFFFFFFFu;
+    bs_apply_all(A.N, A.W, A.ptr, A.reg_end, A.front[cur ^ 1], A.L[cur ^ 1], A.front[cur], A.L[cur], ns, hub_count(pk),
+                 nullptr);
+    if (!bar.sync()) return;
+    cur ^= 1;
+    counts();
+    if (!s_got[0] && !s_got[1]) break;
+    if (A.delta != kNoWindow)
+    {
+      const uint32_t lo = (uint32_t) s_got[2];
+      limit = lo > kNoWindow - 1 - A.delta ? kNoWindow - 1 : lo + A.delta;
+    }
+  }
+  if (tid == 0)
+  {
+    A.out[0] = iters;
+    A.out[1] = iters > 1000000 ? 2 : 1;
   }
 }
 
@@ -636,15 +565,10 @@ extern "C" int la3g_bfs_batch(la3g_graph* G, const uint32_t* roots, uint32_t nro
   cudaStream_t s = G->stream;
   if (hops_out)
   {
-    // the by-id rows go into the hop array itself (N x W x 64 >= nroots x N
-    // bytes), which the next batch re-initialises
-    DevBuf tpos;
-    LA3G_TRY(tpos.alloc((size_t) nroots * N));
-    k_ms_out_pos<<<num_sms() * 8, 256, 0, s>>>(N, nroots, (nroots + 63) / 64, b->hops, tpos.as<uint8_t>());
+    LA3G_TRY(batch_out_buffer(G, b, (size_t) nroots * N));
+    k_ms_out<<<num_sms() * 8, 256, 0, s>>>(N, nroots, (nroots + 63) / 64, g.pos_of_id, b->hops, b->tpos);
     LA3G_LAUNCHED();
-    k_ms_out_id<<<num_sms() * 8, 256, 0, s>>>(N, nroots, g.pos_of_id, tpos.as<uint8_t>(), b->hops);
-    LA3G_LAUNCHED();
-    LA3G_CUDA(cudaMemcpyAsync(hops_out, b->hops, (size_t) nroots * N, cudaMemcpyDeviceToHost, s));
+    LA3G_CUDA(cudaMemcpyAsync(hops_out, b->tpos, (size_t) nroots * N, cudaMemcpyDeviceToHost, s));
     LA3G_CUDA(cudaStreamSynchronize(s));
   }
   LA3G_TRY(T.finish());
@@ -775,51 +699,40 @@ static int sssp_batch_chunk(la3g_graph* G, BatchScratch* b, const uint32_t* root
                                               b->sfront[0]);
   LA3G_LAUNCHED();
   tls_launches += 3;
-  int cur = 0;
-  uint32_t iters = 0;
   // the distance window: roots at distance <= limit relax, the rest wait;
-  // after each iteration limit = (smallest distance left in the frontier) +
-  // delta, which ctr[6] collects (atomicMin over the relax kernel's warps)
+  // after each iteration limit = (smallest distance left in the frontier) + delta
   const uint32_t delta = b->sssp_delta ? b->sssp_delta : sssp_auto_delta(b->max_w, b->max_reg_deg);
-  uint32_t limit = delta;
-  unsigned int* pend = (unsigned int*) (b->ctr + 6);
-  // two alternating pair lists; ctr[c] / ctr[2 + c] count list c's small
-  // pairs and its packed hub slots / tasks
-  PairList L[2];
-  for (int c = 0; c < 2; c++) L[c] = PairList{b->sact[c], b->shub[c], b->shub_t0[c], b->ctr + c, b->ctr + 2 + c};
+  BsArgs A;
+  A.ptr = g.out_ptr;
+  A.reg_end = b->reg_end;
+  A.row = g.out_row;
+  A.wgt = g.out_w;
+  A.N = N;
+  A.R = R;
+  A.W = W;
+  for (int c = 0; c < 2; c++)
+  {
+    A.front[c] = b->sfront[c];
+    A.L[c] = PairList{b->sact[c], b->shub[c], b->shub_t0[c], b->ctr + c, b->ctr + 2 + c};
+  }
+  A.dist = b->sdist;
+  A.ctr = b->ctr;
+  A.bar = b->bar;
+  A.delta = delta;
+  A.out = b->hctr;
+  b->hctr[1] = 0;
   LA3G_CUDA(cudaMemsetAsync(b->ctr, 0, 4 * 8, s));
-  k_bs_list<<<num_sms() * 8, 256, 0, s>>>((uint64_t) N * W, W, g.out_ptr, b->reg_end, b->sfront[0], L[0]);
+  LA3G_CUDA(cudaMemsetAsync(b->ctr + 4, 0xFF, 2 * 8, s));
+  LA3G_CUDA(cudaMemsetAsync(b->bar, 0, 8, s));
+  k_bs_list<<<num_sms() * 8, 256, 0, s>>>((uint64_t) N * W, W, g.out_ptr, b->reg_end, b->sfront[0], A.L[0]);
   LA3G_LAUNCHED();
   tls_launches++;
-  for (;;)
+  unsigned grid = 0;
+  LA3G_TRY(cooperative_blocks((const void*) k_bs_run, 256, std::max<uint64_t>((uint64_t) N * W, g.nent * 2), 4, &grid));
   {
-    if (iters > 1000000) return set_error(LA3G_ETIMEOUT, "batched sssp did not converge");
-    iters++;
-    if (delta != kNoWindow) LA3G_CUDA(cudaMemsetAsync(pend, 0xFF, 4, s));
-    {
-      ProfileScope p("sssp_batch_relax", s, 0.0);
-      k_bs_relax<<<num_sms() * 16, 256, 0, s>>>(g.out_ptr, b->reg_end, g.out_row, g.out_w, R, W, b->sfront[cur], L[cur],
-                                           b->sfront[cur ^ 1], b->sdist, delta == kNoWindow ? kNoWindow : limit,
-                                           delta == kNoWindow ? nullptr : pend);
-      LA3G_LAUNCHED();
-    }
-    LA3G_CUDA(cudaMemsetAsync(b->ctr + (cur ^ 1), 0, 8, s));
-    LA3G_CUDA(cudaMemsetAsync(b->ctr + 2 + (cur ^ 1), 0, 8, s));
-    k_bs_apply<<<num_sms() * 8, 256, 0, s>>>(N, W, g.out_ptr, b->reg_end, b->sfront[cur ^ 1], L[cur ^ 1], b->sfront[cur],
-                                        L[cur]);
-    LA3G_LAUNCHED();
-    tls_launches += 2;
-    unsigned long long act[7] = {0, 0, 0, 0, 0, 0, 0};
-    LA3G_CUDA(cudaMemcpyAsync(act, b->ctr, 7 * 8, cudaMemcpyDeviceToHost, s));
-    LA3G_CUDA(cudaStreamSynchronize(s));
-    cur ^= 1;
-    if (!act[cur] && !act[2 + cur]) break;
-    if (delta != kNoWindow)
-    {
-      uint32_t lo;
-      std::memcpy(&lo, &act[6], 4);
-      limit = lo > kNoWindow - 1 - delta ? kNoWindow - 1 : lo + delta;
-    }
+    void* args[] = {(void*) &A};
+    ProfileScope p("sssp_batch", s, 0.0);
+    LA3G_CUDA(cudaLaunchCooperativeKernel((const void*) k_bs_run, grid, 256, args, 0, s));
   }
   if (g.nsink)
   {
@@ -830,19 +743,20 @@ static int sssp_batch_chunk(la3g_graph* G, BatchScratch* b, const uint32_t* root
   }
   if (dist_out)
   {
-    DevBuf tmp;
-    LA3G_TRY(tmp.alloc((size_t) N * R * 4));
-    k_bs_out<<<num_sms() * 8, 256, 0, s>>>(N, R, g.id_of_pos, b->sdist, tmp.as<uint32_t>());
+    LA3G_TRY(batch_out_buffer(G, b, (size_t) N * R * 4));
+    k_bs_out<<<num_sms() * 8, 256, 0, s>>>(N, R, g.pos_of_id, b->sdist, (uint32_t*) b->tpos);
     LA3G_LAUNCHED();
-    LA3G_CUDA(cudaMemcpyAsync(dist_out, tmp.p, (size_t) N * R * 4, cudaMemcpyDeviceToHost, s));
-    LA3G_CUDA(cudaStreamSynchronize(s));
+    LA3G_CUDA(cudaMemcpyAsync(dist_out, b->tpos, (size_t) N * R * 4, cudaMemcpyDeviceToHost, s));
   }
-  *iters_out = iters;
+  LA3G_CUDA(cudaStreamSynchronize(s));
+  if (b->hctr[1] != 1)
+    return set_error(LA3G_ETIMEOUT, b->hctr[1] ? "batched sssp did not converge" : "batched sssp: a grid barrier wait ran out");
+  *iters_out = (uint32_t) b->hctr[0];
   return LA3G_OK;
 }
 
 // Project autotuner for the batched BFS: times every combination of level
-// mode (per-level CUDA graph / persistent kernel), block size and push
+// mode (pushing and pulling levels / pulling only), block size and push
 // threshold on the caller's roots and keeps the fastest for this graph.
 extern "C" int la3g_batch_autotune(la3g_graph* G, const uint32_t* roots, uint32_t nroots, char* report, size_t cap)
 {
@@ -860,7 +774,7 @@ extern "C" int la3g_batch_autotune(la3g_graph* G, const uint32_t* roots, uint32_
     for (int block : blocks)
       for (double frac : fracs)
       {
-        if (mode == 1 && frac != 0.0) continue;  // the persistent kernel runs pull levels only
+        if (mode == 1 && frac != 0.0) continue;  // mode 1 pulls only
         BatchConfig c;
         c.mode = mode;
         c.block = block;

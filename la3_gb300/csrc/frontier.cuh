@@ -84,6 +84,28 @@ __device__ __forceinline__ void hops_record(uint8_t* block, uint64_t nb, uint8_t
   }
 }
 
+// The same for 32 consecutive pairs, lane l's at block0 + 64 l, by the whole
+// warp: eight lanes take a pair's 64 bytes, so that a step touches 256
+// contiguous bytes (a lane per pair touches 32 separate sectors with each of
+// its eight accesses).
+__device__ __forceinline__ void hops_record_warp(uint8_t* block0, uint64_t nb, uint8_t hop, int lane)
+{
+  const unsigned any = __ballot_sync(0xffffffffu, nb != 0);
+  const uint64_t hx = 0x0101010101010101ull * hop;
+#pragma unroll
+  for (int it = 0; it < 8; it++)
+  {
+    if (!((any >> (4 * it)) & 0xFu)) continue;
+    const int src = it * 4 + (lane >> 3);
+    const uint64_t w = __shfl_sync(0xffffffffu, nb, src);
+    const uint32_t m = (uint32_t) (w >> (8 * (lane & 7))) & 0xFFu;
+    if (!m) continue;
+    uint64_t* q = reinterpret_cast<uint64_t*>(block0) + src * 8 + (lane & 7);
+    const uint64_t M = spread_bits_to_bytes(m);
+    *q = (*q & ~M) | (hx & M);
+  }
+}
+
 // Bottom-up scan of one (vertex, word) pair of a multi-source BFS: the OR of
 // the frontier words front[u W + w] over the in-neighbours u of v, stopping
 // once every bit of `want` is found.  Called by all 32 lanes of a warp with
@@ -103,7 +125,7 @@ __device__ __forceinline__ uint64_t warp_or64(uint64_t a)
 
 __device__ __forceinline__ uint64_t pull_scan(uint32_t v, uint32_t w, uint32_t W, uint64_t want,
                                               const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col,
-                                              const uint64_t* __restrict__ front, int lane)
+                                              const uint64_t* front, int lane)
 {
   uint64_t acc = 0;
   uint32_t e = 0, end = 0;

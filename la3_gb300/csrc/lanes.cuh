@@ -183,7 +183,7 @@ static __device__ __forceinline__ void bs_relax_dense(uint32_t k0, uint32_t k1, 
 // either relaxed or carried, so the shortest distances are the same.
 static __device__ __forceinline__ void bs_relax_range(uint32_t i, uint32_t k0, uint32_t k1, int lane, uint32_t R, uint32_t W,
                                                const uint32_t* __restrict__ row, const uint32_t* __restrict__ wgt,
-                                               const uint64_t* __restrict__ front, uint64_t* next, uint32_t* dist,
+                                               const uint64_t* front, uint64_t* next, uint32_t* dist,
                                                uint32_t limit, uint32_t& lmin)
 {
   const uint32_t u = i / W, w = i % W;
@@ -210,16 +210,15 @@ static __device__ __forceinline__ void bs_relax_range(uint32_t i, uint32_t k0, u
   else bs_relax_sparse(k0, k1, lane, R, W, row, wgt, u, w, f, k, next, dist, lmin);
 }
 
-static __global__ void __launch_bounds__(256, 4)
-k_bs_relax(const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ reg_end, const uint32_t* __restrict__ row,
-           const uint32_t* __restrict__ wgt, uint32_t R, uint32_t W, const uint64_t* __restrict__ front, PairList L,
-           uint64_t* next, uint32_t* dist, uint32_t limit = kNoWindow, unsigned int* pend_min = nullptr)
+static __device__ __forceinline__ void bs_relax_all(const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ reg_end,
+                                             const uint32_t* __restrict__ row, const uint32_t* __restrict__ wgt, uint32_t R,
+                                             uint32_t W, const uint64_t* front, const PairList& L, uint32_t ns,
+                                             unsigned long long pk, uint64_t* next, uint32_t* dist, uint32_t limit,
+                                             unsigned int* pend_min)
 {
   const int lane = threadIdx.x & 31;
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  const uint32_t ns = (uint32_t) *L.nsmall;
-  const unsigned long long pk = *L.packed;
   const uint32_t nbig = hub_count(pk), ntasks = hub_tasks(pk);
   uint32_t lmin = 0xFFFFFFFFu;
   for (uint32_t a = warp; a < ntasks + ns; a += nwarps)
@@ -244,16 +243,24 @@ k_bs_relax(const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ reg_en
   }
 }
 
+static __global__ void __launch_bounds__(256, 4)
+k_bs_relax(const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ reg_end, const uint32_t* __restrict__ row,
+           const uint32_t* __restrict__ wgt, uint32_t R, uint32_t W, const uint64_t* __restrict__ front, PairList L,
+           uint64_t* next, uint32_t* dist)
+{
+  bs_relax_all(ptr, reg_end, row, wgt, R, W, front, L, (uint32_t) *L.nsmall, *L.packed, next, dist, kNoWindow, nullptr);
+}
+
 // After a relaxation: the old frontier words are cleared (they become the
 // next "next" buffer) and the words holding newly lowered roots form the next
 // active list.  alive (W words, optional) collects the roots that still have
 // a frontier.
-static __global__ void k_bs_apply(uint32_t N, uint32_t W, const uint32_t* __restrict__ ptr,
-                                  const uint32_t* __restrict__ reg_end, const uint64_t* __restrict__ next,
-                                  PairList out, uint64_t* front_old, PairList old, uint64_t* alive = nullptr)
+static __device__ __forceinline__ void bs_apply_all(uint32_t N, uint32_t W, const uint32_t* __restrict__ ptr,
+                                             const uint32_t* __restrict__ reg_end, const uint64_t* next,
+                                             const PairList& out, uint64_t* front_old, const PairList& old, uint64_t ns,
+                                             uint64_t nb, uint64_t* alive)
 {
   const uint64_t tid = (uint64_t) blockIdx.x * blockDim.x + threadIdx.x, nth = (uint64_t) gridDim.x * blockDim.x;
-  const uint64_t ns = *old.nsmall, nb = hub_count(*old.packed);
   for (uint64_t k = tid; k < ns; k += nth) front_old[old.small[k]] = 0;
   for (uint64_t k = tid; k < nb; k += nth) front_old[old.hub[k]] = 0;
   const uint64_t NW = (uint64_t) N * W;
@@ -267,19 +274,24 @@ static __global__ void k_bs_apply(uint32_t N, uint32_t W, const uint32_t* __rest
   }
 }
 
+static __global__ void k_bs_apply(uint32_t N, uint32_t W, const uint32_t* __restrict__ ptr,
+                                  const uint32_t* __restrict__ reg_end, const uint64_t* __restrict__ next,
+                                  PairList out, uint64_t* front_old, PairList old, uint64_t* alive)
+{
+  bs_apply_all(N, W, ptr, reg_end, next, out, front_old, old, *old.nsmall, hub_count(*old.packed), alive);
+}
+
 // Top-down step of a multi-source BFS over a split list of frontier
 // (vertex, word) pairs (small pairs a warp each, hub edges as kHubTask-edge
 // tasks): each edge's target gets the word's bits that it has not visited,
 // ORed into its next word (skipped when already there).
 static __device__ __forceinline__ void ms_push_pairs(const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col,
-                                                     uint32_t W, const uint64_t* __restrict__ front,
-                                                     const uint64_t* __restrict__ vis, uint64_t* next, const PairList& L)
+                                                     uint32_t W, const uint64_t* front, const uint64_t* vis, uint64_t* next,
+                                                     const PairList& L, uint32_t ns, unsigned long long pk)
 {
   const int lane = threadIdx.x & 31;
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  const uint32_t ns = (uint32_t) *L.nsmall;
-  const unsigned long long pk = *L.packed;
   const uint32_t nbig = hub_count(pk), ntasks = hub_tasks(pk);
   for (uint32_t a = warp; a < ntasks + ns; a += nwarps)
   {

@@ -160,7 +160,7 @@ __global__ void k_lb_list(uint64_t NW, uint32_t W, const uint32_t* __restrict__ 
 __global__ void k_lb_push(const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col, uint32_t W,
                           const uint64_t* __restrict__ front, const uint64_t* __restrict__ vis, uint64_t* next, PairList list)
 {
-  ms_push_pairs(ptr, col, W, front, vis, next, list);
+  ms_push_pairs(ptr, col, W, front, vis, next, list, (uint32_t) *list.nsmall, *list.packed);
 }
 
 // After a push: new bits = next & ~visited; the old frontier words of the
