@@ -487,10 +487,12 @@ struct BsArgs
 __global__ void __launch_bounds__(256, 4) k_bs_run(BsArgs A)
 {
   __shared__ unsigned long long s_got[3];
+  __shared__ unsigned int s_taken;
   GridBarrier bar{A.bar, (int*) (A.bar + 1), kDefaultWaitPolls};
   const uint64_t tid = (uint64_t) blockIdx.x * blockDim.x + threadIdx.x;
   uint32_t iters = 0, limit = A.delta;
   int cur = 0;
+  if (threadIdx.x == 0) s_taken = 0;
   auto counts = [&]() {
     if (threadIdx.x < 3) s_got[threadIdx.x] = __ldcg(&A.ctr[2 * threadIdx.x + cur]);
     __syncthreads();
@@ -505,11 +507,12 @@ __global__ void __launch_bounds__(256, 4) k_bs_run(BsArgs A)
     unsigned int* pend = (unsigned int*) &A.ctr[4 + (cur ^ 1)];
     if (tid == 0) A.ctr[cur ^ 1] = A.ctr[2 + (cur ^ 1)] = 0;  // the list formed next
     bs_relax_all(A.ptr, A.reg_end, A.row, A.wgt, A.R, A.W, A.front[cur], A.L[cur], (uint32_t) ns, pk, A.front[cur ^ 1],
-                 A.dist, A.delta == kNoWindow ? kNoWindow : limit, A.delta == kNoWindow ? nullptr : pend);
+                 A.dist, A.delta == kNoWindow ? kNoWindow : limit, A.delta == kNoWindow ? nullptr : pend, &s_taken);
     if (!bar.sync()) return;
     // every block has read this list's smallest distance: it starts over for
     // the list after the next
     if (tid == 0) *(unsigned int*) &A.ctr[4 + cur] = 0xFFFFFFFFu;
+    if (threadIdx.x == 0) s_taken = 0;
     bs_apply_all(A.N, A.W, A.ptr, A.reg_end, A.front[cur ^ 1], A.L[cur ^ 1], A.front[cur], A.L[cur], ns, hub_count(pk),
                  nullptr);
     if (!bar.sync()) return;
@@ -586,6 +589,14 @@ extern "C" int la3g_bfs_batch(la3g_graph* G, const uint32_t* roots, uint32_t nro
   return LA3G_OK;
 }
 
+// Distances (vertices x roots of a chunk) up to which the iterations run in one
+// kernel.  There the host's round trips weigh most (ER 50k, 64 roots: 0.95 ms
+// against 1.72; R-MAT 2^19, 64 roots: 3.4 against 3.9); with more, distances
+// miss the L2 cache and the four-fold grid of a launch per iteration keeps more
+// warps ready than the resident one (R-MAT 2^22, 16 roots: 9.2 ms against 10.2;
+// ER 2^22, 64 roots: 64 against 79).
+static constexpr uint64_t kBsOneKernel = 40ull << 20;
+
 static constexpr uint32_t kSsspChunk = 256;  // roots per device pass (bounds the [N][R] state)
 
 // Default window width of the batched SSSP.  The window pays where degrees
@@ -638,6 +649,39 @@ extern "C" int la3g_sssp_batch(la3g_graph* G, const uint32_t* roots, uint32_t nr
   LA3G_TRY(T.finish());
   if (st) st->iterations = iters;
   return LA3G_OK;
+}
+
+// The iterations of k_bs_run stepped from the host.
+static int bs_stepped(la3g_graph* G, BatchScratch* b, const BsArgs& A)
+{
+  cudaStream_t s = G->stream;
+  int cur = 0;
+  uint32_t limit = A.delta;
+  for (uint32_t iters = 1;; iters++)
+  {
+    unsigned int* pend = A.delta == kNoWindow ? nullptr : (unsigned int*) (b->ctr + 4);
+    if (pend) LA3G_CUDA(cudaMemsetAsync(pend, 0xFF, 4, s));
+    {
+      ProfileScope p("sssp_batch_relax", s, 0.0);
+      k_bs_relax<<<num_sms() * 16, 256, 0, s>>>(A.ptr, A.reg_end, A.row, A.wgt, A.R, A.W, A.front[cur], A.L[cur],
+                                                A.front[cur ^ 1], A.dist, pend ? limit : kNoWindow, pend);
+      LA3G_LAUNCHED();
+    }
+    LA3G_CUDA(cudaMemsetAsync(b->ctr + (cur ^ 1), 0, 8, s));
+    LA3G_CUDA(cudaMemsetAsync(b->ctr + 2 + (cur ^ 1), 0, 8, s));
+    k_bs_apply<<<num_sms() * 8, 256, 0, s>>>(A.N, A.W, A.ptr, A.reg_end, A.front[cur ^ 1], A.L[cur ^ 1], A.front[cur], A.L[cur]);
+    LA3G_LAUNCHED();
+    tls_launches += 2;
+    unsigned long long act[5] = {0, 0, 0, 0, 0};
+    LA3G_CUDA(cudaMemcpyAsync(act, b->ctr, 5 * 8, cudaMemcpyDeviceToHost, s));
+    LA3G_CUDA(cudaStreamSynchronize(s));
+    cur ^= 1;
+    b->hctr[0] = iters;
+    b->hctr[1] = iters > 1000000 ? 2 : 1;
+    if ((!act[cur] && !act[2 + cur]) || iters > 1000000) return LA3G_OK;
+    const uint32_t lo = (uint32_t) act[4];
+    if (pend) limit = lo > kNoWindow - 1 - A.delta ? kNoWindow - 1 : lo + A.delta;
+  }
 }
 
 static int sssp_batch_chunk(la3g_graph* G, BatchScratch* b, const uint32_t* roots, uint32_t R, uint32_t* dist_out,
@@ -727,13 +771,15 @@ static int sssp_batch_chunk(la3g_graph* G, BatchScratch* b, const uint32_t* root
   k_bs_list<<<num_sms() * 8, 256, 0, s>>>((uint64_t) N * W, W, g.out_ptr, b->reg_end, b->sfront[0], A.L[0]);
   LA3G_LAUNCHED();
   tls_launches++;
-  unsigned grid = 0;
-  LA3G_TRY(cooperative_blocks((const void*) k_bs_run, 256, std::max<uint64_t>((uint64_t) N * W, g.nent * 2), 4, &grid));
+  if ((uint64_t) N * R <= kBsOneKernel)
   {
+    unsigned grid = 0;
+    LA3G_TRY(cooperative_blocks((const void*) k_bs_run, 256, std::max<uint64_t>((uint64_t) N * W, g.nent * 2), 4, &grid));
     void* args[] = {(void*) &A};
     ProfileScope p("sssp_batch", s, 0.0);
     LA3G_CUDA(cudaLaunchCooperativeKernel((const void*) k_bs_run, grid, 256, args, 0, s));
   }
+  else LA3G_TRY(bs_stepped(G, b, A));
   if (g.nsink)
   {
     k_bs_sinks<<<num_sms() * 8, 256, 0, s>>>(g.in_ptr, g.in_col, g.in_w, g.nreg, g.nsink, R, b->rpos, g.src_base(),

@@ -214,15 +214,26 @@ static __device__ __forceinline__ void bs_relax_all(const uint32_t* __restrict__
                                              const uint32_t* __restrict__ row, const uint32_t* __restrict__ wgt, uint32_t R,
                                              uint32_t W, const uint64_t* front, const PairList& L, uint32_t ns,
                                              unsigned long long pk, uint64_t* next, uint32_t* dist, uint32_t limit,
-                                             unsigned int* pend_min)
+                                             unsigned int* pend_min, unsigned int* taken)
 {
   const int lane = threadIdx.x & 31;
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
   const uint32_t nbig = hub_count(pk), ntasks = hub_tasks(pk);
   uint32_t lmin = 0xFFFFFFFFu;
-  for (uint32_t a = warp; a < ntasks + ns; a += nwarps)
+  // with `taken` (the block's, zero at the start) a block's warps take its items,
+  // every gridDim-th one, as they come free: hubs' neighbours differ in cost too
+  // much for fixed shares, and one counter for the whole grid is too slow
+  const uint32_t total = ntasks + ns;
+  for (uint32_t a = warp;; a += nwarps)
   {
+    if (taken)
+    {
+      uint32_t k = 0;
+      if (lane == 0) k = atomicAdd(taken, 1u);
+      a = blockIdx.x + gridDim.x * __shfl_sync(0xffffffffu, k, 0);
+    }
+    if (a >= total) break;
     if (a < ntasks)
     {
       const uint32_t slot = hub_of_task(L.hub_t0, nbig, a);
@@ -246,9 +257,10 @@ static __device__ __forceinline__ void bs_relax_all(const uint32_t* __restrict__
 static __global__ void __launch_bounds__(256, 4)
 k_bs_relax(const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ reg_end, const uint32_t* __restrict__ row,
            const uint32_t* __restrict__ wgt, uint32_t R, uint32_t W, const uint64_t* __restrict__ front, PairList L,
-           uint64_t* next, uint32_t* dist)
+           uint64_t* next, uint32_t* dist, uint32_t limit = kNoWindow, unsigned int* pend_min = nullptr)
 {
-  bs_relax_all(ptr, reg_end, row, wgt, R, W, front, L, (uint32_t) *L.nsmall, *L.packed, next, dist, kNoWindow, nullptr);
+  bs_relax_all(ptr, reg_end, row, wgt, R, W, front, L, (uint32_t) *L.nsmall, *L.packed, next, dist, limit, pend_min,
+               nullptr);
 }
 
 // After a relaxation: the old frontier words are cleared (they become the
@@ -276,7 +288,7 @@ static __device__ __forceinline__ void bs_apply_all(uint32_t N, uint32_t W, cons
 
 static __global__ void k_bs_apply(uint32_t N, uint32_t W, const uint32_t* __restrict__ ptr,
                                   const uint32_t* __restrict__ reg_end, const uint64_t* __restrict__ next,
-                                  PairList out, uint64_t* front_old, PairList old, uint64_t* alive)
+                                  PairList out, uint64_t* front_old, PairList old, uint64_t* alive = nullptr)
 {
   bs_apply_all(N, W, ptr, reg_end, next, out, front_old, old, *old.nsmall, hub_count(*old.packed), alive);
 }
