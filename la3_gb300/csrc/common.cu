@@ -123,11 +123,6 @@ ProfileScope::~ProfileScope()
 
 bool profile_enabled() { return prof_on; }
 
-DeviceLoop::~DeviceLoop()
-{
-  if (exec) cudaGraphExecDestroy(exec);
-}
-
 void profile_add_bytes(const char* name, double bytes)
 {
   if (!prof_on) return;

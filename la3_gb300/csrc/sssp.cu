@@ -19,10 +19,18 @@
 // activated; INF if never): one dense pass over the regular rows after each
 // iteration finds those rows, scatters their new distance and forms the next
 // frontier, so the relaxations themselves only do a non-returning atomicMin.
+//
+// All iterations run in one cooperative kernel with a grid barrier between its
+// phases; every block decides for itself, from counters in global memory,
+// whether an iteration pushes or pulls.  (As a graph with conditional nodes an
+// iteration was five launches, 18 us on a graph whose iterations take a few us
+// of work.)
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
 #include <vector>
+
+#include <cub/device/device_radix_sort.cuh>
 
 #include "frontier.cuh"
 #include "la3g_internal.h"
@@ -30,168 +38,76 @@
 namespace la3g {
 
 static constexpr uint32_t kInf = 0x7FFFFFFFu;
-static constexpr uint32_t kPullLong = 64;     // pull rows longer than this are cut into tasks
+static constexpr uint32_t kPullLong = 256;    // pull rows longer than this are cut into tasks
 static constexpr uint32_t kPullChunk = 512;   // in-edges per long-row task (one warp)
 static constexpr uint32_t kPullLanes = 4;     // lanes per short row in a pull step
 
-// The frontier is two lists: vertices with at most kBigDeg out-edges into
-// regular rows (one warp each) and hubs (their edges shared by the grid).
-struct SsspScratch
+struct SsspCounters  // what an iteration activates
 {
-  uint32_t* dist = nullptr;
-  uint32_t* msg = nullptr;        // the distance each vertex scattered at its last activation (INF if never)
-  uint32_t* reg_end = nullptr;   // [nslots] end of each vertex's out-edges into regular rows
-  uint32_t* small[1] = {nullptr};      // push steps: the frontier's split lists
-  uint32_t* big[1] = {nullptr};
-  uint32_t* big_task0[1] = {nullptr};
-  // [0] activated count, [1] their regular out-degree sum, [2] activated with regular out-edges,
-  // [3] scratch, [4] scratch, [5] the next frontier's smallest message
-  unsigned long long* ctr = nullptr;
-  unsigned long long* hctr = nullptr;
-  uint32_t* fbits = nullptr;      // [nslots / 32 + 1] the current frontier, one bit per vertex
-  unsigned long long* fctr = nullptr;  // push steps: [0] small-list length, [1] hub slots and tasks
-  uint32_t* fmsg = nullptr;       // pull steps: msg of the current frontier's vertices, INF elsewhere
-  uint32_t* long_rows = nullptr;  // regular rows with more than kPullLong in-edges
-  uint32_t nlong = 0;
-  uint32_t* task_row = nullptr;   // pull tasks over the long rows: kPullChunk in-edges each
-  uint32_t* task_begin = nullptr;
-  uint32_t ntasks = 0;
-  uint64_t task_edges = 0;        // in-edges of the long rows
-  uint32_t* ymin = nullptr;       // [nlong] partial minima of the long rows (INF between steps)
-  uint64_t reg_in = 0;            // in-edges of the regular rows
-  uint32_t max_w = 0;             // largest weight: pull steps need INF + w to stay in uint32
-  uint32_t min_w = 0;             // smallest weight of a regular row's in-edge
-  uint32_t* by_id = nullptr;      // [nslots] distances reordered by id before they leave the device
-  unsigned long long* state = nullptr;  // the iteration loop's state (kSt* slots), device side
-  DeviceLoop* loop = nullptr;     // the device-driven loop graph (built on first use)
+  unsigned long long count, deg, out, fmin;  // vertices, their regular out-degrees' sum, those that have any, smallest message
 };
 
-// Loop state slots (unsigned long long each).
-enum : int {
-  kStIter = 0,      // iterations, counted as the reference counts them
-  kStExamined,      // edges relaxed or gathered
-  kStStatus,        // 1: the iteration limit was reached
-  kStFirst,         // 1 until the first decision (the root's frontier is in kStNlist0 / kStDeg0)
-  kStNlist0,        // the root's frontier: 1 if it scatters
-  kStDeg0,          // the root's regular out-degree
-  kStMode,          // the body chosen last: kPull, kPush or kDone
-  kStSrcRoot,       // the root's position if it is a source (the sink pass reads it), else ~0
-  kStFrontDeg,      // the chosen step's frontier out-degree sum
-  kStNlist,         // the chosen step's frontier: vertices with regular out-edges
-  kStPulls,         // pull steps run
-  kStPushes,        // push steps run
-  kStFmin,          // the chosen step's frontier minimum (what the pull's settled test reads)
-  kStSlots = 16
+struct SsspStats  // pinned, written by the kernel at its end
+{
+  unsigned long long iterations, examined, status, reached_deg;
 };
-enum : unsigned { kPull = 0, kPush = 1, kDone = 2 };
+static constexpr unsigned long long kSsspRunning = 2;  // status until the kernel has ended properly
+
+struct SsspArgs
+{
+  // the graph: push CSR (regular rows first, up to reg_end), pull CSR (offsets
+  // of all rows; columns and weights are read for the sinks only)
+  const uint32_t *out_ptr, *out_row, *out_w, *reg_end, *in_ptr, *in_col, *in_w, *pos_of_id;
+  uint32_t N, nreg, nsink, src_base, iso_base;
+  uint64_t reg_in;                // in-edges of the regular rows
+  uint32_t min_w, max_w;          // pull steps need INF + max_w to stay in uint32
+  uint64_t limit;                 // most iterations
+  // pull steps: the regular rows' entries, slot of the column and weight, each
+  // row in ascending order of weight >> wshift.  Slots number the columns by
+  // descending out-degree: the hot ones' messages share sectors.
+  const uint32_t* slot;
+  const uint2* entry;
+  int wshift;
+  // rows with more than kPullLong in-edges, cut into tasks of kPullChunk
+  const uint32_t *task_row, *task_begin;  // row; [begins | ends]
+  uint32_t ntasks;
+  uint32_t* dist;
+  uint32_t* msg;                  // the distance each vertex scattered at its last activation (INF if never)
+  uint32_t* fmsg;                 // by slot: msg of the frontier a pull step reads, INF elsewhere
+  uint32_t *fbits, *pbits;        // the current frontier; the one fmsg holds
+  // push steps: the frontier's lists, vertices with at most kBigDeg regular
+  // out-edges (one warp each) and hubs (their edges shared by the grid)
+  uint32_t *small, *big, *big_task0;
+  unsigned long long* fctr;       // [0] small-list length, [1] hub slots and tasks
+  SsspCounters* ctr;              // [3]
+  unsigned long long* reached;
+  unsigned int* bar;
+  uint32_t root;
+  uint32_t* dist_out;             // by id, or null
+  SsspStats* stats;
+};
+
+struct SsspScratch
+{
+  SsspArgs A{};
+  SsspStats* stats = nullptr;     // pinned
+  uint32_t* by_id = nullptr;      // [nslots] distances reordered by id before they leave the device
+  uint32_t* reg_end = nullptr;    // [nslots] end of each vertex's out-edges into regular rows
+  uint32_t* long_rows = nullptr;
+  uint32_t nlong = 0;
+  uint32_t* slot = nullptr;
+  uint2* entry = nullptr;
+  uint64_t reg_in = 0;
+  uint32_t max_w = 0, min_w = 0;  // largest weight; smallest of a regular row's in-edge
+  int wshift = 0;
+  unsigned grid = 0;
+};
 
 static void sssp_scratch_free(void* p)
 {
   SsspScratch* s = (SsspScratch*) p;
-  if (s->hctr) cudaFreeHost(s->hctr);
-  delete s->loop;
+  if (s->stats) cudaFreeHost(s->stats);
   delete s;
-}
-
-__global__ void k_sssp_init(uint32_t N, uint32_t* dist, uint32_t* msg, uint32_t* fmsg)
-{
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < N; p += gridDim.x * blockDim.x)
-  {
-    dist[p] = kInf;
-    msg[p] = kInf;
-    fmsg[p] = kInf;
-  }
-}
-
-// The root (an id; none if it is outside the graph): distance 0, scattered
-// (msg 0); regular and source vertices scatter, so they form the first
-// frontier (even with no regular out-edge: the first iteration runs).
-__global__ void k_sssp_root(uint32_t root, uint32_t N, const uint32_t* __restrict__ pos_of_id,
-                            const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ reg_end, uint32_t nreg,
-                            uint32_t src_base, uint32_t iso_base, uint32_t* dist, uint32_t* msg, uint32_t* fbits,
-                            unsigned long long* state)
-{
-  for (int k = 0; k < kStSlots; k++) state[k] = 0;
-  state[kStFirst] = 1;
-  state[kStSrcRoot] = ~0ull;
-  if (root >= N) return;
-  const uint32_t rp = pos_of_id[root];
-  const bool src = rp >= src_base && rp < iso_base;
-  dist[rp] = 0;
-  msg[rp] = 0;
-  if (src) state[kStSrcRoot] = rp;
-  if (rp < nreg || src)
-  {
-    fbits[rp >> 5] = 1u << (rp & 31);
-    state[kStNlist0] = 1;
-    state[kStDeg0] = reg_end[rp] - ptr[rp];
-  }
-}
-
-// Start of every iteration (one thread): reads the counters the last dense
-// apply left (or the root's frontier), ends the loop as the reference's
-// execute loop does (nothing activated; or activated vertices with no
-// regular out-edge, which take one more, empty iteration), and otherwise
-// counts the iteration and picks pull (frontier out-degree sum above the
-// regular rows' in-edges / divisor, after the first iteration, with weights
-// that keep INF + w in uint32) or push.
-// It also clears the counters the step's kernels accumulate into (the dense
-// apply's, keeping the frontier minimum for the pull in the state; the push
-// split's), so that no memset node sits between the iterations.
-__global__ void k_sssp_decide(unsigned long long* state, unsigned long long* ctr, unsigned long long* fctr,
-                              uint64_t reg_in, uint32_t max_w, double divisor, uint64_t limit,
-                              cudaGraphConditionalHandle cont, cudaGraphConditionalHandle mode)
-{
-  unsigned long long it = state[kStIter], nlist, deg;
-  bool done = false;
-  if (state[kStFirst])
-  {
-    state[kStFirst] = 0;
-    nlist = state[kStNlist0];
-    deg = state[kStDeg0];
-  }
-  else
-  {
-    deg = ctr[1];
-    nlist = ctr[2];
-    if (ctr[0] == 0) done = true;
-    else if (nlist == 0)
-    {
-      it++;  // the next iteration runs with messages that reach no regular row
-      done = true;
-    }
-  }
-  unsigned m = kDone;
-  if (!done)
-  {
-    if (it > limit) state[kStStatus] = 1;
-    else
-    {
-      it++;
-      if (nlist)
-        m = it > 1 && max_w <= 0x80000000u && (double) deg * divisor > (double) reg_in ? kPull : kPush;
-    }
-  }
-  state[kStIter] = it;
-  state[kStMode] = m;
-  state[kStFrontDeg] = deg;
-  state[kStNlist] = nlist;
-  state[kStFmin] = ctr[5];
-  ctr[0] = ctr[1] = ctr[2] = 0;
-  ctr[5] = ~0ull;  // the next frontier's minimum
-  fctr[0] = fctr[1] = 0;
-  if (m == kPull)
-  {
-    state[kStExamined] += reg_in;
-    state[kStPulls]++;
-  }
-  else if (m == kPush)
-  {
-    state[kStExamined] += deg;
-    state[kStPushes]++;
-  }
-  loop_set(cont, m != kDone);
-  loop_set(mode, m);
 }
 
 // End of the regular-row part of every out-edge list (rows ascend, so the
@@ -221,64 +137,47 @@ __device__ __forceinline__ void relax(uint32_t v, uint32_t cand, bool valid, uin
 // edges), then one warp per small vertex.  Messages are the distances the
 // frontier vertices held when they were activated (msg), as the reference's
 // scatter values are.
-__global__ void __launch_bounds__(256)
-k_sssp_push(const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ reg_end, const uint32_t* __restrict__ row,
-            const uint32_t* __restrict__ w, const uint32_t* __restrict__ small, const uint32_t* __restrict__ big,
-            const uint32_t* __restrict__ big_task0, const unsigned long long* __restrict__ fctr,
-            const uint32_t* __restrict__ msg, uint32_t* dist)
+__device__ __forceinline__ void sssp_push(const SsspArgs& A, uint32_t nsmall, unsigned long long packed, uint32_t warp,
+                                          uint32_t nwarps, uint32_t lane)
 {
-  const uint32_t nsmall = (uint32_t) fctr[0];
-  const uint32_t nbig = hub_count(fctr[1]), ntasks = hub_tasks(fctr[1]);
-  const int lane = threadIdx.x & 31;
-  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+  const uint32_t nbig = hub_count(packed), ntasks = hub_tasks(packed);
   for (uint32_t t = warp; t < ntasks; t += nwarps)
   {
-    const uint32_t slot = hub_of_task(big_task0, nbig, t);
-    const uint32_t u = big[slot];
-    const uint32_t mu = msg[u];
-    const uint32_t b = ptr[u] + (t - big_task0[slot]) * kHubTask;
-    const uint32_t e = min(b + kHubTask, reg_end[u]);
-    for (uint32_t i = b + lane; i < e; i += 32) relax(row[i], mu + w[i], true, dist);
+    const uint32_t slot = hub_of_task(A.big_task0, nbig, t);
+    const uint32_t u = A.big[slot], mu = A.msg[u];
+    const uint32_t b = A.out_ptr[u] + (t - A.big_task0[slot]) * kHubTask;
+    const uint32_t e = min(b + kHubTask, A.reg_end[u]);
+    for (uint32_t i = b + lane; i < e; i += 32) relax(__ldg(&A.out_row[i]), mu + __ldg(&A.out_w[i]), true, A.dist);
   }
   for (uint32_t f = warp; f < nsmall; f += nwarps)
   {
-    const uint32_t u = small[f];
-    const uint32_t mu = msg[u];
-    const uint32_t b = ptr[u], e = reg_end[u];
-    for (uint32_t i = b + lane; i < e; i += 32) relax(row[i], mu + w[i], true, dist);
+    const uint32_t u = A.small[f], mu = A.msg[u];
+    const uint32_t b = A.out_ptr[u], e = A.reg_end[u];
+    for (uint32_t i = b + lane; i < e; i += 32) relax(__ldg(&A.out_row[i]), mu + __ldg(&A.out_w[i]), true, A.dist);
   }
 }
 
 // After an iteration: the regular rows whose distance fell below their
 // message were activated.  They scatter (msg = dist) and form the next
-// frontier: one bit per vertex (a warp writes a whole word, so every word of
-// the bitmap is rewritten) and the pull step's message array (fmsg: msg for
-// the frontier, INF elsewhere); the counters get the frontier's size, its
-// regular out-degree sum, how many of it have regular out-edges, and its
-// smallest message.
-__global__ void __launch_bounds__(256)
-k_sssp_dense_apply(uint32_t nreg, uint32_t words, const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ reg_end,
-                   const uint32_t* __restrict__ dist, uint32_t* msg, uint32_t* fmsg, uint32_t* fbits,
-                   unsigned long long* ctr)
+// frontier, one bit per vertex (a warp writes a whole word, so every word of
+// the bitmap is rewritten); the counters describe it.
+__device__ __forceinline__ void sssp_dense_apply(const SsspArgs& A, uint32_t words, SsspCounters* ctr, uint32_t warp,
+                                                 uint32_t nwarps, uint32_t lane)
 {
-  const uint32_t lane = threadIdx.x & 31;
-  unsigned long long deg = 0, cnt = 0, out = 0;
-  uint32_t fmin = 0xFFFFFFFFu;
-  const uint32_t nth = gridDim.x * blockDim.x;
-  for (uint32_t v0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); v0 < words * 32u; v0 += nth)
+  unsigned long long deg = 0;
+  uint32_t cnt = 0, out = 0, fmin = 0xFFFFFFFFu;
+  for (uint32_t w = warp; w < words; w += nwarps)
   {
-    const uint32_t v = v0 + lane;
+    const uint32_t v = w * 32 + lane;
     bool act = false;
-    if (v < nreg)
+    if (v < A.nreg)
     {
-      const uint32_t dv = dist[v];
-      act = dv < msg[v];
-      fmsg[v] = act ? dv : kInf;
+      const uint32_t dv = A.dist[v];
+      act = dv < A.msg[v];
       if (act)
       {
-        msg[v] = dv;
-        const uint32_t d = reg_end[v] - ptr[v];
+        A.msg[v] = dv;
+        const uint32_t d = A.reg_end[v] - A.out_ptr[v];
         deg += d;
         cnt++;
         out += d != 0;
@@ -286,40 +185,51 @@ k_sssp_dense_apply(uint32_t nreg, uint32_t words, const uint32_t* __restrict__ p
       }
     }
     const unsigned m = __ballot_sync(0xffffffffu, act);
-    if (lane == 0) fbits[v0 >> 5] = m;
+    if (lane == 0) A.fbits[w] = m;
   }
-  cnt = block_sum_u64(cnt);
+  const unsigned long long co = block_sum_u64((unsigned long long) cnt << 32 | out);
   deg = block_sum_u64(deg);
-  out = block_sum_u64(out);
   fmin = block_min_u32(fmin);
-  if (threadIdx.x == 0)
+  if (threadIdx.x == 0 && co)
   {
-    if (cnt) atomicAdd(&ctr[0], cnt);
-    if (deg) atomicAdd(&ctr[1], deg);
-    if (out) atomicAdd(&ctr[2], out);
-    if (fmin != 0xFFFFFFFFu) atomicMin(&ctr[5], (unsigned long long) fmin);
+    atomicAdd(&ctr->count, co >> 32);
+    atomicAdd(&ctr->out, co & 0xFFFFFFFFull);
+    if (deg) atomicAdd(&ctr->deg, deg);
+    atomicMin(&ctr->fmin, (unsigned long long) fmin);
+  }
+}
+
+// Pull steps only: the frontier's messages by slot, INF again for the frontier
+// of the last pull step.
+__device__ __forceinline__ void sssp_front(const SsspArgs& A, uint32_t words, uint32_t warp, uint32_t nwarps, uint32_t lane)
+{
+  for (uint32_t w = warp; w < words; w += nwarps)
+  {
+    const uint32_t now = A.fbits[w], was = A.pbits[w];
+    if ((now | was) >> lane & 1)
+    {
+      const uint32_t v = w * 32 + lane;
+      A.fmsg[A.slot[v]] = now >> lane & 1 ? A.msg[v] : kInf;
+    }
+    __syncwarp();
+    if (lane == 0 && now != was) A.pbits[w] = now;
   }
 }
 
 // Push steps only: the frontier bitmap into the split lists (vertices with
 // up to kBigDeg regular out-edges, appended a warp at a time; hubs with their
 // edge tasks).
-__global__ void __launch_bounds__(256)
-k_sssp_split(const uint32_t* __restrict__ fbits, uint32_t words, const uint32_t* __restrict__ ptr,
-             const uint32_t* __restrict__ reg_end, uint32_t* small, uint32_t* big, uint32_t* big_task0,
-             unsigned long long* fctr)
+__device__ __forceinline__ void sssp_split(const SsspArgs& A, uint32_t words, uint32_t warp, uint32_t nwarps, uint32_t lane)
 {
-  const uint32_t lane = threadIdx.x & 31;
-  const uint32_t nth = gridDim.x * blockDim.x;
-  for (uint32_t w0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); w0 < words; w0 += nth)
+  for (uint32_t w0 = warp * 32; w0 < words; w0 += nwarps * 32)
   {
     const uint32_t w = w0 + lane;
-    uint32_t bits = w < words ? fbits[w] : 0u, c = 0;
+    uint32_t bits = w < words ? A.fbits[w] : 0u, c = 0;
     for (uint32_t x = bits; x; x &= x - 1)
     {
       const uint32_t v = w * 32 + (__ffs(x) - 1);
-      const uint32_t d = reg_end[v] - ptr[v];
-      if (d > kBigDeg) hub_append(v, d, big, big_task0, &fctr[1]);
+      const uint32_t d = A.reg_end[v] - A.out_ptr[v];
+      if (d > kBigDeg) hub_append(v, d, A.big, A.big_task0, &A.fctr[1]);
       else c += d != 0;
     }
     uint32_t incl = c;
@@ -331,13 +241,13 @@ k_sssp_split(const uint32_t* __restrict__ fbits, uint32_t words, const uint32_t*
     const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
     if (!total) continue;
     uint32_t base = 0;
-    if (lane == 31) base = (uint32_t) atomicAdd(&fctr[0], (unsigned long long) total);
+    if (lane == 31) base = (uint32_t) atomicAdd(&A.fctr[0], (unsigned long long) total);
     base = __shfl_sync(0xffffffffu, base, 31) + incl - c;
     for (uint32_t x = bits; x; x &= x - 1)
     {
       const uint32_t v = w * 32 + (__ffs(x) - 1);
-      const uint32_t d = reg_end[v] - ptr[v];
-      if (d && d <= kBigDeg) small[base++] = v;
+      const uint32_t d = A.reg_end[v] - A.out_ptr[v];
+      if (d && d <= kBigDeg) A.small[base++] = v;
     }
   }
 }
@@ -348,98 +258,111 @@ k_sssp_split(const uint32_t* __restrict__ fbits, uint32_t words, const uint32_t*
 // that lowers it.  fmsg holds msg for the frontier and INF for every other
 // vertex, so each edge is one load and one add: INF + w (w <= 2^31) stays
 // above INF in uint32 and never lowers a row.  Short rows are owned by one
-// lane group and long rows are cut into tasks whose minima meet in ymin,
-// so dist needs no atomics; fmsg is not written while the step runs.
+// lane group, long rows are cut into tasks that lower the row's distance by
+// atomicMin; the messages are not written while the step runs.
 // Sources are frontier vertices only in the first iteration, which always
 // pushes.
-__device__ __forceinline__ void sssp_pull_edge(uint32_t e, const uint32_t* __restrict__ col,
-                                               const uint32_t* __restrict__ w, const uint32_t* __restrict__ fmsg,
-                                               uint32_t& y)
+//
+// Every candidate of a step is at least the frontier's smallest message plus
+// its edge's weight, and a row's entries ascend by weight (exactly, or by its
+// leading bits), so a row is done as soon as that sum reaches what it already
+// has: most of its edges' messages, random reads that bound the step at 240 G a
+// second however they are arranged, are never read.  R-MAT 2^22: the five pulls
+// of a call 1343 us over the CSR by position, 1095 with the messages by slot,
+// 486 with the rows by weight.
+__device__ __forceinline__ bool sssp_past(unsigned long long fmin, uint32_t w, int wshift, uint32_t have)
 {
-  y = min(y, fmsg[col[e]] + w[e]);
+  return fmin + ((w >> wshift) << wshift) >= have;
 }
 
-__global__ void __launch_bounds__(256)
-k_sssp_pull(const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col, const uint32_t* __restrict__ w,
-            uint32_t nreg, const uint32_t* __restrict__ task_row, const uint32_t* __restrict__ task_begin,
-            uint32_t ntasks, uint32_t task_warps, uint32_t* ymin, const uint32_t* __restrict__ fmsg,
-            uint32_t* dist, const uint32_t* __restrict__ long_rows, const unsigned long long* __restrict__ fmin_ptr,
-            uint32_t min_w)
+__global__ void k_sssp_slot_keys(const uint32_t* __restrict__ ptr, uint32_t N, uint32_t* key, uint32_t* iota)
 {
-  const unsigned long long fmin = *fmin_ptr;  // the frontier's smallest message
+  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < N; p += gridDim.x * blockDim.x)
+  {
+    key[p] = ~(ptr[p + 1] - ptr[p]);
+    iota[p] = p;
+  }
+}
+
+__global__ void k_sssp_slots(const uint32_t* __restrict__ order, uint32_t N, uint32_t* slot)
+{
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) slot[order[i]] = i;
+}
+
+// Sort keys (row, leading bits of the weight) and values (slot, weight) of the
+// regular rows' entries, a warp per row.
+template <class K>
+__global__ void __launch_bounds__(256)
+k_sssp_entries(const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col, const uint32_t* __restrict__ w,
+               uint32_t nreg, const uint32_t* __restrict__ slot, int wbits, int wshift, K* key, uint2* entry)
+{
+  const uint32_t lane = threadIdx.x & 31, nw = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < nreg; r += nw)
+    for (uint32_t e = ptr[r] + lane; e < ptr[r + 1]; e += 32)
+    {
+      key[e] = (K) r << wbits | (K) (w[e] >> wshift);
+      entry[e] = make_uint2(slot[col[e]], w[e]);
+    }
+}
+
+__device__ __forceinline__ void sssp_pull(const SsspArgs& A, unsigned long long fmin, uint32_t warp, uint32_t nwarps,
+                                          uint32_t lane)
+{
   // Every candidate of this step is a frontier message plus a weight, so at
   // least fmin + min_w: a row already at or below that cannot be lowered and
   // its in-edges are not read (the result is the same).
   const uint32_t settled =
-      fmin == ~0ull ? 0u : (fmin + min_w < kInf ? (uint32_t) (fmin + min_w) : kInf);
-  const int lane = threadIdx.x & 31;
-  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (warp < task_warps)
+      fmin == ~0ull ? 0u : (fmin + A.min_w < kInf ? (uint32_t) (fmin + A.min_w) : kInf);
+  const uint2* __restrict__ entry = A.entry;
+  const uint32_t* fmsg = A.fmsg;
+  // long rows first
+  for (uint32_t t = warp; t < A.ntasks; t += nwarps)
   {
-    // long rows: each task's minimum goes to the row's partial slot
-    for (uint32_t t = warp; t < ntasks; t += task_warps)
+    uint32_t* const at = &A.dist[A.task_row[t]];
+    uint32_t y = *(volatile uint32_t*) at;  // with what the row's other tasks found so far
+    if (y <= settled) continue;
+    const uint32_t b = A.task_begin[t], e = A.task_begin[A.ntasks + t], had = y;
+    for (uint32_t i0 = b; i0 < e; i0 += 128)
     {
-      const uint32_t k = task_row[t];  // index into the long-row list
-      if (dist[long_rows[k]] <= settled) continue;
-      const uint32_t b = task_begin[t], e = task_begin[ntasks + t];  // [begins | ends]
-      uint32_t y = kInf;
-      for (uint32_t i = b + lane; i < e; i += 32) sssp_pull_edge(i, col, w, fmsg, y);
-      for (int o = 16; o > 0; o >>= 1) y = min(y, __shfl_xor_sync(0xffffffffu, y, o));
-      if (lane == 0 && y < kInf) atomicMin(&ymin[k], y);
+      uint2 x[4];
+      uint32_t m[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) x[u] = i0 + u * 32 + lane < e ? __ldcs(&entry[i0 + u * 32 + lane]) : make_uint2(0u, kInf);
+      if (sssp_past(fmin, __shfl_sync(0xffffffffu, x[0].y, 0), A.wshift, y)) break;
+#pragma unroll
+      for (int u = 0; u < 4; u++) m[u] = fmsg[x[u].x];
+#pragma unroll
+      for (int u = 0; u < 4; u++) y = min(y, m[u] + x[u].y);
+      y = __reduce_min_sync(0xffffffffu, y);
     }
-    return;
+    if (lane == 0 && y < had) atomicMin(at, y);
   }
   // short rows: a group of kPullLanes lanes per row; each lane keeps four
-  // independent loads in flight per step (indices, then frontier words,
-  // then messages), since the step is bound by memory latency
+  // independent loads in flight per step (entries, then messages), since the
+  // step is bound by memory latency
   constexpr uint32_t G = kPullLanes;
-  const uint32_t sub = lane & (G - 1);
-  const uint32_t group = (((blockIdx.x * blockDim.x + threadIdx.x) >> 5) - task_warps) * (32 / G) + lane / G;
-  const uint32_t ngroups = (((gridDim.x * blockDim.x) >> 5) - task_warps) * (32 / G);
-  const uint32_t rounds = (nreg + ngroups - 1) / ngroups;
-  for (uint32_t k = 0; k < rounds; k++)
+  const uint32_t sub = lane & (G - 1), group = warp * (32 / G) + lane / G, ngroups = nwarps * (32 / G);
+  const unsigned group_mask = ((1u << G) - 1) << (lane & ~(G - 1));
+  for (uint32_t v = group; v < A.nreg; v += ngroups)
   {
-    const uint32_t v = group + k * ngroups;
-    uint32_t y = kInf, dv = 0;
-    bool mine = false;
-    if (v < nreg)
+    const uint32_t b = A.in_ptr[v], dv = A.dist[v];
+    uint32_t e = A.in_ptr[v + 1], y = dv;  // y: the same in the group's lanes after each step
+    if (e - b > kPullLong || dv <= settled) e = b;
+    for (uint32_t i = b; i < e; i += 4 * G)
     {
-      const uint32_t b = ptr[v], e = ptr[v + 1];
-      dv = dist[v];
-      mine = e - b <= kPullLong && dv > settled;
-      if (mine)
-        for (uint32_t i = b + sub; i < e; i += 4 * G)
-        {
-          uint32_t c[4], ww[4], m[4];
+      uint2 x[4];
+      uint32_t m[4];
 #pragma unroll
-          for (int u = 0; u < 4; u++)
-          {
-            const bool ok = i + u * G < e;
-            c[u] = ok ? col[i + u * G] : 0u;
-            ww[u] = ok ? w[i + u * G] : kInf;
-          }
+      for (uint32_t u = 0; u < 4; u++) x[u] = i + u * G + sub < e ? __ldcs(&entry[i + u * G + sub]) : make_uint2(0u, kInf);
+      if (sssp_past(fmin, __shfl_sync(group_mask, x[0].y, 0, G), A.wshift, y)) break;
 #pragma unroll
-          for (int u = 0; u < 4; u++) m[u] = fmsg[c[u]];
+      for (int u = 0; u < 4; u++) m[u] = fmsg[x[u].x];
 #pragma unroll
-          for (int u = 0; u < 4; u++) y = min(y, m[u] + ww[u]);
-        }
+      for (int u = 0; u < 4; u++) y = min(y, m[u] + x[u].y);
+#pragma unroll
+      for (int o = G / 2; o > 0; o >>= 1) y = min(y, __shfl_xor_sync(group_mask, y, o));
     }
-#pragma unroll
-    for (int o = G / 2; o > 0; o >>= 1) y = min(y, __shfl_xor_sync(0xffffffffu, y, o));
-    if (mine && sub == 0 && y < dv) dist[v] = y;
-  }
-}
-
-// Long rows after a pull step: apply the partial minimum, reset it.
-__global__ void k_sssp_pull_long(const uint32_t* __restrict__ long_rows, uint32_t nlong, uint32_t* ymin, uint32_t* dist)
-{
-  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nlong; k += gridDim.x * blockDim.x)
-  {
-    const uint32_t y = ymin[k];
-    if (y == kInf) continue;
-    ymin[k] = kInf;
-    const uint32_t v = long_rows[k];
-    if (y < dist[v]) dist[v] = y;
+    if (sub == 0 && y < dv) A.dist[v] = y;
   }
 }
 
@@ -475,47 +398,139 @@ __global__ void k_sssp_long_rows(const uint32_t* __restrict__ ptr, const uint32_
 }
 
 // A step pulls when its frontier's out-degree sum exceeds the regular rows'
-// in-edges / kPullDivisor (measured on R-MAT s22: 2 and 4 give 1.90 ms per
-// call, 6 to 16 give 2.16-2.18 ms).
+// in-edges / kPullDivisor (8 roots each: R-MAT 2^22 2: 8.2 ms, 4: 7.3, 8: 7.3;
+// ER 2^22 2: 34.8, 4: 35.2, 8: 38.8).
 static constexpr double kPullDivisor = 4.0;
+static constexpr int kSsspThreads = 512;
 
-// Sink pass: y = min over in-neighbours (regular: final dist; the root if it
-// is a source: its message 0) of msg + w; dist = min(dist, y).
-__global__ void k_sssp_sinks(const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col,
-                             const uint32_t* __restrict__ w, uint32_t nreg, uint32_t nsink,
-                             const unsigned long long* __restrict__ state, uint32_t* dist)
+__global__ void __launch_bounds__(kSsspThreads, 3) k_sssp_run(SsspArgs A)
 {
-  const uint32_t src_root = (uint32_t) state[kStSrcRoot];
-  for (uint32_t v = nreg + blockIdx.x * blockDim.x + threadIdx.x; v < nreg + nsink; v += gridDim.x * blockDim.x)
+  __shared__ SsspCounters s_got;
+  __shared__ unsigned long long s_list[2];
+  GridBarrier bar{A.bar, (int*) (A.bar + 1), kBarrierPolls};
+  const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
+  const uint32_t lane = threadIdx.x & 31, warp = tid >> 5, nwarps = nth >> 5;
+  const uint32_t words = A.N / 32 + 1;
+  // The root (none if it is outside the graph): distance 0, scattered (msg 0);
+  // regular and source vertices scatter, so they form the first frontier (even
+  // with no regular out-edge: the first iteration runs).
+  const uint32_t rp = A.root < A.N ? A.pos_of_id[A.root] : 0xFFFFFFFFu;
+  const bool src = rp >= A.src_base && rp < A.iso_base, scatters = rp < A.nreg || src;
+  for (uint32_t p = tid; p < A.N; p += nth)
+  {
+    A.dist[p] = A.msg[p] = p == rp ? 0u : kInf;
+    A.fmsg[p] = kInf;
+  }
+  for (uint32_t w = tid; w < words; w += nth)
+  {
+    A.fbits[w] = scatters && w == rp >> 5 ? 1u << (rp & 31) : 0u;
+    A.pbits[w] = 0;
+  }
+  if (tid == 0)
+  {
+    for (int k = 0; k < 3; k++) A.ctr[k] = SsspCounters{0, 0, 0, ~0ull};
+    A.fctr[0] = A.fctr[1] = *A.reached = 0;
+  }
+  if (!bar.sync()) return;
+  // the loop's state, the same in every thread.  It ends as the reference's
+  // execute loop does: nothing activated, or activated vertices with no
+  // regular out-edge, which take one more, empty iteration.
+  unsigned long long it = 0, examined = 0, nlist = scatters, deg = scatters ? A.reg_end[rp] - A.out_ptr[rp] : 0, fmin = ~0ull;
+  bool failed = false;
+  for (;;)
+  {
+    if (it > A.limit)
+    {
+      failed = true;
+      break;
+    }
+    it++;
+    if (!nlist) break;
+    SsspCounters* const next = A.ctr + it % 3;
+    if (tid == 0) A.ctr[(it + 1) % 3] = SsspCounters{0, 0, 0, ~0ull};  // read last before the barrier just passed
+    if (it > 1 && A.max_w <= 0x80000000u && (double) deg * kPullDivisor > (double) A.reg_in)
+    {
+      examined += A.reg_in;
+      sssp_front(A, words, warp, nwarps, lane);
+      if (!bar.sync()) return;
+      sssp_pull(A, fmin, warp, nwarps, lane);
+    }
+    else
+    {
+      examined += deg;
+      sssp_split(A, words, warp, nwarps, lane);
+      if (!bar.sync()) return;
+      if (threadIdx.x < 2) s_list[threadIdx.x] = __ldcg(&A.fctr[threadIdx.x]);
+      __syncthreads();
+      sssp_push(A, (uint32_t) s_list[0], s_list[1], warp, nwarps, lane);
+    }
+    if (!bar.sync()) return;
+    if (tid == 0) A.fctr[0] = A.fctr[1] = 0;
+    sssp_dense_apply(A, words, next, warp, nwarps, lane);
+    if (!bar.sync()) return;
+    if (threadIdx.x == 0) s_got = {__ldcg(&next->count), __ldcg(&next->deg), __ldcg(&next->out), __ldcg(&next->fmin)};
+    __syncthreads();
+    const unsigned long long count = s_got.count;
+    deg = s_got.deg;
+    nlist = s_got.out;
+    fmin = s_got.fmin;
+    __syncthreads();  // s_got is free
+    if (!count) break;
+  }
+  // Sink pass: y = min over in-neighbours (regular: final dist; the root if it
+  // is a source: its message 0) of msg + w; dist = min(dist, y).
+  for (uint32_t v = A.nreg + tid; v < A.nreg + A.nsink; v += nth)
   {
     uint32_t y = kInf;
-    for (uint32_t i = ptr[v]; i < ptr[v + 1]; i++)
+    for (uint32_t i = A.in_ptr[v]; i < A.in_ptr[v + 1]; i++)
     {
-      const uint32_t c = col[i];
+      const uint32_t c = A.in_col[i];
       uint32_t cand;
-      if (c < nreg) cand = dist[c] + w[i];
-      else if (c == src_root) cand = 0u + w[i];
+      if (c < A.nreg) cand = A.dist[c] + A.in_w[i];
+      else if (src && c == rp) cand = A.in_w[i];
       else continue;
       y = min(y, cand);
     }
-    dist[v] = min(dist[v], y);
+    if (y < A.dist[v]) A.dist[v] = y;
   }
+  if (!bar.sync()) return;
+  unsigned long long r = 0;
+  for (uint32_t i = tid; i < A.N; i += nth)
+  {
+    if (A.dist_out) A.dist_out[i] = A.dist[A.pos_of_id[i]];
+    if (A.dist[i] != kInf) r += A.out_ptr[i + 1] - A.out_ptr[i];
+  }
+  r = block_sum_u64(r);
+  if (threadIdx.x == 0 && r) atomicAdd(A.reached, r);
+  if (!bar.sync()) return;
+  if (tid == 0) *A.stats = SsspStats{it, examined, failed ? 1ull : 0ull, __ldcg(A.reached)};
 }
 
-__global__ void k_reached_outdeg(const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ dist, uint32_t N,
-                                 unsigned long long* out)
+// The pull's entries; rows ascend by position, so the regular rows' come first.
+template <class K>
+static int sssp_entries(la3g_graph* G, SsspScratch* ss, int rbits, int wbits)
 {
-  unsigned long long s = 0;
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < N; v += gridDim.x * blockDim.x)
-    if (dist[v] != kInf) s += ptr[v + 1] - ptr[v];
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0 && s) atomicAdd(out, s);
-}
-
-__global__ void k_u32_by_id(uint32_t N, const uint32_t* __restrict__ id_of_pos, const uint32_t* __restrict__ val,
-                            uint32_t* __restrict__ out)
-{
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < N; p += gridDim.x * blockDim.x) out[id_of_pos[p]] = val[p];
+  const uint64_t m = ss->reg_in;
+  LA3G_TRY(galloc(G, &ss->entry, m + 1));
+  if (!m) return LA3G_OK;
+  cub::DoubleBuffer<K> k(nullptr, nullptr);
+  cub::DoubleBuffer<uint2> v(nullptr, nullptr);
+  size_t tb = 0;
+  LA3G_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, k, v, (int64_t) m, 0, rbits + wbits, G->stream));
+  const size_t kb = (m * sizeof(K) + 255) & ~(size_t) 255, vb = (m * 8 + 255) & ~(size_t) 255;
+  DevBuf tmp;
+  LA3G_TRY(tmp.alloc(2 * kb + vb + tb));
+  char* p = tmp.as<char>();
+  k = cub::DoubleBuffer<K>((K*) p, (K*) (p + kb));
+  v = cub::DoubleBuffer<uint2>(ss->entry, (uint2*) (p + 2 * kb));
+  k_sssp_entries<K><<<grid_for((uint64_t) G->g.nreg * 32, 256), 256, 0, G->stream>>>(
+      G->g.in_ptr, G->g.in_col, G->g.in_w, G->g.nreg, ss->slot, wbits, ss->wshift, k.Current(), v.Current());
+  LA3G_LAUNCHED();
+  LA3G_CUDA(cub::DeviceRadixSort::SortPairs(p + 2 * kb + vb, tb, k, v, (int64_t) m, 0, rbits + wbits, G->stream));
+  if (v.Current() != ss->entry)
+    LA3G_CUDA(cudaMemcpyAsync(ss->entry, v.Current(), m * 8, cudaMemcpyDeviceToDevice, G->stream));
+  LA3G_CUDA(cudaStreamSynchronize(G->stream));  // before the temporaries go
+  return LA3G_OK;
 }
 
 static int sssp_scratch(la3g_graph* G, SsspScratch** out)
@@ -526,213 +541,117 @@ static int sssp_scratch(la3g_graph* G, SsspScratch** out)
   if (!ss) return set_error(LA3G_ENOMEM, "out of host memory");
   G->slot[kSlotSssp] = ss;
   G->slot_free[kSlotSssp] = sssp_scratch_free;
-  const uint32_t N = G->g.nslots;
-  LA3G_TRY(galloc(G, &ss->dist, N));
-  LA3G_TRY(galloc(G, &ss->msg, N));
-  LA3G_TRY(galloc(G, &ss->reg_end, N));
-  LA3G_TRY(galloc(G, &ss->small[0], N));
-  LA3G_TRY(galloc(G, &ss->big[0], N));
-  LA3G_TRY(galloc(G, &ss->big_task0[0], N));
-  LA3G_TRY(galloc(G, &ss->ctr, 8));
-  LA3G_TRY(galloc(G, &ss->fctr, 2));
-  LA3G_TRY(galloc(G, &ss->fbits, (size_t) N / 32 + 2));
-  LA3G_TRY(galloc(G, &ss->by_id, N));
-  LA3G_TRY(galloc(G, &ss->state, kStSlots));
-  LA3G_CUDA(cudaHostAlloc(&ss->hctr, kStSlots * sizeof(unsigned long long), cudaHostAllocDefault));
-  k_sssp_reg_end<<<grid_for(N, 256), 256, 0, G->stream>>>(G->g.out_ptr, G->g.out_row, N, G->g.nreg, ss->reg_end);
-  LA3G_LAUNCHED();
-  LA3G_TRY(galloc(G, &ss->long_rows, std::max<uint32_t>(G->g.nreg, 1)));
-  LA3G_TRY(galloc(G, &ss->fmsg, N));
-  LA3G_CUDA(cudaMemsetAsync(ss->ctr, 0, 8 * sizeof(unsigned long long), G->stream));
-  LA3G_CUDA(cudaMemsetAsync(ss->ctr + 3, 0xFF, sizeof(unsigned long long), G->stream));
-  k_sssp_long_rows<<<grid_for(G->g.nreg, 256), 256, 0, G->stream>>>(G->g.in_ptr, G->g.in_w, G->g.nreg, ss->long_rows,
-                                                                     ss->ctr, ss->ctr + 1, (unsigned int*) (ss->ctr + 2),
-                                                                     (unsigned int*) (ss->ctr + 3));
-  LA3G_LAUNCHED();
-  LA3G_CUDA(cudaMemcpyAsync(ss->hctr, ss->ctr, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, G->stream));
-  LA3G_CUDA(cudaStreamSynchronize(G->stream));
-  ss->nlong = (uint32_t) ss->hctr[0];
-  ss->reg_in = ss->hctr[1];
-  ss->max_w = (uint32_t) ss->hctr[2];
-  ss->min_w = (uint32_t) ss->hctr[3];
-  if (ss->nlong)
-  {
-    // cut the long rows into tasks of kPullChunk in-edges (host side: few rows)
-    std::vector<uint32_t> rows(ss->nlong), b(ss->nlong), e(ss->nlong), ptr((size_t) G->g.nreg + 1);
-    LA3G_CUDA(cudaMemcpy(rows.data(), ss->long_rows, ss->nlong * 4, cudaMemcpyDeviceToHost));
-    LA3G_CUDA(cudaMemcpy(ptr.data(), G->g.in_ptr, ptr.size() * 4, cudaMemcpyDeviceToHost));
-    for (uint32_t k = 0; k < ss->nlong; k++)
-    {
-      b[k] = ptr[rows[k]];
-      e[k] = ptr[rows[k] + 1];
-    }
-    std::vector<uint32_t> trow, tbeg;
-    for (uint32_t k = 0; k < ss->nlong; k++)
-    {
-      ss->task_edges += e[k] - b[k];
-      for (uint32_t x = b[k]; x < e[k]; x += kPullChunk)
-      {
-        trow.push_back(k);
-        tbeg.push_back(x);
-      }
-    }
-    ss->ntasks = (uint32_t) trow.size();
-    LA3G_TRY(galloc(G, &ss->task_row, trow.size()));
-    LA3G_TRY(galloc(G, &ss->task_begin, 2 * trow.size()));  // [begins | ends]
-    LA3G_TRY(galloc(G, &ss->ymin, ss->nlong));
-    std::vector<uint32_t> be(2 * trow.size());
-    for (size_t t = 0; t < trow.size(); t++)
-    {
-      be[t] = tbeg[t];
-      be[trow.size() + t] = std::min<uint32_t>(tbeg[t] + kPullChunk, e[trow[t]]);
-    }
-    LA3G_CUDA(cudaMemcpy(ss->task_row, trow.data(), trow.size() * 4, cudaMemcpyHostToDevice));
-    LA3G_CUDA(cudaMemcpy(ss->task_begin, be.data(), be.size() * 4, cudaMemcpyHostToDevice));
-    std::vector<uint32_t> inf(ss->nlong, kInf);
-    LA3G_CUDA(cudaMemcpy(ss->ymin, inf.data(), ss->nlong * 4, cudaMemcpyHostToDevice));
-  }
-  *out = ss;
-  return LA3G_OK;
-}
-
-// One iteration's body, k = kPull or kPush: the relaxation step, then the
-// dense apply that forms the next frontier and its counters.  `deg` and
-// `nlist` (the frontier's out-degree sum and size) only size the profile
-// entries' bytes; the kernels read every count they need on the device.
-static int sssp_body(la3g_graph* G, SsspScratch* ss, cudaStream_t s, unsigned k, double deg, double nlist)
-{
-  DevGraph& g = G->g;
-  const uint32_t words = g.nslots / 32 + 1;
-  if (k == kPull)
-  {
-    // in-edges of every regular row (index + weight), the frontier
-    // messages of their columns, one dist read per row
-    ProfileScope p("sssp_pull", s, 8.0 * ss->reg_in + 8.0 * ss->reg_in + 8.0 * g.nreg);
-    // warps split between long-row tasks and short rows in proportion to their in-edges
-    const uint32_t all_warps = num_sms() * 8 * 8;
-    const uint32_t task_warps =
-        ss->ntasks ? std::min<uint32_t>(ss->ntasks, std::max<uint32_t>(1, (uint32_t) ((double) all_warps *
-                                                                                        ss->task_edges /
-                                                                                        std::max<uint64_t>(ss->reg_in, 1))))
-                   : 0;
-    k_sssp_pull<<<num_sms() * 8, 256, 0, s>>>(g.in_ptr, g.in_col, g.in_w, g.nreg, ss->task_row, ss->task_begin,
-                                              ss->ntasks, task_warps, ss->ymin, ss->fmsg, ss->dist, ss->long_rows,
-                                              ss->state + kStFmin, ss->min_w);
-    LA3G_LAUNCHED();
-    if (ss->nlong)
-    {
-      k_sssp_pull_long<<<grid_for(ss->nlong, 256), 256, 0, s>>>(ss->long_rows, ss->nlong, ss->ymin, ss->dist);
-      LA3G_LAUNCHED();
-      tls_launches++;
-    }
-  }
-  else
-  {
-    k_sssp_split<<<grid_for(words, 256), 256, 0, s>>>(ss->fbits, words, g.out_ptr, ss->reg_end, ss->small[0],
-                                                      ss->big[0], ss->big_task0[0], ss->fctr);
-    LA3G_LAUNCHED();
-    tls_launches++;
-    ProfileScope p("sssp_push", s, 8.0 * deg + 12.0 * nlist);
-    k_sssp_push<<<num_sms() * 8, 256, 0, s>>>(g.out_ptr, ss->reg_end, g.out_row, g.out_w, ss->small[0], ss->big[0],
-                                              ss->big_task0[0], ss->fctr, ss->msg, ss->dist);
-    LA3G_LAUNCHED();
-  }
-  k_sssp_dense_apply<<<grid_for((uint64_t) words * 32, 256, num_sms() * 4), 256, 0, s>>>(
-      g.nreg, words, g.out_ptr, ss->reg_end, ss->dist, ss->msg, ss->fmsg, ss->fbits, ss->ctr);
-  LA3G_LAUNCHED();
-  tls_launches++;
-  return LA3G_OK;
-}
-
-// Iteration limit: with non-negative weights every distance is final after
-// at most N + 1 iterations (Bellman-Ford), so a loop past N + 2 is a fault.
-static uint64_t sssp_limit(const DevGraph& g) { return (uint64_t) g.nslots + 2; }
-
-static int sssp_decide(la3g_graph* G, SsspScratch* ss, cudaStream_t s, cudaGraphConditionalHandle cont,
-                       cudaGraphConditionalHandle mode)
-{
-  k_sssp_decide<<<1, 1, 0, s>>>(ss->state, ss->ctr, ss->fctr, ss->reg_in, ss->max_w, kPullDivisor, sssp_limit(G->g),
-                                cont, mode);
-  LA3G_LAUNCHED();
-  tls_launches++;
-  return LA3G_OK;
-}
-
-// Runs SSSP from `root` with the distances left on the device (positions).
-// The iterations run as one device-driven graph (no host round trip per
-// iteration); with profiling on they are stepped from the host instead, so
-// that each kernel is timed.
-static int sssp_run(la3g_graph* G, SsspScratch* ss, uint32_t root, la3g_stats* st)
-{
   DevGraph& g = G->g;
   cudaStream_t s = G->stream;
   const uint32_t N = g.nslots;
-  const uint32_t words = N / 32 + 1;
-  k_sssp_init<<<grid_for(N, 256), 256, 0, s>>>(N, ss->dist, ss->msg, ss->fmsg);
+  SsspArgs& A = ss->A;
+  LA3G_TRY(galloc(G, &A.dist, N));
+  LA3G_TRY(galloc(G, &A.msg, N));
+  LA3G_TRY(galloc(G, &A.fmsg, N));
+  LA3G_TRY(galloc(G, &ss->reg_end, N));
+  LA3G_TRY(galloc(G, &A.small, N));
+  LA3G_TRY(galloc(G, &A.big, N));
+  LA3G_TRY(galloc(G, &A.big_task0, N));
+  LA3G_TRY(galloc(G, &A.ctr, 3));
+  LA3G_TRY(galloc(G, &A.fctr, 4));  // with `reached` and the barrier
+  A.reached = A.fctr + 2;
+  A.bar = (unsigned int*) (A.fctr + 3);
+  LA3G_TRY(galloc(G, &A.fbits, (size_t) N / 32 + 2));
+  LA3G_TRY(galloc(G, &A.pbits, (size_t) N / 32 + 2));
+  LA3G_TRY(galloc(G, &ss->by_id, N));
+  LA3G_CUDA(cudaHostAlloc(&ss->stats, sizeof(SsspStats), cudaHostAllocMapped));
+  k_sssp_reg_end<<<grid_for(N, 256), 256, 0, s>>>(g.out_ptr, g.out_row, N, g.nreg, ss->reg_end);
   LA3G_LAUNCHED();
-  LA3G_CUDA(cudaMemsetAsync(ss->fbits, 0, (size_t) words * 4, s));
-  k_sssp_root<<<1, 1, 0, s>>>(root, N, g.pos_of_id, g.out_ptr, ss->reg_end, g.nreg, g.src_base(), g.iso_base(),
-                              ss->dist, ss->msg, ss->fbits, ss->state);
-  LA3G_LAUNCHED();
-  tls_launches += 2;
-  if (!profile_enabled())
+  LA3G_TRY(galloc(G, &ss->long_rows, std::max<uint32_t>(g.nreg, 1)));
   {
-    if (!ss->loop)
-    {
-      ss->loop = new (std::nothrow) DeviceLoop();
-      if (!ss->loop) return set_error(LA3G_ENOMEM, "out of host memory");
-      const int rc = device_loop_build(
-          ss->loop, 2,
-          [&](cudaStream_t c, cudaGraphConditionalHandle cont, cudaGraphConditionalHandle mode) {
-            return sssp_decide(G, ss, c, cont, mode);
-          },
-          [&](cudaStream_t c, int k) { return sssp_body(G, ss, c, (unsigned) k, 0.0, 0.0); });
-      if (rc != LA3G_OK)
-      {
-        delete ss->loop;
-        ss->loop = nullptr;
-        return rc;
-      }
-    }
-    LA3G_CUDA(cudaGraphLaunch(ss->loop->exec, s));
-  }
-  else
-  {
-    for (;;)
-    {
-      LA3G_TRY(sssp_decide(G, ss, s, 0, 0));
-      LA3G_CUDA(cudaMemcpyAsync(ss->hctr, ss->state, kStSlots * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-      LA3G_CUDA(cudaStreamSynchronize(s));
-      const unsigned m = (unsigned) ss->hctr[kStMode];
-      if (m == kDone) break;
-      LA3G_TRY(sssp_body(G, ss, s, m, (double) ss->hctr[kStFrontDeg], (double) ss->hctr[kStNlist]));
-    }
-  }
-  if (g.nsink)
-  {
-    // the sink rows' in-edges only (index + weight, and the column's
-    // distance), their offsets and the distance read and written
-    const double sink_in = (double) (g.nent - ss->reg_in);
-    ProfileScope p("sssp_sinks", s, 12.0 * sink_in + 12.0 * g.nsink);
-    k_sssp_sinks<<<grid_for(g.nsink, 256), 256, 0, s>>>(g.in_ptr, g.in_col, g.in_w, g.nreg, g.nsink, ss->state,
-                                                         ss->dist);
+    // [0] long rows [1] regular in-edges [2] largest weight [3] smallest
+    unsigned long long* c = (unsigned long long*) A.ctr;
+    unsigned long long h[4];
+    LA3G_CUDA(cudaMemsetAsync(c, 0, 3 * sizeof(unsigned long long), s));
+    LA3G_CUDA(cudaMemsetAsync(c + 3, 0xFF, sizeof(unsigned long long), s));
+    k_sssp_long_rows<<<grid_for(g.nreg, 256), 256, 0, s>>>(g.in_ptr, g.in_w, g.nreg, ss->long_rows, c, c + 1,
+                                                           (unsigned int*) (c + 2), (unsigned int*) (c + 3));
     LA3G_LAUNCHED();
+    LA3G_CUDA(cudaMemcpyAsync(h, c, sizeof h, cudaMemcpyDeviceToHost, s));
+    LA3G_CUDA(cudaStreamSynchronize(s));
+    ss->nlong = (uint32_t) h[0];
+    ss->reg_in = h[1];
+    ss->max_w = (uint32_t) h[2];
+    ss->min_w = (uint32_t) h[3];
   }
-  LA3G_CUDA(cudaMemcpyAsync(ss->hctr, ss->state, kStSlots * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-  LA3G_CUDA(cudaStreamSynchronize(s));
-  if (ss->hctr[kStStatus]) return set_error(LA3G_ETIMEOUT, "sssp did not converge");
-  if (ss->loop && !profile_enabled())
+  if (ss->nlong)
   {
-    // the graph's launches: one decide per pass, each body's kernels per step
-    const uint64_t passes = ss->hctr[kStPulls] + ss->hctr[kStPushes] + 1;
-    tls_launches += (uint32_t) (passes + ss->hctr[kStPulls] * ss->loop->body_launches[kPull] +
-                                ss->hctr[kStPushes] * ss->loop->body_launches[kPush]);
+    // cut the long rows into tasks of kPullChunk in-edges (host side: few rows)
+    std::vector<uint32_t> rows(ss->nlong), ptr((size_t) g.nreg + 1);
+    LA3G_CUDA(cudaMemcpy(rows.data(), ss->long_rows, ss->nlong * 4, cudaMemcpyDeviceToHost));
+    LA3G_CUDA(cudaMemcpy(ptr.data(), g.in_ptr, ptr.size() * 4, cudaMemcpyDeviceToHost));
+    std::vector<uint32_t> trow, tbeg, tend;
+    for (uint32_t r : rows)
+      for (uint64_t x = ptr[r]; x < ptr[r + 1]; x += kPullChunk)
+      {
+        trow.push_back(r);
+        tbeg.push_back((uint32_t) x);
+        tend.push_back((uint32_t) std::min<uint64_t>(x + kPullChunk, ptr[r + 1]));
+      }
+    const size_t nt = trow.size();
+    uint32_t *row = nullptr, *be = nullptr;
+    LA3G_TRY(galloc(G, &row, nt));
+    LA3G_TRY(galloc(G, &be, 2 * nt));
+    LA3G_CUDA(cudaMemcpy(row, trow.data(), nt * 4, cudaMemcpyHostToDevice));
+    LA3G_CUDA(cudaMemcpy(be, tbeg.data(), nt * 4, cudaMemcpyHostToDevice));
+    LA3G_CUDA(cudaMemcpy(be + nt, tend.data(), nt * 4, cudaMemcpyHostToDevice));
+    A.task_row = row;
+    A.task_begin = be;
+    A.ntasks = (uint32_t) nt;
   }
-  if (st)
   {
-    st->iterations = (uint32_t) ss->hctr[kStIter];
-    st->edges_examined = ss->hctr[kStExamined];
+    DevBuf tmp;
+    size_t tb = 0;
+    uint32_t* z = nullptr;
+    LA3G_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, z, z, z, z, (int64_t) N, 0, 32, G->stream));
+    LA3G_TRY(tmp.alloc((size_t) N * 16 + tb + 256));
+    uint32_t *key = tmp.as<uint32_t>(), *key2 = key + N, *iota = key2 + N, *order = iota + N;
+    void* lib = (void*) (((uintptr_t) (order + N) + 255) & ~(uintptr_t) 255);
+    k_sssp_slot_keys<<<grid_for(N, 256), 256, 0, G->stream>>>(G->g.out_ptr, N, key, iota);
+    LA3G_LAUNCHED();
+    LA3G_CUDA(cub::DeviceRadixSort::SortPairs(lib, tb, key, key2, iota, order, (int64_t) N, 0, 32, G->stream));
+    LA3G_TRY(galloc(G, &ss->slot, N));
+    k_sssp_slots<<<grid_for(N, 256), 256, 0, G->stream>>>(order, N, ss->slot);
+    LA3G_LAUNCHED();
+    int rbits = 1, wbits = 1;
+    while ((uint64_t) G->g.nreg >> rbits) rbits++;
+    while (wbits < 32 && ss->max_w >> wbits) wbits++;
+    // eight leading bits of the weight order a row well enough
+    ss->wshift = std::max(0, wbits - 8);
+    wbits -= ss->wshift;
+    if (rbits + wbits <= 32) LA3G_TRY(sssp_entries<uint32_t>(G, ss, rbits, wbits));
+    else LA3G_TRY(sssp_entries<uint64_t>(G, ss, rbits, wbits));
+    LA3G_CUDA(cudaStreamSynchronize(G->stream));
   }
+  A.out_ptr = g.out_ptr;
+  A.out_row = g.out_row;
+  A.out_w = g.out_w;
+  A.reg_end = ss->reg_end;
+  A.in_ptr = g.in_ptr;
+  A.in_col = g.in_col;
+  A.in_w = g.in_w;
+  A.pos_of_id = g.pos_of_id;
+  A.N = N;
+  A.nreg = g.nreg;
+  A.nsink = g.nsink;
+  A.src_base = g.src_base();
+  A.iso_base = g.iso_base();
+  A.reg_in = ss->reg_in;
+  A.min_w = ss->min_w;
+  A.max_w = ss->max_w;
+  // with non-negative weights every distance is final after at most N + 1
+  // iterations (Bellman-Ford), so a loop past N + 2 is a fault
+  A.limit = (uint64_t) N + 2;
+  A.slot = ss->slot;
+  A.entry = ss->entry;
+  A.wshift = ss->wshift;
+  A.stats = ss->stats;
+  *out = ss;
   return LA3G_OK;
 }
 
@@ -752,26 +671,33 @@ extern "C" int la3g_sssp(la3g_graph* G, uint32_t root, uint32_t* dist_out, la3g_
   LA3G_TRY(sssp_scratch(G, &ss));
   cudaStream_t s = G->stream;
   const uint32_t N = g.nslots;
+  SsspArgs A = ss->A;
+  A.root = root;
+  A.dist_out = dist_out ? ss->by_id : nullptr;
+  ss->stats->status = kSsspRunning;
+  if (!ss->grid)  // few blocks for a small graph: a barrier takes longer the more there are
+    LA3G_TRY(cooperative_blocks((const void*) k_sssp_run, kSsspThreads, std::max<uint64_t>(N, g.nent / 8), 3, &ss->grid));
   T.device_begin();
-  LA3G_TRY(sssp_run(G, ss, root, st));
+  LA3G_CUDA(cudaMemsetAsync(A.bar, 0, 8, s));
+  {
+    // distances and messages; the edges examined are added below
+    ProfileScope p("sssp", s, 8.0 * N);
+    void* args[] = {(void*) &A};
+    LA3G_CUDA(cudaLaunchCooperativeKernel((const void*) k_sssp_run, ss->grid, kSsspThreads, args, 0, s));
+  }
   T.device_end();
+  if (dist_out) LA3G_CUDA(cudaMemcpyAsync(dist_out, ss->by_id, (size_t) N * 4, cudaMemcpyDeviceToHost, s));
+  LA3G_TRY(T.finish());
+  const SsspStats r = *ss->stats;
+  if (r.status == kSsspRunning) return set_error(LA3G_ETIMEOUT, "sssp: a grid barrier wait ran out");
+  if (r.status) return set_error(LA3G_ETIMEOUT, "sssp did not converge");
+  profile_add_bytes("sssp", 8.0 * (double) r.examined);
   if (st)
   {
-    LA3G_CUDA(cudaMemsetAsync(ss->ctr + 2, 0, 8, s));
-    k_reached_outdeg<<<grid_for(N, 256), 256, 0, s>>>(g.out_ptr, ss->dist, N, ss->ctr + 2);
-    LA3G_LAUNCHED();
-    LA3G_CUDA(cudaMemcpyAsync(ss->hctr + 2, ss->ctr + 2, 8, cudaMemcpyDeviceToHost, s));
-    LA3G_CUDA(cudaStreamSynchronize(s));
-    st->teps_edges = ss->hctr[2];
-    st->algo_bytes = st->edges_examined * 8 + (uint64_t) N * 8;
+    st->iterations = (uint32_t) r.iterations;
+    st->edges_examined = r.examined;
+    st->teps_edges = r.reached_deg;
+    st->algo_bytes = r.examined * 8 + (uint64_t) N * 8;
   }
-  if (dist_out)
-  {
-    // the graph's own reorder buffer: no allocation per call
-    k_u32_by_id<<<grid_for(N, 256), 256, 0, s>>>(N, g.id_of_pos, ss->dist, ss->by_id);
-    LA3G_LAUNCHED();
-    LA3G_CUDA(cudaMemcpyAsync(dist_out, ss->by_id, (size_t) N * 4, cudaMemcpyDeviceToHost, s));
-    LA3G_CUDA(cudaStreamSynchronize(s));
-  }
-  return T.finish();
+  return LA3G_OK;
 }
