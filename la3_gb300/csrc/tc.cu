@@ -58,6 +58,7 @@ static constexpr uint32_t kTcMidSlots = 2048;     // hash slots of its table (>=
 static constexpr uint32_t kTcBlockCap = 2048;     // |N+(y)| up to this: a large block table; longer: global search
 static constexpr uint32_t kTcBlockSlots = 8192;   // hash slots of a large block table (>= 4 kTcBlockCap)
 static constexpr uint32_t kTcBlockPairs = 1024;   // pairs per block task (both block sizes; R-MAT s20 call: 4096 4.96 ms, 2048 4.83, 1024 4.73, 512 4.74, 256 5.01)
+static constexpr uint32_t kTcLong = 64;           // suffixes this long are walked by themselves (same call: 24 4.62 ms, 32 4.51, 64 4.35, 128 4.42)
 static constexpr int kTcWarpKernelWarps = 8;
 static constexpr int kTcMidThreads = 256;
 static constexpr int kTcBlockThreads = 512;
@@ -412,6 +413,21 @@ __device__ __forceinline__ uint32_t tc_mid3(uint32_t a, uint32_t b, uint32_t c)
 
 __device__ __forceinline__ uint32_t tc_hash(uint32_t w, int lg) { return (w * 0x9E3779B1u) >> (32 - lg); }
 
+// How N+(y) is held while its pairs are walked.
+//   kTcHash    a hash table, see TcTable;
+//   kTcBits    a bitmap over the ranks above y, with the index of each word's
+//              first element: a probe is one word and a bit test, a hit's index
+//              a count of bits, and neighbouring ranks share words (no bank
+//              conflicts).  Degree order puts the y with long rows, which hold
+//              nine tenths of what is walked on R-MAT, near the top: at 2^20
+//              none with more than 128 elements spans over 22,192 ranks;
+//   kTcSearch  neither fits: binary search in the sorted row in global memory.
+// R-MAT 2^20: a hash probe of 32 elements took 80 warp instructions, 14 of them
+// branches (probe chains); the rows above 128 elements took 2830 us hashed, 2365
+// us as bitmaps.  What bounds them now is the instructions left, about 50 per 32
+// elements at three a clock and SM: every hit has an id to compare and a counter.
+enum : int { kTcHash, kTcBits, kTcSearch };
+
 // The table of one task's N+(y): open addressing (rank -> index in the row)
 // with at least 4 slots per element, so that nearly every probe ends at its
 // first slot; the ids of the row's elements (lid) and one counter per
@@ -425,6 +441,10 @@ struct TcTable
   uint32_t* cn;
   uint32_t mask;
   int lg;
+  // kTcBits: 32 ranks of base .. base + span - 1 each: their bits, and the index
+  // in the row of the first one set
+  const uint2* word;
+  uint32_t base, span;
 };
 
 // Per-warp round state (shared memory): the compacted pairs' (suffix start
@@ -438,19 +458,11 @@ struct TcRound
   uint32_t cx[32];
 };
 
-// Counts the element w (of the suffix of the pair at lane k of this round)
-// against N+(y): a hit closes {x, y, w}; its middle id takes the count - x
-// in the round's cx[k], y in cy, w in cn[j].  SEARCH: N+(y) too long for a
-// table, binary search in the sorted global row, w's count straight to ntri.
-template <class IDX, bool SEARCH>
-__device__ __forceinline__ void tc_probe(uint32_t w, uint32_t k, uint32_t xo, uint32_t yid, const TcTable<IDX>& T,
-                                         const uint32_t* __restrict__ row, uint32_t d,
-                                         const uint32_t* __restrict__ id_of_rank, TcRound& R, uint32_t& cy,
-                                         uint32_t* ntri)
+// Index of w in N+(y), or -1.
+template <class IDX, int FORM>
+__device__ __forceinline__ int tc_find(uint32_t w, const TcTable<IDX>& T, const uint32_t* __restrict__ row, uint32_t d)
 {
-  if (w == kEmpty) return;
-  int j = -1;
-  if (SEARCH)
+  if (FORM == kTcSearch)
   {
     uint32_t lo = 0, hi = d;
     while (lo < hi)
@@ -459,35 +471,100 @@ __device__ __forceinline__ void tc_probe(uint32_t w, uint32_t k, uint32_t xo, ui
       if (row[mid] < w) lo = mid + 1;
       else hi = mid;
     }
-    if (lo < d && row[lo] == w) j = (int) lo;
+    return lo < d && row[lo] == w ? (int) lo : -1;
   }
-  else
+  if (FORM == kTcBits)
   {
-    uint32_t sl = tc_hash(w, T.lg), kk = T.key[sl];
-    while (kk != w && kk != kEmpty)
-    {
-      sl = (sl + 1) & T.mask;
-      kk = T.key[sl];
-    }
-    if (kk == w) j = T.idx[sl];
+    const uint32_t r = w - T.base;  // the walked ranks are above y
+    if (r >= T.span) return -1;
+    const uint2 x = T.word[r >> 5];
+    const uint32_t bit = 1u << (r & 31);
+    return x.x & bit ? (int) (x.y + __popc(x.x & (bit - 1))) : -1;
   }
+  uint32_t sl = tc_hash(w, T.lg), kk = T.key[sl];
+  while (kk != w && kk != kEmpty)
+  {
+    sl = (sl + 1) & T.mask;
+    kk = T.key[sl];
+  }
+  return kk == w ? (int) T.idx[sl] : -1;
+}
+
+// Counts the element w (of the suffix of the pair at lane k of this round)
+// against N+(y): a hit closes {x, y, w}; its middle id takes the count - x
+// in the round's cx[k], y in cy, w in cn[j], or without a table (kTcSearch) straight in ntri.
+template <class IDX, int FORM>
+__device__ __forceinline__ void tc_probe(uint32_t w, uint32_t k, uint32_t xo, uint32_t yid, const TcTable<IDX>& T,
+                                         const uint32_t* __restrict__ row, uint32_t d,
+                                         const uint32_t* __restrict__ id_of_rank, TcRound& R, uint32_t& cy,
+                                         uint32_t* ntri)
+{
+  if (w == kEmpty) return;
+  const int j = tc_find<IDX, FORM>(w, T, row, d);
   if (j < 0) return;
-  const uint32_t wid = SEARCH ? id_of_rank[w] : T.lid[j];
+  const uint32_t wid = FORM == kTcSearch ? id_of_rank[w] : T.lid[j];
   const uint32_t mid = tc_mid3(xo, yid, wid);
   cy += mid == yid;
-  uint32_t* const at_w = SEARCH ? &ntri[wid] : &T.cn[j];
+  uint32_t* const at_w = FORM == kTcSearch ? &ntri[wid] : &T.cn[j];
   if (mid != yid) atomicAdd(mid == xo ? &R.cx[k] : at_w, 1u);
 }
 
-// One warp walks one round: pairs [p0, p1) (at most 32) of y.  The pairs'
-// suffixes are concatenated and read 64 elements per step (two 32-element
-// windows whose loads are in flight together).  Element t belongs to the
+// One pair with a long suffix (L elements from s), walked by the whole warp:
+// no element's owner is looked up, and the triangles counted at x or y, whose
+// ids are the same for all lanes, add up in registers.
+template <class IDX, int FORM>
+__device__ __forceinline__ void tc_long(uint32_t s, uint32_t L, uint32_t xid, uint32_t yid,
+                                        const uint32_t* __restrict__ pcol, const uint32_t* __restrict__ id_of_rank,
+                                        const TcTable<IDX>& T, const uint32_t* __restrict__ row, uint32_t d, uint32_t& cy,
+                                        uint32_t* ntri)
+{
+  const uint32_t lane = threadIdx.x & 31, lo = min(xid, yid), hi = max(xid, yid);
+  uint32_t below = 0, above = 0;  // hits with an id below both, above both
+  for (uint32_t t0 = 0; t0 < L; t0 += 128)
+  {
+    uint32_t w[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) w[u] = t0 + u * 32 + lane < L ? pcol[s + t0 + u * 32 + lane] : kEmpty;
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+    {
+      if (FORM == kTcBits)
+      {
+        // without branches: a miss takes an id that counts nowhere
+        const uint32_t r = w[u] - T.base, at = r & 31;
+        const uint2 x = r < T.span ? T.word[r >> 5] : make_uint2(0u, 0u);
+        const bool hit = x.x >> at & 1;
+        const uint32_t j = x.y + __popc(x.x & ~(0xFFFFFFFFu << at)), wid = hit ? T.lid[j] : lo;
+        below += wid < lo;
+        above += wid > hi;
+        if (wid > lo && wid < hi) atomicAdd(&T.cn[j], 1u);
+        continue;
+      }
+      if (w[u] == kEmpty) continue;
+      const int j = tc_find<IDX, FORM>(w[u], T, row, d);
+      if (j < 0) continue;
+      const uint32_t wid = FORM == kTcSearch ? id_of_rank[w[u]] : T.lid[j];
+      below += wid < lo;
+      above += wid > hi;
+      if (wid > lo && wid < hi) atomicAdd(FORM == kTcSearch ? &ntri[wid] : &T.cn[j], 1u);
+    }
+  }
+  // the middle of {x, y, w} is the lower of x and y when w is below both
+  cy += xid < yid ? above : below;
+  const uint32_t cx = __reduce_add_sync(0xffffffffu, xid < yid ? below : above);
+  if (lane == 0 && cx) atomicAdd(&ntri[xid], cx);
+}
+
+// One warp walks one round: pairs [p0, p1) (at most 32) of y.  Suffixes of
+// kTcLong elements or more, which hold most of what is walked on R-MAT, are
+// walked one after another (tc_long); the rest are concatenated and read 64
+// elements per step (two 32-element windows whose loads are in flight together).  Element t belongs to the
 // compacted pair k whose walk offset is the last at or below t: k = (pairs
 // started before the window) + (pairs starting in the window at or below
 // the lane) - 1, from one OR-reduction of the window's start bits; the
 // owner's (start - offset) and x id come from its lane by shuffle, so the
 // address of element t is so[k] + t.
-template <class IDX, bool SEARCH>
+template <class IDX, int FORM>
 __device__ __forceinline__ void tc_round(uint32_t p0, uint32_t p1, const uint2* __restrict__ pairs,
                                          const uint32_t* __restrict__ pptr, const uint32_t* __restrict__ pcol,
                                          const uint32_t* __restrict__ id_of_rank, uint32_t yid, const TcTable<IDX>& T,
@@ -506,7 +583,16 @@ __device__ __forceinline__ void tc_round(uint32_t p0, uint32_t p1, const uint2* 
     L = pptr[px.y + 1] - s;
     xid = id_of_rank[px.y];
   }
+  walked += L;
+  for (unsigned m = __ballot_sync(full, L >= kTcLong); m; m &= m - 1)
+  {
+    const int k = __ffs(m) - 1;
+    tc_long<IDX, FORM>(__shfl_sync(full, s, k), __shfl_sync(full, L, k), __shfl_sync(full, xid, k), yid, pcol,
+                       id_of_rank, T, row, d, cy, ntri);
+  }
+  if (L >= kTcLong) L = 0;
   const unsigned nz = __ballot_sync(full, L > 0);
+  if (!nz) return;
   uint32_t incl = L;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1)
@@ -550,11 +636,10 @@ __device__ __forceinline__ void tc_round(uint32_t p0, uint32_t p1, const uint2* 
     slip |= (va && ka >= np) || (vb && kb >= np);
     const uint32_t wa = (va && ka < np) ? pcol[soa + ta] : kEmpty;
     const uint32_t wb = (vb && kb < np) ? pcol[sob + tb] : kEmpty;
-    tc_probe<IDX, SEARCH>(wa, ka, xa, yid, T, row, d, id_of_rank, R, cy, ntri);
-    tc_probe<IDX, SEARCH>(wb, kb, xb, yid, T, row, d, id_of_rank, R, cy, ntri);
+    tc_probe<IDX, FORM>(wa, ka, xa, yid, T, row, d, id_of_rank, R, cy, ntri);
+    tc_probe<IDX, FORM>(wb, kb, xb, yid, T, row, d, id_of_rank, R, cy, ntri);
   }
   if (slip) atomicAdd(err, 1ull);
-  walked += total;
   __syncwarp();
   if (lane < np && R.cx[lane]) atomicAdd(&ntri[my_x], R.cx[lane]);
   __syncwarp();
@@ -577,6 +662,21 @@ __device__ __forceinline__ void tc_build(const uint32_t* __restrict__ row, uint3
     uint32_t sl = tc_hash(w, lg);
     while (atomicCAS(&key[sl], kEmpty, w) != kEmpty) sl = (sl + 1) & mask;
     idx[sl] = (IDX) j;
+  }
+}
+
+// The same as a bitmap: `words` words cleared by the caller.
+__device__ __forceinline__ void tc_build_bits(const uint32_t* __restrict__ row, uint32_t d, uint32_t base,
+                                              const uint32_t* __restrict__ id_of_rank, uint2* word, uint32_t* lid,
+                                              uint32_t* cn, uint32_t tid, uint32_t nthreads)
+{
+  for (uint32_t j = tid; j < d; j += nthreads)
+  {
+    const uint32_t w = row[j], q = (w - base) >> 5;
+    lid[j] = id_of_rank[w];
+    cn[j] = 0;
+    atomicOr(&word[q].x, 1u << ((w - base) & 31));
+    if (j == 0 || (row[j - 1] - base) >> 5 != q) word[q].y = j;
   }
 }
 
@@ -625,11 +725,11 @@ k_tc_count_warp(const uint32_t* __restrict__ pptr, const uint32_t* __restrict__ 
     tc_build<uint8_t>(pcol + yb, d, lg, id_of_rank, key, idx, lid, cn, lane, 32);
     __syncwarp();
     built += d;
-    const TcTable<uint8_t> T{key, idx, lid, cn, (1u << lg) - 1, lg};
+    const TcTable<uint8_t> T{key, idx, lid, cn, (1u << lg) - 1, lg, nullptr, 0, 0};
     const uint32_t yid = id_of_rank[y];
     uint32_t cy = 0;
     for (uint32_t q = p0; q < p1; q += 32)
-      tc_round<uint8_t, false>(q, min(q + 32u, p1), pairs, pptr, pcol, id_of_rank, yid, T, nullptr, d, s_r[wi], cy,
+      tc_round<uint8_t, kTcHash>(q, min(q + 32u, p1), pairs, pptr, pcol, id_of_rank, yid, T, nullptr, d, s_r[wi], cy,
                                walked, ntri, ctr + 5);
     for (int o = 16; o > 0; o >>= 1) cy += __shfl_xor_sync(0xffffffffu, cy, o);
     if (lane == 0 && cy) atomicAdd(&ntri[yid], cy);
@@ -638,6 +738,7 @@ k_tc_count_warp(const uint32_t* __restrict__ pptr, const uint32_t* __restrict__ 
       if (cn[j]) atomicAdd(&ntri[lid[j]], cn[j]);
     __syncwarp();
   }
+  for (int o = 16; o > 0; o >>= 1) walked += __shfl_xor_sync(0xffffffffu, walked, o);
   if (lane == 0)
   {
     atomicAdd(&ctr[2], walked);
@@ -661,9 +762,11 @@ k_tc_count_block(const uint32_t* __restrict__ pptr, const uint32_t* __restrict__
   constexpr int WARPS = THREADS / 32;
   extern __shared__ __align__(16) uint32_t tc_smem[];
   uint32_t* key = tc_smem;                          // [SLOTS]
-  uint32_t* lid = key + SLOTS;                      // [CAP]
+  uint16_t* idx = (uint16_t*) (key + SLOTS);        // [SLOTS]
+  uint2* word = (uint2*) tc_smem;                   // [WORDS], in the place of both
+  uint32_t* lid = (uint32_t*) (idx + SLOTS);        // [CAP]
   uint32_t* cn = lid + CAP;                         // [CAP]
-  uint16_t* idx = (uint16_t*) (cn + CAP);           // [SLOTS]
+  constexpr uint32_t WORDS = SLOTS * 6 / 8;
   __shared__ TcRound s_r[WARPS];
   __shared__ uint32_t s_t, s_cy, s_round;
   const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
@@ -684,16 +787,22 @@ k_tc_count_block(const uint32_t* __restrict__ pptr, const uint32_t* __restrict__
     const uint32_t y = tk.x, p0 = tk.y, p1 = min(p0 + kTcBlockPairs, mptr[y + 1]);
     const uint32_t yb = pptr[y], d = pptr[y + 1] - yb;
     const bool search = d > CAP;
+    // a bitmap of the ranks above y if it fits the hash table's place: it is the
+    // faster one at every length that has a block task
+    const uint32_t base = y + 1, span = d ? pcol[yb + d - 1] - y : 0;
+    const bool bits = span <= WORDS * 32;
     const int lg = search ? 5 : tc_lg(d);
     if (!search)
     {
-      for (uint32_t i = threadIdx.x; i < (1u << lg); i += THREADS) key[i] = kEmpty;
+      const uint32_t words = bits ? 2 * ((span + 31) / 32) : 1u << lg;
+      for (uint32_t i = threadIdx.x; i < words; i += THREADS) key[i] = bits ? 0u : kEmpty;
       __syncthreads();
-      tc_build<uint16_t>(pcol + yb, d, lg, id_of_rank, key, idx, lid, cn, threadIdx.x, THREADS);
+      if (bits) tc_build_bits(pcol + yb, d, base, id_of_rank, word, lid, cn, threadIdx.x, THREADS);
+      else tc_build<uint16_t>(pcol + yb, d, lg, id_of_rank, key, idx, lid, cn, threadIdx.x, THREADS);
       if (threadIdx.x == 0) built += d;
     }
     __syncthreads();
-    const TcTable<uint16_t> T{key, idx, lid, cn, (1u << lg) - 1, lg};
+    const TcTable<uint16_t> T{key, idx, lid, cn, (1u << lg) - 1, lg, word, base, span};
     const uint32_t yid = id_of_rank[y];
     uint32_t cy = 0;
     for (;;)
@@ -704,11 +813,14 @@ k_tc_count_block(const uint32_t* __restrict__ pptr, const uint32_t* __restrict__
       const uint32_t q = p0 + 32u * r;
       if (q >= p1) break;
       if (search)
-        tc_round<uint16_t, true>(q, min(q + 32u, p1), pairs, pptr, pcol, id_of_rank, yid, T, pcol + yb, d, s_r[wi],
-                                 cy, walked, ntri, ctr + 5);
+        tc_round<uint16_t, kTcSearch>(q, min(q + 32u, p1), pairs, pptr, pcol, id_of_rank, yid, T, pcol + yb, d, s_r[wi],
+                                      cy, walked, ntri, ctr + 5);
+      else if (bits)
+        tc_round<uint16_t, kTcBits>(q, min(q + 32u, p1), pairs, pptr, pcol, id_of_rank, yid, T, nullptr, d, s_r[wi], cy,
+                                    walked, ntri, ctr + 5);
       else
-        tc_round<uint16_t, false>(q, min(q + 32u, p1), pairs, pptr, pcol, id_of_rank, yid, T, nullptr, d, s_r[wi],
-                                  cy, walked, ntri, ctr + 5);
+        tc_round<uint16_t, kTcHash>(q, min(q + 32u, p1), pairs, pptr, pcol, id_of_rank, yid, T, nullptr, d, s_r[wi], cy,
+                                    walked, ntri, ctr + 5);
     }
     for (int o = 16; o > 0; o >>= 1) cy += __shfl_xor_sync(0xffffffffu, cy, o);
     if (lane == 0 && cy) atomicAdd(&s_cy, cy);
@@ -719,7 +831,7 @@ k_tc_count_block(const uint32_t* __restrict__ pptr, const uint32_t* __restrict__
         if (cn[j]) atomicAdd(&ntri[lid[j]], cn[j]);
     __syncthreads();
   }
-  // every lane of a warp holds the warp's walked count
+  for (int o = 16; o > 0; o >>= 1) walked += __shfl_xor_sync(0xffffffffu, walked, o);
   if (lane == 0 && walked) atomicAdd(&ctr[2], walked);
   if (threadIdx.x == 0 && built) atomicAdd(&ctr[3], built);
 }
