@@ -19,9 +19,10 @@
 //   and w lies in the part of N+(x) ranked above y (a suffix of the row).
 //
 // Pass 1 (list building, every call): degrees, ranks (one radix sort of the
-// vertices), N+ rows by an edge-parallel count / scan / fill, a segmented
-// sort of the rows, and the transposed pair lists: for each y the pairs
-// (x, start of the suffix of N+(x) after y), i.e. every oriented edge once.
+// vertices), N+ rows by an edge-parallel count / scan / fill, a sort of each
+// row, and with it the transposed pair lists: for each y the pairs (x, start
+// of the suffix of N+(x) after y), i.e. every oriented edge once.  Its atomics
+// bound it (three per edge).
 //
 // Pass 2 (counting) is y-centric: a task is a vertex y and a slice of its
 // pairs; N+(y) goes into a shared-memory hash table (rank -> index, at least
@@ -79,7 +80,7 @@ struct TcScratch
   uint32_t* id_of_rank = nullptr;   // [N]
   uint32_t* dplus = nullptr;        // [N + 1] |N+| by rank, then the row offsets' input
   uint32_t* pptr = nullptr;         // [N + 1] N+ row offsets (rows = ranks)
-  uint32_t* fill = nullptr;         // [N] fill cursors
+  uint32_t* fill = nullptr;         // [N + 31] counters, then cursors (tc_spread)
   uint32_t* pcol_raw = nullptr;     // [m] N+ rows as filled (ranks)
   uint32_t* pcol = nullptr;         // [m] N+ rows, each ascending
   uint32_t* mcount = nullptr;       // [N + 1] pairs per y
@@ -149,16 +150,25 @@ __device__ __forceinline__ uint32_t tc_row_of(const uint32_t* __restrict__ ptr, 
   return lo;
 }
 
+// Where rank y's counter or cursor stands in an array of them (N + 31 entries):
+// the highest ranks take most of the atomics, so neighbouring ranks lie in
+// different lines.  R-MAT 2^20, in rank order and spread: the sort, which appends
+// the pairs, 811 and 566 us, the fill 256 and 214, the count 166 and 151.
+__device__ __forceinline__ uint32_t tc_spread(uint32_t y, uint32_t N)
+{
+  const uint32_t rows = (N + 31) / 32;
+  return (y % rows) * 32 + y / rows;
+}
+
 // Every undirected edge once (the pull CSR of the id-oriented graph: row =
 // higher id, column = lower id); each thread takes kTcEdgesPerThread
-// consecutive entries, so a hub row spreads over many threads.  PLUS = false
-// counts |N+| per lower-rank end; PLUS = true writes the higher-rank end into
+// consecutive entries, so a hub row spreads over many threads.  FILL = false
+// counts |N+| per lower-rank end; FILL = true writes the higher-rank end into
 // the lower end's row.
 template <bool FILL>
 __global__ void __launch_bounds__(256)
 k_tc_orient(const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col, uint32_t nrows, uint64_t m,
-            const uint32_t* __restrict__ rank_of_pos, uint32_t* count_or_fill, const uint32_t* __restrict__ pptr,
-            uint32_t* pcol)
+            const uint32_t* __restrict__ rank_of_pos, uint32_t N, uint32_t* count_or_fill, uint32_t* pcol)
 {
   const uint64_t e0 = ((uint64_t) blockIdx.x * blockDim.x + threadIdx.x) * kTcEdgesPerThread;
   if (e0 >= m) return;
@@ -176,15 +186,22 @@ k_tc_orient(const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ col, 
     }
     const uint32_t ru = rank_of_pos[col[e]];
     const uint32_t lo = min(rr, ru), hi = max(rr, ru);
-    if (FILL) pcol[pptr[lo] + atomicAdd(&count_or_fill[lo], 1u)] = hi;
-    else atomicAdd(&count_or_fill[lo], 1u);
+    uint32_t* const at = &count_or_fill[tc_spread(lo, N)];
+    if (FILL) pcol[atomicAdd(at, 1u)] = hi;
+    else atomicAdd(at, 1u);
   }
 }
 
-// Pairs per y (a y with an empty N+(y) closes no triangle as the middle
-// rank) and the tasks they form.
+__global__ void k_tc_dplus(uint32_t N, const uint32_t* __restrict__ count, uint32_t* dplus)
+{
+  for (uint32_t y = blockIdx.x * blockDim.x + threadIdx.x; y <= N; y += gridDim.x * blockDim.x)
+    dplus[y] = y < N ? count[tc_spread(y, N)] : 0;
+}
+
+// Pairs per y and the tasks they form (none where N+(y) is empty: no triangle
+// has such a y as its middle rank).
 __global__ void k_tc_pair_counts(uint32_t N, const uint32_t* __restrict__ pptr, const uint32_t* __restrict__ deg_of_rank,
-                                 uint32_t* mcount, unsigned long long* tcount, uint32_t* tcount2)
+                                 uint32_t* fill, uint32_t* mcount, unsigned long long* tcount, uint32_t* tcount2)
 {
   for (uint32_t y = blockIdx.x * blockDim.x + threadIdx.x; y <= N; y += gridDim.x * blockDim.x)
   {
@@ -193,8 +210,9 @@ __global__ void k_tc_pair_counts(uint32_t N, const uint32_t* __restrict__ pptr, 
     if (y < N)
     {
       const uint32_t dp = pptr[y + 1] - pptr[y];
-      c = dp ? deg_of_rank[y] - dp : 0u;
-      if (c)
+      fill[tc_spread(y, N)] = pptr[y];
+      c = deg_of_rank[y] - dp;
+      if (c && dp)
       {
         if (dp <= kTcWarpCap) t = (c + kTcWarpPairs - 1) / kTcWarpPairs;
         else if (dp <= kTcMidCap) t = (unsigned long long) ((c + kTcBlockPairs - 1) / kTcBlockPairs) << 32;
@@ -207,84 +225,12 @@ __global__ void k_tc_pair_counts(uint32_t N, const uint32_t* __restrict__ pptr, 
   }
 }
 
-// Index of rank y in the ascending row [b, e) (y is known to be there).
-__device__ __forceinline__ uint32_t tc_find_in_row(const uint32_t* __restrict__ pcol, uint32_t b, uint32_t e, uint32_t y)
-{
-  while (b < e)
-  {
-    const uint32_t mid = (b + e) >> 1;
-    if (pcol[mid] < y) b = mid + 1;
-    else e = mid;
-  }
-  return b;
-}
-
-// Pair lists by y, built from each y's own adjacency (its in- and out-rows in
-// the id-oriented graph), so that a hub's many pairs come from consecutive
-// entries: the lanes of a warp that hold the same y reserve their slots with
-// one atomic.  A neighbour x of lower rank gives the pair (s, x), s the
-// index after y in the sorted row N+(x).  Thread chunks [0, m8) cover the
-// in-rows' m entries, [m8, m8 + m) the out-rows' (m8 = m rounded up to the
-// chunk size, so that no chunk straddles the two).
-__global__ void __launch_bounds__(256)
-k_tc_pairs(const uint32_t* __restrict__ iptr, const uint32_t* __restrict__ icol, const uint32_t* __restrict__ optr,
-           const uint32_t* __restrict__ orow, uint32_t nrows, uint32_t N, uint64_t m,
-           const uint32_t* __restrict__ rank_of_pos, const uint32_t* __restrict__ pptr,
-           const uint32_t* __restrict__ pcol, const uint32_t* __restrict__ mptr, uint32_t* fill, uint2* pairs)
-{
-  const int lane = threadIdx.x & 31;
-  const uint64_t m8 = (m + kTcEdgesPerThread - 1) / kTcEdgesPerThread * kTcEdgesPerThread;
-  const uint64_t e0 = ((uint64_t) blockIdx.x * blockDim.x + threadIdx.x) * kTcEdgesPerThread;
-  const bool in_part = e0 < m8;
-  const uint32_t* ptr = in_part ? iptr : optr;
-  const uint32_t* col = in_part ? icol : orow;
-  const uint64_t base = in_part ? 0 : m8;
-  const uint64_t lim = in_part ? m : m8 + m;
-  const bool live = e0 < lim;
-  uint32_t r = 0, ry = 0;
-  uint64_t rend = 0;
-  if (live)
-  {
-    r = tc_row_of(ptr, in_part ? nrows : N, e0 - base);
-    ry = rank_of_pos[r];
-    rend = ptr[r + 1] + base;
-  }
-  for (uint32_t u = 0; u < kTcEdgesPerThread; u++)
-  {
-    const uint64_t e = e0 + u;
-    bool emit = false;
-    uint32_t x = 0;
-    if (live && e < lim)
-    {
-      if (e >= rend)  // the next non-empty row (sinks' out-rows are empty, in runs)
-      {
-        r = tc_row_of(ptr, in_part ? nrows : N, e - base);
-        ry = rank_of_pos[r];
-        rend = ptr[r + 1] + base;
-      }
-      x = rank_of_pos[col[e - base]];
-      emit = x < ry && pptr[ry + 1] > pptr[ry];
-    }
-    const unsigned want = __ballot_sync(0xffffffffu, emit);
-    if (!want) continue;
-    const unsigned grp = __match_any_sync(0xffffffffu, emit ? ry : 0xFFFFFFFFu);
-    if (emit)
-    {
-      const int leader = __ffs(grp) - 1;
-      uint32_t slot = 0;
-      if (lane == leader) slot = atomicAdd(&fill[ry], (uint32_t) __popc(grp));
-      slot = __shfl_sync(grp, slot, leader) + __popc(grp & ((1u << lane) - 1));
-      const uint32_t sidx = tc_find_in_row(pcol, pptr[x], pptr[x + 1], ry);
-      pairs[mptr[ry] + slot] = make_uint2(sidx + 1, x);
-    }
-  }
-}
-
 __global__ void k_tc_tasks(uint32_t N, const unsigned long long* __restrict__ toff, const uint32_t* __restrict__ toff2,
-                           const uint32_t* __restrict__ mptr, uint2* wtasks, uint2* mtasks, uint2* btasks)
+                           const uint32_t* __restrict__ mptr, uint32_t* fill, uint2* wtasks, uint2* mtasks, uint2* btasks)
 {
   for (uint32_t y = blockIdx.x * blockDim.x + threadIdx.x; y < N; y += gridDim.x * blockDim.x)
   {
+    fill[tc_spread(y, N)] = mptr[y];
     const unsigned long long c = toff[y + 1] - toff[y];
     const uint32_t nw = (uint32_t) c, nm = (uint32_t) (c >> 32), nb = toff2[y + 1] - toff2[y];
     const uint32_t wo = (uint32_t) toff[y], mo = (uint32_t) (toff[y] >> 32), bo = toff2[y];
@@ -296,25 +242,43 @@ __global__ void k_tc_tasks(uint32_t N, const unsigned long long* __restrict__ to
 
 // ---------------------------------------------------------------- row sort
 
+// The pair that the element w at index e of pcol, in the sorted row of x, makes
+// for w as a middle rank: the suffix from e + 1 on.  Grouped by w; the order
+// within a group is free.
+__device__ __forceinline__ void tc_emit(uint32_t e, uint32_t x, uint32_t w, uint32_t N, uint32_t* fill, uint2* pairs)
+{
+  pairs[atomicAdd(&fill[tc_spread(w, N)], 1u)] = make_uint2(e + 1, x);
+}
+
 // Sorts every N+ row ascending (pass 1 fills them in arbitrary order): up to
 // 32 elements in a warp's registers (a bitonic network over shuffles), up to
 // kTcSortWarpCap in a warp's shared buffer; longer rows are listed for
-// k_tc_sort_big.
+// k_tc_sort_big.  Each element's pair is appended as its row is written out: the
+// start of its suffix is known there (a pass of its own searched the rows for
+// it: R-MAT 2^20 577 us).  Rows are taken by position, which orders the pair
+// lists about so too, and the tasks that run together then walk the same rows
+// (a call: by rank 4.17 ms, by position 4.06).
 template <int WARPS>
 __global__ void __launch_bounds__(WARPS * 32)
-k_tc_sort_rows(const uint32_t* __restrict__ pptr, uint32_t N, const uint32_t* __restrict__ raw, uint32_t* out,
-               uint32_t* big_rows, unsigned long long* nbig)
+k_tc_sort_rows(const uint32_t* __restrict__ pptr, uint32_t N, const uint32_t* __restrict__ rank_of_pos,
+               const uint32_t* __restrict__ raw, uint32_t* out,
+               uint32_t* fill, uint2* pairs, uint32_t* big_rows, unsigned long long* nbig)
 {
   __shared__ uint32_t s_buf[WARPS][kTcSortWarpCap];
   const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
   uint32_t* buf = s_buf[wi];
   const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t x = gw; x < N; x += nw)
+  for (uint32_t p = gw; p < N; p += nw)
   {
-    const uint32_t b = pptr[x], d = pptr[x + 1] - b;
+    const uint32_t x = rank_of_pos[p], b = pptr[x], d = pptr[x + 1] - b;
     if (d <= 1)
     {
-      if (d == 1 && lane == 0) out[b] = raw[b];
+      if (d == 1 && lane == 0)
+      {
+        const uint32_t w = raw[b];
+        out[b] = w;
+        tc_emit(b, x, w, N, fill, pairs);
+      }
       continue;
     }
     if (d <= 32)
@@ -329,7 +293,11 @@ k_tc_sort_rows(const uint32_t* __restrict__ pptr, uint32_t N, const uint32_t* __
           const bool asc = (lane & k) == 0, low = (lane & j) == 0;
           v = (low == asc) ? min(v, o) : max(v, o);
         }
-      if ((uint32_t) lane < d) out[b + lane] = v;
+      if ((uint32_t) lane < d)
+      {
+        out[b + lane] = v;
+        tc_emit(b + lane, x, v, N, fill, pairs);
+      }
       continue;
     }
     if (d > kTcSortWarpCap)
@@ -346,7 +314,7 @@ k_tc_sort_rows(const uint32_t* __restrict__ pptr, uint32_t N, const uint32_t* __
       {
         for (uint32_t q = lane; q < n / 2; q += 32)
         {
-          const uint32_t i = 2 * j * (q / j) + (q % j), l = i + j;
+          const uint32_t i = 2 * q - (q & (j - 1)), l = i + j;
           const uint32_t a = buf[i], c = buf[l];
           if ((a > c) == ((i & k) == 0))
           {
@@ -356,17 +324,22 @@ k_tc_sort_rows(const uint32_t* __restrict__ pptr, uint32_t N, const uint32_t* __
         }
         __syncwarp();
       }
-    for (uint32_t i = lane; i < d; i += 32) out[b + i] = buf[i];
+    for (uint32_t i = lane; i < d; i += 32)
+    {
+      out[b + i] = buf[i];
+      tc_emit(b + i, x, buf[i], N, fill, pairs);
+    }
     __syncwarp();
   }
 }
 
 // Rows longer than kTcSortWarpCap, one block each, in dynamic shared memory
-// (up to kTcSortBlockCap elements); longer ones are counted in *over so that
-// the call sorts with the library's segmented sort instead.
+// (up to kTcSortBlockCap elements); longer ones are copied as they are and
+// counted in *over so that the call sorts with the library's segmented sort
+// instead.
 __global__ void __launch_bounds__(1024)
-k_tc_sort_big(const uint32_t* __restrict__ pptr, const uint32_t* __restrict__ raw, uint32_t* out,
-              const uint32_t* __restrict__ big_rows, const unsigned long long* __restrict__ nbig,
+k_tc_sort_big(const uint32_t* __restrict__ pptr, const uint32_t* __restrict__ raw, uint32_t N, uint32_t* out,
+              uint32_t* fill, uint2* pairs, const uint32_t* __restrict__ big_rows, const unsigned long long* __restrict__ nbig,
               unsigned long long* over)
 {
   extern __shared__ uint32_t sbig[];
@@ -378,6 +351,11 @@ k_tc_sort_big(const uint32_t* __restrict__ pptr, const uint32_t* __restrict__ ra
     if (d > kTcSortBlockCap)
     {
       if (threadIdx.x == 0) atomicAdd(over, 1ull);
+      for (uint32_t i = threadIdx.x; i < d; i += blockDim.x)
+      {
+        out[b + i] = raw[b + i];
+        tc_emit(b + i, x, raw[b + i], N, fill, pairs);
+      }
       continue;
     }
     uint32_t n = 64;
@@ -389,7 +367,7 @@ k_tc_sort_big(const uint32_t* __restrict__ pptr, const uint32_t* __restrict__ ra
       {
         for (uint32_t q = threadIdx.x; q < n / 2; q += blockDim.x)
         {
-          const uint32_t i = 2 * j * (q / j) + (q % j), l = i + j;
+          const uint32_t i = 2 * q - (q & (j - 1)), l = i + j;
           const uint32_t a = sbig[i], c = sbig[l];
           if ((a > c) == ((i & k) == 0))
           {
@@ -399,9 +377,23 @@ k_tc_sort_big(const uint32_t* __restrict__ pptr, const uint32_t* __restrict__ ra
         }
         __syncthreads();
       }
-    for (uint32_t i = threadIdx.x; i < d; i += blockDim.x) out[b + i] = sbig[i];
+    for (uint32_t i = threadIdx.x; i < d; i += blockDim.x)
+    {
+      out[b + i] = sbig[i];
+      tc_emit(b + i, x, sbig[i], N, fill, pairs);
+    }
     __syncthreads();
   }
+}
+
+// The pairs of rows that the library sorted: a warp per row.
+__global__ void __launch_bounds__(256)
+k_tc_pairs(const uint32_t* __restrict__ pptr, uint32_t N, const uint32_t* __restrict__ pcol, uint32_t* fill,
+           uint2* pairs)
+{
+  const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t x = gw; x < N; x += nw)
+    for (uint32_t e = pptr[x] + (threadIdx.x & 31); e < pptr[x + 1]; e += 32) tc_emit(e, x, pcol[e], N, fill, pairs);
 }
 
 // ---------------------------------------------------------------- pass 2
@@ -528,6 +520,7 @@ __device__ __forceinline__ void tc_long(uint32_t s, uint32_t L, uint32_t xid, ui
 #pragma unroll
     for (int u = 0; u < 4; u++)
     {
+      if (t0 + u * 32 >= L) break;
       if (FORM == kTcBits)
       {
         // without branches: a miss takes an id that counts nowhere
@@ -871,7 +864,7 @@ static int tc_scratch(la3g_graph* G, TcScratch** out)
   LA3G_TRY(galloc(G, &ts->id_of_rank, N));
   LA3G_TRY(galloc(G, &ts->dplus, (size_t) N + 1));
   LA3G_TRY(galloc(G, &ts->pptr, (size_t) N + 1));
-  LA3G_TRY(galloc(G, &ts->fill, N));
+  LA3G_TRY(galloc(G, &ts->fill, (size_t) N + 31));
   LA3G_TRY(galloc(G, &ts->pcol_raw, m + 1));
   LA3G_TRY(galloc(G, &ts->pcol, m + 1));
   LA3G_TRY(galloc(G, &ts->mcount, (size_t) N + 1));
@@ -916,8 +909,7 @@ static int tc_lists(la3g_graph* G, TcScratch* ts, bool library_sort)
   const unsigned eblocks = (unsigned) std::max<uint64_t>(1, (m + 256ull * kTcEdgesPerThread - 1) /
                                                                 (256ull * kTcEdgesPerThread));
   size_t tb = ts->temp_bytes;
-  LA3G_CUDA(cudaMemsetAsync(ts->dplus, 0, ((size_t) N + 1) * 4, s));
-  LA3G_CUDA(cudaMemsetAsync(ts->fill, 0, (size_t) N * 4, s));
+  LA3G_CUDA(cudaMemsetAsync(ts->fill, 0, ((size_t) N + 31) * 4, s));
   LA3G_CUDA(cudaMemsetAsync(ts->ctr, 0, kTcCounters * sizeof(unsigned long long), s));
   k_tc_deg<<<grid_for(N, 256), 256, 0, s>>>(g.in_ptr, g.out_ptr, N, ts->deg, ts->iota);
   LA3G_LAUNCHED();
@@ -928,17 +920,32 @@ static int tc_lists(la3g_graph* G, TcScratch* ts, bool library_sort)
   tls_launches += 2;
   if (m)
   {
-    k_tc_orient<false><<<eblocks, 256, 0, s>>>(g.in_ptr, g.in_col, g.nrows(), m, ts->rank_of_pos, ts->dplus, nullptr,
-                                               nullptr);
+    k_tc_orient<false><<<eblocks, 256, 0, s>>>(g.in_ptr, g.in_col, g.nrows(), m, ts->rank_of_pos, N, ts->fill, nullptr);
     LA3G_LAUNCHED();
     tls_launches++;
   }
+  k_tc_dplus<<<grid_for((uint64_t) N + 1, 256), 256, 0, s>>>(N, ts->fill, ts->dplus);
+  LA3G_LAUNCHED();
+  tls_launches++;
   tb = ts->temp_bytes;
   LA3G_CUDA(cub::DeviceScan::ExclusiveSum(ts->temp, tb, ts->dplus, ts->pptr, (int) N + 1, s));
+  k_tc_pair_counts<<<grid_for((uint64_t) N + 1, 256), 256, 0, s>>>(N, ts->pptr, ts->deg_of_rank, ts->fill, ts->mcount,
+                                                                   ts->tcount, ts->tcount2);
+  LA3G_LAUNCHED();
+  tls_launches++;
+  tb = ts->temp_bytes;
+  LA3G_CUDA(cub::DeviceScan::ExclusiveSum(ts->temp, tb, ts->mcount, ts->mptr, (int) N + 1, s));
+  tb = ts->temp_bytes;
+  LA3G_CUDA(cub::DeviceScan::ExclusiveSum(ts->temp, tb, ts->tcount, ts->toff, (int) N + 1, s));
+  tb = ts->temp_bytes;
+  LA3G_CUDA(cub::DeviceScan::ExclusiveSum(ts->temp, tb, ts->tcount2, ts->toff2, (int) N + 1, s));
   if (m)
   {
-    k_tc_orient<true><<<eblocks, 256, 0, s>>>(g.in_ptr, g.in_col, g.nrows(), m, ts->rank_of_pos, ts->fill, ts->pptr,
-                                              ts->pcol_raw);
+    k_tc_orient<true><<<eblocks, 256, 0, s>>>(g.in_ptr, g.in_col, g.nrows(), m, ts->rank_of_pos, N, ts->fill, ts->pcol_raw);
+    LA3G_LAUNCHED();
+    tls_launches++;
+    k_tc_tasks<<<grid_for(N, 256), 256, 0, s>>>(N, ts->toff, ts->toff2, ts->mptr, ts->fill, ts->wtasks, ts->mtasks,
+                                                ts->btasks);
     LA3G_LAUNCHED();
     tls_launches++;
     if (library_sort)
@@ -952,40 +959,21 @@ static int tc_lists(la3g_graph* G, TcScratch* ts, bool library_sort)
       tb = ts->seg_bytes;
       LA3G_CUDA(cub::DeviceSegmentedSort::SortKeys(ts->seg_temp, tb, ts->pcol_raw, ts->pcol, (int64_t) m, (int64_t) N,
                                                    ts->pptr, ts->pptr + 1, s));
+      k_tc_pairs<<<grid_for((uint64_t) N * 32, 256), 256, 0, s>>>(ts->pptr, N, ts->pcol, ts->fill, ts->pairs);
+      LA3G_LAUNCHED();
+      tls_launches++;
     }
     else
     {
-      k_tc_sort_rows<8><<<num_sms() * 8, 256, 0, s>>>(ts->pptr, N, ts->pcol_raw, ts->pcol, ts->big_rows, ts->ctr + 6);
+      k_tc_sort_rows<8><<<num_sms() * 8, 256, 0, s>>>(ts->pptr, N, ts->rank_of_pos, ts->pcol_raw, ts->pcol, ts->fill,
+                                                      ts->pairs, ts->big_rows, ts->ctr + 6);
       LA3G_LAUNCHED();
-      k_tc_sort_big<<<num_sms(), 1024, kTcSortBigSmem, s>>>(ts->pptr, ts->pcol_raw, ts->pcol, ts->big_rows, ts->ctr + 6,
-                                                       ts->ctr + 7);
+      k_tc_sort_big<<<num_sms(), 1024, kTcSortBigSmem, s>>>(ts->pptr, ts->pcol_raw, N, ts->pcol, ts->fill, ts->pairs,
+                                                            ts->big_rows, ts->ctr + 6, ts->ctr + 7);
       LA3G_LAUNCHED();
       tls_launches += 2;
     }
   }
-  k_tc_pair_counts<<<grid_for((uint64_t) N + 1, 256), 256, 0, s>>>(N, ts->pptr, ts->deg_of_rank, ts->mcount,
-                                                                   ts->tcount, ts->tcount2);
-  LA3G_LAUNCHED();
-  tls_launches++;
-  tb = ts->temp_bytes;
-  LA3G_CUDA(cub::DeviceScan::ExclusiveSum(ts->temp, tb, ts->mcount, ts->mptr, (int) N + 1, s));
-  tb = ts->temp_bytes;
-  LA3G_CUDA(cub::DeviceScan::ExclusiveSum(ts->temp, tb, ts->tcount, ts->toff, (int) N + 1, s));
-  tb = ts->temp_bytes;
-  LA3G_CUDA(cub::DeviceScan::ExclusiveSum(ts->temp, tb, ts->tcount2, ts->toff2, (int) N + 1, s));
-  if (m)
-  {
-    LA3G_CUDA(cudaMemsetAsync(ts->fill, 0, (size_t) N * 4, s));
-    const uint64_t m8 = (m + kTcEdgesPerThread - 1) / kTcEdgesPerThread * kTcEdgesPerThread;
-    const unsigned pblocks = (unsigned) ((m8 + m + 256ull * kTcEdgesPerThread - 1) / (256ull * kTcEdgesPerThread));
-    k_tc_pairs<<<pblocks, 256, 0, s>>>(g.in_ptr, g.in_col, g.out_ptr, g.out_row, g.nrows(), N, m, ts->rank_of_pos,
-                                       ts->pptr, ts->pcol, ts->mptr, ts->fill, ts->pairs);
-    LA3G_LAUNCHED();
-    tls_launches++;
-  }
-  k_tc_tasks<<<grid_for(N, 256), 256, 0, s>>>(N, ts->toff, ts->toff2, ts->mptr, ts->wtasks, ts->mtasks, ts->btasks);
-  LA3G_LAUNCHED();
-  tls_launches++;
   return LA3G_OK;
 }
 
@@ -1023,10 +1011,9 @@ extern "C" int la3g_tc(la3g_graph* G, uint64_t* total_out, uint32_t* per_vertex_
     {
       // pass 1: degrees, ranks, N+ rows (count, fill, sort), pair lists,
       // tasks; compulsory bytes: the edge list read by the count and fill
-      // passes, the rows written, sorted (read + write), the adjacency read
-      // once more for the pair lists (8 B per pair), plus the per-vertex
-      // arrays (about 48 B per vertex)
-      ProfileScope p("tc_lists", s, 4.0 * m + 8.0 * m + 8.0 * m + 8.0 * m + 8.0 * m + 48.0 * N);
+      // passes, the rows written, sorted (read + write), the pairs (8 B each),
+      // plus the per-vertex arrays (about 48 B per vertex)
+      ProfileScope p("tc_lists", s, 4.0 * m + 8.0 * m + 8.0 * m + 8.0 * m + 48.0 * N);
       LA3G_TRY(tc_lists(G, ts, attempt == 1));
     }
     LA3G_CUDA(cudaMemsetAsync(ts->ntri, 0, (size_t) N * 4, s));
@@ -1070,7 +1057,7 @@ extern "C" int la3g_tc(la3g_graph* G, uint64_t* total_out, uint32_t* per_vertex_
     st->iterations = 2;
     st->teps_edges = g.nent;
     st->edges_examined = (uint64_t) walked;
-    st->algo_bytes = (uint64_t) (4.0 * walked + 16.0 * m + 8.0 * built + 36.0 * m + 48.0 * N);
+    st->algo_bytes = (uint64_t) (4.0 * walked + 16.0 * m + 8.0 * built + 28.0 * m + 48.0 * N);
   }
   return LA3G_OK;
 }
