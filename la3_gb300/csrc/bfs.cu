@@ -400,12 +400,20 @@ static int bfs_launch(BfsArgs& A, unsigned* grid, cudaStream_t s)
   return LA3G_OK;
 }
 
+// Up to this many vertices the kernel writes the outputs by id straight into
+// pinned host memory, copied to the caller's once it has ended.  Two copies from
+// the device take longer up to about twice this (R-MAT x 8, hops and parents: 2^12
+// 79 us copied, 65 direct; 2^14 87 and 77; 2^16 155 and 154; 2^18 200 and 262).
+static constexpr uint32_t kBfsDirect = 1u << 15;
+static_assert(sizeof(BfsStats) <= 256, "the outputs start 256 bytes behind");
+
 struct BfsScratch
 {
   BfsArgs A{};
   BfsStats* stats = nullptr;   // pinned
   uint8_t* hops_id = nullptr;  // [nslots] outputs by id
   uint32_t* parent_id = nullptr;
+  bool direct = false;         // they are in pinned host memory, behind stats
   unsigned grid = 0;
 };
 
@@ -453,8 +461,14 @@ static int bfs_scratch(la3g_graph* G, BfsScratch** out)
   A.nent = g.nent;
   A.limit = (uint64_t) N + 2;  // every level visits at least one new vertex: more is a fault
   A.pos_of_id = g.pos_of_id;
-  LA3G_CUDA(cudaHostAlloc(&bs->stats, sizeof(BfsStats), cudaHostAllocMapped));
+  bs->direct = N <= kBfsDirect;
+  LA3G_CUDA(cudaHostAlloc(&bs->stats, bs->direct ? 256 + n4 + n1 : sizeof(BfsStats), cudaHostAllocMapped));
   A.stats = bs->stats;
+  if (bs->direct)
+  {
+    bs->parent_id = (uint32_t*) ((char*) bs->stats + 256);
+    bs->hops_id = (uint8_t*) bs->parent_id + n4;
+  }
   *out = bs;
   return LA3G_OK;
 }
@@ -493,9 +507,15 @@ extern "C" int la3g_bfs(la3g_graph* G, uint32_t root, uint8_t* hops_out, uint32_
     LA3G_TRY(bfs_launch<false>(A, &bs->grid, s));
   }
   T.device_end();
-  if (hops_out) LA3G_CUDA(cudaMemcpyAsync(hops_out, bs->hops_id, N, cudaMemcpyDeviceToHost, s));
-  if (parent_out) LA3G_CUDA(cudaMemcpyAsync(parent_out, bs->parent_id, (size_t) N * 4, cudaMemcpyDeviceToHost, s));
+  if (hops_out && !bs->direct) LA3G_CUDA(cudaMemcpyAsync(hops_out, bs->hops_id, N, cudaMemcpyDeviceToHost, s));
+  if (parent_out && !bs->direct)
+    LA3G_CUDA(cudaMemcpyAsync(parent_out, bs->parent_id, (size_t) N * 4, cudaMemcpyDeviceToHost, s));
   LA3G_TRY(T.finish());
+  if (bs->direct)
+  {
+    if (hops_out) std::memcpy(hops_out, bs->hops_id, N);
+    if (parent_out) std::memcpy(parent_out, bs->parent_id, (size_t) N * 4);
+  }
   if (none)
   {
     if (st) st->iterations = 1;

@@ -1172,25 +1172,20 @@ extern "C" int la3g_pr(la3g_graph* G, uint32_t iters, double* rank_out, uint32_t
     st->edges_examined = (uint64_t) it * g.nent + g.nent;
     st->algo_bytes = (uint64_t) ((4.0 * g.nent + 28.0 * N) * it);
   }
-  if (rank_out || degree_out)
+  // the results by id, in the message buffers, which are free now (a buffer for
+  // each call cost its allocation and release, 65 us of a 680 us call at 2^16)
+  if (rank_out)
   {
-    DevBuf tmp;
-    LA3G_TRY(tmp.alloc((size_t) N * 8));
-    if (rank_out)
-    {
-      k_rank_by_id<double><<<grid_for(N, 256), 256, 0, s>>>(N, g.nrows(), ps->L.qpos, g.id_of_pos, ps->rank,
-                                                              tmp.as<double>());
-      LA3G_LAUNCHED();
-      LA3G_CUDA(cudaMemcpyAsync(rank_out, tmp.p, (size_t) N * 8, cudaMemcpyDeviceToHost, s));
-      LA3G_CUDA(cudaStreamSynchronize(s));
-    }
-    if (degree_out)
-    {
-      k_scatter_pos_u32<<<grid_for(N, 256), 256, 0, s>>>(N, g.id_of_pos, ps->deg, tmp.as<uint32_t>());
-      LA3G_LAUNCHED();
-      LA3G_CUDA(cudaMemcpyAsync(degree_out, tmp.p, (size_t) N * 4, cudaMemcpyDeviceToHost, s));
-      LA3G_CUDA(cudaStreamSynchronize(s));
-    }
+    k_rank_by_id<double><<<grid_for(N, 256), 256, 0, s>>>(N, g.nrows(), ps->L.qpos, g.id_of_pos, ps->rank, ps->x[0]);
+    LA3G_LAUNCHED();
+    LA3G_CUDA(cudaMemcpyAsync(rank_out, ps->x[0], (size_t) N * 8, cudaMemcpyDeviceToHost, s));
+  }
+  if (degree_out)
+  {
+    uint32_t* out = (uint32_t*) ps->x[1];
+    k_scatter_pos_u32<<<grid_for(N, 256), 256, 0, s>>>(N, g.id_of_pos, ps->deg, out);
+    LA3G_LAUNCHED();
+    LA3G_CUDA(cudaMemcpyAsync(degree_out, out, (size_t) N * 4, cudaMemcpyDeviceToHost, s));
   }
   return T.finish();
 }
@@ -1211,8 +1206,10 @@ static int pr_f32_run(la3g_graph* G, uint32_t iters, double tol, double* rank_ou
   if (!ps->rankf)
   {
     LA3G_TRY(galloc(G, &ps->rankf, N));
-    LA3G_TRY(galloc(G, &ps->xf[0], (size_t) N + 1));
-    LA3G_TRY(galloc(G, &ps->xf[1], (size_t) N + 1));
+    // one block of memory: the results by id, 8 B each, take the place of both
+    const size_t stride = ((size_t) N + 1 + 63) & ~(size_t) 63;
+    LA3G_TRY(galloc(G, &ps->xf[0], 2 * stride));
+    ps->xf[1] = ps->xf[0] + stride;
     LA3G_TRY(galloc(G, &ps->resid, 1));
   }
   if (tiled && !ps->tile_col)
@@ -1301,11 +1298,10 @@ static int pr_f32_run(la3g_graph* G, uint32_t iters, double tol, double* rank_ou
   }
   if (rank_out)
   {
-    DevBuf tmp;
-    LA3G_TRY(tmp.alloc((size_t) N * 8));
-    k_rank_by_id<float><<<grid_for(N, 256), 256, 0, s>>>(N, g.nrows(), L.qpos, g.id_of_pos, ps->rankf, tmp.as<double>());
+    double* out = (double*) ps->xf[0];  // the messages are no longer needed
+    k_rank_by_id<float><<<grid_for(N, 256), 256, 0, s>>>(N, g.nrows(), L.qpos, g.id_of_pos, ps->rankf, out);
     LA3G_LAUNCHED();
-    LA3G_CUDA(cudaMemcpyAsync(rank_out, tmp.p, (size_t) N * 8, cudaMemcpyDeviceToHost, s));
+    LA3G_CUDA(cudaMemcpyAsync(rank_out, out, (size_t) N * 8, cudaMemcpyDeviceToHost, s));
   }
   LA3G_TRY(T.finish());
   if (residual_out) *residual_out = res;

@@ -71,3 +71,19 @@ def test_levels(gpu, oracle, tmp_path, kind):
                                                  C.c_void_p(torch.cuda.current_stream().cuda_stream), C.byref(st)))
         assert np.array_equal(hops.cpu().numpy(), oh) and np.array_equal(parent.cpu().numpy().view(np.uint32), opar), root
         assert st.iterations == oit, root
+
+
+@pytest.mark.parametrize("n", [32766, 32767, 32768, 32769])
+def test_small_outputs(gpu, oracle, tmp_path, n):
+    """Outputs written to host memory by the kernel, up to a size, else copied."""
+    rec = np.random.default_rng(9).integers(1, n + 1, (3 * n, 2)).astype(np.uint32)
+    p = tmp_path / "g.bin"
+    rec.tofile(p)
+    g = gpu.Graph.load_undirected(p, n)
+    og = oracle.OracleGraph(p, n, 0)
+    for root in (1, 0, n, n + 9, int(rec[0, 0])):
+        oh, op, _ = og.bfs(root)
+        for want in ((True, True), (True, False), (False, True)):
+            hops, parent, _ = gpu.bfs(g, root, *want)
+            assert hops is None or np.array_equal(hops, oh)
+            assert parent is None or np.array_equal(parent, op)
