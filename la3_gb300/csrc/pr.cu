@@ -376,6 +376,36 @@ __device__ __forceinline__ ParityFn exact_scan(ParityFn f, int lane)
   return f;
 }
 
+// Adds a warp's entries, kExactPer per lane in lane order, to s.
+__device__ __forceinline__ void exact_add_warp(const double (&v)[kExactPer], ExactSum& s, int lane)
+{
+  int from = 0;  // lanes below are in the sum already
+  for (;;)
+  {
+    const ParityFn f = exact_scan(lane >= from ? exact_mine(v, s.e) : ParityFn{0, 0}, lane);
+    const uint64_t incl = s.m + ((s.m & 1) ? f.b : f.a);
+    const unsigned over = __ballot_sync(0xffffffffu, incl >= kExactTop);
+    if (!over)
+    {
+      s.m = __shfl_sync(0xffffffffu, incl, 31);
+      return;
+    }
+    const int L = __ffs(over) - 1;
+    uint64_t before = __shfl_up_sync(0xffffffffu, incl, 1);
+    if (lane == 0) before = s.m;
+    double acc = 0.0;
+    if (lane == L)
+    {
+      acc = exact_double(before, s.e);
+#pragma unroll
+      for (int k = 0; k < kExactPer; k++) acc = __dadd_rn(acc, v[k]);
+    }
+    s = exact_of(__shfl_sync(0xffffffffu, acc, L));
+    from = L + 1;
+    if (from == 32) return;
+  }
+}
+
 // One row of n entries (a multiple of 4) by one warp.
 __device__ __forceinline__ double exact_row_warp(const uint32_t* __restrict__ col, const double* __restrict__ x,
                                                  uint32_t n, int lane)
@@ -385,38 +415,15 @@ __device__ __forceinline__ double exact_row_warp(const uint32_t* __restrict__ co
   exact_load(col, x, lane * kExactPer, n, v);
   for (uint32_t base = 0; base < n; base += 32 * kExactPer)  // a warp's rows end at kLongRow
   {
-    int from = 0;  // lanes below are in the sum already
-    for (;;)
-    {
-      const ParityFn f = exact_scan(lane >= from ? exact_mine(v, s.e) : ParityFn{0, 0}, lane);
-      const uint64_t incl = s.m + ((s.m & 1) ? f.b : f.a);
-      const unsigned over = __ballot_sync(0xffffffffu, incl >= kExactTop);
-      if (!over)
-      {
-        s.m = __shfl_sync(0xffffffffu, incl, 31);
-        break;
-      }
-      const int L = __ffs(over) - 1;
-      uint64_t before = __shfl_up_sync(0xffffffffu, incl, 1);
-      if (lane == 0) before = s.m;
-      double acc = 0.0;
-      if (lane == L)
-      {
-        acc = exact_double(before, s.e);
-#pragma unroll
-        for (int k = 0; k < kExactPer; k++) acc = __dadd_rn(acc, v[k]);
-      }
-      s = exact_of(__shfl_sync(0xffffffffu, acc, L));
-      from = L + 1;
-      if (from == 32) break;
-    }
+    exact_add_warp(v, s, lane);
     if (base + 32 * kExactPer < n) exact_load(col, x, base + (32 + lane) * kExactPer, n, v);
   }
   return exact_double(s.m, s.e);
 }
 
-// One row of n entries (a multiple of 4) by one block (WARPS warps): the warps' functions meet in shared
-// memory, every thread composes them and keeps its own copy of the sum.
+// One row of n entries (a multiple of 4) by one block (WARPS warps): the warps'
+// functions meet in shared memory, every thread composes them and keeps its own
+// copy of the sum.
 template <int WARPS>
 __device__ __forceinline__ double exact_row_block(const uint32_t* __restrict__ col, const double* __restrict__ x,
                                                   uint64_t n)
@@ -431,11 +438,21 @@ __device__ __forceinline__ double exact_row_block(const uint32_t* __restrict__ c
   int buf = 0;
   const uint32_t at = threadIdx.x * kExactPer;
   exact_load(col, x, at, (uint32_t) min(n, (uint64_t) kStep), v);
+  // the first entries leave a binade every few additions, and each time costs the
+  // block two barriers: one warp takes them (20 iterations at 2^16 x 16, which the
+  // longest row bounds: 612 us without this, 588 with)
+  if (w == 0)
+  {
+    exact_add_warp(v, s, lane);
+    if (lane == 0) s_acc = exact_double(s.m, s.e);
+  }
+  __syncthreads();
+  s = exact_of(s_acc);
   for (uint64_t base = 0; base < n; base += kStep)
   {
     const uint64_t next = base + kStep;
     if (next < n) exact_load(col + next, x, at, (uint32_t) min(n - next, (uint64_t) kStep), nv);
-    int from = 0;
+    int from = base ? 0 : 32;
     for (;;)
     {
       const ParityFn f = exact_scan((int) threadIdx.x >= from ? exact_mine(v, s.e) : ParityFn{0, 0}, lane);
