@@ -592,12 +592,20 @@ static int pr_prepare(la3g_graph* G, PrScratch** out)
   }
   const uint32_t N = g.nslots, nrows = g.nrows();
   PrLayout& L = ps->L;
-  LA3G_TRY(galloc(G, &ps->deg, N));
-  LA3G_TRY(galloc(G, &ps->flag, 4));
-  LA3G_TRY(galloc(G, &L.qpos, N));
-  LA3G_TRY(galloc(G, &L.xi, N));
-  LA3G_TRY(galloc(G, &L.degq, N));
-  LA3G_TRY(galloc(G, &L.off, (size_t) nrows + 1));
+  // Three allocations (an allocation costs 35 us or more, which a first call on a
+  // small graph would feel): what is kept, the entries, and the working memory,
+  // which holds the temporaries here and the ranks and messages of a call.
+  auto round = [](size_t b) { return (b + 255) & ~(size_t) 255; };
+  const size_t n4 = round((size_t) N * 4), n8 = round((size_t) N * 8 + 8);
+  char* kept = nullptr;
+  LA3G_TRY(galloc(G, &kept, 4 * n4 + n8 + 256));
+  ps->deg = (uint32_t*) kept;
+  L.qpos = (uint32_t*) (kept + n4);
+  L.xi = (uint32_t*) (kept + 2 * n4);
+  L.degq = (uint32_t*) (kept + 3 * n4);
+  L.off = (decltype(L.off)) (kept + 4 * n4);
+  ps->flag = (int*) (kept + 4 * n4 + n8);
+  ps->resid = (double*) (ps->flag + 4);
   LA3G_CUDA(cudaMemsetAsync(ps->deg, 0, (size_t) N * 4, s));
   if (g.nent)
   {
@@ -609,17 +617,15 @@ static int pr_prepare(la3g_graph* G, PrScratch** out)
   int bits = 1;
   while (((uint64_t) (N - 1) >> bits) != 0) bits++;
   const uint32_t mask = (1u << bits) - 1;
-  // one allocation for the temporaries: four key / value arrays, the rows'
-  // entry counts, the library calls' storage, the class bounds
+  // temporaries: four key / value arrays and the slots, the rows' entry counts,
+  // the class bounds, the library calls' storage
   size_t tb0 = 0, tb1 = 0;
   uint32_t* null32 = nullptr;
   uint64_t* null64 = nullptr;
   LA3G_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb0, null32, null32, null32, null32, (int64_t) N, 0, bits + 1, s));
   LA3G_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb1, null64, null64, (int64_t) nrows + 1, s));
-  const size_t n4 = ((size_t) N * 4 + 255) & ~(size_t) 255, n8 = ((size_t) N * 8 + 8 + 255) & ~(size_t) 255;
-  DevBuf tmp;
-  LA3G_TRY(tmp.alloc(5 * n4 + n8 + 256 + std::max(tb0, tb1)));
-  char* t = tmp.as<char>();
+  char* t = nullptr;
+  LA3G_TRY(galloc(G, &t, std::max(5 * n4 + n8 + 256 + std::max(tb0, tb1), 3 * n8)));
   uint32_t *key = (uint32_t*) t, *rkey = (uint32_t*) (t + n4), *key2 = (uint32_t*) (t + 2 * n4);
   uint32_t *iota = (uint32_t*) (t + 3 * n4), *slot = (uint32_t*) (t + 4 * n4);
   uint64_t* take = (uint64_t*) (t + 5 * n4);
@@ -658,6 +664,14 @@ static int pr_prepare(la3g_graph* G, PrScratch** out)
     LA3G_LAUNCHED();
   }
   LA3G_CUDA(cudaStreamSynchronize(s));
+  // the FP64 and the FP32 form share the memory: neither leaves anything in it
+  // for a later call
+  ps->rank = (double*) t;
+  ps->x[0] = (double*) (t + n8);
+  ps->x[1] = (double*) (t + 2 * n8);
+  ps->xf[0] = (float*) t;  // the results by id, 8 B each, take the place of both
+  ps->xf[1] = (float*) (t + n8 / 2);
+  ps->rankf = (float*) (t + n8);
   ps->ready = true;
   *out = ps;
   return LA3G_OK;
@@ -1150,12 +1164,6 @@ extern "C" int la3g_pr(la3g_graph* G, uint32_t iters, double* rank_out, uint32_t
   LA3G_TRY(pr_prepare(G, &ps));
   cudaStream_t s = G->stream;
   const uint32_t N = g.nslots;
-  if (!ps->rank)
-  {
-    LA3G_TRY(galloc(G, &ps->rank, N));
-    LA3G_TRY(galloc(G, &ps->x[0], (size_t) N + 1));
-    LA3G_TRY(galloc(G, &ps->x[1], (size_t) N + 1));
-  }
   T.device_begin();
   k_pr_init<double><<<grid_for((uint64_t) N + 1, 256), 256, 0, s>>>(N, g.nreg, g.src_base(), g.iso_base(), ps->L.degq,
                                                                     ps->L.xi, ps->rank, ps->x[0], ps->x[1]);
@@ -1220,15 +1228,6 @@ static int pr_f32_run(la3g_graph* G, uint32_t iters, double tol, double* rank_ou
   LA3G_TRY(pr_prepare(G, &ps));
   cudaStream_t s = G->stream;
   const uint32_t N = g.nslots;
-  if (!ps->rankf)
-  {
-    LA3G_TRY(galloc(G, &ps->rankf, N));
-    // one block of memory: the results by id, 8 B each, take the place of both
-    const size_t stride = ((size_t) N + 1 + 63) & ~(size_t) 63;
-    LA3G_TRY(galloc(G, &ps->xf[0], 2 * stride));
-    ps->xf[1] = ps->xf[0] + stride;
-    LA3G_TRY(galloc(G, &ps->resid, 1));
-  }
   if (tiled && !ps->tile_col)
   {
     LA3G_TRY(pr_build_tiles(G, ps));
