@@ -40,6 +40,13 @@ static constexpr uint32_t kLongRow = 1024;  // longer rows: a block each
 // FP32 on R-MAT 2^22 (50 iterations: 14.8, 14.5, 13.5, 14.3 ms) and as good as
 // any for FP64 on R-MAT 2^16.
 static constexpr uint32_t kShortRow = 256;
+// On graphs of few rows, which leave SMs idle, a lane's chain of additions is
+// what an iteration waits for, and more rows get a warp (limits 256, 64, 32;
+// R-MAT, 50 FP32 / 20 FP64 iterations: 1024 x 8, 771, 463, 459 / 336, 297, 295 us;
+// 33,001 x 12, 1080, 957, 898 / 507, 460, 494; 65,000 x 16, which has more rows
+// than the line, 1305, 1512, 1531 / 596, 632, 648).
+static constexpr uint32_t kShortRowFew = 64;
+static constexpr uint32_t kFewRows = 1u << 15;
 static constexpr int kWarpsPerBlock = 8;
 
 // ---- the pull layout --------------------------------------------------------
@@ -61,7 +68,7 @@ static constexpr int kWarpsPerBlock = 8;
 // messages in shared memory nor L1 eviction hints were faster).
 struct PrRange  // q's of one class (regular rows or sinks)
 {
-  uint32_t q0, q1, q2, q3;  // [q0, q1) above kLongRow, [q1, q2) above kShortRow, [q2, q3) slices
+  uint32_t q0, q1, q2, q3;  // [q0, q1) above kLongRow, [q1, q2) above the slices' limit, [q2, q3) slices
 };
 
 struct PrLayout
@@ -121,10 +128,10 @@ __global__ void k_pr_keys(uint32_t N, uint32_t nrows, uint32_t nreg, uint32_t ma
 
 // Row classes from the sorted keys: bounds[0..3] = q1, q2 of the regular rows,
 // q1, q2 of the sinks (one thread each).
-__global__ void k_pr_bounds(uint32_t nrows, uint32_t nreg, uint32_t mask, const uint32_t* __restrict__ rkey,
-                            uint32_t* bounds)
+__global__ void k_pr_bounds(uint32_t nrows, uint32_t nreg, uint32_t mask, uint32_t short_row,
+                            const uint32_t* __restrict__ rkey, uint32_t* bounds)
 {
-  const uint32_t t = threadIdx.x, lim = (t & 1) ? kShortRow : kLongRow;
+  const uint32_t t = threadIdx.x, lim = (t & 1) ? short_row : kLongRow;
   uint32_t lo = t < 2 ? 0 : nreg, hi = t < 2 ? nreg : nrows;
   const uint32_t key = (t < 2 ? 0u : mask + 1) + (mask > lim ? mask - lim : 0u);  // the first row with lim or fewer
   while (lo < hi)
@@ -640,7 +647,7 @@ static int pr_prepare(la3g_graph* G, PrScratch** out)
   if (nrows)
   {
     LA3G_CUDA(cub::DeviceRadixSort::SortPairs(lib, tb0, rkey, key, iota, L.qpos, (int64_t) nrows, 0, bits + 1, s));
-    k_pr_bounds<<<1, 4, 0, s>>>(nrows, g.nreg, mask, key, bounds);
+    k_pr_bounds<<<1, 4, 0, s>>>(nrows, g.nreg, mask, nrows <= kFewRows ? kShortRowFew : kShortRow, key, bounds);
     LA3G_LAUNCHED();
   }
   k_pr_rows<<<grid_for(N, 256), 256, 0, s>>>(N, nrows, g.nreg, mask, key, bounds, ps->deg, slot, L.qpos, L.xi, L.degq,
@@ -1258,7 +1265,8 @@ static int pr_f32_run(la3g_graph* G, uint32_t iters, double tol, double* rank_ou
   const double it_bytes = 4.0 * g.nent + 4.0 * (g.nreg + 1) + 4.0 * N + 8.0 * g.nreg + 8.0 * g.nreg + 4.0 * g.nreg;
   for (; it < iters;)
   {
-    LA3G_CUDA(cudaMemsetAsync(ps->resid, 0, 8, s));
+    // the residual is looked at after every iteration, or after the last one only
+    if (tol > 0 || it + 1 == iters) LA3G_CUDA(cudaMemsetAsync(ps->resid, 0, 8, s));
     if (tiled)
     {
       // per tile: its non-empty columns (index, offset, message) and 2 B per
