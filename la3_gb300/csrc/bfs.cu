@@ -58,8 +58,8 @@ struct BfsArgs
   uint32_t root;
   uint8_t* hops;
   // [N] while the hops fit a byte (the first 254 levels): 0, or the parent's
-  // key + 1, which a level's visitors raise by atomicMax; later: a level's
-  // candidate, moved to `parent` at its end
+  // key + 1 (bfs_code), which a level's visitors raise by atomicMax; later: a
+  // level's candidate, moved to `parent` at its end
   uint32_t* cand;
   uint32_t* parent;                 // [N] later levels' parents
   uint32_t* list[2];                // [N] frontier lists
@@ -117,6 +117,28 @@ struct HubList
 __device__ __forceinline__ FrontierCounters bfs_counters(const FrontierCounters* c)
 {
   return {__ldcg(&c->raw), __ldcg(&c->degsum), __ldcg(&c->nsmall), __ldcg(&c->packed)};
+}
+
+// A parent's key as cand holds it: above 0, ascending with the key.  A caller's
+// keys (CHECK) may be any 32-bit numbers; the two largest share a code.
+template <bool CHECK>
+__device__ __forceinline__ uint32_t bfs_code(uint32_t key)
+{
+  return CHECK ? key + (key != 0xFFFFFFFFu) : key + 1;
+}
+
+// The key behind the code x of v, which was reached at `hop`: where two keys
+// share it, the larger one if a neighbour with that key was in the frontier.
+template <bool CHECK>
+__device__ __forceinline__ uint32_t bfs_key_of(const BfsArgs& A, uint32_t v, uint32_t x, uint8_t hop)
+{
+  if (CHECK && x == 0xFFFFFFFFu)
+    for (uint32_t i = A.ptr[v + 1]; i > A.ptr[v]; i--)
+    {
+      const uint32_t u = A.col[i - 1];
+      if (u < A.N && A.key[u] == x && A.hops[u] == (uint8_t) (hop - 1)) return x;
+    }
+  return x - 1;
 }
 
 // CHECK: the CSR comes from the caller; neighbour ids outside the graph are
@@ -269,7 +291,7 @@ __global__ void __launch_bounds__(kBfsThreads, 3) k_bfs_run(BfsArgs A)
             {
               A.hops[v] = hop;
               if (wide) A.parent[v] = A.key[from];
-              else A.cand[v] = A.key[from] + 1;
+              else A.cand[v] = bfs_code<CHECK>(A.key[from]);
               deg += e - b;
               cnt++;
             }
@@ -324,14 +346,14 @@ __global__ void __launch_bounds__(kBfsThreads, 3) k_bfs_run(BfsArgs A)
       if (!wide)
         for (uint32_t t = warp; t < ntasks; t += nwarps)
         {
-          const uint32_t slot = H.of_task(nbig, t), u = H.big[-(int64_t) slot], hu = A.key[u] + 1;
+          const uint32_t slot = H.of_task(nbig, t), u = H.big[-(int64_t) slot], hu = bfs_code<CHECK>(A.key[u]);
           const uint32_t b = A.ptr[u] + (t - H.task0[(int64_t) slot * H.dir]) * kHubTask;
           const uint32_t e = min(b + kHubTask, A.ptr[u + 1]);
           for (uint32_t i0 = b; i0 < e; i0 += 32) visit(i0 + lane, e, hu);
         }
       for (uint32_t f = warp; f < nsmall + (wide ? nbig : 0); f += nwarps)
       {
-        const uint32_t u = f < nsmall ? A.list[c][f] : H.big[-(int64_t) (f - nsmall)], hu = A.key[u] + 1;
+        const uint32_t u = f < nsmall ? A.list[c][f] : H.big[-(int64_t) (f - nsmall)], hu = bfs_code<CHECK>(A.key[u]);
         const uint32_t b = A.ptr[u], e = A.ptr[u + 1];
         for (uint32_t i0 = b; i0 < e; i0 += 32) visit(i0 + lane, e, hu);
       }
@@ -343,7 +365,7 @@ __global__ void __launch_bounds__(kBfsThreads, 3) k_bfs_run(BfsArgs A)
         {
           const uint32_t v = A.list[c ^ 1][i];
           A.hops[v] = hop;
-          A.parent[v] = A.cand[v] - 1;
+          A.parent[v] = bfs_key_of<CHECK>(A, v, A.cand[v], hop);
           A.cand[v] = 0;
           deg += A.ptr[v + 1] - A.ptr[v];
         }
@@ -370,7 +392,7 @@ __global__ void __launch_bounds__(kBfsThreads, 3) k_bfs_run(BfsArgs A)
     if (A.parent_out)
     {
       const uint32_t x = A.cand[p];
-      A.parent_out[i] = x ? x - 1 : wide ? A.parent[p] : 0;
+      A.parent_out[i] = x ? bfs_key_of<CHECK>(A, p, x, A.hops[p]) : wide ? A.parent[p] : 0;
     }
   }
   if (wide)
