@@ -204,6 +204,14 @@ int la3g_bfs(la3g_graph* g, uint32_t root, uint8_t* hops_out, uint32_t* parent_o
  * 2147483647 = unreached. */
 int la3g_sssp(la3g_graph* g, uint32_t root, uint32_t* dist_out, la3g_stats* st);
 
+/* la3g_bfs and la3g_sssp run as one kernel whose blocks wait for one another
+ * at grid barriers.  A block waits at most `polls` polls (polls < 0: the
+ * default); when one runs out, every block leaves the kernel, and the call
+ * returns LA3G_ETIMEOUT with the device left usable and the outputs undefined.
+ * No counterpart in the reference (it has no device waits); polls = 0 makes
+ * any wait give up at once, which exercises that error path. */
+int la3g_set_wait_limit(la3g_graph* g, long long polls);
+
 /* Connected components (src/apps/graph_analytics/cc.cpp:11-31, cc.h:11-38)
  * on an undirected graph: labels as the reference computes them (the least
  * vertex id of each component when vertex 0 has no edges). */
@@ -287,9 +295,9 @@ int la3g_batch_autotune(la3g_graph* g, const uint32_t* roots, uint32_t nroots, c
 int la3g_batch_config(la3g_graph* g, int mode, int block, double push_frac);
 
 /* In mode 1 the batched-BFS kernel's grid barriers wait at most `polls`
- * polls per block (default 2^26, restored by polls < 0); a block that runs
- * out sets an error word, every block leaves its kernel, and the call returns
- * LA3G_ETIMEOUT with the device left usable.  No counterpart in the
+ * polls per block (default 2^26, restored by polls < 0); when a block runs
+ * out, every block leaves its kernel, and the call returns LA3G_ETIMEOUT with
+ * the device left usable.  No counterpart in the
  * reference (it has no device waits); polls = 0 makes any wait give up at
  * once, which exercises that error path. */
 int la3g_batch_set_wait_limit(la3g_graph* g, long long polls);

@@ -121,6 +121,10 @@ class Graph:
         torch.cuda.current_stream().cuda_stream); None = the graph's own."""
         N.check(N.lib().la3g_graph_set_stream(self._h, C.c_void_p(cuda_stream) if cuda_stream else None))
 
+    def set_wait_limit(self, polls: int = -1) -> None:
+        """Grid-barrier poll limit of bfs and sssp on this graph (< 0: the default)."""
+        N.check(N.lib().la3g_set_wait_limit(self._h, polls))
+
     def positions(self) -> tuple[np.ndarray, np.ndarray]:
         pos = np.empty(self.nslots, np.uint32)
         ids = np.empty(self.nslots, np.uint32)

@@ -137,6 +137,7 @@ SIGNATURES = {
     "la3g_graph_free": (None, [_P]),
     "la3g_graph_info_get": (C.c_int, [_P, C.POINTER(GraphInfo)]),
     "la3g_graph_set_stream": (C.c_int, [_P, _P]),
+    "la3g_set_wait_limit": (C.c_int, [_P, C.c_longlong]),
     "la3g_graph_positions": (C.c_int, [_P, _u32p, _u32p]),
     "la3g_graph_device_view": (C.c_int, [_P, C.POINTER(DeviceGraph)]),
     "la3g_graph_push_view": (C.c_int, [_P, C.POINTER(_P), C.POINTER(_P)]),

@@ -47,8 +47,8 @@ struct BatchConfig
   bool tuned = false;
 };
 
-// Polls a block makes at a grid barrier before it gives up (sets the error
-// word, every block leaves, the call returns LA3G_ETIMEOUT);
+// Polls a block makes at a grid barrier before it gives up (every block leaves,
+// the call returns LA3G_ETIMEOUT);
 // la3g_batch_set_wait_limit changes it per graph for mode 1.
 static constexpr long long kDefaultWaitPolls = 1ll << 26;
 
@@ -69,7 +69,7 @@ struct BatchScratch
   // hubs, [4 + c] smallest distance list c holds
   unsigned long long* ctr = nullptr;
   unsigned long long* hctr = nullptr;  // pinned, written by the kernels: [0] levels / iterations, [1] status
-  unsigned int* bar = nullptr;         // grid barrier: count, error word
+  unsigned long long* bar = nullptr;   // grid barrier's count
   uint8_t* tpos = nullptr;             // results by root and id, before they leave the device
   size_t tpos_bytes = 0;
   BatchConfig cfg;                           // set by hand, or the default
@@ -139,7 +139,7 @@ struct MsArgs
   uint8_t* hops;
   PairList list;       // pushing levels: the frontier's pairs
   unsigned long long* ctr;
-  unsigned int* bar;
+  unsigned long long* bar;
   long long wait_polls;
   // a level pushes when its new bits x mean degree stay below the limit
   double mean_deg, push_limit;
@@ -177,7 +177,7 @@ __device__ __forceinline__ uint32_t ms_found(const MsArgs& A, uint64_t base, boo
 __global__ void __launch_bounds__(512) k_ms_run(MsArgs A)
 {
   __shared__ unsigned long long s_alive[kMsAliveShared], s_got[3];
-  GridBarrier bar{A.bar, (int*) (A.bar + 1), A.wait_polls};
+  GridBarrier bar{A.bar, A.wait_polls};
   const int lane = threadIdx.x & 31;
   const uint64_t tid = (uint64_t) blockIdx.x * blockDim.x + threadIdx.x, nth = (uint64_t) gridDim.x * blockDim.x;
   const uint64_t NW = (uint64_t) A.nrows * A.W;
@@ -300,7 +300,7 @@ static int batch_scratch(la3g_graph* G, BatchScratch** out)
     G->slot[kSlotBatch] = b;
     G->slot_free[kSlotBatch] = batch_scratch_free;
     LA3G_TRY(galloc(G, &b->ctr, 8));
-    LA3G_TRY(galloc(G, &b->bar, 2));
+    LA3G_TRY(galloc(G, &b->bar, 1));
     LA3G_CUDA(cudaHostAlloc(&b->hctr, 2 * sizeof(unsigned long long), cudaHostAllocMapped));
   }
   *out = b;
@@ -475,7 +475,7 @@ struct BsArgs
   PairList L[2];            // their counters: ctr[c], ctr[2 + c]
   uint32_t* dist;
   unsigned long long* ctr;
-  unsigned int* bar;
+  unsigned long long* bar;
   uint32_t delta;           // kNoWindow: no window
   unsigned long long* out;  // pinned: iterations, status
 };
@@ -488,7 +488,7 @@ __global__ void __launch_bounds__(256, 4) k_bs_run(BsArgs A)
 {
   __shared__ unsigned long long s_got[3];
   __shared__ unsigned int s_taken;
-  GridBarrier bar{A.bar, (int*) (A.bar + 1), kDefaultWaitPolls};
+  GridBarrier bar{A.bar, kDefaultWaitPolls};
   const uint64_t tid = (uint64_t) blockIdx.x * blockDim.x + threadIdx.x;
   uint32_t iters = 0, limit = A.delta;
   int cur = 0;

@@ -66,7 +66,8 @@ struct BfsArgs
   uint32_t* task0;                  // [N] first task numbers of the hubs: even levels from the front, odd from the back
   uint32_t* bits[2];                // [N / 32 + 1] frontier bitmaps
   FrontierCounters* ctr;            // [3]
-  unsigned int* bar;                // barrier count, then the error word
+  unsigned long long* bar;          // barrier count
+  long long wait_polls;
   const uint32_t* pos_of_id;        // null: ids are positions
   uint8_t* hops_out;                // by id, or null
   uint32_t* parent_out;             // by id, or null
@@ -147,7 +148,7 @@ template <bool CHECK>
 __global__ void __launch_bounds__(kBfsThreads, 3) k_bfs_run(BfsArgs A)
 {
   __shared__ FrontierCounters s_next;
-  GridBarrier bar{A.bar, (int*) (A.bar + 1), kBarrierPolls};
+  GridBarrier bar{A.bar, A.wait_polls};
   const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
   const uint32_t lane = threadIdx.x & 31, warp = tid >> 5, nwarps = nth >> 5;
   const uint32_t words = (A.N + 31) / 32;
@@ -474,7 +475,7 @@ static int bfs_scratch(la3g_graph* G, BfsScratch** out)
   A.bits[0] = (uint32_t*) take(nb);
   A.bits[1] = (uint32_t*) take(nb);
   A.ctr = (FrontierCounters*) take(256);
-  A.bar = (unsigned int*) take(256);
+  A.bar = (unsigned long long*) take(256);
   A.ptr = g.in_ptr;
   A.col = g.in_col;
   A.key = g.hash_of_pos;
@@ -521,6 +522,7 @@ extern "C" int la3g_bfs(la3g_graph* G, uint32_t root, uint8_t* hops_out, uint32_
   {
     BfsArgs A = bs->A;
     A.root = root;
+    A.wait_polls = G->wait_polls < 0 ? kBarrierPolls : G->wait_polls;
     bs->stats->status = kBfsRunning;
     A.hops_out = hops_out ? bs->hops_id : nullptr;
     A.parent_out = parent_out ? bs->parent_id : nullptr;
@@ -592,7 +594,7 @@ static constexpr size_t kNaBits0Off = kNaList1Off + na_round(sizeof(uint32_t) * 
 static constexpr size_t kNaBits1Off = kNaBits0Off + na_round(sizeof(uint32_t) * kNaWords);
 static constexpr size_t kNaCtrOff = kNaBits1Off + na_round(sizeof(uint32_t) * kNaWords);
 static constexpr size_t kNaBarOff = kNaCtrOff + na_round(3 * sizeof(FrontierCounters));
-static constexpr size_t kNaStatsOff = kNaBarOff + na_round(2 * sizeof(unsigned int));
+static constexpr size_t kNaStatsOff = kNaBarOff + na_round(sizeof(unsigned long long));
 static constexpr size_t kNoAllocScratchBytes = kNaStatsOff + na_round(sizeof(BfsStats));
 
 static __device__ __align__(256) unsigned char g_bfs_noalloc_scratch[kNoAllocScratchBytes];
@@ -676,7 +678,8 @@ static int bfs_noalloc_run(const uint32_t* row_ptr, const uint32_t* col, const u
     A.bits[0] = (uint32_t*) (base + kNaBits0Off);
     A.bits[1] = (uint32_t*) (base + kNaBits1Off);
     A.ctr = (FrontierCounters*) (base + kNaCtrOff);
-    A.bar = (unsigned int*) (base + kNaBarOff);
+    A.bar = (unsigned long long*) (base + kNaBarOff);
+    A.wait_polls = kBarrierPolls;
     A.stats = (BfsStats*) (base + kNaStatsOff);
     unsigned grid = 0;
     LA3G_CUDA(cudaMemsetAsync(&A.stats->status, 0xFF, sizeof r.status, s));

@@ -520,6 +520,13 @@ extern "C" int la3g_graph_set_stream(la3g_graph* g, void* cuda_stream)
   return LA3G_OK;
 }
 
+extern "C" int la3g_set_wait_limit(la3g_graph* g, long long polls)
+{
+  if (!g) return set_error(LA3G_EINVAL, "null graph");
+  g->wait_polls = polls;
+  return LA3G_OK;
+}
+
 extern "C" int la3g_graph_from_records(const void* records, uint64_t nrec, uint32_t n, uint32_t nright,
                                        uint32_t flags, la3g_graph** out)
 {

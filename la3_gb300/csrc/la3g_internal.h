@@ -115,40 +115,49 @@ __device__ __forceinline__ uint32_t block_min_u32(uint32_t v)
   return v;
 }
 
-// Barrier over the blocks of a cooperative launch.  `count` starts at zero; a
-// block that waits more than `limit` polls sets *err and every block leaves its
-// kernel at its next barrier (sync() returns false in all its threads).  Every
-// thread of every block calls sync() the same number of times.  Like
+// Barrier over the blocks of a cooperative launch.  `count` starts at zero.  A
+// block that waits more than `limit` polls gives up: sync() returns false in all
+// its threads, which then leave the kernel, and so does every other block's.  A
+// barrier is passed by every block or by none, so that what lies between two of
+// them is done whole or the kernel does not get past it: giving up sets the
+// count's top bit, only while the count is below the barrier's target.  No block
+// then gets to the next barrier, so a count above the target, which only blocks
+// at the next one can have made, says that the bit was set there.
+// Every thread of every block calls sync() the same number of times.  Like
 // cooperative groups' grid barrier it is a fence at device scope, after which
 // ordinary loads see what the other blocks wrote before it.
 struct GridBarrier
 {
-  unsigned int* count;
-  int* err;
+  static constexpr unsigned long long kGaveUp = 1ull << 63;
+  unsigned long long* count;
   long long limit;
-  unsigned int phase = 0;
+  unsigned long long target = 0;
   __device__ bool sync()
   {
     __shared__ int s_ok;
-    phase++;
+    target += gridDim.x;
     __syncthreads();
     if (threadIdx.x == 0)
     {
-      const unsigned int target = phase * gridDim.x;
       __threadfence();
-      atomicAdd(count, 1u);
-      volatile unsigned int* c = count;
+      atomicAdd(count, 1ull);
+      volatile unsigned long long* c = count;
       long long polls = 0;
-      int ok = 1;
-      while ((int) (*c - target) < 0)
-        if (++polls > limit || ((polls & 63) == 0 && *(volatile int*) err))
+      for (;;)
+      {
+        const unsigned long long x = *c, arrived = x & ~kGaveUp;
+        if (x & kGaveUp ? arrived > target : arrived >= target)
         {
-          atomicExch(err, 1);
-          ok = 0;
+          s_ok = 1;
           break;
         }
+        if (x & kGaveUp || (++polls > limit && atomicCAS(count, x, x | kGaveUp) == x))
+        {
+          s_ok = 0;
+          break;
+        }
+      }
       __threadfence();
-      s_ok = ok;
     }
     __syncthreads();
     return s_ok;
@@ -254,6 +263,7 @@ struct la3g_graph
   cudaStream_t stream = nullptr;       // stream the calls run on
   cudaStream_t own_stream = nullptr;   // the graph's own stream
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  long long wait_polls = -1;           // la3g_set_wait_limit; < 0: the default
   std::vector<void*> allocations;
   uint64_t device_bytes = 0;
   void* slot[la3g::kSlotCount] = {};

@@ -81,7 +81,8 @@ struct SsspArgs
   unsigned long long* fctr;       // [0] small-list length, [1] hub slots and tasks
   SsspCounters* ctr;              // [3]
   unsigned long long* reached;
-  unsigned int* bar;
+  unsigned long long* bar;
+  long long wait_polls;
   uint32_t root;
   uint32_t* dist_out;             // by id, or null
   SsspStats* stats;
@@ -407,7 +408,7 @@ __global__ void __launch_bounds__(kSsspThreads, 3) k_sssp_run(SsspArgs A)
 {
   __shared__ SsspCounters s_got;
   __shared__ unsigned long long s_list[2];
-  GridBarrier bar{A.bar, (int*) (A.bar + 1), kBarrierPolls};
+  GridBarrier bar{A.bar, A.wait_polls};
   const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
   const uint32_t lane = threadIdx.x & 31, warp = tid >> 5, nwarps = nth >> 5;
   const uint32_t words = A.N / 32 + 1;
@@ -555,7 +556,7 @@ static int sssp_scratch(la3g_graph* G, SsspScratch** out)
   LA3G_TRY(galloc(G, &A.ctr, 3));
   LA3G_TRY(galloc(G, &A.fctr, 4));  // with `reached` and the barrier
   A.reached = A.fctr + 2;
-  A.bar = (unsigned int*) (A.fctr + 3);
+  A.bar = A.fctr + 3;
   LA3G_TRY(galloc(G, &A.fbits, (size_t) N / 32 + 2));
   LA3G_TRY(galloc(G, &A.pbits, (size_t) N / 32 + 2));
   LA3G_TRY(galloc(G, &ss->by_id, N));
@@ -673,6 +674,7 @@ extern "C" int la3g_sssp(la3g_graph* G, uint32_t root, uint32_t* dist_out, la3g_
   const uint32_t N = g.nslots;
   SsspArgs A = ss->A;
   A.root = root;
+  A.wait_polls = G->wait_polls < 0 ? kBarrierPolls : G->wait_polls;
   A.dist_out = dist_out ? ss->by_id : nullptr;
   ss->stats->status = kSsspRunning;
   if (!ss->grid)  // few blocks for a small graph: a barrier takes longer the more there are
