@@ -206,7 +206,8 @@ int la3g_sssp(la3g_graph* g, uint32_t root, uint32_t* dist_out, la3g_stats* st);
 
 /* la3g_bfs and la3g_sssp run as one kernel whose blocks wait for one another
  * at grid barriers.  A block waits at most `polls` polls (polls < 0: the
- * default); when one runs out, every block leaves the kernel, and the call
+ * default, 2^26 and 8 per stored entry, above what any list of the graph takes
+ * to walk); when one runs out, every block leaves the kernel, and the call
  * returns LA3G_ETIMEOUT with the device left usable and the outputs undefined.
  * No counterpart in the reference (it has no device waits); polls = 0 makes
  * any wait give up at once, which exercises that error path. */
@@ -295,11 +296,11 @@ int la3g_batch_autotune(la3g_graph* g, const uint32_t* roots, uint32_t nroots, c
 int la3g_batch_config(la3g_graph* g, int mode, int block, double push_frac);
 
 /* In mode 1 the batched-BFS kernel's grid barriers wait at most `polls`
- * polls per block (default 2^26, restored by polls < 0); when a block runs
- * out, every block leaves its kernel, and the call returns LA3G_ETIMEOUT with
- * the device left usable.  No counterpart in the
- * reference (it has no device waits); polls = 0 makes any wait give up at
- * once, which exercises that error path. */
+ * polls per block (polls < 0: the default, as for la3g_set_wait_limit); when a
+ * block runs out, every block leaves its kernel, and the call returns
+ * LA3G_ETIMEOUT with the device left usable.  No counterpart in the reference
+ * (it has no device waits); polls = 0 makes any wait give up at once, which
+ * exercises that error path. */
 int la3g_batch_set_wait_limit(la3g_graph* g, long long polls);
 
 /* The batched SSSP's distance window: an iteration relaxes only the roots
@@ -403,7 +404,9 @@ void la3g_server_free(la3g_server* s);
  * one fixed device array of about 12.8 MB, so nvertices is limited to
  * 1048576 (2^20); larger graphs are rejected with LA3G_EINVAL.  Each call
  * looks up the array's address on the current device (no allocation).  The
- * call waits for its stream before it returns, also after an error.
+ * call waits for its stream before it returns, also after an error.  Its
+ * kernel's grid barriers wait as long as la3g_bfs's by default
+ * (la3g_set_wait_limit); LA3G_ETIMEOUT if a wait runs out.
  * Calls share the array, so calls that overlap on the GPU race; run them one
  * at a time.  row_ptr must be non-decreasing with row_ptr[nvertices] = the
  * entry count; that is not checked, while neighbour ids >= nvertices are

@@ -47,14 +47,9 @@ struct BatchConfig
   bool tuned = false;
 };
 
-// Polls a block makes at a grid barrier before it gives up (every block leaves,
-// the call returns LA3G_ETIMEOUT);
-// la3g_batch_set_wait_limit changes it per graph for mode 1.
-static constexpr long long kDefaultWaitPolls = 1ll << 26;
-
 struct BatchScratch
 {
-  long long wait_polls = kDefaultWaitPolls;  // grid-barrier poll limit in mode 1
+  long long wait_polls = -1; // grid-barrier poll limit in mode 1 (la3g_batch_set_wait_limit; < 0: the default)
   uint32_t cap_r = 0;        // roots the buffers were sized for
   uint64_t* vis = nullptr;   // [N][W]
   uint64_t* buf[2] = {nullptr, nullptr};  // frontier / next, [N][W]
@@ -367,7 +362,7 @@ static int ms_bfs_run(la3g_graph* G, BatchScratch* b, const uint32_t* roots_host
   A.list = PairList{b->active, b->phub, b->phub_t0, b->ctr + 3, b->ctr + 4};
   A.ctr = b->ctr;
   A.bar = b->bar;
-  A.wait_polls = cfg.mode == 1 ? b->wait_polls : kDefaultWaitPolls;
+  A.wait_polls = barrier_polls(cfg.mode == 1 ? b->wait_polls : -1, g.nent);
   A.mean_deg = (double) g.nent / std::max<uint32_t>(1, nrows);
   A.push_limit = cfg.mode == 1 ? 0.0 : cfg.push_frac * (double) g.nent * 64.0 * W;
   A.out = b->hctr;
@@ -476,6 +471,7 @@ struct BsArgs
   uint32_t* dist;
   unsigned long long* ctr;
   unsigned long long* bar;
+  long long wait_polls;
   uint32_t delta;           // kNoWindow: no window
   unsigned long long* out;  // pinned: iterations, status
 };
@@ -488,7 +484,7 @@ __global__ void __launch_bounds__(256, 4) k_bs_run(BsArgs A)
 {
   __shared__ unsigned long long s_got[3];
   __shared__ unsigned int s_taken;
-  GridBarrier bar{A.bar, kDefaultWaitPolls};
+  GridBarrier bar{A.bar, A.wait_polls};
   const uint64_t tid = (uint64_t) blockIdx.x * blockDim.x + threadIdx.x;
   uint32_t iters = 0, limit = A.delta;
   int cur = 0;
@@ -762,6 +758,7 @@ static int sssp_batch_chunk(la3g_graph* G, BatchScratch* b, const uint32_t* root
   A.dist = b->sdist;
   A.ctr = b->ctr;
   A.bar = b->bar;
+  A.wait_polls = barrier_polls(-1, g.nent);
   A.delta = delta;
   A.out = b->hctr;
   b->hctr[1] = 0;
@@ -869,7 +866,7 @@ extern "C" int la3g_batch_set_wait_limit(la3g_graph* G, long long polls)
   if (!G) return set_error(LA3G_EINVAL, "null graph");
   BatchScratch* b = nullptr;
   LA3G_TRY(batch_scratch(G, &b));
-  b->wait_polls = polls < 0 ? kDefaultWaitPolls : polls;
+  b->wait_polls = polls;
   return LA3G_OK;
 }
 

@@ -67,7 +67,7 @@ struct BfsArgs
   uint32_t* bits[2];                // [N / 32 + 1] frontier bitmaps
   FrontierCounters* ctr;            // [3]
   unsigned long long* bar;          // barrier count
-  long long wait_polls;
+  long long wait_polls;             // < 0: the default
   const uint32_t* pos_of_id;        // null: ids are positions
   uint8_t* hops_out;                // by id, or null
   uint32_t* parent_out;             // by id, or null
@@ -148,12 +148,12 @@ template <bool CHECK>
 __global__ void __launch_bounds__(kBfsThreads, 3) k_bfs_run(BfsArgs A)
 {
   __shared__ FrontierCounters s_next;
-  GridBarrier bar{A.bar, A.wait_polls};
   const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
   const uint32_t lane = threadIdx.x & 31, warp = tid >> 5, nwarps = nth >> 5;
   const uint32_t words = (A.N + 31) / 32;
   const uint32_t rp = A.pos_of_id ? A.pos_of_id[A.root] : A.root;
   const uint64_t nent = CHECK ? A.ptr[A.N] : A.nent;
+  GridBarrier bar{A.bar, barrier_polls(A.wait_polls, nent)};
   const uint32_t rdeg = rp < A.nrows ? A.ptr[rp + 1] - A.ptr[rp] : 0;
 
   // everything unvisited, the root at 0 and in the first frontier
@@ -522,7 +522,7 @@ extern "C" int la3g_bfs(la3g_graph* G, uint32_t root, uint8_t* hops_out, uint32_
   {
     BfsArgs A = bs->A;
     A.root = root;
-    A.wait_polls = G->wait_polls < 0 ? kBarrierPolls : G->wait_polls;
+    A.wait_polls = G->wait_polls;
     bs->stats->status = kBfsRunning;
     A.hops_out = hops_out ? bs->hops_id : nullptr;
     A.parent_out = parent_out ? bs->parent_id : nullptr;
@@ -679,7 +679,7 @@ static int bfs_noalloc_run(const uint32_t* row_ptr, const uint32_t* col, const u
     A.bits[1] = (uint32_t*) (base + kNaBits1Off);
     A.ctr = (FrontierCounters*) (base + kNaCtrOff);
     A.bar = (unsigned long long*) (base + kNaBarOff);
-    A.wait_polls = kBarrierPolls;
+    A.wait_polls = -1;
     A.stats = (BfsStats*) (base + kNaStatsOff);
     unsigned grid = 0;
     LA3G_CUDA(cudaMemsetAsync(&A.stats->status, 0xFF, sizeof r.status, s));

@@ -164,8 +164,16 @@ struct GridBarrier
   }
 };
 
-// Polls of a barrier before it gives up (a few seconds).
-static constexpr long long kBarrierPolls = 1ll << 23;
+// Polls of a barrier before it gives up, by default: 2^26 (ten seconds or more;
+// a poll takes 0.15 us) and kEntryPolls for each entry of the matrix, since a
+// lane may walk a whole list between two barriers (the neighbours of a vertex in
+// a bottom-up level, a sink's in-edges: 0.05 and 0.14 us an entry, up to four
+// times that where the reads miss L2): work that is only long is waited for.
+static constexpr long long kBarrierPolls = 1ll << 26, kEntryPolls = 8;
+__host__ __device__ inline long long barrier_polls(long long set, uint64_t entries)
+{
+  return set < 0 ? kBarrierPolls + kEntryPolls * (long long) entries : set;
+}
 
 // Blocks of a cooperative launch of `f`: enough for `want` threads, at most
 // as many as are resident at once (and max_per_sm per SM).

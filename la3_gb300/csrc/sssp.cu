@@ -674,7 +674,7 @@ extern "C" int la3g_sssp(la3g_graph* G, uint32_t root, uint32_t* dist_out, la3g_
   const uint32_t N = g.nslots;
   SsspArgs A = ss->A;
   A.root = root;
-  A.wait_polls = G->wait_polls < 0 ? kBarrierPolls : G->wait_polls;
+  A.wait_polls = barrier_polls(G->wait_polls, g.nent);
   A.dist_out = dist_out ? ss->by_id : nullptr;
   ss->stats->status = kSsspRunning;
   if (!ss->grid)  // few blocks for a small graph: a barrier takes longer the more there are

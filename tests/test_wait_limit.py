@@ -61,3 +61,34 @@ def test_runs_out_in_the_last_level(gpu):
         with pytest.raises(L.N.LA3GError) as e:
             L.bfs(g, 1)
         assert e.value.status == ETIMEOUT
+
+
+def test_long_sink_is_waited_for(gpu):
+    """One lane walks the in-edges of a sink (seconds): slow, but an answer."""
+    L = gpu
+    m = (1 << 24) - 1
+    i = np.arange(2, m + 2, dtype=np.uint32)
+    rec = np.full((3 * m, 3), 7, np.uint32)
+    rec[:m, 0], rec[:m, 1] = 1, i
+    rec[m: 2 * m, 0], rec[m: 2 * m, 1] = i, 1  # regular vertices: their distances are looked up
+    rec[2 * m:, 0], rec[2 * m:, 1] = i, m + 2
+    g = L.Graph.from_records(rec, m + 2, L.DIRECTED | L.WEIGHTED)
+    want = np.full(m + 3, 7, np.uint32)
+    want[[0, 1, m + 2]] = 0x7FFFFFFF, 0, 14
+    assert np.array_equal(L.sssp(g, 1)[0], want)
+
+
+def test_long_unreached_hub_is_waited_for(gpu):
+    """One lane looks through all neighbours of a hub that the root does not reach."""
+    L = gpu
+    k, m, b = 64, 98_304, 36 << 20
+    mid = np.arange(2, 2 + k, dtype=np.uint32)
+    leaf = np.arange(2 + k, 2 + k + m, dtype=np.uint32)
+    hub = 2 + k + m
+    rec = np.concatenate([np.stack([np.full(k, 1, np.uint32), mid], 1), np.stack([np.repeat(mid, m), np.tile(leaf, k)], 1),
+                          np.stack([np.full(b, hub, np.uint32), np.arange(hub + 1, hub + 1 + b, dtype=np.uint32)], 1)])
+    g = L.Graph.from_records(rec, hub + b, 0)
+    want = np.full(g.nslots, 255, np.uint8)
+    want[1], want[mid], want[leaf] = 0, 1, 2
+    hops, _, st = L.bfs(g, 1, want_parent=False)
+    assert st.pull_iterations > 0 and np.array_equal(hops, want)
