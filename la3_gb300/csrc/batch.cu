@@ -55,7 +55,7 @@ struct BatchScratch
   uint64_t* buf[2] = {nullptr, nullptr};  // frontier / next, [N][W]
   uint64_t* alive[3] = {nullptr, nullptr, nullptr};  // [W] per-word "discovered something" masks
   uint8_t* hops = nullptr;   // [N][W * 64] by position (vertex-major)
-  uint32_t* rpos = nullptr;  // root positions
+  uint32_t* rpos = nullptr;  // [R] root ids, then positions
   uint32_t* active = nullptr;  // push: active (vertex, word) pairs of small vertices
   uint32_t* phub = nullptr;    // push: pairs of hub vertices, and their first task numbers
   uint32_t* phub_t0 = nullptr;
@@ -320,11 +320,11 @@ static int ms_bfs_alloc(la3g_graph* G, BatchScratch* b, uint32_t R)
   return LA3G_OK;
 }
 
-__global__ void k_root_pos(const uint32_t* __restrict__ ids, uint32_t R, uint32_t N, const uint32_t* __restrict__ pos_of_id,
-                           uint32_t* out)
+// Root ids -> positions, in place.
+__global__ void k_root_pos(uint32_t R, uint32_t N, const uint32_t* __restrict__ pos_of_id, uint32_t* rpos)
 {
   for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < R; r += gridDim.x * blockDim.x)
-    out[r] = ids[r] < N ? pos_of_id[ids[r]] : 0xFFFFFFFFu;
+    rpos[r] = rpos[r] < N ? pos_of_id[rpos[r]] : 0xFFFFFFFFu;
 }
 
 // Runs one batch; hops by position stay in b->hops.  Returns the level count
@@ -336,8 +336,8 @@ static int ms_bfs_run(la3g_graph* G, BatchScratch* b, const uint32_t* roots_host
   cudaStream_t s = G->stream;
   const uint32_t N = g.nslots, nrows = g.nrows(), W = (R + 63) / 64;
   LA3G_TRY(ms_bfs_alloc(G, b, R));
-  LA3G_CUDA(cudaMemcpyAsync(b->active, roots_host, (size_t) R * 4, cudaMemcpyHostToDevice, s));
-  k_root_pos<<<grid_for(R, 256), 256, 0, s>>>(b->active, R, N, g.pos_of_id, b->rpos);
+  LA3G_CUDA(cudaMemcpyAsync(b->rpos, roots_host, (size_t) R * 4, cudaMemcpyHostToDevice, s));
+  k_root_pos<<<grid_for(R, 256), 256, 0, s>>>(R, N, g.pos_of_id, b->rpos);
   LA3G_LAUNCHED();
   k_ms_init<<<num_sms() * 8, 256, 0, s>>>(N, W, R, b->vis, b->buf[0], b->buf[1]);
   LA3G_LAUNCHED();
@@ -730,8 +730,8 @@ static int sssp_batch_chunk(la3g_graph* G, BatchScratch* b, const uint32_t* root
     b->cap_sr = R;
   }
   if (R > b->cap_r) LA3G_TRY(ms_bfs_alloc(G, b, R));
-  LA3G_CUDA(cudaMemcpyAsync(b->active, roots, (size_t) R * 4, cudaMemcpyHostToDevice, s));
-  k_root_pos<<<grid_for(R, 256), 256, 0, s>>>(b->active, R, N, g.pos_of_id, b->rpos);
+  LA3G_CUDA(cudaMemcpyAsync(b->rpos, roots, (size_t) R * 4, cudaMemcpyHostToDevice, s));
+  k_root_pos<<<grid_for(R, 256), 256, 0, s>>>(R, N, g.pos_of_id, b->rpos);
   LA3G_LAUNCHED();
   k_bs_init<<<num_sms() * 8, 256, 0, s>>>((uint64_t) N * R, b->sdist, (uint64_t) N * W, b->sfront[0], b->sfront[1]);
   LA3G_LAUNCHED();
