@@ -320,7 +320,11 @@ __device__ __forceinline__ void sssp_pull(const SsspArgs& A, unsigned long long 
   for (uint32_t t = warp; t < A.ntasks; t += nwarps)
   {
     uint32_t* const at = &A.dist[A.task_row[t]];
-    uint32_t y = *(volatile uint32_t*) at;  // with what the row's other tasks found so far
+    // with what the row's other tasks found so far: one lane's read for all, since
+    // they lower it meanwhile and the lanes leave the loops below together
+    uint32_t y = 0;
+    if (lane == 0) y = *(volatile uint32_t*) at;
+    y = __shfl_sync(0xffffffffu, y, 0);
     if (y <= settled) continue;
     const uint32_t b = A.task_begin[t], e = A.task_begin[A.ntasks + t], had = y;
     for (uint32_t i0 = b; i0 < e; i0 += 128)
