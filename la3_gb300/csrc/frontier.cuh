@@ -43,8 +43,9 @@ __device__ __forceinline__ uint32_t hub_tasks(unsigned long long packed)
   return (uint32_t) (packed & ((1ull << kHubSlotShift) - 1));
 }
 
-// Slot whose task range holds task t (task0 ascends with the slot).
-__device__ __forceinline__ uint32_t hub_of_task(const uint32_t* __restrict__ task0, uint32_t nbig, uint32_t t)
+// Slot whose task range holds task t (task0 ascends with the slot; not
+// __restrict__: kernels that run all levels rewrite it between barriers).
+__device__ __forceinline__ uint32_t hub_of_task(const uint32_t* task0, uint32_t nbig, uint32_t t)
 {
   uint32_t lo = 0, hi = nbig;
   while (hi - lo > 1)
