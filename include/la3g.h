@@ -437,6 +437,12 @@ void la3g_profile_reset(void);
  * the length needed (excluding the terminating NUL). */
 size_t la3g_profile_report(char* buf, size_t cap);
 
+/* For tests of what happens when memory runs out: of the calling thread's
+ * device allocations from now on, the n-th (0: the next) fails, once, with
+ * LA3G_ENOMEM; n < 0: none.  A call that fails so can be made again.  Returns
+ * what was left of the number set before (< 0: it has failed, or none was set). */
+int64_t la3g_fail_allocation(int64_t n);
+
 #ifdef __cplusplus
 }
 #endif

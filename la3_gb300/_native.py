@@ -179,6 +179,7 @@ SIGNATURES = {
     "la3g_profile_enable": (None, [C.c_int]),
     "la3g_profile_reset": (None, []),
     "la3g_profile_report": (C.c_size_t, [C.c_char_p, C.c_size_t]),
+    "la3g_fail_allocation": (C.c_int64, [C.c_int64]),
 }
 
 _lib = None

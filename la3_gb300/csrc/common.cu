@@ -63,19 +63,41 @@ double now_ms()
   return duration<double, std::milli>(steady_clock::now().time_since_epoch()).count();
 }
 
-int galloc_bytes(la3g_graph* G, void** p, size_t bytes)
+static thread_local int64_t tls_fail_alloc = -1;
+
+int device_alloc(void** p, size_t bytes)
 {
   *p = nullptr;
-  cudaError_t e = cudaMalloc(p, bytes ? bytes : 16);
+  const bool fail = tls_fail_alloc == 0;
+  if (tls_fail_alloc >= 0) tls_fail_alloc--;
+  if (fail) return set_error(LA3G_ENOMEM, "device allocation of %zu bytes failed: asked for", bytes);
+  const cudaError_t e = cudaMalloc(p, bytes ? bytes : 16);
   if (e != cudaSuccess)
   {
     cudaGetLastError();
     *p = nullptr;
     return set_error(LA3G_ENOMEM, "device allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
   }
-  G->allocations.push_back(*p);
+  return LA3G_OK;
+}
+
+int galloc_bytes(la3g_graph* G, void** p, size_t bytes)
+{
+  LA3G_TRY(device_alloc(p, bytes));
+  G->allocations.emplace_back(*p, bytes);
   G->device_bytes += bytes;
   return LA3G_OK;
+}
+
+GallocScope::~GallocScope()
+{
+  if (kept || G->allocations.size() == from) return;
+  cudaStreamSynchronize(G->stream);
+  for (; G->allocations.size() > from; G->allocations.pop_back())
+  {
+    cudaFree(G->allocations.back().first);
+    G->device_bytes -= G->allocations.back().second;
+  }
 }
 
 // ---------------------------------------------------------------- profiling
@@ -174,6 +196,8 @@ extern "C" const char* la3g_status_string(int s)
     default: return "unknown status";
   }
 }
+
+extern "C" int64_t la3g_fail_allocation(int64_t n) { return std::exchange(tls_fail_alloc, n < 0 ? -1 : n); }
 
 extern "C" void la3g_profile_enable(int on)
 {

@@ -449,12 +449,21 @@ int build_push_csr(la3g_graph* G)
   DevGraph& g = G->g;
   if (g.out_ptr) return LA3G_OK;
   const uint64_t N = g.nslots, m = g.nent;
-  LA3G_TRY(galloc(G, &g.out_ptr, N + 1));
-  LA3G_TRY(galloc(G, &g.out_row, m + 1));
-  if (g.weighted()) LA3G_TRY(galloc(G, &g.out_w, m + 1));
+  GallocScope scope(G);
+  uint32_t *ptr = nullptr, *row = nullptr, *w = nullptr;
+  LA3G_TRY(galloc(G, &ptr, N + 1));
+  LA3G_TRY(galloc(G, &row, m + 1));
+  if (g.weighted()) LA3G_TRY(galloc(G, &w, m + 1));
+  g.out_ptr = ptr;
+  g.out_row = row;
+  g.out_w = w;
   const int rc = g.weighted() ? push_csr<uint64_t>(G) : push_csr<uint32_t>(G);
-  if (rc) g.out_ptr = nullptr;  // not built: the next call tries again
-  return rc;
+  if (rc)
+  {
+    g.out_ptr = g.out_row = g.out_w = nullptr;  // not built: the next call tries again
+    return rc;
+  }
+  return scope.keep();
 }
 
 static int new_graph(uint32_t n, uint32_t nright, uint32_t flags, la3g_graph** out, la3g_graph** G)
@@ -505,7 +514,7 @@ extern "C" void la3g_graph_free(la3g_graph* g)
   if (g->own_stream && g->own_stream != g->stream) cudaStreamSynchronize(g->own_stream);
   for (int i = 0; i < kSlotCount; i++)
     if (g->slot[i] && g->slot_free[i]) g->slot_free[i](g->slot[i]);
-  for (void* p : g->allocations) cudaFree(p);
+  for (const auto& a : g->allocations) cudaFree(a.first);
   if (g->ev0) cudaEventDestroy(g->ev0);
   if (g->ev1) cudaEventDestroy(g->ev1);
   if (g->own_stream) cudaStreamDestroy(g->own_stream);

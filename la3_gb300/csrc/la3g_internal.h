@@ -4,7 +4,9 @@
 
 #include <cstdint>
 #include <cstdio>
+#include <new>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "la3g.h"
@@ -198,6 +200,9 @@ void profile_add_bytes(const char* name, double bytes);
 
 extern thread_local uint32_t tls_launches;
 
+// cudaMalloc, or LA3G_ENOMEM (also as la3g_fail_allocation asks).
+int device_alloc(void** p, size_t bytes);
+
 // Scoped device buffer for temporaries.
 struct DevBuf
 {
@@ -213,13 +218,7 @@ struct DevBuf
     if (p) cudaFree(p);
     p = nullptr;
     bytes = 0;
-    cudaError_t e = cudaMalloc(&p, n ? n : 16);
-    if (e != cudaSuccess)
-    {
-      cudaGetLastError();
-      p = nullptr;
-      return set_error(LA3G_ENOMEM, "device allocation of %zu bytes failed: %s", n, cudaGetErrorString(e));
-    }
+    LA3G_TRY(device_alloc(&p, n));
     bytes = n;
     return LA3G_OK;
   }
@@ -272,7 +271,7 @@ struct la3g_graph
   cudaStream_t own_stream = nullptr;   // the graph's own stream
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   long long wait_polls = -1;           // la3g_set_wait_limit; < 0: the default
-  std::vector<void*> allocations;
+  std::vector<std::pair<void*, uint64_t>> allocations;  // and their bytes
   uint64_t device_bytes = 0;
   void* slot[la3g::kSlotCount] = {};
   void (*slot_free[la3g::kSlotCount])(void*) = {};
@@ -287,6 +286,24 @@ int galloc(la3g_graph* G, T** p, size_t count)
 {
   return galloc_bytes(G, (void**) p, count * sizeof(T));
 }
+
+// Graph allocations made while it lives are released again unless keep() is
+// called: what is built in several allocations stands whole or not at all.
+struct GallocScope
+{
+  la3g_graph* G;
+  size_t from;
+  bool kept = false;
+  explicit GallocScope(la3g_graph* G_) : G(G_), from(G_->allocations.size()) {}
+  GallocScope(const GallocScope&) = delete;
+  GallocScope& operator=(const GallocScope&) = delete;
+  ~GallocScope();
+  int keep()
+  {
+    kept = true;
+    return LA3G_OK;
+  }
+};
 
 int build_push_csr(la3g_graph* G);
 // Bipartite corpus: the position of the first term row (docs come first).
