@@ -287,37 +287,53 @@ static int batch_out_buffer(la3g_graph* G, BatchScratch* b, size_t bytes)
 
 static int batch_scratch(la3g_graph* G, BatchScratch** out)
 {
-  BatchScratch* b = (BatchScratch*) G->slot[kSlotBatch];
-  if (!b)
-  {
-    b = new (std::nothrow) BatchScratch();
-    if (!b) return set_error(LA3G_ENOMEM, "out of host memory");
-    G->slot[kSlotBatch] = b;
-    G->slot_free[kSlotBatch] = batch_scratch_free;
+  return graph_scratch(G, kSlotBatch, batch_scratch_free, out, [&](BatchScratch* b) -> int {
     LA3G_TRY(galloc(G, &b->ctr, 8));
     LA3G_TRY(galloc(G, &b->bar, 1));
     LA3G_CUDA(cudaHostAlloc(&b->hctr, 2 * sizeof(unsigned long long), cudaHostAllocMapped));
-  }
-  *out = b;
-  return LA3G_OK;
+    return LA3G_OK;
+  });
 }
 
+// Larger buffers take the place of those in use when all of them are there; the
+// old ones stay owned by the graph.
 static int ms_bfs_alloc(la3g_graph* G, BatchScratch* b, uint32_t R)
 {
   if (R <= b->cap_r) return LA3G_OK;
   const uint32_t N = G->g.nslots, W = (R + 63) / 64;
-  // buffers sized for the new R; the old ones stay owned by the graph
-  LA3G_TRY(galloc(G, &b->vis, (size_t) N * W));
-  LA3G_TRY(galloc(G, &b->buf[0], (size_t) N * W));
-  LA3G_TRY(galloc(G, &b->buf[1], (size_t) N * W));
-  for (int k = 0; k < 3; k++) LA3G_TRY(galloc(G, &b->alive[k], W));
-  LA3G_TRY(galloc(G, &b->hops, (size_t) N * W * 64));
-  LA3G_TRY(galloc(G, &b->rpos, R));
-  LA3G_TRY(galloc(G, &b->active, (size_t) N * W));
-  LA3G_TRY(galloc(G, &b->phub, (size_t) N * W));
-  LA3G_TRY(galloc(G, &b->phub_t0, (size_t) N * W));
-  b->cap_r = R;
-  return LA3G_OK;
+  GallocScope scope(G);
+  BatchScratch t = *b;
+  LA3G_TRY(galloc(G, &t.vis, (size_t) N * W));
+  LA3G_TRY(galloc(G, &t.buf[0], (size_t) N * W));
+  LA3G_TRY(galloc(G, &t.buf[1], (size_t) N * W));
+  for (int k = 0; k < 3; k++) LA3G_TRY(galloc(G, &t.alive[k], W));
+  LA3G_TRY(galloc(G, &t.hops, (size_t) N * W * 64));
+  LA3G_TRY(galloc(G, &t.rpos, R));
+  LA3G_TRY(galloc(G, &t.active, (size_t) N * W));
+  LA3G_TRY(galloc(G, &t.phub, (size_t) N * W));
+  LA3G_TRY(galloc(G, &t.phub_t0, (size_t) N * W));
+  t.cap_r = R;
+  *b = t;
+  return scope.keep();
+}
+
+static int bs_alloc(la3g_graph* G, BatchScratch* b, uint32_t R)
+{
+  if (R <= b->cap_sr) return LA3G_OK;
+  const uint32_t N = G->g.nslots, W = (R + 63) / 64;
+  GallocScope scope(G);
+  BatchScratch t = *b;
+  LA3G_TRY(galloc(G, &t.sdist, (size_t) N * R));
+  for (int c = 0; c < 2; c++)
+  {
+    LA3G_TRY(galloc(G, &t.sfront[c], (size_t) N * W));
+    LA3G_TRY(galloc(G, &t.sact[c], (size_t) N * W));
+    LA3G_TRY(galloc(G, &t.shub[c], (size_t) N * W));
+    LA3G_TRY(galloc(G, &t.shub_t0[c], (size_t) N * W));
+  }
+  t.cap_sr = R;
+  *b = t;
+  return scope.keep();
 }
 
 // Root ids -> positions, in place.
@@ -716,20 +732,8 @@ static int sssp_batch_chunk(la3g_graph* G, BatchScratch* b, const uint32_t* root
     *iters_out = 0;
     return LA3G_OK;
   }
-  if (R > b->cap_sr)
-  {
-    LA3G_TRY(galloc(G, &b->sdist, (size_t) N * R));
-    LA3G_TRY(galloc(G, &b->sfront[0], (size_t) N * W));
-    LA3G_TRY(galloc(G, &b->sfront[1], (size_t) N * W));
-    LA3G_TRY(galloc(G, &b->sact[0], (size_t) N * W));
-    LA3G_TRY(galloc(G, &b->sact[1], (size_t) N * W));
-    LA3G_TRY(galloc(G, &b->shub[0], (size_t) N * W));
-    LA3G_TRY(galloc(G, &b->shub[1], (size_t) N * W));
-    LA3G_TRY(galloc(G, &b->shub_t0[0], (size_t) N * W));
-    LA3G_TRY(galloc(G, &b->shub_t0[1], (size_t) N * W));
-    b->cap_sr = R;
-  }
-  if (R > b->cap_r) LA3G_TRY(ms_bfs_alloc(G, b, R));
+  LA3G_TRY(bs_alloc(G, b, R));
+  LA3G_TRY(ms_bfs_alloc(G, b, R));
   LA3G_CUDA(cudaMemcpyAsync(b->rpos, roots, (size_t) R * 4, cudaMemcpyHostToDevice, s));
   k_root_pos<<<grid_for(R, 256), 256, 0, s>>>(R, N, g.pos_of_id, b->rpos);
   LA3G_LAUNCHED();

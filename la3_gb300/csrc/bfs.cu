@@ -447,14 +447,8 @@ static void bfs_scratch_free(void* p)
   delete s;
 }
 
-static int bfs_scratch(la3g_graph* G, BfsScratch** out)
+static int bfs_scratch_build(la3g_graph* G, BfsScratch* bs)
 {
-  BfsScratch* bs = (BfsScratch*) G->slot[kSlotBfs];
-  if (bs) { *out = bs; return LA3G_OK; }
-  bs = new (std::nothrow) BfsScratch();
-  if (!bs) return set_error(LA3G_ENOMEM, "out of host memory");
-  G->slot[kSlotBfs] = bs;
-  G->slot_free[kSlotBfs] = bfs_scratch_free;
   DevGraph& g = G->g;
   const uint32_t N = g.nslots;
   // one allocation: eight arrays of a word per vertex, two of a byte, two bitmaps
@@ -492,8 +486,12 @@ static int bfs_scratch(la3g_graph* G, BfsScratch** out)
     bs->parent_id = (uint32_t*) ((char*) bs->stats + 256);
     bs->hops_id = (uint8_t*) bs->parent_id + n4;
   }
-  *out = bs;
   return LA3G_OK;
+}
+
+static int bfs_scratch(la3g_graph* G, BfsScratch** out)
+{
+  return graph_scratch(G, kSlotBfs, bfs_scratch_free, out, [&](BfsScratch* bs) { return bfs_scratch_build(G, bs); });
 }
 
 }  // namespace la3g

@@ -149,20 +149,18 @@ __global__ void k_f32_by_id(uint32_t N, const uint32_t* __restrict__ id_of_pos, 
   for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < N; p += gridDim.x * blockDim.x) out[id_of_pos[p]] = v[p];
 }
 
-static int bm25_scratch(la3g_graph* G, Bm25Scratch** out)
+static int bm25_scratch_build(la3g_graph* G, Bm25Scratch* b)
 {
-  Bm25Scratch* b = (Bm25Scratch*) G->slot[kSlotBm25];
-  if (b) { *out = b; return LA3G_OK; }
-  b = new (std::nothrow) Bm25Scratch();
-  if (!b) return set_error(LA3G_ENOMEM, "out of host memory");
-  G->slot[kSlotBm25] = b;
-  G->slot_free[kSlotBm25] = bm25_scratch_free;
   const uint32_t N = G->g.nslots;
   LA3G_TRY(galloc(G, &b->length, N));
   LA3G_TRY(galloc(G, &b->tok, 1));
   LA3G_TRY(ir_scratch(G, &b->ir));
-  *out = b;
   return LA3G_OK;
+}
+
+static int bm25_scratch(la3g_graph* G, Bm25Scratch** out)
+{
+  return graph_scratch(G, kSlotBm25, bm25_scratch_free, out, [&](Bm25Scratch* b) { return bm25_scratch_build(G, b); });
 }
 
 // First term row: positions ascend with ids, docs (ids <= D) come first.

@@ -329,20 +329,18 @@ __global__ void k_ccb_by_id(uint32_t N, const uint32_t* __restrict__ id_of_pos, 
   for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < N; p += gridDim.x * blockDim.x) out[id_of_pos[p]] = lab[p];
 }
 
-static int cc_scratch(la3g_graph* G, CcScratch** out)
+static int cc_scratch_build(la3g_graph* G, CcScratch* cs)
 {
-  CcScratch* cs = (CcScratch*) G->slot[kSlotCc];
-  if (cs) { *out = cs; return LA3G_OK; }
-  cs = new (std::nothrow) CcScratch();
-  if (!cs) return set_error(LA3G_ENOMEM, "out of host memory");
-  G->slot[kSlotCc] = cs;
-  G->slot_free[kSlotCc] = cc_scratch_free;
   LA3G_TRY(galloc(G, &cs->label, G->g.nslots));
   LA3G_TRY(galloc(G, &cs->flag, 1));
   LA3G_TRY(galloc(G, &cs->walked, 2));
   LA3G_CUDA(cudaHostAlloc(&cs->hwalked, 2 * sizeof(unsigned long long), cudaHostAllocDefault));
-  *out = cs;
   return LA3G_OK;
+}
+
+static int cc_scratch(la3g_graph* G, CcScratch** out)
+{
+  return graph_scratch(G, kSlotCc, cc_scratch_free, out, [&](CcScratch* cs) { return cc_scratch_build(G, cs); });
 }
 
 }  // namespace la3g
@@ -375,11 +373,13 @@ extern "C" int la3g_cc(la3g_graph* G, uint32_t* label_out, la3g_stats* st)
   {
     if (!cs->parent)
     {
+      GallocScope scope(G);
       LA3G_TRY(galloc(G, &cs->least, nrows));
       LA3G_TRY(galloc(G, &cs->deep, kCcFlags));
       LA3G_TRY(galloc(G, &cs->probe, kCcSamples));
       LA3G_TRY(galloc(G, &cs->giant, 2));
-      LA3G_TRY(galloc(G, &cs->parent, nrows));
+      LA3G_TRY(galloc(G, &cs->parent, nrows));  // last: it says that all are there
+      scope.keep();
     }
     int nflat = 0;
     auto flatten = [&](const uint32_t* share) -> int {
@@ -462,10 +462,12 @@ extern "C" int la3g_cc(la3g_graph* G, uint32_t* label_out, la3g_stats* st)
   {
     if (!cs->lab_pos)
     {
-      LA3G_TRY(galloc(G, &cs->lab_pos, N));
+      GallocScope scope(G);
       LA3G_TRY(galloc(G, &cs->msg, 2 * (size_t) N));
       LA3G_TRY(galloc(G, &cs->active[0], N));
       LA3G_TRY(galloc(G, &cs->active[1], N));
+      LA3G_TRY(galloc(G, &cs->lab_pos, N));  // last
+      scope.keep();
     }
     uint32_t* msg[2] = {cs->msg, cs->msg + N};
     k_ccb_init<<<grid_for(N, 256), 256, 0, s>>>(N, nrows, g.id_of_pos, cs->lab_pos, msg[0], cs->active[0]);

@@ -505,8 +505,13 @@ static int ir_query(la3g_graph* G, IrScratch* b, const Scorer& S, const float* l
   {
     if (nterms > b->qcap)
     {
-      LA3G_TRY(galloc(G, &b->qin, nterms));
-      LA3G_TRY(galloc(G, &b->qpos, 1 + 2 * (size_t) nterms));
+      GallocScope scope(G);
+      uint32_t *qin = nullptr, *qpos = nullptr;
+      LA3G_TRY(galloc(G, &qin, nterms));
+      LA3G_TRY(galloc(G, &qpos, 1 + 2 * (size_t) nterms));
+      scope.keep();
+      b->qin = qin;
+      b->qpos = qpos;
       b->qcap = nterms;
     }
     Q.pairs = b->qpos;

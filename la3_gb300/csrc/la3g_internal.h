@@ -305,6 +305,31 @@ struct GallocScope
   }
 };
 
+// An app's scratch on the graph, made by build(scratch) on first use.  It is put
+// in its slot only when it is complete: a call after a failed one builds it anew.
+template <class S, class Build>
+int graph_scratch(la3g_graph* G, AppSlot slot, void (*free_scratch)(void*), S** out, Build build)
+{
+  if (!G->slot[slot])
+  {
+    S* s = new (std::nothrow) S();
+    if (!s) return set_error(LA3G_ENOMEM, "out of host memory");
+    GallocScope scope(G);
+    const int rc = build(s);
+    if (rc != LA3G_OK)
+    {
+      cudaStreamSynchronize(G->stream);  // kernels that write to it
+      free_scratch(s);
+      return rc;
+    }
+    scope.keep();
+    G->slot[slot] = s;
+    G->slot_free[slot] = free_scratch;
+  }
+  *out = (S*) G->slot[slot];
+  return LA3G_OK;
+}
+
 int build_push_csr(la3g_graph* G);
 // Bipartite corpus: the position of the first term row (docs come first).
 int bipartite_first_term_row(la3g_graph* G, uint32_t* out);

@@ -98,21 +98,19 @@ struct LmScorer
   }
 };
 
-static int lm_scratch(la3g_graph* G, LmScratch** out)
+static int lm_scratch_build(la3g_graph* G, LmScratch* b)
 {
-  LmScratch* b = (LmScratch*) G->slot[kSlotLm];
-  if (b) { *out = b; return LA3G_OK; }
-  b = new (std::nothrow) LmScratch();
-  if (!b) return set_error(LA3G_ENOMEM, "out of host memory");
-  G->slot[kSlotLm] = b;
-  G->slot_free[kSlotLm] = lm_scratch_free;
   const uint32_t N = G->g.nslots;
   LA3G_TRY(galloc(G, &b->length, N));
   LA3G_TRY(galloc(G, &b->factor, N));
   LA3G_TRY(galloc(G, &b->tok, 1));
   LA3G_TRY(ir_scratch(G, &b->ir));
-  *out = b;
   return LA3G_OK;
+}
+
+static int lm_scratch(la3g_graph* G, LmScratch** out)
+{
+  return graph_scratch(G, kSlotLm, lm_scratch_free, out, [&](LmScratch* b) { return lm_scratch_build(G, b); });
 }
 
 }  // namespace la3g

@@ -604,6 +604,7 @@ static int pr_prepare(la3g_graph* G, PrScratch** out)
   // which holds the temporaries here and the ranks and messages of a call.
   auto round = [](size_t b) { return (b + 255) & ~(size_t) 255; };
   const size_t n4 = round((size_t) N * 4), n8 = round((size_t) N * 8 + 8);
+  GallocScope scope(G);
   char* kept = nullptr;
   LA3G_TRY(galloc(G, &kept, 4 * n4 + n8 + 256));
   ps->deg = (uint32_t*) kept;
@@ -681,7 +682,7 @@ static int pr_prepare(la3g_graph* G, PrScratch** out)
   ps->rankf = (float*) (t + n8);
   ps->ready = true;
   *out = ps;
-  return LA3G_OK;
+  return scope.keep();
 }
 
 static int pr_launch(la3g_graph* G, PrScratch* ps, const PrRange& r, const double* x, double* xnext, int* flag,

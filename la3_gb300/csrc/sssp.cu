@@ -538,14 +538,8 @@ static int sssp_entries(la3g_graph* G, SsspScratch* ss, int rbits, int wbits)
   return LA3G_OK;
 }
 
-static int sssp_scratch(la3g_graph* G, SsspScratch** out)
+static int sssp_scratch_build(la3g_graph* G, SsspScratch* ss)
 {
-  SsspScratch* ss = (SsspScratch*) G->slot[kSlotSssp];
-  if (ss) { *out = ss; return LA3G_OK; }
-  ss = new (std::nothrow) SsspScratch();
-  if (!ss) return set_error(LA3G_ENOMEM, "out of host memory");
-  G->slot[kSlotSssp] = ss;
-  G->slot_free[kSlotSssp] = sssp_scratch_free;
   DevGraph& g = G->g;
   cudaStream_t s = G->stream;
   const uint32_t N = g.nslots;
@@ -656,8 +650,12 @@ static int sssp_scratch(la3g_graph* G, SsspScratch** out)
   A.entry = ss->entry;
   A.wshift = ss->wshift;
   A.stats = ss->stats;
-  *out = ss;
   return LA3G_OK;
+}
+
+static int sssp_scratch(la3g_graph* G, SsspScratch** out)
+{
+  return graph_scratch(G, kSlotSssp, sssp_scratch_free, out, [&](SsspScratch* ss) { return sssp_scratch_build(G, ss); });
 }
 
 }  // namespace la3g

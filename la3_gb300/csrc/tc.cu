@@ -844,14 +844,8 @@ __global__ void k_tc_sum(uint32_t N, const uint32_t* __restrict__ ntri, unsigned
   if ((threadIdx.x & 31) == 0 && s) atomicAdd(total, s);
 }
 
-static int tc_scratch(la3g_graph* G, TcScratch** out)
+static int tc_scratch_build(la3g_graph* G, TcScratch* ts)
 {
-  TcScratch* ts = (TcScratch*) G->slot[kSlotTc];
-  if (ts) { *out = ts; return LA3G_OK; }
-  ts = new (std::nothrow) TcScratch();
-  if (!ts) return set_error(LA3G_ENOMEM, "out of host memory");
-  G->slot[kSlotTc] = ts;
-  G->slot_free[kSlotTc] = tc_scratch_free;
   const uint32_t N = G->g.nslots;
   const uint64_t m = G->g.nent;
   ts->N = N;
@@ -893,8 +887,12 @@ static int tc_scratch(la3g_graph* G, TcScratch** out)
   LA3G_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, c2, ts->tcount2, ts->toff2, (int) N + 1));
   ts->temp_bytes = std::max(std::max(a, b), std::max(c, c2));
   LA3G_TRY(galloc_bytes(G, &ts->temp, ts->temp_bytes));
-  *out = ts;
   return LA3G_OK;
+}
+
+static int tc_scratch(la3g_graph* G, TcScratch** out)
+{
+  return graph_scratch(G, kSlotTc, tc_scratch_free, out, [&](TcScratch* ts) { return tc_scratch_build(G, ts); });
 }
 
 // Pass 1: the rank-ordered N+ rows and the per-y pair lists and tasks.

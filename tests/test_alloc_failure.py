@@ -49,6 +49,70 @@ def records():
     return n, rec, zero
 
 
+@pytest.mark.parametrize("case", ["bfs", "cc", "cc_zero", "sssp", "tc", "pagerank", "pagerank_f32", "bfs_batch", "sssp_batch",
+                                  "sssp_batch_huge"])
+def test_graph_calls(gpu, records, case):
+    L = gpu
+    n, rec, zero = records
+    pairs = np.ascontiguousarray(rec[:, :2])
+    roots = np.arange(1, 130, dtype=np.uint32)
+    graph = {
+        "bfs": (pairs, 0), "bfs_batch": (pairs, 0), "cc": (pairs, 0), "cc_zero": (np.ascontiguousarray(zero[:, :2]), 0),
+        "tc": (pairs, L.DIRECTED | L.ACYCLIC), "pagerank": (pairs, L.DIRECTED), "pagerank_f32": (pairs, L.DIRECTED),
+    }.get(case, (rec, L.DIRECTED | L.WEIGHTED))
+    if case == "sssp_batch_huge":  # weights that make the batch run its roots one by one
+        graph = rec * np.array([1, 1, 1 << 19], np.uint32), graph[1]
+        roots = roots[:3]
+    call = {
+        "bfs": lambda g: L.bfs(g, 7)[:2], "cc": lambda g: L.cc(g)[:1], "cc_zero": lambda g: L.cc(g)[:1],
+        "sssp": lambda g: L.sssp(g, 7)[:1], "tc": lambda g: L.tc(g)[:2], "pagerank": lambda g: L.pagerank(g, 3)[:2],
+        "pagerank_f32": lambda g: L.pagerank_f32(g, 3)[:1], "bfs_batch": lambda g: L.bfs_batch(g, roots)[:1],
+    }.get(case, lambda g: L.sssp_batch(g, roots)[:1])
+    assert _each(L, lambda: L.Graph.from_records(graph[0], n, graph[1]), call) > 0
+
+
+def test_growing_batches(gpu, records):
+    """A batch that cannot get larger buffers leaves the ones that smaller batches use."""
+    L = gpu
+    n, rec, _ = records
+    few, many = np.arange(1, 20, dtype=np.uint32), np.arange(1, 300, dtype=np.uint32)
+    fail = L.N.lib().la3g_fail_allocation
+    for flags, data, call in ((0, np.ascontiguousarray(rec[:, :2]), L.bfs_batch),
+                              (L.DIRECTED | L.WEIGHTED, rec, L.sssp_batch)):
+        ref = L.Graph.from_records(data, n, flags)
+        want = {len(r): call(ref, r)[0] for r in (few, many)}
+        for k in range(200):
+            g = L.Graph.from_records(data, n, flags)
+            call(g, few)
+            fail(k)
+            try:
+                assert np.array_equal(call(g, many)[0], want[len(many)])
+            except L.N.LA3GError as e:
+                assert e.status == ENOMEM
+            done = fail(-1) >= 0
+            for r in (few, many, few):
+                assert np.array_equal(call(g, r)[0], want[len(r)]), (k, len(r))
+            if done:
+                break
+
+
+@pytest.mark.parametrize("app", ["bm25", "lm"])
+def test_queries(gpu, app):
+    L = gpu
+    rng = np.random.default_rng(4)
+    docs, terms = 500, 150
+    rec = np.stack([rng.integers(1, docs + 1, 6000), rng.integers(1, terms + 1, 6000), rng.integers(1, 9, 6000)], 1)
+    rec = rec.astype(np.uint32)
+    longer = docs + 1 + rng.permutation(terms)[:90]  # above the terms that go by value
+    make = L.BM25 if app == "bm25" else L.LM
+
+    def call(g):
+        q = make(g)
+        return [x for t in (longer[:3], longer, longer[:3]) for x in q.query(t, 10)[:2]]
+
+    assert _each(L, lambda: L.Graph.from_records(rec, docs, L.BIPARTITE | L.WEIGHTED, terms), call) > 0
+
+
 @pytest.mark.parametrize("weighted", [False, True])
 def test_push_view(gpu, records, weighted):
     """The push CSR: built on demand, whole or not at all."""
