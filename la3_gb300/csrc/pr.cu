@@ -103,6 +103,7 @@ struct PrScratch
   float* trankf = nullptr;       // [nslots] by position
   float* txf[2] = {nullptr, nullptr};  // [nslots] by position
   int tile_blocks = 0;           // resident blocks per SM of the tiled kernel
+  bool tiles_ready = false;
 };
 
 static void pr_scratch_free(void* p) { delete (PrScratch*) p; }
@@ -908,12 +909,11 @@ __global__ void k_tile_cols(const uint32_t* __restrict__ order, uint64_t n, cons
   }
 }
 
+// The push CSR has to be there.
 static int pr_build_tiles(la3g_graph* G, PrScratch* ps)
 {
-  if (ps->tile_col) return LA3G_OK;
   DevGraph& g = G->g;
   cudaStream_t s = G->stream;
-  LA3G_TRY(build_push_csr(G));
   const uint64_t m = g.nent;
   const uint32_t ntiles = (g.nreg + kTileRows - 1) / kTileRows;
   DevBuf colof, key, key2, idx, idx2, flag, slot, tmp, kept;
@@ -1236,8 +1236,10 @@ static int pr_f32_run(la3g_graph* G, uint32_t iters, double tol, double* rank_ou
   LA3G_TRY(pr_prepare(G, &ps));
   cudaStream_t s = G->stream;
   const uint32_t N = g.nslots;
-  if (tiled && !ps->tile_col)
+  if (tiled && !ps->tiles_ready)
   {
+    LA3G_TRY(build_push_csr(G));
+    GallocScope scope(G);
     LA3G_TRY(pr_build_tiles(G, ps));
     LA3G_CUDA(cudaFuncSetAttribute(k_prf_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) (kTileRows * 4)));
     LA3G_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ps->tile_blocks, k_prf_tiles, kTileThreads,
@@ -1245,6 +1247,8 @@ static int pr_f32_run(la3g_graph* G, uint32_t iters, double tol, double* rank_ou
     LA3G_TRY(galloc(G, &ps->trankf, N));
     LA3G_TRY(galloc(G, &ps->txf[0], N));
     LA3G_TRY(galloc(G, &ps->txf[1], N));
+    ps->tiles_ready = true;
+    scope.keep();
   }
   const PrLayout& L = ps->L;
   const uint32_t nlong = L.reg.q1;  // regular rows above kLongRow: qpos[0 .. nlong)

@@ -14,7 +14,7 @@ def _same(a, b):
     return all(x == y if isinstance(x, int) else np.array_equal(x, y) for x, y in zip(a, b, strict=True))
 
 
-def _each(L, make, call):
+def _each(L, make, call, same=_same):
     """Returns how many allocations the call makes."""
     fail = L.N.lib().la3g_fail_allocation
     want = call(make())
@@ -30,8 +30,8 @@ def _each(L, make, call):
                 assert fail(-1) < 0
             else:
                 done |= fail(-1) >= 0 and not again
-                assert _same(got, want), n
-        assert _same(call(g), want), n
+                assert same(got, want), n
+        assert same(call(g), want), n
         if done:
             return n
     raise AssertionError("too many allocations")
@@ -69,6 +69,17 @@ def test_graph_calls(gpu, records, case):
         "pagerank_f32": lambda g: L.pagerank_f32(g, 3)[:1], "bfs_batch": lambda g: L.bfs_batch(g, roots)[:1],
     }.get(case, lambda g: L.sssp_batch(g, roots)[:1])
     assert _each(L, lambda: L.Graph.from_records(graph[0], n, graph[1]), call) > 0
+
+
+def test_tiled_pagerank(gpu, records):
+    """Its rows are FP32 sums in any order: of at most 1024 positive numbers each,
+    1023 x 2^-24 of relative difference, three iterations (and the long rows', in
+    fixed order) below 2e-4."""
+    L = gpu
+    n, rec, _ = records
+    calls = _each(L, lambda: L.Graph.from_records(np.ascontiguousarray(rec[:, :2]), n, L.DIRECTED),
+                  lambda g: [L.pagerank_f32(g, 3, tiled=True)[0]], lambda a, b: np.allclose(a[0], b[0], rtol=2e-4, atol=0))
+    assert calls > 0
 
 
 def test_growing_batches(gpu, records):
