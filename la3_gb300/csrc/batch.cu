@@ -275,10 +275,13 @@ __global__ void __launch_bounds__(256) k_ms_out(uint32_t N, uint32_t R, uint32_t
   }
 }
 
-// The buffer results are put in order in before they leave the device.
+// The buffer results are put in order in before they leave the device: one, of
+// the largest size asked for.
 static int batch_out_buffer(la3g_graph* G, BatchScratch* b, size_t bytes)
 {
   if (bytes <= b->tpos_bytes) return LA3G_OK;
+  galloc_release(G, b->tpos);
+  b->tpos = nullptr;
   b->tpos_bytes = 0;
   LA3G_TRY(galloc(G, &b->tpos, bytes));
   b->tpos_bytes = bytes;
@@ -295,8 +298,7 @@ static int batch_scratch(la3g_graph* G, BatchScratch** out)
   });
 }
 
-// Larger buffers take the place of those in use when all of them are there; the
-// old ones stay owned by the graph.
+// Larger buffers take the place of those in use when all of them are there.
 static int ms_bfs_alloc(la3g_graph* G, BatchScratch* b, uint32_t R)
 {
   if (R <= b->cap_r) return LA3G_OK;
@@ -313,8 +315,13 @@ static int ms_bfs_alloc(la3g_graph* G, BatchScratch* b, uint32_t R)
   LA3G_TRY(galloc(G, &t.phub, (size_t) N * W));
   LA3G_TRY(galloc(G, &t.phub_t0, (size_t) N * W));
   t.cap_r = R;
+  scope.keep();
+  for (void* p : {(void*) b->vis, (void*) b->buf[0], (void*) b->buf[1], (void*) b->alive[0], (void*) b->alive[1],
+                  (void*) b->alive[2], (void*) b->hops, (void*) b->rpos, (void*) b->active, (void*) b->phub,
+                  (void*) b->phub_t0})
+    galloc_release(G, p);
   *b = t;
-  return scope.keep();
+  return LA3G_OK;
 }
 
 static int bs_alloc(la3g_graph* G, BatchScratch* b, uint32_t R)
@@ -332,8 +339,12 @@ static int bs_alloc(la3g_graph* G, BatchScratch* b, uint32_t R)
     LA3G_TRY(galloc(G, &t.shub_t0[c], (size_t) N * W));
   }
   t.cap_sr = R;
+  scope.keep();
+  galloc_release(G, b->sdist);
+  for (int c = 0; c < 2; c++)
+    for (void* p : {(void*) b->sfront[c], (void*) b->sact[c], (void*) b->shub[c], (void*) b->shub_t0[c]}) galloc_release(G, p);
   *b = t;
-  return scope.keep();
+  return LA3G_OK;
 }
 
 // Root ids -> positions, in place.

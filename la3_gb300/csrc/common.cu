@@ -89,6 +89,18 @@ int galloc_bytes(la3g_graph* G, void** p, size_t bytes)
   return LA3G_OK;
 }
 
+void galloc_release(la3g_graph* G, void* p)
+{
+  for (auto a = G->allocations.begin(); p && a != G->allocations.end(); ++a)
+    if (a->first == p)
+    {
+      cudaFree(p);
+      G->device_bytes -= a->second;
+      G->allocations.erase(a);
+      return;
+    }
+}
+
 GallocScope::~GallocScope()
 {
   if (kept || G->allocations.size() == from) return;

@@ -330,6 +330,9 @@ int graph_scratch(la3g_graph* G, AppSlot slot, void (*free_scratch)(void*), S** 
   return LA3G_OK;
 }
 
+// Releases a graph allocation that another one replaces (null: nothing).
+void galloc_release(la3g_graph* G, void* p);
+
 int build_push_csr(la3g_graph* G);
 // Bipartite corpus: the position of the first term row (docs come first).
 int bipartite_first_term_row(la3g_graph* G, uint32_t* out);
