@@ -201,7 +201,9 @@ int la3g_bfs(la3g_graph* g, uint32_t root, uint8_t* hops_out, uint32_t* parent_o
 
 /* SSSP (src/apps/graph_analytics/sssp.cpp:11-37, sssp.h:11-46) on a graph
  * loaded with LA3G_DIRECTED | LA3G_WEIGHTED: uint32 distances,
- * 2147483647 = unreached. */
+ * 2147483647 = unreached.  The first call orders the in-edges by weight for the
+ * later ones (8 B per edge kept, 16 to 24 more meanwhile); where that memory is
+ * not there it goes on without, with the same results. */
 int la3g_sssp(la3g_graph* g, uint32_t root, uint32_t* dist_out, la3g_stats* st);
 
 /* la3g_bfs and la3g_sssp run as one kernel whose blocks wait for one another
@@ -363,10 +365,12 @@ int la3g_server_create(uint64_t budget_bytes, uint32_t bfs_lanes, uint32_t sssp_
 /* Makes a loaded graph resident in the server: undirected graphs serve BFS,
  * DIRECTED|WEIGHTED graphs SSSP, BIPARTITE graphs BM25 and LM (both
  * prepared here if needed; LM's first-query leftover activity is taken here,
- * so every served LM query sees the reference's steady state).  The graph's device bytes plus its engine's lane state must fit
- * in the budget left (the lane count is halved down to 64 first), else
- * LA3G_EBUDGET.  The caller keeps ownership but must not use the graph while
- * it is served; la3g_server_free releases it. */
+ * so every served LM query sees the reference's steady state).  The graph's
+ * device bytes plus its engine's lane state must fit in the budget left (the
+ * lane count is halved down to 64 first), else LA3G_EBUDGET.  An SSSP query
+ * answered alone uses the in-edges as an earlier la3g_sssp on the graph has
+ * ordered them, and orders none itself.  The caller keeps ownership but must
+ * not use the graph while it is served; la3g_server_free releases it. */
 int la3g_server_add_graph(la3g_server* s, la3g_graph* g, uint32_t* graph_id);
 /* Queues a query and returns its ticket at once; thread-safe.  The query's
  * output buffers must stay valid until the ticket is polled done. */

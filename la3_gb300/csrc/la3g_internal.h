@@ -334,6 +334,9 @@ int graph_scratch(la3g_graph* G, AppSlot slot, void (*free_scratch)(void*), S** 
 void galloc_release(la3g_graph* G, void* p);
 
 int build_push_csr(la3g_graph* G);
+// la3g_sssp; order: if they are not there yet, the in-edges are first ordered for
+// its pull steps (sssp.cu).
+int sssp_run(la3g_graph* G, uint32_t root, uint32_t* dist_out, la3g_stats* st, bool order);
 // Bipartite corpus: the position of the first term row (docs come first).
 int bipartite_first_term_row(la3g_graph* G, uint32_t* out);
 

@@ -640,11 +640,13 @@ int bfs_retire(Engine* E, const std::vector<uint32_t>& lanes_in, bool deliver, u
 
 // Runs one query alone through the single-root entry point (used for BFS
 // lanes that would pass 254 levels and for SSSP graphs whose weights could
-// reach INF).
+// reach INF).  SSSP takes the ordered in-edges if an earlier la3g_sssp on the
+// graph has made them, and makes none itself: 8 bytes per edge, and more while
+// they are made, that admission has not counted.
 int run_single(Engine* E, Ticket* t)
 {
   if (E->kind == kEngBfs) return la3g_bfs(E->G, t->q.root, (uint8_t*) t->q.out, nullptr, nullptr);
-  return la3g_sssp(E->G, t->q.root, (uint32_t*) t->q.out, nullptr);
+  return sssp_run(E->G, t->q.root, (uint32_t*) t->q.out, nullptr, false);
 }
 
 // Completes a ticket whose root has no vertex: nothing is reached

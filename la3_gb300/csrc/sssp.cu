@@ -55,16 +55,17 @@ static constexpr unsigned long long kSsspRunning = 2;  // status until the kerne
 
 struct SsspArgs
 {
-  // the graph: push CSR (regular rows first, up to reg_end), pull CSR (offsets
-  // of all rows; columns and weights are read for the sinks only)
+  // the graph: push CSR (regular rows first, up to reg_end), pull CSR (columns
+  // and weights are read for the sinks, and in plain pull steps)
   const uint32_t *out_ptr, *out_row, *out_w, *reg_end, *in_ptr, *in_col, *in_w, *pos_of_id;
   uint32_t N, nreg, nsink, src_base, iso_base;
   uint64_t reg_in;                // in-edges of the regular rows
   uint32_t min_w, max_w;          // pull steps need INF + max_w to stay in uint32
   uint64_t limit;                 // most iterations
-  // pull steps: the regular rows' entries, slot of the column and weight, each
-  // row in ascending order of weight >> wshift.  Slots number the columns by
-  // descending out-degree: the hot ones' messages share sectors.
+  // ordered pull steps: the regular rows' entries, slot of the column and weight,
+  // each row in ascending order of weight >> wshift.  Slots number the columns by
+  // descending out-degree: the hot ones' messages share sectors.  (Plain ones go
+  // over the pull CSR; a column's slot is its position.)
   const uint32_t* slot;
   const uint2* entry;
   int wshift;
@@ -96,12 +97,12 @@ struct SsspScratch
   uint32_t* reg_end = nullptr;    // [nslots] end of each vertex's out-edges into regular rows
   uint32_t* long_rows = nullptr;
   uint32_t nlong = 0;
-  uint32_t* slot = nullptr;
-  uint2* entry = nullptr;
   uint64_t reg_in = 0;
   uint32_t max_w = 0, min_w = 0;  // largest weight; smallest of a regular row's in-edge
-  int wshift = 0;
-  unsigned grid = 0;
+  int rbits = 1, wbits = 1, wshift = 0;  // bits of a row, of a weight's leading bits; those below
+  bool ordered = false;           // slot and entry are there
+  bool order_failed = false;      // there was no memory for them
+  unsigned grid[2] = {0, 0};      // plain, ordered
 };
 
 static void sssp_scratch_free(void* p)
@@ -202,6 +203,7 @@ __device__ __forceinline__ void sssp_dense_apply(const SsspArgs& A, uint32_t wor
 
 // Pull steps only: the frontier's messages by slot, INF again for the frontier
 // of the last pull step.
+template <bool ORDERED>
 __device__ __forceinline__ void sssp_front(const SsspArgs& A, uint32_t words, uint32_t warp, uint32_t nwarps, uint32_t lane)
 {
   for (uint32_t w = warp; w < words; w += nwarps)
@@ -210,7 +212,7 @@ __device__ __forceinline__ void sssp_front(const SsspArgs& A, uint32_t words, ui
     if ((now | was) >> lane & 1)
     {
       const uint32_t v = w * 32 + lane;
-      A.fmsg[A.slot[v]] = now >> lane & 1 ? A.msg[v] : kInf;
+      A.fmsg[ORDERED ? A.slot[v] : v] = now >> lane & 1 ? A.msg[v] : kInf;
     }
     __syncwarp();
     if (lane == 0 && now != was) A.pbits[w] = now;
@@ -270,7 +272,9 @@ __device__ __forceinline__ void sssp_split(const SsspArgs& A, uint32_t words, ui
 // has: most of its edges' messages, random reads that bound the step at 240 G a
 // second however they are arranged, are never read.  R-MAT 2^22: the five pulls
 // of a call 1343 us over the CSR by position, 1095 with the messages by slot,
-// 486 with the rows by weight.
+// 486 with the rows by weight.  The ordered copy takes 8 B per in-edge, and 16
+// to 24 more while it is made: where the memory is not there, or not granted (a
+// server's budget), the pulls go over the CSR.
 __device__ __forceinline__ bool sssp_past(unsigned long long fmin, uint32_t w, int wshift, uint32_t have)
 {
   return fmin + ((w >> wshift) << wshift) >= have;
@@ -306,6 +310,7 @@ k_sssp_entries(const uint32_t* __restrict__ ptr, const uint32_t* __restrict__ co
     }
 }
 
+template <bool ORDERED>
 __device__ __forceinline__ void sssp_pull(const SsspArgs& A, unsigned long long fmin, uint32_t warp, uint32_t nwarps,
                                           uint32_t lane)
 {
@@ -315,6 +320,8 @@ __device__ __forceinline__ void sssp_pull(const SsspArgs& A, unsigned long long 
   const uint32_t settled =
       fmin == ~0ull ? 0u : (fmin + A.min_w < kInf ? (uint32_t) (fmin + A.min_w) : kInf);
   const uint2* __restrict__ entry = A.entry;
+  const uint32_t *__restrict__ col = A.in_col, *__restrict__ wgt = A.in_w;
+  auto load = [&](uint32_t i) { return ORDERED ? __ldcs(&entry[i]) : make_uint2(__ldcs(&col[i]), __ldcs(&wgt[i])); };
   const uint32_t* fmsg = A.fmsg;
   // long rows first
   for (uint32_t t = warp; t < A.ntasks; t += nwarps)
@@ -332,8 +339,8 @@ __device__ __forceinline__ void sssp_pull(const SsspArgs& A, unsigned long long 
       uint2 x[4];
       uint32_t m[4];
 #pragma unroll
-      for (int u = 0; u < 4; u++) x[u] = i0 + u * 32 + lane < e ? __ldcs(&entry[i0 + u * 32 + lane]) : make_uint2(0u, kInf);
-      if (sssp_past(fmin, __shfl_sync(0xffffffffu, x[0].y, 0), A.wshift, y)) break;
+      for (int u = 0; u < 4; u++) x[u] = i0 + u * 32 + lane < e ? load(i0 + u * 32 + lane) : make_uint2(0u, kInf);
+      if (ORDERED && sssp_past(fmin, __shfl_sync(0xffffffffu, x[0].y, 0), A.wshift, y)) break;
 #pragma unroll
       for (int u = 0; u < 4; u++) m[u] = fmsg[x[u].x];
 #pragma unroll
@@ -358,8 +365,8 @@ __device__ __forceinline__ void sssp_pull(const SsspArgs& A, unsigned long long 
       uint2 x[4];
       uint32_t m[4];
 #pragma unroll
-      for (uint32_t u = 0; u < 4; u++) x[u] = i + u * G + sub < e ? __ldcs(&entry[i + u * G + sub]) : make_uint2(0u, kInf);
-      if (sssp_past(fmin, __shfl_sync(group_mask, x[0].y, 0, G), A.wshift, y)) break;
+      for (uint32_t u = 0; u < 4; u++) x[u] = i + u * G + sub < e ? load(i + u * G + sub) : make_uint2(0u, kInf);
+      if (ORDERED && sssp_past(fmin, __shfl_sync(group_mask, x[0].y, 0, G), A.wshift, y)) break;
 #pragma unroll
       for (int u = 0; u < 4; u++) m[u] = fmsg[x[u].x];
 #pragma unroll
@@ -408,6 +415,7 @@ __global__ void k_sssp_long_rows(const uint32_t* __restrict__ ptr, const uint32_
 static constexpr double kPullDivisor = 4.0;
 static constexpr int kSsspThreads = 512;
 
+template <bool ORDERED>
 __global__ void __launch_bounds__(kSsspThreads, 3) k_sssp_run(SsspArgs A)
 {
   __shared__ SsspCounters s_got;
@@ -456,9 +464,9 @@ __global__ void __launch_bounds__(kSsspThreads, 3) k_sssp_run(SsspArgs A)
     if (it > 1 && A.max_w <= 0x80000000u && (double) deg * kPullDivisor > (double) A.reg_in)
     {
       examined += A.reg_in;
-      sssp_front(A, words, warp, nwarps, lane);
+      sssp_front<ORDERED>(A, words, warp, nwarps, lane);
       if (!bar.sync()) return;
-      sssp_pull(A, fmin, warp, nwarps, lane);
+      sssp_pull<ORDERED>(A, fmin, warp, nwarps, lane);
     }
     else
     {
@@ -509,33 +517,6 @@ __global__ void __launch_bounds__(kSsspThreads, 3) k_sssp_run(SsspArgs A)
   if (threadIdx.x == 0 && r) atomicAdd(A.reached, r);
   if (!bar.sync()) return;
   if (tid == 0) *A.stats = SsspStats{it, examined, failed ? 1ull : 0ull, __ldcg(A.reached)};
-}
-
-// The pull's entries; rows ascend by position, so the regular rows' come first.
-template <class K>
-static int sssp_entries(la3g_graph* G, SsspScratch* ss, int rbits, int wbits)
-{
-  const uint64_t m = ss->reg_in;
-  LA3G_TRY(galloc(G, &ss->entry, m + 1));
-  if (!m) return LA3G_OK;
-  cub::DoubleBuffer<K> k(nullptr, nullptr);
-  cub::DoubleBuffer<uint2> v(nullptr, nullptr);
-  size_t tb = 0;
-  LA3G_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, k, v, (int64_t) m, 0, rbits + wbits, G->stream));
-  const size_t kb = (m * sizeof(K) + 255) & ~(size_t) 255, vb = (m * 8 + 255) & ~(size_t) 255;
-  DevBuf tmp;
-  LA3G_TRY(tmp.alloc(2 * kb + vb + tb));
-  char* p = tmp.as<char>();
-  k = cub::DoubleBuffer<K>((K*) p, (K*) (p + kb));
-  v = cub::DoubleBuffer<uint2>(ss->entry, (uint2*) (p + 2 * kb));
-  k_sssp_entries<K><<<grid_for((uint64_t) G->g.nreg * 32, 256), 256, 0, G->stream>>>(
-      G->g.in_ptr, G->g.in_col, G->g.in_w, G->g.nreg, ss->slot, wbits, ss->wshift, k.Current(), v.Current());
-  LA3G_LAUNCHED();
-  LA3G_CUDA(cub::DeviceRadixSort::SortPairs(p + 2 * kb + vb, tb, k, v, (int64_t) m, 0, rbits + wbits, G->stream));
-  if (v.Current() != ss->entry)
-    LA3G_CUDA(cudaMemcpyAsync(ss->entry, v.Current(), m * 8, cudaMemcpyDeviceToDevice, G->stream));
-  LA3G_CUDA(cudaStreamSynchronize(G->stream));  // before the temporaries go
-  return LA3G_OK;
 }
 
 static int sssp_scratch_build(la3g_graph* G, SsspScratch* ss)
@@ -603,30 +584,11 @@ static int sssp_scratch_build(la3g_graph* G, SsspScratch* ss)
     A.task_begin = be;
     A.ntasks = (uint32_t) nt;
   }
-  {
-    DevBuf tmp;
-    size_t tb = 0;
-    uint32_t* z = nullptr;
-    LA3G_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, z, z, z, z, (int64_t) N, 0, 32, G->stream));
-    LA3G_TRY(tmp.alloc((size_t) N * 16 + tb + 256));
-    uint32_t *key = tmp.as<uint32_t>(), *key2 = key + N, *iota = key2 + N, *order = iota + N;
-    void* lib = (void*) (((uintptr_t) (order + N) + 255) & ~(uintptr_t) 255);
-    k_sssp_slot_keys<<<grid_for(N, 256), 256, 0, G->stream>>>(G->g.out_ptr, N, key, iota);
-    LA3G_LAUNCHED();
-    LA3G_CUDA(cub::DeviceRadixSort::SortPairs(lib, tb, key, key2, iota, order, (int64_t) N, 0, 32, G->stream));
-    LA3G_TRY(galloc(G, &ss->slot, N));
-    k_sssp_slots<<<grid_for(N, 256), 256, 0, G->stream>>>(order, N, ss->slot);
-    LA3G_LAUNCHED();
-    int rbits = 1, wbits = 1;
-    while ((uint64_t) G->g.nreg >> rbits) rbits++;
-    while (wbits < 32 && ss->max_w >> wbits) wbits++;
-    // eight leading bits of the weight order a row well enough
-    ss->wshift = std::max(0, wbits - 8);
-    wbits -= ss->wshift;
-    if (rbits + wbits <= 32) LA3G_TRY(sssp_entries<uint32_t>(G, ss, rbits, wbits));
-    else LA3G_TRY(sssp_entries<uint64_t>(G, ss, rbits, wbits));
-    LA3G_CUDA(cudaStreamSynchronize(G->stream));
-  }
+  while ((uint64_t) g.nreg >> ss->rbits) ss->rbits++;
+  while (ss->wbits < 32 && ss->max_w >> ss->wbits) ss->wbits++;
+  // eight leading bits of the weight order a row well enough
+  ss->wshift = std::max(0, ss->wbits - 8);
+  ss->wbits -= ss->wshift;
   A.out_ptr = g.out_ptr;
   A.out_row = g.out_row;
   A.out_w = g.out_w;
@@ -646,48 +608,105 @@ static int sssp_scratch_build(la3g_graph* G, SsspScratch* ss)
   // with non-negative weights every distance is final after at most N + 1
   // iterations (Bellman-Ford), so a loop past N + 2 is a fault
   A.limit = (uint64_t) N + 2;
-  A.slot = ss->slot;
-  A.entry = ss->entry;
   A.wshift = ss->wshift;
   A.stats = ss->stats;
+  LA3G_CUDA(cudaStreamSynchronize(s));
   return LA3G_OK;
 }
 
 static int sssp_scratch(la3g_graph* G, SsspScratch** out)
 {
+  LA3G_TRY(build_push_csr(G));
   return graph_scratch(G, kSlotSssp, sssp_scratch_free, out, [&](SsspScratch* ss) { return sssp_scratch_build(G, ss); });
 }
 
-}  // namespace la3g
+// The ordered pull's arrays; rows ascend by position, so the regular rows'
+// entries come first.  First the slots' sort, then the entries', in the same
+// temporary memory.
+template <class K>
+static int sssp_order(la3g_graph* G, SsspScratch* ss)
+{
+  DevGraph& g = G->g;
+  cudaStream_t s = G->stream;
+  const size_t N = g.nslots, m = ss->reg_in;
+  auto round = [](size_t b) { return (b + 255) & ~(size_t) 255; };
+  const size_t n4 = round(N * 4), kb = round(m * sizeof(K)), vb = round(m * 8);
+  size_t slot_lib = 0, entry_lib = 0;
+  {
+    uint32_t* z = nullptr;
+    cub::DoubleBuffer<K> k(nullptr, nullptr);
+    cub::DoubleBuffer<uint2> v(nullptr, nullptr);
+    LA3G_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, slot_lib, z, z, z, z, (int64_t) N, 0, 32, s));
+    if (m) LA3G_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, entry_lib, k, v, (int64_t) m, 0, ss->rbits + ss->wbits, s));
+  }
+  GallocScope scope(G);
+  uint32_t* slot = nullptr;
+  uint2* entry = nullptr;
+  LA3G_TRY(galloc(G, &slot, N));
+  LA3G_TRY(galloc(G, &entry, m + 1));
+  DevBuf tmp;
+  LA3G_TRY(tmp.alloc(std::max(4 * n4 + slot_lib, 2 * kb + vb + entry_lib)));
+  char* p = tmp.as<char>();
+  {
+    uint32_t *key = (uint32_t*) p, *key2 = (uint32_t*) (p + n4), *iota = (uint32_t*) (p + 2 * n4);
+    uint32_t* order = (uint32_t*) (p + 3 * n4);
+    k_sssp_slot_keys<<<grid_for(N, 256), 256, 0, s>>>(g.out_ptr, (uint32_t) N, key, iota);
+    LA3G_LAUNCHED();
+    LA3G_CUDA(cub::DeviceRadixSort::SortPairs(p + 4 * n4, slot_lib, key, key2, iota, order, (int64_t) N, 0, 32, s));
+    k_sssp_slots<<<grid_for(N, 256), 256, 0, s>>>(order, (uint32_t) N, slot);
+    LA3G_LAUNCHED();
+  }
+  if (m)
+  {
+    cub::DoubleBuffer<K> k((K*) p, (K*) (p + kb));
+    cub::DoubleBuffer<uint2> v(entry, (uint2*) (p + 2 * kb));
+    k_sssp_entries<K><<<grid_for((uint64_t) g.nreg * 32, 256), 256, 0, s>>>(g.in_ptr, g.in_col, g.in_w, g.nreg, slot,
+                                                                            ss->wbits, ss->wshift, k.Current(), v.Current());
+    LA3G_LAUNCHED();
+    LA3G_CUDA(cub::DeviceRadixSort::SortPairs(p + 2 * kb + vb, entry_lib, k, v, (int64_t) m, 0, ss->rbits + ss->wbits, s));
+    if (v.Current() != entry) LA3G_CUDA(cudaMemcpyAsync(entry, v.Current(), m * 8, cudaMemcpyDeviceToDevice, s));
+  }
+  LA3G_CUDA(cudaStreamSynchronize(s));  // before the temporaries go
+  scope.keep();
+  ss->A.slot = slot;
+  ss->A.entry = entry;
+  ss->ordered = true;
+  return LA3G_OK;
+}
 
-using namespace la3g;
-
-extern "C" int la3g_sssp(la3g_graph* G, uint32_t root, uint32_t* dist_out, la3g_stats* st)
+int sssp_run(la3g_graph* G, uint32_t root, uint32_t* dist_out, la3g_stats* st, bool order)
 {
   if (!G) return set_error(LA3G_EINVAL, "null graph");
   DevGraph& g = G->g;
   if (!g.directed() || !g.weighted() || (g.flags & (LA3G_REVERSE | LA3G_ACYCLIC | LA3G_BIPARTITE)))
     return set_error(LA3G_EINVAL, "sssp needs a graph loaded with LA3G_DIRECTED | LA3G_WEIGHTED");
   CallTimer T(G, st);
-  LA3G_TRY(build_push_csr(G));
   SsspScratch* ss = nullptr;
   LA3G_TRY(sssp_scratch(G, &ss));
+  if (order && !ss->ordered && !ss->order_failed)
+  {
+    const int rc = ss->rbits + ss->wbits <= 32 ? sssp_order<uint32_t>(G, ss) : sssp_order<uint64_t>(G, ss);
+    if (rc != LA3G_OK && rc != LA3G_ENOMEM) return rc;
+    ss->order_failed = rc == LA3G_ENOMEM;  // the plain pulls give the same
+  }
   cudaStream_t s = G->stream;
   const uint32_t N = g.nslots;
+  const void* kernel = ss->ordered ? (const void*) k_sssp_run<true> : (const void*) k_sssp_run<false>;
+  unsigned& grid = ss->grid[ss->ordered];
   SsspArgs A = ss->A;
   A.root = root;
   A.wait_polls = barrier_polls(G->wait_polls, g.nent);
   A.dist_out = dist_out ? ss->by_id : nullptr;
   ss->stats->status = kSsspRunning;
-  if (!ss->grid)  // few blocks for a small graph: a barrier takes longer the more there are
-    LA3G_TRY(cooperative_blocks((const void*) k_sssp_run, kSsspThreads, std::max<uint64_t>(N, g.nent / 8), 3, &ss->grid));
+  if (!grid)  // few blocks for a small graph: a barrier takes longer the more there are
+    LA3G_TRY(cooperative_blocks(kernel, kSsspThreads, std::max<uint64_t>(N, g.nent / 8), 3, &grid));
   T.device_begin();
   LA3G_CUDA(cudaMemsetAsync(A.bar, 0, 8, s));
   {
     // distances and messages; the edges examined are added below
     ProfileScope p("sssp", s, 8.0 * N);
     void* args[] = {(void*) &A};
-    LA3G_CUDA(cudaLaunchCooperativeKernel((const void*) k_sssp_run, ss->grid, kSsspThreads, args, 0, s));
+    LA3G_CUDA(cudaLaunchCooperativeKernel(kernel, grid, kSsspThreads, args, 0, s));
   }
   T.device_end();
   if (dist_out) LA3G_CUDA(cudaMemcpyAsync(dist_out, ss->by_id, (size_t) N * 4, cudaMemcpyDeviceToHost, s));
@@ -704,4 +723,13 @@ extern "C" int la3g_sssp(la3g_graph* G, uint32_t root, uint32_t* dist_out, la3g_
     st->algo_bytes = r.examined * 8 + (uint64_t) N * 8;
   }
   return LA3G_OK;
+}
+
+}  // namespace la3g
+
+using namespace la3g;
+
+extern "C" int la3g_sssp(la3g_graph* G, uint32_t root, uint32_t* dist_out, la3g_stats* st)
+{
+  return sssp_run(G, root, dist_out, st, true);
 }
