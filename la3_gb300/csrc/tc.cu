@@ -887,6 +887,10 @@ static int tc_scratch_build(la3g_graph* G, TcScratch* ts)
   LA3G_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, c2, ts->tcount2, ts->toff2, (int) N + 1));
   ts->temp_bytes = std::max(std::max(a, b), std::max(c, c2));
   LA3G_TRY(galloc_bytes(G, &ts->temp, ts->temp_bytes));
+  // per function and device, so for every graph
+  LA3G_CUDA(cudaFuncSetAttribute(TC_BIG_KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) kTcBlockSmem));
+  LA3G_CUDA(cudaFuncSetAttribute(TC_MID_KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) kTcMidSmem));
+  LA3G_CUDA(cudaFuncSetAttribute(k_tc_sort_big, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) kTcSortBigSmem));
   return LA3G_OK;
 }
 
@@ -990,14 +994,6 @@ extern "C" int la3g_tc(la3g_graph* G, uint64_t* total_out, uint32_t* per_vertex_
   LA3G_TRY(build_push_csr(G));
   TcScratch* ts = nullptr;
   LA3G_TRY(tc_scratch(G, &ts));
-  static bool smem_set = false;  // the opt-ins are per function and device; idempotent
-  if (!smem_set)
-  {
-    LA3G_CUDA(cudaFuncSetAttribute(TC_BIG_KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) kTcBlockSmem));
-    LA3G_CUDA(cudaFuncSetAttribute(TC_MID_KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) kTcMidSmem));
-    LA3G_CUDA(cudaFuncSetAttribute(k_tc_sort_big, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) kTcSortBigSmem));
-    smem_set = true;
-  }
   cudaStream_t s = G->stream;
   const uint32_t N = g.nslots;
   const double m = (double) g.nent;
