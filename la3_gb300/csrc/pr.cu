@@ -19,9 +19,10 @@
 //
 // Kernel layout: the calls run over a copy of the matrix made for them once
 // per graph (see "the pull layout"): rows in descending length, columns
-// renumbered in descending out-degree.  Rows of at most kShortRow in-edges go
-// a lane each, longer ones a warp each, the longest a block each; FP64 rows are
-// summed in parallel with the result of the sequential sum (see "exact sums").
+// renumbered in descending out-degree.  Rows of at most kShortRow in-edges
+// (kShortRowFew on a graph of few rows) go a lane each, longer ones a warp each,
+// the longest a block each; FP64 rows are summed in parallel with the result of
+// the sequential sum (see "exact sums").
 #include <algorithm>
 #include <cstring>
 #include <vector>
@@ -720,7 +721,7 @@ __device__ __forceinline__ double prf_finish(uint32_t q, float acc, const PrLayo
 // One FP32 pull over the rows of R, FP32 accumulation.  A row of at most
 // kLongRow entries has four partial sums, entry i in sum i % 4, combined
 // (0 + 2) + (1 + 3): a lane holds all four in a slice, a group of four lanes
-// one each above kShortRow.  A longer row has one per thread of its block.
+// one each above the slices' limit.  A longer row has one per thread of its block.
 // The L1 residual is reduced in FP64.
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 k_prf_pull(PrRange R, PrBlocks B, PrLayout L, uint32_t zero, const float* __restrict__ x, float* __restrict__ xnext,
