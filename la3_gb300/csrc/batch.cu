@@ -64,7 +64,7 @@ struct BatchScratch
   // hubs, [4 + c] smallest distance list c holds
   unsigned long long* ctr = nullptr;
   unsigned long long* hctr = nullptr;  // pinned, written by the kernels: [0] levels / iterations, [1] status
-  unsigned long long* bar = nullptr;   // grid barrier's count
+  unsigned int* bar = nullptr;         // grid barrier's count
   uint8_t* tpos = nullptr;             // results by root and id, before they leave the device
   size_t tpos_bytes = 0;
   BatchConfig cfg;                           // set by hand, or the default
@@ -134,7 +134,7 @@ struct MsArgs
   uint8_t* hops;
   PairList list;       // pushing levels: the frontier's pairs
   unsigned long long* ctr;
-  unsigned long long* bar;
+  unsigned int* bar;
   long long wait_polls;
   // a level pushes when its new bits x mean degree stay below the limit
   double mean_deg, push_limit;
@@ -371,7 +371,7 @@ static int ms_bfs_run(la3g_graph* G, BatchScratch* b, const uint32_t* roots_host
   LA3G_CUDA(cudaMemsetAsync(b->hops, 0xFF, (size_t) N * W * 64, s));
   for (int k = 0; k < 3; k++) LA3G_CUDA(cudaMemsetAsync(b->alive[k], 0, (size_t) W * 8, s));
   LA3G_CUDA(cudaMemsetAsync(b->ctr, 0, 8 * 8, s));
-  LA3G_CUDA(cudaMemsetAsync(b->bar, 0, 8, s));
+  LA3G_CUDA(cudaMemsetAsync(b->bar, 0, sizeof *b->bar, s));
   k_ms_roots<<<grid_for(R, 256), 256, 0, s>>>(b->rpos, R, N, W, b->vis, b->buf[0], b->hops, b->alive[0]);
   LA3G_LAUNCHED();
   tls_launches += 3;
@@ -497,7 +497,7 @@ struct BsArgs
   PairList L[2];            // their counters: ctr[c], ctr[2 + c]
   uint32_t* dist;
   unsigned long long* ctr;
-  unsigned long long* bar;
+  unsigned int* bar;
   long long wait_polls;
   uint32_t delta;           // kNoWindow: no window
   unsigned long long* out;  // pinned: iterations, status
@@ -779,7 +779,7 @@ static int sssp_batch_chunk(la3g_graph* G, BatchScratch* b, const uint32_t* root
   b->hctr[1] = 0;
   LA3G_CUDA(cudaMemsetAsync(b->ctr, 0, 4 * 8, s));
   LA3G_CUDA(cudaMemsetAsync(b->ctr + 4, 0xFF, 2 * 8, s));
-  LA3G_CUDA(cudaMemsetAsync(b->bar, 0, 8, s));
+  LA3G_CUDA(cudaMemsetAsync(b->bar, 0, sizeof *b->bar, s));
   k_bs_list<<<num_sms() * 8, 256, 0, s>>>((uint64_t) N * W, W, g.out_ptr, b->reg_end, b->sfront[0], A.L[0]);
   LA3G_LAUNCHED();
   tls_launches++;

@@ -66,7 +66,7 @@ struct BfsArgs
   uint32_t* task0;                  // [N] first task numbers of the hubs: even levels from the front, odd from the back
   uint32_t* bits[2];                // [N / 32 + 1] frontier bitmaps
   FrontierCounters* ctr;            // [3]
-  unsigned long long* bar;          // barrier count
+  unsigned int* bar;                // barrier count
   long long wait_polls;             // < 0: the default
   const uint32_t* pos_of_id;        // null: ids are positions
   uint8_t* hops_out;                // by id, or null
@@ -417,7 +417,7 @@ static int bfs_launch(BfsArgs& A, unsigned* grid, cudaStream_t s)
 {
   // few blocks for a small graph: a barrier takes longer the more there are
   if (!*grid) LA3G_TRY(cooperative_blocks((const void*) k_bfs_run<CHECK>, kBfsThreads, std::max<uint64_t>(A.N, A.nent / 8), 3, grid));
-  LA3G_CUDA(cudaMemsetAsync(A.bar, 0, 8, s));
+  LA3G_CUDA(cudaMemsetAsync(A.bar, 0, sizeof *A.bar, s));
   void* args[] = {(void*) &A};
   LA3G_CUDA(cudaLaunchCooperativeKernel((const void*) k_bfs_run<CHECK>, *grid, kBfsThreads, args, 0, s));
   return LA3G_OK;
@@ -469,7 +469,7 @@ static int bfs_scratch_build(la3g_graph* G, BfsScratch* bs)
   A.bits[0] = (uint32_t*) take(nb);
   A.bits[1] = (uint32_t*) take(nb);
   A.ctr = (FrontierCounters*) take(256);
-  A.bar = (unsigned long long*) take(256);
+  A.bar = (unsigned int*) take(256);
   A.ptr = g.in_ptr;
   A.col = g.in_col;
   A.key = g.hash_of_pos;
@@ -592,7 +592,7 @@ static constexpr size_t kNaBits0Off = kNaList1Off + na_round(sizeof(uint32_t) * 
 static constexpr size_t kNaBits1Off = kNaBits0Off + na_round(sizeof(uint32_t) * kNaWords);
 static constexpr size_t kNaCtrOff = kNaBits1Off + na_round(sizeof(uint32_t) * kNaWords);
 static constexpr size_t kNaBarOff = kNaCtrOff + na_round(3 * sizeof(FrontierCounters));
-static constexpr size_t kNaStatsOff = kNaBarOff + na_round(sizeof(unsigned long long));
+static constexpr size_t kNaStatsOff = kNaBarOff + na_round(sizeof(unsigned int));
 static constexpr size_t kNoAllocScratchBytes = kNaStatsOff + na_round(sizeof(BfsStats));
 
 static __device__ __align__(256) unsigned char g_bfs_noalloc_scratch[kNoAllocScratchBytes];
@@ -676,7 +676,7 @@ static int bfs_noalloc_run(const uint32_t* row_ptr, const uint32_t* col, const u
     A.bits[0] = (uint32_t*) (base + kNaBits0Off);
     A.bits[1] = (uint32_t*) (base + kNaBits1Off);
     A.ctr = (FrontierCounters*) (base + kNaCtrOff);
-    A.bar = (unsigned long long*) (base + kNaBarOff);
+    A.bar = (unsigned int*) (base + kNaBarOff);
     A.wait_polls = -1;
     A.stats = (BfsStats*) (base + kNaStatsOff);
     unsigned grid = 0;

@@ -82,7 +82,7 @@ struct SsspArgs
   unsigned long long* fctr;       // [0] small-list length, [1] hub slots and tasks
   SsspCounters* ctr;              // [3]
   unsigned long long* reached;
-  unsigned long long* bar;
+  unsigned int* bar;
   long long wait_polls;
   uint32_t root;
   uint32_t* dist_out;             // by id, or null
@@ -535,7 +535,7 @@ static int sssp_scratch_build(la3g_graph* G, SsspScratch* ss)
   LA3G_TRY(galloc(G, &A.ctr, 3));
   LA3G_TRY(galloc(G, &A.fctr, 4));  // with `reached` and the barrier
   A.reached = A.fctr + 2;
-  A.bar = A.fctr + 3;
+  A.bar = (unsigned int*) (A.fctr + 3);
   LA3G_TRY(galloc(G, &A.fbits, (size_t) N / 32 + 2));
   LA3G_TRY(galloc(G, &A.pbits, (size_t) N / 32 + 2));
   LA3G_TRY(galloc(G, &ss->by_id, N));
@@ -701,7 +701,7 @@ int sssp_run(la3g_graph* G, uint32_t root, uint32_t* dist_out, la3g_stats* st, b
   if (!grid)  // few blocks for a small graph: a barrier takes longer the more there are
     LA3G_TRY(cooperative_blocks(kernel, kSsspThreads, std::max<uint64_t>(N, g.nent / 8), 3, &grid));
   T.device_begin();
-  LA3G_CUDA(cudaMemsetAsync(A.bar, 0, 8, s));
+  LA3G_CUDA(cudaMemsetAsync(A.bar, 0, sizeof *A.bar, s));
   {
     // distances and messages; the edges examined are added below
     ProfileScope p("sssp", s, 8.0 * N);
