@@ -1096,9 +1096,9 @@ def serve_measure(args, rates, seconds: float) -> dict:
     peaks = measured_peaks()
     bm25_gbs = prof["bytes"] / (prof["ms"] / 1e3) / 1e9 if prof["ms"] else None
     bm25 = {"queries": len(bm_q), "device_ms_mean": statistics.mean(bm_ms), "device_ms_p50": _pct(bm_ms, 50),
-            "postings_per_query": bm_post / len(bm_q), "term_kernel_gbs": bm25_gbs,
-            "term_kernel_frac": (bm25_gbs / peaks["hbm_gbs"]) if bm25_gbs else None,
-            "term_kernel_launches": prof["launches"]}
+            "postings_per_query": bm_post / len(bm_q), "query_gbs": bm25_gbs,
+            "query_frac": (bm25_gbs / peaks["hbm_gbs"]) if bm25_gbs else None,
+            "query_launches": prof["launches"]}
 
     # warm both arms (allocations, first launches)
     arr, qs = make_stream(2000.0, 200)
@@ -1262,8 +1262,8 @@ def next_line(args, rank, world, local) -> dict | None:
                                f"s{args.scale}; graph simulation on R-MAT s{gs_scale} (5-vertex query, 6 labels)",
                    "lm": {"queries": nq, "device_ms_mean": statistics.mean(lm_dev),
                           "device_ms_p50": _pct(lm_dev, 50), "device_ms_p99": _pct(lm_dev, 99),
-                          "postings_per_query": sum(r[1] for r in res) / nq, "term_kernel_gbs": lm_gbs,
-                          "term_kernel_frac": (lm_gbs / peaks["hbm_gbs"]) if lm_gbs else None,
+                          "postings_per_query": sum(r[1] for r in res) / nq, "query_gbs": lm_gbs,
+                          "query_frac": (lm_gbs / peaks["hbm_gbs"]) if lm_gbs else None,
                           "prepare_s": round(lm_prepare_s, 2)},
                    "degree": {"device_ms": deg_ms, "gteps": gd.info.nentries / (deg_ms / 1e3) / 1e9},
                    "graphsim": {"ms": gs_s * 1e3, "iterations": res[-1][6], "matches": res[-1][5],

@@ -12,7 +12,7 @@
 // record which roots still discovered something; words whose roots are all
 // finished are skipped (done-masks).  All levels run inside one cooperative
 // kernel with a grid barrier whose waits are bounded (a barrier that waits too
-// long records an error and every block returns): with a host round trip per
+// long makes every block return): with a host round trip per
 // level a batch of 64 roots on R-MAT 2^18 spent a third of its time between
 // kernels.
 // BFS levels are order-free, so hops equal the single-root runs; a batch

@@ -451,7 +451,7 @@ static int bfs_scratch_build(la3g_graph* G, BfsScratch* bs)
 {
   DevGraph& g = G->g;
   const uint32_t N = g.nslots;
-  // one allocation: eight arrays of a word per vertex, two of a byte, two bitmaps
+  // one allocation: six arrays of a word per vertex, two of a byte, two bitmaps
   auto round = [](size_t b) { return (b + 255) & ~(size_t) 255; };
   const size_t n4 = round((size_t) N * 4), n1 = round(N), nb = round(((size_t) N / 32 + 1) * 4);
   char* p = nullptr;

@@ -223,7 +223,8 @@ __global__ void __launch_bounds__(kCcSamples) k_cc_giant(const uint32_t* __restr
 // walks what is left, and has nothing to do otherwise.  (Walking every chain to
 // its end at once, 2^20 vertices hooked one under the other took 19 ms; finds
 // with path halving cannot be used here, since a late halving store may
-// overwrite a root.)
+// overwrite what another thread has compressed already, and leave the vertex
+// short of its root.)
 static constexpr uint32_t kCcWalk = 512;
 __global__ void k_cc_flatten(uint32_t nrows, const uint32_t* __restrict__ giant_share, uint32_t* parent, uint32_t* deep,
                              int second)

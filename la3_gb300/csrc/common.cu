@@ -155,8 +155,6 @@ ProfileScope::~ProfileScope()
   k.bytes += bytes;
 }
 
-bool profile_enabled() { return prof_on; }
-
 void profile_add_bytes(const char* name, double bytes)
 {
   if (!prof_on) return;

@@ -357,9 +357,6 @@ struct CallTimer
 
 double now_ms();
 
-// True while kernel-level profiling is on (la3g_profile_enable).
-bool profile_enabled();
-
 }  // namespace la3g
 
 #endif  // __CUDACC__

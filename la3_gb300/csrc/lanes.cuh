@@ -179,7 +179,7 @@ static __device__ __forceinline__ void bs_relax_dense(uint32_t k0, uint32_t k1, 
 // limit relax; the others keep their bit, carried into the next frontier, as
 // delta-stepping keeps a vertex in a later bucket.  lmin collects the smallest
 // distance the next frontier will hold (carried distances and lowered
-// candidates), from which the host sets the next window.  Every active bit is
+// candidates), from which the next window is set.  Every active bit is
 // either relaxed or carried, so the shortest distances are the same.
 static __device__ __forceinline__ void bs_relax_range(uint32_t i, uint32_t k0, uint32_t k1, int lane, uint32_t R, uint32_t W,
                                                const uint32_t* __restrict__ row, const uint32_t* __restrict__ wgt,

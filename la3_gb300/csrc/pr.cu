@@ -94,7 +94,7 @@ struct PrScratch
   double* resid = nullptr;
   bool ready = false;
   // tiled layout of the regular rows (la3g_pr_f32_tiled), built on first use
-  uint32_t tile_rows = 0, ntiles = 0;
+  uint32_t ntiles = 0;
   uint64_t tile_ncols = 0, tile_nent = 0;
   uint32_t* tile_col = nullptr;  // [ntiles + 1] first non-empty-column slot of each tile
   uint32_t* tcol = nullptr;      // [ncols] column positions, ascending within a tile
@@ -985,7 +985,6 @@ static int pr_build_tiles(la3g_graph* G, PrScratch* ps)
   for (int64_t t = (int64_t) ntiles - 1; t >= 0; t--) tc[t] = std::min(tc[t], tc[t + 1]);
   LA3G_CUDA(cudaMemcpyAsync(ps->tile_col, tc.data(), tc.size() * 4, cudaMemcpyHostToDevice, s));
   LA3G_CUDA(cudaStreamSynchronize(s));
-  ps->tile_rows = kTileRows;
   ps->ntiles = ntiles;
   ps->tile_ncols = ncols;
   ps->tile_nent = n;
