@@ -187,9 +187,12 @@ int la3g_pr_f32(la3g_graph* g, uint32_t iters, double tol, double* rank_out, dou
  * src/matrix/matrix2d.hpp:6-25): non-empty columns with offsets and a 16-bit
  * row per entry (hypersparse tiles also keep each entry's column and are
  * walked by entry); the tile's row accumulators live in shared memory; rows
- * with more than 1024 in-edges are summed from the flat CSR, a block each.  Built on the device
- * on the first call (about 14 B per entry).  Results agree with
- * la3g_pr_f32 to FP32 rounding (addition order inside a row differs). */
+ * with more than 1024 in-edges are summed from the flat CSR, a block each.
+ * Built on the device on the first call (about 14 B per entry).  Results agree
+ * with la3g_pr_f32 to FP32 rounding (addition order inside a row differs).
+ * The faster one of the two where in-degrees are even (ER 2^24: 1.7x); where a
+ * few columns are behind most edges la3g_pr_f32 is (R-MAT 2^24: this takes 1.4x
+ * its time). */
 int la3g_pr_f32_tiled(la3g_graph* g, uint32_t iters, double tol, double* rank_out, double* residual_out,
                       la3g_stats* st);
 
@@ -212,7 +215,9 @@ int la3g_sssp(la3g_graph* g, uint32_t root, uint32_t* dist_out, la3g_stats* st);
  * to walk); when one runs out, every block leaves the kernel, and the call
  * returns LA3G_ETIMEOUT with the device left usable and the outputs undefined.
  * No counterpart in the reference (it has no device waits); polls = 0 makes
- * any wait give up at once, which exercises that error path. */
+ * any wait give up at once, which exercises that error path.  The whole grid (up
+ * to three blocks of 512 threads per SM, fewer for a small graph) starts at
+ * once: the call waits for other kernels that hold the SMs to end. */
 int la3g_set_wait_limit(la3g_graph* g, long long polls);
 
 /* Connected components (src/apps/graph_analytics/cc.cpp:11-31, cc.h:11-38)
