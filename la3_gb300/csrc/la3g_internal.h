@@ -168,11 +168,11 @@ struct GridBarrier
   }
 };
 
-// Polls of a barrier before it gives up, by default: 2^26 (ten seconds or more;
-// a poll takes 0.15 us) and kEntryPolls for each entry of the matrix, since a
-// lane may walk a whole list between two barriers (the neighbours of a vertex in
-// a bottom-up level, a sink's in-edges: 0.05 and 0.14 us an entry, up to four
-// times that where the reads miss L2): work that is only long is waited for.
+// Polls of a barrier before it gives up, by default: 2^26 (ten seconds; a poll
+// takes 0.15 us) and kEntryPolls for each entry of the matrix, since a lane may
+// walk a whole list between two barriers (the neighbours of a vertex in a
+// bottom-up level, a sink's in-edges: 0.05 and 0.14 us an entry out of L2; eight
+// polls leave room for reads that miss it): work that is only long is waited for.
 static constexpr long long kBarrierPolls = 1ll << 26, kEntryPolls = 8;
 __host__ __device__ inline long long barrier_polls(long long set, uint64_t entries)
 {
